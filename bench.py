@@ -41,20 +41,27 @@ SEED_A, SEED_B = 24001, 24002
 
 def algorithmic_bytes(na: int, nb: int, n: int) -> int:
     """Minimum HBM traffic of one product: u32 operands in and product out
-    (8(na+nb)) plus eight N-element u64 sweeps (64N) of a two-pass schedule."""
-    return 8 * (na + nb) + 64 * n
+    (8(na+nb)) plus the residue sweeps of a two-pass schedule. n is the
+    16-bit-digit length; the residues are three u32 for each of its n/2
+    32-bit digits (6n bytes a sweep): both operands out of the first pass, in
+    and out of the fused pass (one product out), in and out of the inverse
+    pass, into the carry -- eight sweeps."""
+    return 8 * (na + nb) + 8 * 6 * n
 
 
-def kernel_bytes(kind: str, na: int, nb: int, n: int, operand: int) -> int:
-    """Algorithmic bytes of one launch of each kernel kind (N = transform length)."""
+def kernel_bytes(kind: str, na: int, nb: int, n: int) -> int:
+    """Algorithmic bytes of one launch of each kernel kind; forward passes
+    cover both operands, residues are 6n bytes per operand."""
     if kind == "fwd_first":
-        return 4 * operand + 8 * n
-    if kind in ("fwd_mid", "fwd_last", "inv_mid"):
-        return 16 * n
-    if kind == "fused_last":
+        return 4 * (na + nb) + 12 * n
+    if kind == "fwd_mid":
         return 24 * n
+    if kind == "fused_last":
+        return 18 * n
+    if kind in ("inv_mid", "r3_inv"):
+        return 12 * n
     if kind == "carry":
-        return 8 * n + 4 * (na + nb)
+        return 6 * n + 4 * (na + nb)
     return 8 * (na + nb)  # mul_small
 
 
@@ -271,16 +278,11 @@ def run_ours(args) -> None:
                                         olen.data_ptr(), sp) for _ in range(args.trace_steps)]
     per_kind: dict[str, list[float]] = {}
     per_launch_bytes: dict[str, int] = {}
-    first_seen = 0
     for tr in traces:
-        first_seen = 0
         for kind, logr, ms in tr:
             key = f"{kind}<{logr}>" if kind not in ("carry",) else kind
-            operand = na if (kind == "fwd_first" and first_seen == 0) else nb
-            if kind == "fwd_first":
-                first_seen += 1
             per_kind.setdefault(key, []).append(ms)
-            per_launch_bytes[key] = kernel_bytes(kind, na, nb, n, operand)
+            per_launch_bytes[key] = kernel_bytes(kind, na, nb, n)
     kinds = {k: {"launches_per_product": len(v) // len(traces), "avg_ms": statistics.mean(v),
                  "share": sum(v) / sum(sum(x) for x in per_kind.values())} for k, v in per_kind.items()}
     dominant = max(kinds, key=lambda k: kinds[k]["avg_ms"] * kinds[k]["launches_per_product"])
@@ -359,11 +361,11 @@ def run_ours(args) -> None:
         metric = METRIC if headline else f"ms per {na} x {nb}-limb multiply"
         workload = ("2^24 x 2^24-limb product, uniform random limbs" if headline
                     else f"{na} x {nb}-limb product, uniform random limbs")
-        wset = 4 * (na + nb) * 2 + 16 * n
+        wset = 4 * (na + nb) * 2 + 12 * n
         line = {
             "metric": metric, "value": round(value, 4), "unit": "ms", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(step_ms, 4), "higher_is_better": False,
-            "scaling": "weak", "vs_baseline": None, "dtype": "u64 (GF(p), p=2^64-2^32+1)",
+            "scaling": "weak", "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
             "data": "synthetic: seeded uniform random u32 limbs (splitmix64), top limb non-zero",
             "config": {"workload": workload, "na": na, "nb": nb,
                        "ntt_length": n, "plan": plan, "products_per_step": world,

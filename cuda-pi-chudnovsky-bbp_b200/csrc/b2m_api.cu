@@ -81,6 +81,7 @@ static void destroy_context(Context* c) {
     if (c->hcopy) cudaStreamSynchronize(c->hcopy);
     if (c->host_dev) cudaFree(c->host_dev);
     twtable_free_all(c);
+    rns_free_tables(c);
     if (c->d_tables) cudaFree(c->d_tables);
     if (c->d_err) cudaFree(c->d_err);
     if (c->hstream) cudaStreamDestroy(c->hstream);
@@ -161,6 +162,7 @@ b2m_status b2m_init(int device, uint64_t hbm_budget_bytes) {
         return cuda_status(e, "cudaMalloc(tables)");
     }
     if ((e = cudaMemcpy(c->d_tables, tables.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = rns_init_tables(c)) != cudaSuccess ||
         (e = cudaMalloc(&c->d_err, 256)) != cudaSuccess || (e = cudaMemset(c->d_err, 0, 256)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->hstream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->hcopy, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -251,7 +253,7 @@ b2m_status b2m_mul_device(const uint32_t* d_a, uint64_t na, const uint32_t* d_b,
     b2m_status st = check_sizes(na, nb, &logn);
     if (st != B2M_OK) return st;
     cudaSetDevice(c->device);
-    const Plan p = product_plan(c, na, nb);
+    Plan p = product_plan(c, na, nb);
     if (cudaError_t te = twtable_ensure(c, p, s)) return cuda_status(te, "twiddle table");
     const uint64_t wsb = workspace_bytes_plan(p);
     if (!budget_reserve(c, wsb)) {
@@ -424,7 +426,7 @@ b2m_status b2m_autotune(uint64_t na, uint64_t nb, b2m_stream stream, b2m_tune_en
     st = take_device_error(c);
     if (st != B2M_OK) return st;
     Plan kept = cands[best_i];
-    kept.three = 0;  // tuned plans are kept per power-of-two length
+    kept.three = kept.rns = 0;  // tuned plans are kept per power-of-two length
     set_tuned(c, logn, kept);
     if (best_i < cnt) out[best_i].chosen = 1;
     if (n) *n = cnt;
@@ -443,7 +445,7 @@ b2m_status b2m_mul_device_traced(const uint32_t* d_a, uint64_t na, const uint32_
     if (st != B2M_OK) return st;
     cudaSetDevice(c->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const Plan p = product_plan(c, na, nb);
+    Plan p = product_plan(c, na, nb);
     if (cudaError_t te = twtable_ensure(c, p, s)) return cuda_status(te, "twiddle table");
     const uint64_t wsb = workspace_bytes_plan(p);
     if (!budget_reserve(c, wsb)) {
@@ -502,7 +504,7 @@ b2m_status b2m_mul_host(const uint32_t* a, uint64_t na, const uint32_t* b, uint6
     if (st != B2M_OK) return st;
     std::lock_guard<std::mutex> lk(c->host_mu);
     cudaSetDevice(c->device);
-    const Plan p = product_plan(c, na, nb);
+    Plan p = product_plan(c, na, nb);
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t ba = al(4 * na), bb = al(4 * nb), bo = al(4 * (na + nb)), bl = 256;
     const uint64_t wsb = workspace_bytes_plan(p);

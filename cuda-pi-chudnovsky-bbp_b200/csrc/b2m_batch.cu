@@ -98,7 +98,7 @@ static cudaError_t autotune_bucket(b2m_batch* bt, Bucket& b, cudaStream_t s) {
     {
         std::lock_guard<std::mutex> lk(c->tune_mu);
         if (c->has_tuned[b.logn]) {
-            b.plan = c->tuned[b.logn];
+            b.plan = c->tuned[b.logn];  // its tables: b2m_batch_create
             return cudaSuccess;
         }
     }
@@ -110,7 +110,7 @@ static cudaError_t autotune_bucket(b2m_batch* bt, Bucket& b, cudaStream_t s) {
     float best = 1e30f;
     Plan best_p = b.plan;
     cudaError_t e = cudaSuccess;
-    for (const Plan& p : cands) {
+    for (Plan& p : cands) {
         float ms_sum = 0;
         if ((e = twtable_ensure(c, p, s)) != cudaSuccess) break;
         for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {

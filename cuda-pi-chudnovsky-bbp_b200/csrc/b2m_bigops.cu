@@ -301,7 +301,7 @@ DV mul(Scope& S, DV a, DV b) {
     const b2m_status st = check_sizes(a.n, b.n, &logn);
     if (st != B2M_OK) throw Err{st};
     Context* c = S.c();
-    const Plan p = product_plan(c, a.n, b.n);
+    Plan p = product_plan(c, a.n, b.n);
     ck(twtable_ensure(c, p, S.s()), "twiddle table");
     DV out = S.vec(a.n + b.n);
     void* ws = p.npass ? S.raw(workspace_bytes_plan(p)) : nullptr;
@@ -674,7 +674,7 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
     const b2m_status st = check_sizes(na, nb, &logn);
     if (st != B2M_OK) throw Err{st};
     Context* c = S.c();
-    const Plan p = product_plan(c, na, nb);
+    Plan p = product_plan(c, na, nb);
     ck(twtable_ensure(c, p, S.s()), "twiddle table");
     const uint64_t npts = plan_points(p);
     u64* spec = nullptr;

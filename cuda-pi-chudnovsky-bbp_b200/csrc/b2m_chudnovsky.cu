@@ -603,13 +603,13 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
                     pair_share = p.npass > 0;
                 }
             }
-            pair_plan = p;
         } else if (pair_share) {
             p = pair_plan;
             use_spec = true;
         }
         const uint64_t npts = plan_points(p);
-        if ((e = twtable_ensure(c, p, s)) != cudaSuccess) break;
+        if (!use_spec && (e = twtable_ensure(c, p, s)) != cudaSuccess) break;
+        if (!second) pair_plan = p;  // the second product reads the first's spectrum: same passes
         const uint64_t wss = !p.npass ? 0
                              : use_spec ? al(8 * npts + carry_scratch_bytes_n(npts))
                                         : al(workspace_bytes_plan(p));

@@ -40,6 +40,20 @@ struct Context {
     };
     std::mutex twt_mu;
     std::vector<TwTable> twt;
+    // Residue-transform tables (rns_launch.cu, under twt_mu): T and its
+    // inverses of 2^rns_log entries per prime, small from the start, full
+    // size on first need; and the tables of weighted parts, per (q, m).
+    uint2* rns_t = nullptr;
+    uint2* rns_base = nullptr;
+    int rns_log = 0;
+    struct RnsWeights {
+        int q, m;
+        uint2* mem;
+        uint64_t bytes;
+        const uint2* tree[2];  // forward, inverse
+        const uint2* col[2];
+    };
+    std::vector<RnsWeights> rns_weights;
     // Autotuned plan per transform length (b2m_autotune, batch autotune);
     // used by every product of that length once set.
     std::mutex tune_mu;
@@ -53,9 +67,13 @@ struct Context {
 // The plan products of (sub-)transform length 2^logn use: the tuned one if
 // any, else the default (three: the radix-3 products' default).
 inline Plan plan_for(Context* c, int logn, int three = 0) {
-    std::lock_guard<std::mutex> lk(c->tune_mu);
-    Plan p = c->has_tuned[logn] ? c->tuned[logn] : make_plan(logn, three);
+    Plan p;
+    {
+        std::lock_guard<std::mutex> lk(c->tune_mu);
+        p = c->has_tuned[logn] ? c->tuned[logn] : make_plan(logn, three);
+    }
     p.three = three;
+    rns_resolve(c, p, nullptr, false);
     return p;
 }
 // The plan of an na x nb product: 2^L points, or 3 * 2^(L-2) when that holds

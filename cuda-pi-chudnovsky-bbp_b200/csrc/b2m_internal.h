@@ -9,6 +9,8 @@
 
 namespace b2m {
 
+struct Context;
+
 constexpr int MAX_LOGN = 30;      // coefficients stay below p for N <= 2^32
 constexpr int SMALL_MAX_LOGN = 13; // one CTA holds both transforms up to here
 constexpr int CARRY_THREADS = 256;
@@ -37,6 +39,11 @@ struct Plan {
     // 1: 3 * 2^logn points -- a radix-3 step (ntt_radix3.cu) around three
     // 2^logn-point transforms that run the passes above (npass >= 2).
     int three = 0;
+    // 1: the product runs on the three-prime residue transforms
+    // (rns_launch.cu), whose passes follow from the length; logn, logr and
+    // logc then only name the length and the workspace. Set where the tables
+    // of that path exist (rns_resolve).
+    int rns = 0;
 };
 
 // Points of a plan's transform, and the workspace and carry scratch a
@@ -84,6 +91,30 @@ struct ProdJob {
     u32* ticket;
 };
 uint64_t carry_scratch_bytes(int logn);
+
+// ---- residue transforms (rns_*.cu) -------------------------------------------
+// Arguments of the transform passes; pointers and lengths of single products
+// are in the struct, batched ones in jobs[blockIdx.y].
+struct RnsArgs {
+    const u32* a;
+    const u32* b;
+    u64 na, nb;
+    u32* bufA;                // residues [prime][nt]
+    u32* bufB;
+    const ProdJob* jobs;
+    u64 nt;                   // points: q * 2^m
+    const uint2* tw;          // T, [prime][ent] (w, floor(2^32 w / p))
+    const uint2* twi;         // its inverses
+    const uint2* wtree;       // weighted sub-transforms: first-pass trees [prime][q][2^logr]
+    const uint2* wcol;        // and column factors [prime][q][2^logs] (forward or inverse)
+    u32 ent;
+    u32 nmask;                // sub-problem index -> tree node
+    int logs;                 // log2 S of the pass
+    int q;
+    int op0;                  // operand of grid z 0..2
+    int square;
+    uint2 ct[3][8];           // c_t of the q sub-transforms
+};
 
 // Optional tracing of a launch sequence: an event is recorded on the stream
 // before every kernel and once after the last one.
@@ -174,8 +205,7 @@ PassGeo pass_geo(const Plan& p, int k);
 // only looks them up, so launch paths that must not allocate still use
 // tables that exist.
 constexpr int TWT_MIN_LOGM = 12;
-struct Context;
-cudaError_t twtable_ensure(Context* c, const Plan& p, cudaStream_t s);
+cudaError_t twtable_ensure(Context* c, Plan& p, cudaStream_t s);
 void twtable_free_all(Context* c);
 
 // Per-family launchers (ntt_fam_*.cu, ntt_carry.cu); each dispatches on the
@@ -206,6 +236,35 @@ cudaError_t launch_mul_small(int logn, const PassGeo& g, cudaStream_t s, const u
 cudaError_t launch_carry(unsigned nchunks, cudaStream_t s, const u64* coef, u32* out, u64 nout,
                          LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                          const ProdJob* jobs = nullptr, unsigned njobs = 1, u64 points = 1);
+// Residue-transform products. rns_resolve sets p.rns when p is the default
+// plan of its length, the length is in range and the tables exist; with
+// `build` it builds missing tables first (when `s` is not capturing and the
+// budget has room for them beside the product's own workspace).
+cudaError_t rns_init_tables(Context* c);
+void rns_free_tables(Context* c);
+cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build);
+int rns_launches(const Plan& p);
+cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout,
+                               u32* bufA, u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,
+                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready);
+cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, cudaStream_t s);
+cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, u32* err, cudaStream_t s,
+                              bool a_ready);
+// CRT constants of the carry: residues r_i = scale * c mod p_i become the
+// coefficient c (rns_carry.cu).
+struct RnsCrt {
+    uint2 kap[3];   // (scale * P / p_i)^-1 mod p_i
+    u32 qlo[3], qhi[3];  // P / p_i
+};
+cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
+                             LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
+                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt);
+cudaError_t rns_launch_first(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_launch_mid(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_launch_inv(int logr, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_configure();
+
 cudaError_t configure_first();
 cudaError_t configure_mid();
 cudaError_t configure_inv();

@@ -416,11 +416,11 @@ b2m_status b2m_server_start(const b2m_server_config* cfg, b2m_server** out) {
     for (int logn = SMALL_MAX_LOGN + 1; logn <= MAX_LOGN; ++logn) {
         const uint64_t pts = 1ull << logn;
         if (2 * 8 * pts > S->cfg.hbm_budget_bytes) break;
-        if (twtable_ensure(c, plan_for(c, logn), S->release_stream) != cudaSuccess) break;
+        Plan p = plan_for(c, logn);
+        if (twtable_ensure(c, p, S->release_stream) != cudaSuccess) break;
         // the sub-transform plan of 3 * 2^logn points may differ
-        if (6 * 8 * pts <= S->cfg.hbm_budget_bytes &&
-            twtable_ensure(c, plan_for(c, logn, 1), S->release_stream) != cudaSuccess)
-            break;
+        p = plan_for(c, logn, 1);
+        if (6 * 8 * pts <= S->cfg.hbm_budget_bytes && twtable_ensure(c, p, S->release_stream) != cudaSuccess) break;
     }
     // Each slot's arena starts at an equal share of half the budget (at most
     // 4 GiB), so that typical dispatches never grow it.

@@ -31,6 +31,22 @@ __device__ __forceinline__ CState cs_then(CState f, CState g) {
 
 __device__ __forceinline__ u64 cs_eval(CState f, u64 c) { return f.h + (c >= f.t ? 1ull : 0ull); }
 
+// The carry function of NL normalised limbs with carry-out c (for a carry-in
+// of 0).
+template <int NL>
+__device__ __forceinline__ CState group_state(const u32* limb, u64 c) {
+    bool upper_ones = true;
+#pragma unroll
+    for (int i = 2; i < NL; ++i) upper_ones &= (limb[i] == 0xFFFFFFFFu);
+    const u64 dl = (u64)limb[0] | ((u64)limb[1] << 32);
+    u64 t = CS_NEVER;
+    if (upper_ones && dl != 0) {
+        const u64 tt = 0ull - dl;  // 2^64 - dl
+        if (tt < (1ull << 62)) t = tt;
+    }
+    return {c, t};
+}
+
 // Normalise G coefficients (each < 2^61) into G/2 limbs; returns the group's
 // carry function. Coefficient 2i lands in the low half of limb i.
 template <int G>
@@ -45,16 +61,7 @@ __device__ __forceinline__ CState group_carry(const u64* coef, u32* limb) {
         c = x1 >> 16;
         limb[i / 2] = (u32)(x0 & 0xFFFFu) | ((u32)(x1 & 0xFFFFu) << 16);
     }
-    bool upper_ones = true;
-#pragma unroll
-    for (int i = 2; i < G / 2; ++i) upper_ones &= (limb[i] == 0xFFFFFFFFu);
-    const u64 dl = (u64)limb[0] | ((u64)limb[1] << 32);
-    u64 t = CS_NEVER;
-    if (upper_ones && dl != 0) {
-        const u64 tt = 0ull - dl;  // 2^64 - dl
-        if (tt < (1ull << 62)) t = tt;
-    }
-    return {c, t};
+    return group_state<G / 2>(limb, c);
 }
 
 // Add a carry-in (< 2^62) into G/2 limbs; overflow past the group is already

@@ -239,8 +239,10 @@ static cudaError_t twtable_ensure_inv0(Context* c, Context::TwTable& t, cudaStre
     return cudaSuccess;
 }
 
-cudaError_t twtable_ensure(Context* c, const Plan& p, cudaStream_t s) {
+cudaError_t twtable_ensure(Context* c, Plan& p, cudaStream_t s) {
     if (!c || p.npass < 2) return cudaSuccess;
+    if (cudaError_t e = rns_resolve(c, p, s, true)) return e;
+    if (p.rns) return cudaSuccess;  // the passes below are not launched
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return cudaSuccess;
     for (int k = 0; k + 1 < p.npass; ++k) {
@@ -360,10 +362,14 @@ cudaError_t configure_kernels() {
     if (e == cudaSuccess) e = configure_last();
     if (e == cudaSuccess) e = configure_fused();
     if (e == cudaSuccess) e = configure_small();
+    if (e == cudaSuccess) e = rns_configure();
     return e;
 }
 
-int plan_launches(const Plan& p) { return p.npass == 0 ? 1 : 3 * p.npass + (p.three ? 3 : 0); }
+int plan_launches(const Plan& p) {
+    if (p.rns) return rns_launches(p);
+    return p.npass == 0 ? 1 : 3 * p.npass + (p.three ? 3 : 0);
+}
 
 static cudaError_t launch_forward(const u32* limbs, uint64_t nlimbs, u64* buf, const Plan& p,
                                   const RootTables& tw, bool fused, const u64* aspec, u64 ninv,
@@ -426,6 +432,12 @@ cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb,
     unsigned long long* ol = out_len ? reinterpret_cast<unsigned long long*>(out_len) : len_tmp;
     if (out_len && (e = cudaMemsetAsync(out_len, 0, sizeof(uint64_t), s)) != cudaSuccess) return e;
 
+    if (p.rns) {
+        e = rns_launch_product(a, na, b, nb, out, nout, reinterpret_cast<u32*>(bufA), reinterpret_cast<u32*>(bufB), slots,
+                               ticket, ol, p, err, s, tr, b_ready);
+        if (tr) tr->end(s);
+        return e;
+    }
     if (a == b && na == nb) {
         // a square: one forward transform, its spectrum squared in the fused pass
         if (b_ready && (e = cudaStreamWaitEvent(s, b_ready, 0)) != cudaSuccess) return e;
@@ -474,6 +486,7 @@ static cudaError_t bucket_forward(const Plan& p, const ProdJob* jobs, unsigned n
 cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const RootTables& tw,
                                    cudaStream_t s) {
     if (p.npass == 0) return cudaErrorInvalidValue;
+    if (p.rns) return rns_launch_spectrum(p, jobs, njobs, s);
     return bucket_forward(p, jobs, njobs, tw, s, 0, 0);
 }
 
@@ -490,6 +503,7 @@ cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, co
         g.smem = 2 * rp * sizeof(u64) + (size_t)T * 2 * sizeof(u64);
         return launch_mul_small(logn, g, s, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, ninv, tw, jobs, njobs);
     }
+    if (p.rns) return rns_launch_bucket(p, jobs, njobs, err, s, a_ready);
     cudaError_t e = cudaSuccess;
     for (int op = a_ready ? 1 : 0; op < 2 && e == cudaSuccess; ++op)
         e = bucket_forward(p, jobs, njobs, tw, s, op, 1);  // N^-1: in the carry

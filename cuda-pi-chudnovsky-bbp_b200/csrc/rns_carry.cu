@@ -1,0 +1,171 @@
+// rns_carry.cu -- CRT and carry: residues of the coefficients modulo three
+// 30-bit primes -> u32 limbs.
+//
+// Same decoupled-lookback scan as ntt_carry.cu (one CTA of 256 threads per
+// 2048 limbs, eight consecutive digits per thread), reading 12 bytes of
+// residues per digit instead of two 8-byte coefficients, with the CRT in
+// front of it. With y_i = r_i (scale P / p_i)^-1 mod p_i,
+//     c = sum y_i P / p_i - t P,   t = floor(sum y_i / p_i) in {0, 1, 2}.
+// t comes from the top 16 bits of each y_i: the estimate of the sum is low by
+// less than 2^-11.7, and c / P <= 2^89 / P = 0.79 leaves room for the 2^-11
+// added back.
+//
+// Reference counterpart: carry_propagate (include/ntt.h:70-91).
+#include <cuda_runtime.h>
+
+#include "b2m_internal.h"
+#include "carry.cuh"
+#include "carry_lookback.cuh"
+#include "rns_field.cuh"
+
+namespace b2m {
+
+constexpr int RCARRY_G = 8;  // digits per thread: CARRY_CHUNK / 2 limbs per CTA, as ntt_carry.cu
+static_assert(CARRY_THREADS * RCARRY_G * 2 == CARRY_CHUNK, "one lookback slot per 2048 limbs");
+
+constexpr u64 RNS_P01 = (u64)RNS_P0 * RNS_P1;
+constexpr u32 RNS_PLO = (u32)((u64)(u32)RNS_P01 * RNS_P2);                                   // P mod 2^32
+constexpr u64 RNS_PHI = (RNS_P01 >> 32) * RNS_P2 + (((u64)(u32)RNS_P01 * RNS_P2) >> 32);     // P >> 32
+__host__ __device__ constexpr u32 rns_kt(int i) { return (u32)((1ull << 44) / rns_prime(i)); }
+
+// One digit: c + carry -> limb and the new carry. The carry in and out is
+// below 2^59.
+__device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& carry) {
+    u32 y[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const u32 v = r[i] * k.kap[i].x - __umulhi(r[i], k.kap[i].y) * rns_prime(i);  // [0, 2p)
+        y[i] = __viaddmin_u32(v, 0u - rns_prime(i), v);                               // [0, p)
+    }
+    u32 s = 1u << 19;  // 2^30 * 2^-11
+#pragma unroll
+    for (int i = 0; i < 3; ++i) s += (y[i] >> 14) * rns_kt(i);
+    const u32 t = s >> 30;
+    u64 lo = 0, hi = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        lo += (u64)y[i] * k.qlo[i];  // three terms below 2^62
+        hi += (u64)y[i] * k.qhi[i];
+    }
+    // (hi : lo) - t P + carry, in words w0 and v
+    const u64 tl = (u64)t * RNS_PLO;
+    u64 v = hi + (lo >> 32) - (u64)t * RNS_PHI - (tl >> 32) + (carry >> 32);
+    u32 w = (u32)lo;
+    v -= w < (u32)tl;
+    w -= (u32)tl;
+    w += (u32)carry;
+    v += w < (u32)carry;
+    carry = v;
+    return w;
+}
+
+__global__ void __launch_bounds__(CARRY_THREADS, 6)
+    k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout, u32 nchunks,
+                LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
+                const ProdJob* __restrict__ jobs, const RnsCrt crt) {
+    if (jobs) {
+        const ProdJob& J = jobs[blockIdx.y];
+        coef = reinterpret_cast<const u32*>(J.bufB);
+        out = J.out;
+        nout = J.na + J.nb;
+        slots = J.slots;
+        ticket = J.ticket;
+        out_len = J.out_len;
+    }
+    __shared__ u32 s_chunk;
+    __shared__ u64 s_cin;
+    __shared__ unsigned long long s_top[CARRY_THREADS / 32];
+    __shared__ u64 s_lasth[CARRY_THREADS / 32];
+    __shared__ CState s_ws[CARRY_THREADS / 32 + 1];
+    if (threadIdx.x == 0) s_chunk = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const u32 chunk = s_chunk;
+    if (chunk >= nchunks) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const u64 base = ((u64)chunk * CARRY_THREADS + threadIdx.x) * RCARRY_G;
+
+    u32 lm[RCARRY_G];
+    CState st;
+    {
+        uint4 r[3][RCARRY_G / 4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < RCARRY_G / 4; ++k)
+                r[i][k] = reinterpret_cast<const uint4*>(coef + (u64)i * nt + base)[k];
+        u64 c = 0;
+#pragma unroll
+        for (int k = 0; k < RCARRY_G / 4; ++k) {
+            const u32 d0[3] = {r[0][k].x, r[1][k].x, r[2][k].x}, d1[3] = {r[0][k].y, r[1][k].y, r[2][k].y},
+                      d2[3] = {r[0][k].z, r[1][k].z, r[2][k].z}, d3[3] = {r[0][k].w, r[1][k].w, r[2][k].w};
+            lm[4 * k] = rns_digit(d0, crt, c);
+            lm[4 * k + 1] = rns_digit(d1, crt, c);
+            lm[4 * k + 2] = rns_digit(d2, crt, c);
+            lm[4 * k + 3] = rns_digit(d3, crt, c);
+        }
+        st = group_state<RCARRY_G>(lm, c);
+    }
+    const u64 h_before = __shfl_up_sync(0xFFFFFFFFu, st.h, 1);
+    if (lane == 31) s_lasth[warp] = st.h;
+    u64 cin;
+    if (!__syncthreads_or(st.t != CS_NEVER)) {
+        // no group's carry-out depends on its carry-in (the usual case)
+        const CState agg{s_lasth[CARRY_THREADS / 32 - 1], CS_NEVER};
+        cin = lane > 0 ? h_before : (warp > 0 ? s_lasth[warp - 1] : 0);
+        if (warp == 0) {
+            const u64 c = warp_lookback(slots, chunk, agg, err);
+            if (lane == 0) cin = c;
+        }
+    } else {
+        bool has_ex;
+        CState agg;
+        const CState ex = block_scan_carry(st, &has_ex, &agg, s_ws);
+        if (warp == 0) {
+            const u64 c = warp_lookback(slots, chunk, agg, err);
+            if (threadIdx.x == 0) s_cin = c;
+        }
+        __syncthreads();
+        const u64 cin_chunk = s_cin;
+        if (threadIdx.x == 0) st_release(&slots[chunk].word, (cs_eval(agg, cin_chunk) << 2) | SLOT_INCL);
+        cin = has_ex ? cs_eval(ex, cin_chunk) : cin_chunk;
+    }
+    group_add_carry<RCARRY_G>(lm, cin);
+
+    unsigned long long top = 0;
+#pragma unroll
+    for (int i = 0; i < RCARRY_G; ++i)
+        if (lm[i] && base + i < nout) top = base + i + 1;
+    if (base + RCARRY_G <= nout && ((reinterpret_cast<uintptr_t>(out + base) & 15) == 0)) {
+        uint4* dst = reinterpret_cast<uint4*>(out + base);
+#pragma unroll
+        for (int i = 0; i < RCARRY_G / 4; ++i)
+            dst[i] = make_uint4(lm[4 * i], lm[4 * i + 1], lm[4 * i + 2], lm[4 * i + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < RCARRY_G; ++i)
+            if (base + i < nout) out[base + i] = lm[i];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
+        top = o > top ? o : top;
+    }
+    if (lane == 0) s_top[warp] = top;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 0; w < CARRY_THREADS / 32; ++w) top = s_top[w] > top ? s_top[w] : top;
+        if (top) atomicMax(out_len, top);
+    }
+}
+
+cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
+                             LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
+                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt) {
+    if (nchunks == 0 || njobs == 0) return cudaSuccess;
+    k_rns_carry<<<dim3(nchunks, njobs), CARRY_THREADS, 0, s>>>(coef, nt, out, nout, nchunks, slots, ticket, out_len,
+                                                               err, jobs, crt);
+    return cudaGetLastError();
+}
+
+}  // namespace b2m

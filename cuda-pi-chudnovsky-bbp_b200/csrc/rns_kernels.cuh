@@ -1,0 +1,422 @@
+// rns_kernels.cuh -- transform passes over the three 30-bit primes.
+//
+// A product of na x nb limbs uses 32-bit digits (one limb each) and
+// N = q * 2^m >= na + nb points. Evaluating at N points means reducing the
+// operand modulo x^M - c_t for q constants c_t (M = 2^m, t < q) and splitting
+// each x^M - c_t down to linear factors by a binary tree:
+//     x^2h - w^2 = (x^h - w)(x^h + w),
+// one butterfly (a, b) -> (a + w b, a - w b) per pair of coefficients, with
+// one twiddle w per tree node, the same for every position inside the node.
+// Nodes are numbered 2k, 2k + 1 below k, so with T[k] = product over the set
+// bits j of k of the 2^(j+2)-th root of unity, node k of every level splits
+// with w = T[k]: one table serves all lengths and all levels, and there are
+// no twiddles between passes. The inverse runs the tree backwards with the
+// inverses. Everything stays in place; the spectrum's order never matters.
+//
+// Passes: pass k handles logr[k] levels. An array is B sub-problems (the
+// nodes at the level where the pass starts) of R rows x S columns, row-major.
+// A block takes C columns of one sub-problem; each thread holds 2^LA
+// elements in registers: stage A does LA levels over rows 2^LB apart, one
+// exchange through shared memory, stage B the remaining LB levels over
+// adjacent rows. Loads and stores go straight between registers and global
+// memory (C columns of a row are contiguous). The last pass (S = 1) keeps a
+// sub-problem inside one warp, transforms both operands, multiplies, and
+// runs the first inverse pass on the product without leaving the registers
+// but for the exchanges, so a product of P passes is P + (P - 1) transform
+// launches for both operands and all primes together.
+//
+// What bounds them: the multiply-add pipe (8 cycles of it per butterfly) with
+// the ALU pipe close behind; see rns_field.cuh.
+//
+// Reference counterpart: the per-stage launches of src/ntt_cuda.cu:99-128;
+// the product is the same integer.
+#pragma once
+#include "b2m_internal.h"
+#include "rns_field.cuh"
+
+namespace b2m {
+
+__device__ __forceinline__ uint2 rns_ld(const uint2* p) { return __ldg(p); }
+__device__ __forceinline__ uint4 rns_ld2(const uint2* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+
+// L levels below node `node` on 2^L registers (element k = position k of the
+// node's 2^L equal parts). N0: the node is node 0, whose leftmost chain has
+// w = 1. HZ (with N0): the upper half is zero, so the first level copies.
+template <int L, bool N0, bool HZ, int LEV = 0>
+__device__ __forceinline__ void rns_dft_fwd(u32* x, const uint2* __restrict__ T, u32 node, const RnsMod& m) {
+    constexpr int half = 1 << (L - 1 - LEV);
+    if constexpr (LEV == 0) {
+        if constexpr (N0 && HZ) {
+#pragma unroll
+            for (int i = 0; i < half; ++i) x[i + half] = x[i];
+        } else if constexpr (N0) {
+#pragma unroll
+            for (int i = 0; i < half; ++i) rns_bfly_fwd1(x[i], x[i + half], m);
+        } else {
+            const uint2 w = rns_ld(T + node);
+#pragma unroll
+            for (int i = 0; i < half; ++i) rns_bfly_fwd(x[i], x[i + half], w, m);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < (1 << LEV); j += 2) {
+            const uint4 w = rns_ld2(T + ((u64)node << LEV) + j);
+#pragma unroll
+            for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
+                if (N0 && j == 0) rns_bfly_fwd1(x[i], x[i + half], m);
+                else rns_bfly_fwd(x[i], x[i + half], make_uint2(w.x, w.y), m);
+            }
+#pragma unroll
+            for (int i = (2 * j + 2) * half; i < (2 * j + 3) * half; ++i)
+                rns_bfly_fwd(x[i], x[i + half], make_uint2(w.z, w.w), m);
+        }
+    }
+    if constexpr (LEV + 1 < L) rns_dft_fwd<L, N0, HZ, LEV + 1>(x, T, node, m);
+}
+
+template <int L, bool N0, int LEV = L - 1>
+__device__ __forceinline__ void rns_dft_inv(u32* x, const uint2* __restrict__ T, u32 node, const RnsMod& m) {
+    constexpr int half = 1 << (L - 1 - LEV);
+    if constexpr (LEV == 0) {
+        if constexpr (N0) {
+#pragma unroll
+            for (int i = 0; i < half; ++i) rns_bfly_inv1(x[i], x[i + half], m);
+        } else {
+            const uint2 w = rns_ld(T + node);
+#pragma unroll
+            for (int i = 0; i < half; ++i) rns_bfly_inv(x[i], x[i + half], w, m);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < (1 << LEV); j += 2) {
+            const uint4 w = rns_ld2(T + ((u64)node << LEV) + j);
+#pragma unroll
+            for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
+                if (N0 && j == 0) rns_bfly_inv1(x[i], x[i + half], m);
+                else rns_bfly_inv(x[i], x[i + half], make_uint2(w.x, w.y), m);
+            }
+#pragma unroll
+            for (int i = (2 * j + 2) * half; i < (2 * j + 3) * half; ++i)
+                rns_bfly_inv(x[i], x[i + half], make_uint2(w.z, w.w), m);
+        }
+        rns_dft_inv<L, N0, LEV - 1>(x, T, node, m);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Column passes. LA >= LB; a block is 256 threads: C columns x 2^LB row
+// groups. Shared memory rows get one pad row every 2^LB, so that the warp's
+// row groups (when C < 32) fall into different banks in both stages.
+// ---------------------------------------------------------------------------
+template <int LOGR>
+struct RnsCol {
+    static constexpr int LA = (LOGR + 1) / 2, LB = LOGR - LA;
+    static constexpr int E = 1 << LA, U = 1 << LB, R = 1 << LOGR;
+    static constexpr int LC = 8 - LB, C = 1 << LC;
+    static constexpr int NB = 1 << (LA - LB);  // stage-B transforms per thread
+    static constexpr int SMEM = (R + (R >> LB)) << LC;  // words
+    static constexpr int THREADS = 256;
+    static constexpr int MINB = E >= 32 ? 3 : 4;
+    __device__ __forceinline__ static int sa(int row, int col) { return ((row + (row >> LB)) << LC) + col; }
+};
+
+template <int LOGR>
+__device__ __forceinline__ void rns_exchange_ab(u32* sm, u32 (&x)[RnsCol<LOGR>::E], int u, int col) {
+    using G = RnsCol<LOGR>;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) sm[G::sa(u + (k << G::LB), col)] = x[k];
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = sm[G::sa(((u + (n << G::LB)) << G::LB) + k, col)];
+}
+template <int LOGR>
+__device__ __forceinline__ void rns_exchange_ba(u32* sm, u32 (&x)[RnsCol<LOGR>::E], int u, int col) {
+    using G = RnsCol<LOGR>;
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) sm[G::sa(((u + (n << G::LB)) << G::LB) + k, col)] = x[n * G::U + k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) x[k] = sm[G::sa(u + (k << G::LB), col)];
+}
+
+// Stage B of a column pass: NB transforms of LB levels at nodes node0 + s.
+template <int LOGR, bool INV>
+__device__ __forceinline__ void rns_stage_b(u32 (&x)[RnsCol<LOGR>::E], const uint2* T, u32 node0, int u,
+                                            const RnsMod& m) {
+    using G = RnsCol<LOGR>;
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n) {
+        u32* y = x + n * G::U;
+        if constexpr (INV) rns_dft_inv<G::LB, false>(y, T, node0 + u + (n << G::LB), m);
+        else rns_dft_fwd<G::LB, false, false>(y, T, node0 + u + (n << G::LB), m);
+    }
+}
+
+// Global addresses are a block-uniform 64-bit base per row plus the thread's
+// 32-bit offset (the row step stays in uniform registers): one instruction
+// per access. With 64-bit indices per element, address arithmetic was more
+// than half of a pass's instructions.
+// Stage-B rows ((u + n 2^LB) 2^LB + k) of the thread's column.
+template <int LOGR>
+__device__ __forceinline__ void rns_store_b(const u32* x, u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR>;
+    const u32 o = ((u32)u << (logs + G::LB)) + col;
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) (base + ((u64)((n << (2 * G::LB)) + k) << logs))[o] = x[n * G::U + k];
+}
+template <int LOGR>
+__device__ __forceinline__ void rns_load_b(u32* x, const u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR>;
+    const u32 o = ((u32)u << (logs + G::LB)) + col;
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = (base + ((u64)((n << (2 * G::LB)) + k) << logs))[o];
+}
+// K stage-A rows of limbs (j0 + k rows of 2^LB), zero at and past n, below
+// 4p (np4 = -4p). Tiles below the operand's end take no per-limb check.
+template <int LOGR, int K>
+__device__ __forceinline__ void rns_load_limbs(u32* x, const u32* limbs, u32 j0, u32 n, int logs, u32 np4) {
+    using G = RnsCol<LOGR>;
+    const int ls = logs + G::LB;
+    // last position the block's K rows touch, plus one (at most 2^26)
+    if (((u32)K << ls) - (1u << logs) + G::C <= n) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) x[k] = __ldg(limbs + ((u64)k << ls) + j0);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) x[k] = j0 + ((u32)k << ls) < n ? __ldg(limbs + ((u64)k << ls) + j0) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[k] = __viaddmin_u32(x[k], np4, x[k]);
+}
+
+// Buffer of operand `op` (0: A, 1: B) and the limbs it is made of.
+__device__ __forceinline__ u32* rns_buf(const RnsArgs& a, int op) {
+    if (a.jobs) {
+        const ProdJob& J = a.jobs[blockIdx.y];
+        return reinterpret_cast<u32*>(op ? J.bufB : J.bufA);
+    }
+    return op ? a.bufB : a.bufA;
+}
+
+// First forward pass: limbs -> residues. Grid x: tiles of the q * M points,
+// y: jobs, z: operand * 3 + prime.
+template <int LOGR>
+__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_first(const RnsArgs a) {
+    using G = RnsCol<LOGR>;
+    extern __shared__ u32 smr[];
+    const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
+    const RnsMod m(pi);
+    const u32* limbs = op ? a.b : a.a;
+    u64 nd = op ? a.nb : a.na;
+    if (a.jobs) {
+        const ProdJob& J = a.jobs[blockIdx.y];
+        limbs = op ? J.b : J.a;
+        nd = op ? J.nb : J.na;
+    }
+    u32* buf = rns_buf(a, op) + (u64)pi * a.nt;
+    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), node = blockIdx.x >> (a.logs - G::LC);
+    const u32 c0 = cg << G::LC;                           // first column of the tile
+    const u32 j0 = ((u32)u << a.logs) + col;              // this thread's first position, less c0
+    const u32 n = (u32)nd;                                // at most 2^26
+    const u32 np4 = 2 * m.np2;
+    u32 x[G::E];
+    const uint2* T = a.tw + (u64)pi * a.ent;
+    if (a.q == 1) {
+        if (2 * nd <= a.nt) {
+            // the upper half of the points is zero for almost every product
+            rns_load_limbs<LOGR, G::E / 2>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+            rns_dft_fwd<G::LA, true, true>(x, T, 0, m);
+        } else {
+            rns_load_limbs<LOGR, G::E>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+            rns_dft_fwd<G::LA, true, false>(x, T, 0, m);
+        }
+        rns_exchange_ab<LOGR>(smr, x, u, col);
+        rns_stage_b<LOGR, false>(x, T, 0, u, m);
+    } else {
+        // modulo x^M - c_t: sum over the filled M-blocks of c_t^i x_i, highest first
+        const int lm = a.logs + LOGR;
+        const uint2 ct = a.ct[pi][node];
+        const u32 last = (n - 1) >> lm;
+        const u32 b0 = (last << lm) + c0;
+        rns_load_limbs<LOGR, G::E>(x, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
+        for (u32 i = last; i-- > 0;) {  // blocks below the last are full
+            const u32* lp = limbs + ((i << lm) + c0);
+            u32 v[G::E];
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) v[k] = __ldg(lp + ((u64)k << (a.logs + G::LB)) + j0);
+#pragma unroll
+            for (int k = 0; k < G::E; ++k)
+                x[k] = rns_red2(__viaddmin_u32(v[k], np4, v[k]), m) + rns_mul(x[k], ct, m);
+        }
+        // roots of unity as the c_t: the nodes of the common tree; otherwise
+        // (weighted) each sub-transform has its own first-pass tree and
+        // leaves a factor theta_t^column
+        const uint2* T1 = a.wtree ? a.wtree + ((u64)(pi * a.q + node) << LOGR) : T;
+        const u32 n0 = a.wtree ? 1u : node;
+        rns_dft_fwd<G::LA, false, false>(x, T1, n0, m);
+        rns_exchange_ab<LOGR>(smr, x, u, col);
+        rns_stage_b<LOGR, false>(x, T1, n0 << G::LA, u, m);
+        if (a.wtree) {
+            const uint2 w = rns_ld(a.wcol + ((u64)(pi * a.q + node) << a.logs) + c0 + col);
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) x[k] = rns_mul(x[k], w, m);
+        }
+    }
+    rns_store_b<LOGR>(x, buf + ((u64)node << (a.logs + LOGR)) + c0, u, col, a.logs);
+}
+
+// A middle forward pass, in place. Grid as above.
+template <int LOGR>
+__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_mid(const RnsArgs a) {
+    using G = RnsCol<LOGR>;
+    extern __shared__ u32 smr[];
+    const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
+    const RnsMod m(pi);
+    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), sub = blockIdx.x >> (a.logs - G::LC);
+    const u32 node = sub & a.nmask;
+    u32* buf = rns_buf(a, op) + (u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + ((u64)cg << G::LC);
+    const uint2* T = a.tw + (u64)pi * a.ent;
+    u32 x[G::E];
+    const u32 o = ((u32)u << a.logs) + col;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) x[k] = (buf + ((u64)k << (a.logs + G::LB)))[o];
+    rns_dft_fwd<G::LA, false, false>(x, T, node, m);
+    rns_exchange_ab<LOGR>(smr, x, u, col);
+    rns_stage_b<LOGR, false>(x, T, node << G::LA, u, m);
+    rns_store_b<LOGR>(x, buf, u, col, a.logs);
+}
+
+// An inverse column pass, in place. Grid z: prime. FIRST: the tree's top
+// levels (pass 0).
+template <int LOGR, bool FIRST>
+__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_inv(const RnsArgs a) {
+    using G = RnsCol<LOGR>;
+    extern __shared__ u32 smr[];
+    const int pi = blockIdx.z;
+    const RnsMod m(pi);
+    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), sub = blockIdx.x >> (a.logs - G::LC);
+    u32* buf = rns_buf(a, 1) + (u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + ((u64)cg << G::LC);
+    const uint2* T = a.twi + (u64)pi * a.ent;
+    u32 node = sub & a.nmask;
+    u32 x[G::E];
+    rns_load_b<LOGR>(x, buf, u, col, a.logs);
+    if constexpr (FIRST) {
+        if (a.wtree) {
+            T = a.wtree + ((u64)(pi * a.q + sub) << LOGR);
+            node = 1;
+            const uint2 w = rns_ld(a.wcol + ((u64)(pi * a.q + sub) << a.logs) + ((u64)cg << G::LC) + col);
+#pragma unroll
+            for (int k = 0; k < G::E; ++k) x[k] = rns_mul(x[k], w, m);
+        }
+    }
+    rns_stage_b<LOGR, true>(x, T, node << G::LA, u, m);
+    rns_exchange_ba<LOGR>(smr, x, u, col);
+    if (FIRST && a.q == 1) rns_dft_inv<G::LA, true>(x, T, 0, m);
+    else rns_dft_inv<G::LA, false>(x, T, node, m);
+    const u32 o = ((u32)u << a.logs) + col;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) (buf + ((u64)k << (a.logs + G::LB)))[o] = x[k];
+}
+
+// ---------------------------------------------------------------------------
+// Last forward pass of both operands, pointwise product, first inverse pass.
+// A sub-problem is R contiguous elements handled by U = 2^LB lanes of one
+// warp (U * 2^LA = R), so the exchanges need no block barrier. Grid x: tiles
+// of 256 * 2^LA elements, y: jobs, z: prime. bufA null: a square.
+// ---------------------------------------------------------------------------
+template <int LOGR>
+struct RnsLast {
+    static constexpr int LA = (LOGR + 1) / 2, LB = LOGR - LA;
+    static constexpr int E = 1 << LA, U = 1 << LB, R = 1 << LOGR;
+    static constexpr int NB = 1 << (LA - LB);
+    static constexpr int THREADS = 256, SUBS = THREADS / U;
+    // padded sub-problem: one word per 2^LB, and sub-problems of one warp
+    // start U banks apart (mod 32), so both stages are free of conflicts
+    static constexpr int RAW = R + (R >> LB);
+    static constexpr int BS = LB >= 5 ? RAW : RAW + ((U - RAW % 32) + 32) % 32;
+    static constexpr int SMEM = BS * SUBS;  // words
+    static constexpr int MINB = E >= 32 ? 2 : 3;
+    __device__ __forceinline__ static int sa(int row) { return row + (row >> LB); }
+};
+
+template <int LOGR>
+__device__ __forceinline__ void rns_last_fwd(u32 (&x)[RnsLast<LOGR>::E], u32* sm, const uint2* T, u32 node, int u,
+                                             const RnsMod& m) {
+    using G = RnsLast<LOGR>;
+    rns_dft_fwd<G::LA, false, false>(x, T, node, m);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) sm[G::sa(u + (k << G::LB))] = x[k];
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n) {
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = sm[G::sa(((u + (n << G::LB)) << G::LB) + k)];
+        u32* y = x + n * G::U;
+        rns_dft_fwd<G::LB, false, false>(y, T, (node << G::LA) + u + (n << G::LB), m);
+    }
+}
+
+template <int LOGR>
+__global__ void __launch_bounds__(256, RnsLast<LOGR>::MINB) k_rns_fused(const RnsArgs a) {
+    using G = RnsLast<LOGR>;
+    extern __shared__ u32 smr[];
+    const int pi = blockIdx.z;
+    const RnsMod m(pi);
+    const int u = threadIdx.x & (G::U - 1), sl = threadIdx.x >> G::LB;
+    const u32 sub = blockIdx.x * G::SUBS + sl;
+    if (((u64)sub << LOGR) >= a.nt) return;  // whole sub-problems: whole groups of U lanes
+    u32* sm = smr + sl * G::BS;
+    const u64 off = (u64)pi * a.nt + ((u64)sub << LOGR) + u;
+    u32* bb = rns_buf(a, 1) + off;
+    const uint2* T = a.tw + (u64)pi * a.ent;
+    const uint2* Ti = a.twi + (u64)pi * a.ent;
+    const u32 node = sub & a.nmask;
+    u32 x[G::E];
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) x[k] = bb[k << G::LB];
+    if (!a.square) {
+        const u32* ab = rns_buf(a, 0) + off;
+        u32 y[G::E];
+#pragma unroll
+        for (int k = 0; k < G::E; ++k) y[k] = ab[k << G::LB];
+        rns_last_fwd<LOGR>(y, sm, T, node, u, m);
+        rns_last_fwd<LOGR>(x, sm, T, node, u, m);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k) x[k] = rns_redc((u64)rns_red2(x[k], m) * rns_red2(y[k], m), pi, m);
+    } else {
+        rns_last_fwd<LOGR>(x, sm, T, node, u, m);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k) {
+            const u32 v = rns_red2(x[k], m);
+            x[k] = rns_redc((u64)v * v, pi, m);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n) {
+        u32* y = x + n * G::U;
+        rns_dft_inv<G::LB, false>(y, Ti, (node << G::LA) + u + (n << G::LB), m);
+#pragma unroll
+        for (int k = 0; k < G::U; ++k) sm[G::sa(((u + (n << G::LB)) << G::LB) + k)] = x[n * G::U + k];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) x[k] = sm[G::sa(u + (k << G::LB))];
+    rns_dft_inv<G::LA, false>(x, Ti, node, m);
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) bb[k << G::LB] = x[k];
+}
+
+}  // namespace b2m

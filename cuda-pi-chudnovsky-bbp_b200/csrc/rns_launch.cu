@@ -1,0 +1,540 @@
+// rns_launch.cu -- products on the three-prime residue transforms: lengths,
+// tables and launch sequences (kernels: rns_kernels.cuh, rns_carry.cu).
+//
+// A product whose 16-bit-digit length is 2^L or 3 * 2^k points takes half as
+// many 32-bit digits: N = q * 2^m with q = 1 or 3, as long as the roots of
+// unity last (q * 2^m <= 2^23); beyond that N splits into q <= 8 parts of at
+// most 2^23 points (N <= 2^26, the CRT's bound on the coefficients: at most
+// 2^25 terms below 2^64 each). Parts evaluate modulo x^M - c_t. Where the
+// 2^23 roots allow, c_t is the constant of tree node t and the parts are the
+// first q nodes of the next power of two (a truncated tree); otherwise
+// c_t = theta_t^M with theta_t a power of the generator, the first pass runs
+// the tree of theta_t and its columns take a factor theta_t^column
+// ("weighted"). The parts of the inverse are put together by the inverse
+// Vandermonde matrix of the c_t (k_rns_combine).
+//
+// Reference counterpart: mul_ntt_cuda (src/ntt_cuda.cu:179-243).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <vector>
+
+#include "b2m.h"
+#include "b2m_context.h"
+#include "b2m_internal.h"
+#include "rns_field.cuh"
+
+namespace b2m {
+
+namespace {
+
+struct RnsShape {
+    int q = 0, m = 0;       // N = q * 2^m
+    bool weighted = false;
+    int npass = 0, logr[3] = {0, 0, 0};
+    u64 points() const { return (u64)q << m; }
+};
+
+// Pass radices of a 2^m-point part.
+constexpr int RNS_MIN_M = 13, RNS_MAX_M = RNS_TWO_ADICITY;
+constexpr int kSplit[RNS_MAX_M - RNS_MIN_M + 1][3] = {
+    {6, 0, 7},   // 2^13
+    {6, 0, 8},   // 2^14
+    {7, 0, 8},   // 2^15
+    {8, 0, 8},   // 2^16
+    {9, 0, 8},   // 2^17
+    {10, 0, 8},  // 2^18
+    {10, 0, 9},  // 2^19
+    {6, 6, 8},   // 2^20
+    {6, 7, 8},   // 2^21
+    {7, 7, 8},   // 2^22
+    {7, 8, 8},   // 2^23
+};
+
+// The shape of a plan's length, q = 0 when these transforms do not take it.
+RnsShape rns_shape(const Plan& p) {
+    RnsShape r;
+    if (p.npass < 2) return r;
+    int m = p.logn - 1, q = p.three ? 3 : 1;  // 32-bit digits
+    while (m > RNS_MAX_M) {
+        --m;
+        q *= 2;
+    }
+    if (m < RNS_MIN_M || q > 8) return r;
+    int lq = 0;
+    while ((1 << lq) < q) ++lq;
+    r.q = q;
+    r.m = m;
+    r.weighted = q > 1 && m + lq > RNS_TWO_ADICITY;
+    const int* s = kSplit[m - RNS_MIN_M];
+    for (int k = 0; k < 3; ++k)
+        if (s[k]) r.logr[r.npass++] = s[k];
+    return r;
+}
+
+// ---- tables -------------------------------------------------------------------
+// T[k] = prod over set bits j of k of root_(2^(j+2)), root[] given per prime
+// (forward, or the inverses).
+struct RootSet {
+    u32 w[3][22];
+};
+
+__device__ __forceinline__ u32 dmulmod(u32 a, u32 b, u32 p) { return (u32)((u64)a * b % p); }
+
+__global__ void k_rns_build(uint2* __restrict__ t, u32 ent, const RootSet fwd, const RootSet inv) {
+    const int i = blockIdx.y % 3;
+    const u32 p = rns_prime(i);
+    const RootSet& r = blockIdx.y < 3 ? fwd : inv;
+    uint2* dst = t + (u64)blockIdx.y * ent;
+    for (u32 k = blockIdx.x * blockDim.x + threadIdx.x; k < ent; k += gridDim.x * blockDim.x) {
+        u32 v = 1;
+        for (u32 b = k; b; b &= b - 1) v = dmulmod(v, r.w[i][__ffs(b) - 1], p);
+        dst[k] = make_uint2(v, (u32)(((u64)v << 32) / p));
+    }
+}
+
+// Weighted parts: w^column (column < 2^logs) of a per-part base w, and the
+// first-pass tree: entry 2^lev + k = (theta^(M / 2^(lev+1))) T[k].
+struct WeightSet {
+    u32 col[3][8];          // theta_t (or its inverse)
+    u32 lev[3][8][10];      // theta_t^(M / 2^(lev+1))
+};
+
+__device__ __forceinline__ u32 dpowmod(u32 a, u32 e, u32 p) {
+    u32 r = 1;
+    for (; e; e >>= 1, a = dmulmod(a, a, p))
+        if (e & 1) r = dmulmod(r, a, p);
+    return r;
+}
+
+__global__ void k_rns_build_weights(uint2* __restrict__ tree, uint2* __restrict__ col, int q, int logr, int logs,
+                                    const uint2* __restrict__ T, u32 ent, const WeightSet w) {
+    const int i = blockIdx.y / q, t = blockIdx.y % q;
+    const u32 p = rns_prime(i);
+    const u32 n1 = 1u << logr, n2 = 1u << logs;
+    for (u32 x = blockIdx.x * blockDim.x + threadIdx.x; x < n1 + n2; x += gridDim.x * blockDim.x) {
+        if (x < n1) {
+            u32 v = 1;
+            if (x) {
+                const int lev = 31 - __clz(x);
+                v = dmulmod(w.lev[i][t][lev], T[(u64)i * ent + (x - (1u << lev))].x, p);
+            }
+            tree[((u64)(i * q + t) << logr) + x] = make_uint2(v, (u32)(((u64)v << 32) / p));
+        } else {
+            const u32 v = dpowmod(w.col[i][t], x - n1, p);
+            col[((u64)(i * q + t) << logs) + (x - n1)] = make_uint2(v, (u32)(((u64)v << 32) / p));
+        }
+    }
+}
+
+RootSet root_set(bool inverse) {
+    RootSet r;
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 22; ++j) {
+            const u32 w = j + 2 <= RNS_TWO_ADICITY ? rns_root(i, j + 2) : 1u;
+            r.w[i][j] = inverse ? rns_invmod(w, rns_prime(i)) : w;
+        }
+    return r;
+}
+
+// T[k] on the host, for small k.
+u32 node_root(int i, u32 k) {
+    u32 v = 1;
+    for (int j = 0; j < 22; ++j)
+        if ((k >> j) & 1) v = rns_mulmod(v, rns_root(i, j + 2), rns_prime(i));
+    return v;
+}
+
+u32 theta(int i, int t) { return rns_powmod(rns_generator(i), t, rns_prime(i)); }
+
+// c_t of part t.
+u32 part_constant(const RnsShape& sh, int i, int t) {
+    const u32 p = rns_prime(i);
+    if (sh.q == 1) return 1;
+    if (sh.weighted) return rns_powmod(theta(i, t), 1ull << sh.m, p);
+    const u32 w = node_root(i, t / 2);  // x^2M - w^2 = (x^M - w)(x^M + w)
+    return (t & 1) ? p - w : w;
+}
+
+// Host constants of a shape, computed once.
+struct CombineArgs {
+    u32 v[3][8][8];  // inverse Vandermonde matrix of the c_t
+};
+struct RnsConst {
+    uint2 ct[3][8];
+    CombineArgs comb;
+    RnsCrt crt;
+};
+
+RnsConst make_const(const RnsShape& sh) {
+    RnsConst k{};
+    const int q = sh.q;
+    for (int i = 0; i < 3; ++i) {
+        const u32 p = rns_prime(i);
+        u32 c[8];
+        for (int t = 0; t < q; ++t) {
+            c[t] = part_constant(sh, i, t);
+            k.ct[i][t] = rns_pair(c[t], p);
+        }
+        // inverse of V[t][s] = c_t^s by Gauss-Jordan
+        u32 a[8][16];
+        for (int t = 0; t < q; ++t) {
+            u32 x = 1;
+            for (int s = 0; s < q; ++s, x = rns_mulmod(x, c[t], p)) {
+                a[t][s] = x;
+                a[t][q + s] = s == t;
+            }
+        }
+        for (int col = 0; col < q; ++col) {
+            int piv = col;
+            while (!a[piv][col]) ++piv;
+            for (int s = 0; s < 2 * q; ++s) std::swap(a[piv][s], a[col][s]);
+            const u32 inv = rns_invmod(a[col][col], p);
+            for (int s = 0; s < 2 * q; ++s) a[col][s] = rns_mulmod(a[col][s], inv, p);
+            for (int r = 0; r < q; ++r) {
+                if (r == col || !a[r][col]) continue;
+                const u32 f = p - a[r][col];
+                for (int s = 0; s < 2 * q; ++s) a[r][s] = (u32)((a[r][s] + (u64)f * a[col][s]) % p);
+            }
+        }
+        for (int s = 0; s < q; ++s)
+            for (int t = 0; t < q; ++t) k.comb.v[i][s][t] = a[s][q + t];
+        // residues arrive as c * 2^m * 2^-32 (Montgomery pointwise product),
+        // times 2^-32 again when k_rns_combine ran
+        u32 scale = rns_invmod(rns_powmod(2, 32, p), p);
+        if (q > 1) scale = rns_mulmod(scale, scale, p);
+        scale = rns_mulmod(scale, rns_powmod(2, sh.m, p), p);
+        const u64 qi = i == 0 ? (u64)RNS_P1 * RNS_P2 : (i == 1 ? (u64)RNS_P0 * RNS_P2 : (u64)RNS_P0 * RNS_P1);
+        k.crt.kap[i] = rns_pair(rns_invmod(rns_mulmod(scale, (u32)(qi % p), p), p), p);
+        k.crt.qlo[i] = (u32)qi;
+        k.crt.qhi[i] = (u32)(qi >> 32);
+    }
+    return k;
+}
+
+const RnsConst& shape_const(const RnsShape& sh) {
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, RnsConst> cache;  // at most a few dozen shapes
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = cache.find({sh.q, sh.m});
+    if (it == cache.end()) it = cache.emplace(std::make_pair(sh.q, sh.m), make_const(sh)).first;
+    return it->second;
+}
+
+// The parts' remainders z_t = f mod (x^M - c_t) -> the M-blocks of f:
+// f_s[j] = sum_t V^-1[s][t] z_t[j], one wide sum and one reduction each.
+// In place; z_t < 2p is brought below p, so q <= 8 terms below 2^59.8 fit.
+__global__ void __launch_bounds__(256) k_rns_combine(u32* buf, const ProdJob* __restrict__ jobs, int q, int m_log,
+                                                     const CombineArgs c) {
+    const int i = blockIdx.z;
+    const RnsMod m(i);
+    const u64 M = 1ull << m_log;
+    if (jobs) buf = reinterpret_cast<u32*>(jobs[blockIdx.y].bufB);
+    buf += (u64)i * q * M;
+    for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < M; j += (u64)gridDim.x * blockDim.x) {
+        u32 z[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+            if (t < q) {
+                z[t] = buf[t * M + j];
+                z[t] = __viaddmin_u32(z[t], 0u - m.p, z[t]);
+            }
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            if (s < q) {
+                u64 acc = 0;
+#pragma unroll
+                for (int t = 0; t < 8; ++t)
+                    if (t < q) acc += (u64)z[t] * c.v[i][s][t];
+                buf[s * M + j] = rns_redc(acc, i, m);
+            }
+    }
+}
+
+// ---- context tables --------------------------------------------------------------
+constexpr int RNS_BASE_LOG = 18, RNS_FULL_LOG = RNS_TWO_ADICITY - 1;  // log2 entries per prime and direction
+
+cudaError_t build_tables(uint2** out, int log_ent, cudaStream_t s) {
+    const u64 bytes = 6ull * sizeof(uint2) << log_ent;
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaSuccess) return e;
+    const u32 ent = 1u << log_ent;
+    k_rns_build<<<dim3(std::min<u32>(4096, ent / 256), 6), 256, 0, s>>>(*out, ent, root_set(false), root_set(true));
+    if ((e = cudaGetLastError()) == cudaSuccess) e = cudaStreamSynchronize(s);  // complete before anyone sees it
+    if (e != cudaSuccess) {
+        cudaFree(*out);
+        *out = nullptr;
+    }
+    return e;
+}
+
+int need_log_ent(const RnsShape& sh) {
+    int lq = 0;
+    if (!sh.weighted)
+        while ((1 << lq) < sh.q) ++lq;
+    return sh.m + lq - 1;
+}
+
+// Caller holds c->twt_mu.
+const Context::RnsWeights* find_weights(Context* c, const RnsShape& sh) {
+    for (const Context::RnsWeights& w : c->rns_weights)
+        if (w.q == sh.q && w.m == sh.m) return &w;
+    return nullptr;
+}
+
+cudaError_t build_weights(Context* c, const RnsShape& sh, Context::RnsWeights* w, cudaStream_t s) {
+    const int logr = sh.logr[0], logs = sh.m - logr;
+    const u64 tree = 3ull * sh.q << logr, col = 3ull * sh.q << logs;
+    cudaError_t e = cudaMalloc(&w->mem, 2 * (tree + col) * sizeof(uint2));
+    if (e != cudaSuccess) return e;
+    for (int dir = 0; dir < 2 && e == cudaSuccess; ++dir) {
+        WeightSet ws{};
+        for (int i = 0; i < 3; ++i)
+            for (int t = 0; t < sh.q; ++t) {
+                u32 th = theta(i, t);
+                if (dir) th = rns_invmod(th, rns_prime(i));
+                ws.col[i][t] = th;
+                for (int l = 0; l < logr; ++l) ws.lev[i][t][l] = rns_powmod(th, 1ull << (sh.m - l - 1), rns_prime(i));
+            }
+        uint2* base = w->mem + dir * (tree + col);
+        k_rns_build_weights<<<dim3(64, 3 * sh.q), 256, 0, s>>>(base, base + tree, sh.q, logr, logs,
+                                                              c->rns_t + (dir ? 3ull << c->rns_log : 0),
+                                                              1u << c->rns_log, ws);
+        e = cudaGetLastError();
+        w->tree[dir] = base;
+        w->col[dir] = base + tree;
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        cudaFree(w->mem);
+        w->mem = nullptr;
+    }
+    return e;
+}
+
+}  // namespace
+
+cudaError_t rns_init_tables(Context* c) {
+    cudaError_t e = build_tables(&c->rns_t, RNS_BASE_LOG, 0);
+    if (e != cudaSuccess) return e;
+    c->rns_base = c->rns_t;
+    c->rns_log = RNS_BASE_LOG;
+    return cudaSuccess;
+}
+
+void rns_free_tables(Context* c) {
+    std::lock_guard<std::mutex> lk(c->twt_mu);
+    if (c->rns_t && c->rns_t != c->rns_base) {
+        cudaFree(c->rns_t);
+        budget_release(c, 6ull * sizeof(uint2) << RNS_FULL_LOG);
+    }
+    if (c->rns_base) cudaFree(c->rns_base);
+    c->rns_t = c->rns_base = nullptr;
+    for (Context::RnsWeights& w : c->rns_weights) {
+        cudaFree(w.mem);
+        budget_release(c, w.bytes);
+    }
+    c->rns_weights.clear();
+}
+
+// Only default plans run here: a plan fixed by b2m_set_plan or kept by an
+// autotuner names passes of the 64-bit transform and gets them.
+static bool is_default_plan(const Plan& p) {
+    for (int three = 0; three < 2; ++three) {
+        const Plan d = make_plan(p.logn, three);
+        bool same = d.npass == p.npass;
+        for (int k = 0; same && k < p.npass; ++k) same = d.logr[k] == p.logr[k] && d.logc[k] == p.logc[k];
+        if (same) return true;
+    }
+    return false;
+}
+
+cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
+    p.rns = 0;
+    const RnsShape sh = rns_shape(p);
+    if (!c || !c->rns_t || sh.q == 0 || !is_default_plan(p)) return cudaSuccess;
+    const int need = need_log_ent(sh);
+    if (build) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) build = false;
+    }
+    std::lock_guard<std::mutex> lk(c->twt_mu);
+    // tables only where they leave the product its workspace
+    auto room = [&](uint64_t bytes) {
+        const uint64_t ws = workspace_bytes_plan(p);
+        if (!budget_reserve(c, bytes + ws)) return false;
+        budget_release(c, ws);
+        return true;
+    };
+    if (need > c->rns_log) {
+        const uint64_t bytes = 6ull * sizeof(uint2) << RNS_FULL_LOG;
+        if (!build || !room(bytes)) return cudaSuccess;
+        uint2* t = nullptr;
+        const cudaError_t e = build_tables(&t, RNS_FULL_LOG, s);
+        if (e != cudaSuccess) {
+            budget_release(c, bytes);
+            if (e != cudaErrorMemoryAllocation) return e;
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        c->rns_t = t;  // the base table stays: launches in flight read it
+        c->rns_log = RNS_FULL_LOG;
+    }
+    if (sh.weighted && !find_weights(c, sh)) {
+        if (!build) return cudaSuccess;
+        Context::RnsWeights w{};
+        w.q = sh.q;
+        w.m = sh.m;
+        w.bytes = 2 * 3ull * sh.q * sizeof(uint2) * ((1ull << sh.logr[0]) + (1ull << (sh.m - sh.logr[0])));
+        if (!room(w.bytes)) return cudaSuccess;
+        const cudaError_t e = build_weights(c, sh, &w, s);
+        if (e != cudaSuccess) {
+            budget_release(c, w.bytes);
+            if (e != cudaErrorMemoryAllocation) return e;
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        c->rns_weights.push_back(w);
+    }
+    p.rns = 1;
+    return cudaSuccess;
+}
+
+int rns_launches(const Plan& p) {
+    const RnsShape sh = rns_shape(p);
+    return 2 * sh.npass - 1 + (sh.q > 1) + 1;
+}
+
+namespace {
+
+struct RnsRun {
+    RnsShape sh;
+    RnsArgs a{};
+    unsigned njobs = 1;
+    const uint2 *wtree[2] = {nullptr, nullptr}, *wcol[2] = {nullptr, nullptr};
+    cudaStream_t s;
+    Tracer* tr = nullptr;
+
+    RnsRun(const Plan& p, cudaStream_t st) : sh(rns_shape(p)), s(st) {
+        Context* c = ctx();
+        std::lock_guard<std::mutex> lk(c->twt_mu);
+        a.nt = sh.points();
+        a.tw = c->rns_t;
+        a.ent = 1u << c->rns_log;
+        a.twi = a.tw + 3ull * a.ent;
+        a.q = sh.q;
+        if (sh.weighted) {
+            const Context::RnsWeights* w = find_weights(c, sh);
+            for (int d = 0; d < 2; ++d) {
+                wtree[d] = w->tree[d];
+                wcol[d] = w->col[d];
+            }
+        }
+        const RnsConst& k = shape_const(sh);
+        for (int i = 0; i < 3; ++i)
+            for (int t = 0; t < 8; ++t) a.ct[i][t] = k.ct[i][t];
+    }
+    // Pass k's stride and node mask.
+    void pass(int k) {
+        int before = 0;
+        for (int i = 0; i < k; ++i) before += sh.logr[i];
+        a.logs = sh.m - before - sh.logr[k];
+        a.nmask = sh.weighted ? (1u << before) - 1 : ~0u;
+    }
+    void weights(int dir, bool on) {
+        a.wtree = on ? wtree[dir] : nullptr;
+        a.wcol = on ? wcol[dir] : nullptr;
+    }
+    // elements per block of a column pass: 256 threads of 2^LA
+    unsigned tiles(int k) const { return (unsigned)(a.nt >> (8 + (sh.logr[k] + 1) / 2)); }
+    // Forward passes but the last, operands op0 .. op0 + nops - 1.
+    cudaError_t forward(int op0, int nops) {
+        cudaError_t e = cudaSuccess;
+        a.op0 = op0;
+        for (int k = 0; k + 1 < sh.npass && e == cudaSuccess; ++k) {
+            pass(k);
+            const dim3 grid(tiles(k), njobs, 3 * nops);
+            if (tr) tr->mark(s, k == 0 ? B2M_K_FWD_FIRST : B2M_K_FWD_MID, sh.logr[k]);
+            weights(0, k == 0);
+            e = k == 0 ? rns_launch_first(sh.logr[k], grid, s, a) : rns_launch_mid(sh.logr[k], grid, s, a);
+        }
+        weights(0, false);
+        return e;
+    }
+    // Last forward pass of both operands, product, inverse passes, parts.
+    cudaError_t finish() {
+        const int last = sh.npass - 1;
+        pass(last);
+        if (tr) tr->mark(s, B2M_K_FUSED_LAST, sh.logr[last]);
+        cudaError_t e = rns_launch_fused(sh.logr[last], dim3(1, njobs, 3), s, a);
+        for (int k = last - 1; k >= 0 && e == cudaSuccess; --k) {
+            pass(k);
+            if (tr) tr->mark(s, B2M_K_INV_MID, sh.logr[k]);
+            weights(1, k == 0);
+            e = rns_launch_inv(sh.logr[k], k == 0, dim3(tiles(k), njobs, 3), s, a);
+        }
+        weights(1, false);
+        if (sh.q > 1 && e == cudaSuccess) {
+            if (tr) tr->mark(s, B2M_K_R3_INV, 0);
+            const unsigned blocks = (unsigned)std::min<u64>(4096, (1ull << sh.m) / 256);
+            k_rns_combine<<<dim3(blocks, njobs, 3), 256, 0, s>>>(a.bufB, a.jobs, sh.q, sh.m, shape_const(sh).comb);
+            e = cudaGetLastError();
+        }
+        return e;
+    }
+    cudaError_t carry(u32* out, u64 nout, LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err) {
+        if (tr) tr->mark(s, B2M_K_CARRY, 0);
+        return rns_launch_carry((unsigned)(a.nt / (CARRY_CHUNK / 2)), s, a.bufB, a.nt, out, nout, slots, ticket,
+                                out_len, err, a.jobs, njobs, shape_const(sh).crt);
+    }
+};
+
+}  // namespace
+
+cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout, u32* bufA,
+                               u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,
+                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready) {
+    RnsRun r(p, s);
+    r.tr = tr;
+    r.a.a = a;
+    r.a.b = b;
+    r.a.na = na;
+    r.a.nb = nb;
+    r.a.bufA = bufA;
+    r.a.bufB = bufB;
+    r.a.square = a == b && na == nb;
+    cudaError_t e = cudaSuccess;
+    if (r.a.square || !b_ready) {
+        if (b_ready) e = cudaStreamWaitEvent(s, b_ready, 0);
+        if (e == cudaSuccess) e = r.forward(r.a.square ? 1 : 0, r.a.square ? 1 : 2);
+    } else {
+        // operand B may still be on its way: A's passes go first
+        e = r.forward(0, 1);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b_ready, 0);
+        if (e == cudaSuccess) e = r.forward(1, 1);
+    }
+    if (e == cudaSuccess) e = r.finish();
+    return e == cudaSuccess ? r.carry(out, nout, slots, ticket, out_len, err) : e;
+}
+
+// Operand a of each job up to the last forward pass, which the fused pass
+// repeats for every product that shares it.
+cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, cudaStream_t s) {
+    RnsRun r(p, s);
+    r.a.jobs = jobs;
+    r.njobs = njobs;
+    return r.forward(0, 1);
+}
+
+cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, u32* err, cudaStream_t s,
+                              bool a_ready) {
+    RnsRun r(p, s);
+    r.a.jobs = jobs;
+    r.njobs = njobs;
+    cudaError_t e = a_ready ? r.forward(1, 1) : r.forward(0, 2);
+    if (e == cudaSuccess) e = r.finish();
+    return e == cudaSuccess ? r.carry(nullptr, 0, nullptr, nullptr, nullptr, err) : e;
+}
+
+}  // namespace b2m

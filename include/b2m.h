@@ -371,7 +371,8 @@ enum {
     B2M_K_CARRY = 6,       /* decoupled-lookback carry into u32 limbs */
     B2M_K_SMALL = 7,       /* whole product in one CTA (transform length <= 2^13) */
     B2M_K_R3_FWD = 8,      /* radix-3 step of a 3 * 2^k-point transform (digits in) */
-    B2M_K_R3_INV = 9       /* inverse radix-3 step (coefficients out, natural order) */
+    B2M_K_R3_INV = 9       /* inverse radix-3 step, or the parts of a residue transform put
+                              together (coefficients out, natural order) */
 };
 
 typedef struct b2m_plan_desc {
@@ -387,7 +388,10 @@ typedef struct b2m_plan_desc {
 /* Describes the transform plan the library uses for an na x nb product (no
  * reference counterpart: the reference always runs radix-2 stages of
  * next_pow2(2na + 2nb) points; this library uses 3 * 2^k points instead when
- * that is fewer and k >= 14). */
+ * that is fewer and k >= 14). Default plans of 2^14 to 2^27 points run on
+ * half as many 32-bit digits modulo three 30-bit primes, with passes of their
+ * own: logr and logc then describe the plan of 16-bit digits that they stand
+ * for (and that b2m_set_plan takes), launches what is launched. */
 b2m_status b2m_plan_describe(uint64_t na, uint64_t nb, b2m_plan_desc* desc);
 
 /* One timed candidate of b2m_autotune. */

@@ -1,0 +1,107 @@
+"""Products on the three-prime residue transforms (csrc/rns_*.cu), which run
+every default plan from 2^14 to 2^27 points of 16-bit digits.
+
+Sizes sit at the edges of the lengths: the shortest and the longest product
+of a length, operands longer than half of it (nothing of the first pass is
+zero), one-limb operands, squares, and lengths put together from 2, 3, 4, 6
+and 8 parts. Up to about a million limbs the oracle gives the product; above
+that the 64-bit transform does (the general path, run by fixing one of its
+plans). Everything is an integer: results are equal or wrong."""
+import numpy as np
+import pytest
+
+import oracle
+from golden_util import gen_operand
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(torch, a):
+    return torch.from_numpy(a.view(np.int32)).cuda()
+
+
+def _mul(b2m, torch, a, na, b, nb):
+    out = torch.full((na + nb,), -1, dtype=torch.int32, device="cuda")
+    olen = torch.zeros(1, dtype=torch.int64, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    b2m.mul_device(a.data_ptr(), na, b.data_ptr(), nb, out.data_ptr(), na + nb, olen.data_ptr(), s)
+    b2m.stream_check(s)
+    return out, int(olen.item())
+
+
+# 32-bit points 2^13 .. 2^20 (two and three passes) and 3 * 2^13, 3 * 2^18
+SMALL = [(4096, 1), (8191, 1), (4097, 4095), (8000, 192), (8192, 8192), (16383, 16384), (30000, 2768),
+         (65535, 65537), (131072, 131072), (200000, 62144), (262143, 262145), (524288, 524288), (1000000, 48576),
+         (12288, 12288), (20000, 4576), (24575, 1), (393216, 393216), (700000, 86432)]
+
+
+@pytest.mark.parametrize("na,nb", SMALL)
+@pytest.mark.parametrize("kind", [0, 1])
+def test_edges_match_oracle(b2m_gpu, na, nb, kind):
+    torch = pytest.importorskip("torch")
+    a, b = gen_operand(na + 3, na, kind), gen_operand(nb + 5, nb, kind)
+    out, n = _mul(b2m_gpu, torch, _dev(torch, a), na, _dev(torch, b), nb)
+    want = oracle.mul_port(a, b)
+    got = out.cpu().numpy().view(np.uint32)
+    assert n == want.size and np.array_equal(got[:n], want) and not got[n:].any()
+
+
+@pytest.mark.parametrize("na", [4096, 12288, 70001, 196608, 300000])
+def test_squares_match_oracle(b2m_gpu, na):
+    torch = pytest.importorskip("torch")
+    a = gen_operand(na, na)
+    t = _dev(torch, a)
+    out, n = _mul(b2m_gpu, torch, t, na, t, na)
+    want = oracle.mul_port(a, a)
+    assert n == want.size and np.array_equal(out.cpu().numpy().view(np.uint32)[:n], want)
+
+
+# (sub-)length of the 64-bit transform and one of its non-default plans,
+# product sizes; parts of the residue transform in the comment
+LARGE = [
+    (22, [7, 7, 8], [5, 5, 4], [(1 << 20, 1 << 20), (1900000, 190000)]),             # 2^21: one part
+    (23, [7, 8, 8], [5, 4, 4], [(3 << 21, 3 << 21), (12000000, 500000)]),           # 3 * 2^22: 3 weighted parts
+    (22, [7, 7, 8], [5, 5, 4], [(3 << 20, 3 << 20), (6000000, 290000)]),             # 3 * 2^21: 3 tree parts
+    (25, [8, 9, 8], [4, 3, 4], [(1 << 23, 1 << 23), (16000000, 700000), (8388609, 8388607)]),  # 2 parts
+    (26, [8, 9, 9], [4, 3, 3], [(1 << 24, 1 << 24), (33000000, 500000)]),            # 4 parts
+    (25, [8, 9, 8], [4, 3, 4], [(25000000, 25000000), (50000000, 300000)]),          # 3 * 2^24: 6 parts
+    (27, [9, 9, 9], [3, 3, 3], [(1 << 25, 1 << 25), (60000000, 7000000)]),           # 8 parts
+]
+
+
+@pytest.mark.parametrize("logn,logr,logc,sizes", LARGE)
+@pytest.mark.parametrize("kind", [0, 1])
+def test_large_lengths_match_the_64_bit_transform(b2m_gpu, logn, logr, logc, sizes, kind):
+    torch = pytest.importorskip("torch")
+    for na, nb in sizes:
+        a = torch.empty(na, dtype=torch.int32, device="cuda")
+        b = torch.empty(nb, dtype=torch.int32, device="cuda")
+        b2m_gpu.gen_operand_device(na + 1, na, kind, a.data_ptr())
+        b2m_gpu.gen_operand_device(nb + 2, nb, kind, b.data_ptr())
+        torch.cuda.synchronize()
+        before = b2m_gpu.plan_describe(na, nb)
+        assert before["ntt_log2"] == logn and before["logr"] != logr
+        out, n = _mul(b2m_gpu, torch, a, na, b, nb)
+        try:
+            b2m_gpu.set_plan(logn, logr, logc)
+            want, nw = _mul(b2m_gpu, torch, a, na, b, nb)
+        finally:
+            b2m_gpu.set_plan(logn, before["logr"], before["logc"])
+        assert n == nw and torch.equal(out, want), (na, nb)
+
+
+def test_spectrum_sharing_and_batches_use_the_same_path(b2m_gpu):
+    """Batched jobs of one length: balanced, unbalanced and one-limb operands
+    side by side in one launch."""
+    torch = pytest.importorskip("torch")
+    sizes = [(8192, 8192), (16000, 300), (16383, 1), (1, 16383), (9000, 7000)]
+    ops = [(gen_operand(7 * i + 1, na), gen_operand(7 * i + 2, nb)) for i, (na, nb) in enumerate(sizes)]
+    dev = [(_dev(torch, a), _dev(torch, b)) for a, b in ops]
+    outs = [torch.full((na + nb,), -1, dtype=torch.int32, device="cuda") for na, nb in sizes]
+    jobs = [(a.data_ptr(), na, b.data_ptr(), nb, o.data_ptr(), na + nb, 0)
+            for (na, nb), (a, b), o in zip(sizes, dev, outs)]
+    b2m_gpu.mul_batch(jobs, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    for (a, b), o in zip(ops, outs):
+        want = oracle.mul_port(a, b)
+        assert np.array_equal(o.cpu().numpy().view(np.uint32)[:want.size], want)
