@@ -30,6 +30,7 @@ struct Bucket {
     Plan plan;
     unsigned first = 0;  // index of the bucket's first job in the device table
     unsigned njobs = 0;
+    JobBufs bufs;
 };
 
 }  // namespace b2m
@@ -66,7 +67,8 @@ static cudaError_t enqueue_batch(b2m_batch* bt, cudaStream_t s) {
     for (size_t i = 0; i < bt->buckets.size(); ++i) {
         const Bucket& b = bt->buckets[i];
         cudaStream_t st = bt->side[i % ns];
-        if ((e = launch_bucket(b.plan, bt->djobs + b.first, b.njobs, c->tw, c->d_err, st)) != cudaSuccess) return e;
+        if ((e = launch_bucket(b.plan, bt->djobs + b.first, b.njobs, b.bufs, c->tw, c->d_err, st)) != cudaSuccess)
+            return e;
     }
     for (size_t i = 0; i < ns; ++i) {
         if ((e = cudaEventRecord(bt->ev[1 + i], bt->side[i])) != cudaSuccess) return e;
@@ -116,7 +118,7 @@ static cudaError_t autotune_bucket(b2m_batch* bt, Bucket& b, cudaStream_t s) {
         for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {
             launch_batch_prep(s, bt->djobs, bt->njobs_all, bt->scratch, bt->scratch_words);
             cudaEventRecord(t0, s);
-            e = launch_bucket(p, bt->djobs + b.first, b.njobs, c->tw, c->d_err, s);
+            e = launch_bucket(p, bt->djobs + b.first, b.njobs, b.bufs, c->tw, c->d_err, s);
             cudaEventRecord(t1, s);
             if (e == cudaSuccess) e = cudaEventSynchronize(t1);
             float ms = 0;
@@ -225,6 +227,7 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
         b.plan = plan_for(c, b.logn, three);
         b.first = (unsigned)hj.size();
         b.njobs = (unsigned)std::min<size_t>(MAX_GRID_Y, it->second.size() - off);
+        if (n > (1ull << SMALL_MAX_LOGN)) b.bufs = {pbuf, 16 * n, pbuf + 8 * n, 16 * n};
         for (size_t k = off; k < off + b.njobs; ++k) {
             const unsigned i = it->second[k];
             ProdJob p = mk(i);

@@ -683,7 +683,7 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
         ProdJob* sj = static_cast<ProdJob*>(S.raw(sizeof(ProdJob)));
         k_dc_spec_job<<<1, 1, 0, S.s()>>>(b, nb, spec, sj);
         ck(cudaGetLastError(), "spectrum job");
-        ck(launch_bucket_spectrum(p, sj, 1, c->tw, S.s()), "shared spectrum");
+        ck(launch_bucket_spectrum(p, sj, 1, {spec, 0, nullptr, 0}, c->tw, S.s()), "shared spectrum");
     }
     const uint64_t wss = !p.npass ? 0
                          : spec   ? ((8 * npts + carry_scratch_bytes_n(npts) + 255) & ~255ull)
@@ -701,7 +701,9 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
                                                                   spec);
         if (wss) k_dc_zero_ws<<<(unsigned)nj, 256, 0, S.s()>>>(jobs, nj, carry_scratch_bytes_n(npts) / 8);
         ck(cudaGetLastError(), "job tables");
-        ck(launch_bucket(p, jobs, (unsigned)nj, c->tw, c->d_err, S.s(), spec != nullptr), "batched product");
+        JobBufs bufs;
+        if (wss) bufs = spec ? JobBufs{spec, 0, ws, wss} : JobBufs{ws, wss, ws + 8 * npts, wss};
+        ck(launch_bucket(p, jobs, (unsigned)nj, bufs, c->tw, c->d_err, S.s(), spec != nullptr), "batched product");
     }
 }
 

@@ -636,7 +636,11 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         for (uint64_t off = 0; off < m2 && e == cudaSuccess; off += 65535) {
             const unsigned nj = (unsigned)std::min<uint64_t>(65535, m2 - off);
-            e = launch_bucket(p, jobs + off, nj, c->tw, c->d_err, s, use_spec);
+            JobBufs bufs;
+            if (wss)
+                bufs = use_spec ? JobBufs{pair_ws + off * pair_wss, pair_wss, ws + off * wss, wss}
+                                : JobBufs{ws + off * wss, wss, ws + off * wss + 8 * npts, wss};
+            e = launch_bucket(p, jobs + off, nj, bufs, c->tw, c->d_err, s, use_spec);
         }
         if (!second) {
             pair_ws = ws;  // job i's bufA starts its workspace slot

@@ -93,14 +93,15 @@ struct ProdJob {
 uint64_t carry_scratch_bytes(int logn);
 
 // ---- residue transforms (rns_*.cu) -------------------------------------------
-// Arguments of the transform passes; pointers and lengths of single products
-// are in the struct, batched ones in jobs[blockIdx.y].
+// Arguments of the transform passes. Operands of single products are in the
+// struct, batched ones in jobs[blockIdx.y]; buffers are job 0's and a stride.
 struct RnsArgs {
     const u32* a;
     const u32* b;
     u64 na, nb;
     u32* bufA;                // residues [prime][nt]
     u32* bufB;
+    u64 stride_a, stride_b;   // between jobs, in residues
     const ProdJob* jobs;
     u64 nt;                   // points: q * 2^m
     const uint2* tw;          // T, [prime][ent] (w, floor(2^32 w / p))
@@ -143,12 +144,21 @@ struct Tracer {
 // its operand a under plan p (a spectrum several products share: the kernels
 // only read bufA), so a's forward passes are skipped. Plans of one CTA
 // (npass == 0) transform both operands themselves and ignore it.
-cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const RootTables& tw, u32* err,
-                          cudaStream_t s, bool a_ready = false);
+// The jobs' transform buffers again as job 0's and the strides in bytes
+// between jobs (0: shared), so that kernels address them from uniform
+// registers; null where the plan has one CTA per product.
+struct JobBufs {
+    void* a = nullptr;
+    u64 stride_a = 0;
+    void* b = nullptr;
+    u64 stride_b = 0;
+};
+cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
+                          const RootTables& tw, u32* err, cudaStream_t s, bool a_ready = false);
 // Only the forward transform of operand a of each job, into its bufA
 // (npass >= 1): the spectrum that later launch_bucket(..., a_ready) calls read.
-cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const RootTables& tw,
-                                   cudaStream_t s);
+cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
+                                   const RootTables& tw, cudaStream_t s);
 
 // Grid-wide passes over u32 limbs (b2m_bigops.cu), ordered on s:
 // out = a +- b mod 2^(32 n) (limbs of a at or past la read as 0, likewise b;
@@ -247,9 +257,10 @@ int rns_launches(const Plan& p);
 cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout,
                                u32* bufA, u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,
                                const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready);
-cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, cudaStream_t s);
-cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, u32* err, cudaStream_t s,
-                              bool a_ready);
+cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
+                                cudaStream_t s);
+cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs, u32* err,
+                              cudaStream_t s, bool a_ready);
 // CRT constants of the carry: residues r_i = scale * c mod p_i become the
 // coefficient c (rns_carry.cu).
 struct RnsCrt {
@@ -259,9 +270,10 @@ struct RnsCrt {
 cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                              const ProdJob* jobs, unsigned njobs, const RnsCrt& crt);
-cudaError_t rns_launch_first(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
-cudaError_t rns_launch_mid(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
-cudaError_t rns_launch_inv(int logr, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a);
+// v: columns per thread (1; or 2 up to logr = 8)
+cudaError_t rns_launch_first(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_launch_mid(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
+cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_configure();
 

@@ -248,7 +248,10 @@ static cudaError_t launch_dispatch(b2m_server* S, Slot& sl, std::vector<Req>& rv
         while (k1 < n && rs[order[k1]]->pts == pts && k1 - k0 < 65535) ++k1;
         Plan p = plan_for(S->c, rs[order[k0]]->logn, rs[order[k0]]->three);
         if ((e = twtable_ensure(S->c, p, s)) != cudaSuccess) return e;
-        if ((e = launch_bucket(p, djobs + k0, (unsigned)(k1 - k0), S->c->tw, S->c->d_err, s)) != cudaSuccess) return e;
+        JobBufs bufs;  // as laid out above: two buffers of pts elements per job, jobs back to back
+        if (pts > (1ull << SMALL_MAX_LOGN)) bufs = {hj[k0].bufA, 16 * pts, hj[k0].bufB, 16 * pts};
+        if ((e = launch_bucket(p, djobs + k0, (unsigned)(k1 - k0), bufs, S->c->tw, S->c->d_err, s)) != cudaSuccess)
+            return e;
         // Residue check of the bucket's products, its grid sized to the
         // bucket's longest operands (not the dispatch's).
         uint64_t maxlen = 0;

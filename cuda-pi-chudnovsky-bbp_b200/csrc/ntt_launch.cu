@@ -483,15 +483,15 @@ static cudaError_t bucket_forward(const Plan& p, const ProdJob* jobs, unsigned n
                    : launch_fused_last(p.logr[last], geo(p, last), s, nullptr, nullptr, ninv, tw, jobs, njobs);
 }
 
-cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const RootTables& tw,
-                                   cudaStream_t s) {
+cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
+                                   const RootTables& tw, cudaStream_t s) {
     if (p.npass == 0) return cudaErrorInvalidValue;
-    if (p.rns) return rns_launch_spectrum(p, jobs, njobs, s);
+    if (p.rns) return rns_launch_spectrum(p, jobs, njobs, bufs, s);
     return bucket_forward(p, jobs, njobs, tw, s, 0, 0);
 }
 
-cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const RootTables& tw, u32* err,
-                          cudaStream_t s, bool a_ready) {
+cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
+                          const RootTables& tw, u32* err, cudaStream_t s, bool a_ready) {
     const int logn = p.logn;
     const u64 ninv = gl_inv(plan_points(p));
     if (p.npass == 0) {
@@ -503,7 +503,7 @@ cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, co
         g.smem = 2 * rp * sizeof(u64) + (size_t)T * 2 * sizeof(u64);
         return launch_mul_small(logn, g, s, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, ninv, tw, jobs, njobs);
     }
-    if (p.rns) return rns_launch_bucket(p, jobs, njobs, err, s, a_ready);
+    if (p.rns) return rns_launch_bucket(p, jobs, njobs, bufs, err, s, a_ready);
     cudaError_t e = cudaSuccess;
     for (int op = a_ready ? 1 : 0; op < 2 && e == cudaSuccess; ++op)
         e = bucket_forward(p, jobs, njobs, tw, s, op, 1);  // N^-1: in the carry

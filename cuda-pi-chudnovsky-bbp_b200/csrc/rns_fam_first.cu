@@ -4,20 +4,24 @@
 
 namespace b2m {
 
-template <int LOGR>
+template <int LOGR, int V>
 static cudaError_t launch(dim3 grid, cudaStream_t s, const RnsArgs& a) {
-    k_rns_first<LOGR><<<grid, RnsCol<LOGR>::THREADS, RnsCol<LOGR>::SMEM * 4, s>>>(a);
+    k_rns_first<LOGR, V><<<grid, RnsCol<LOGR, V>::THREADS, RnsCol<LOGR, V>::SMEM * 4, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t rns_launch_first(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a) {
-    switch (logr) {
-        case 5: return launch<5>(grid, s, a);
-        case 6: return launch<6>(grid, s, a);
-        case 7: return launch<7>(grid, s, a);
-        case 8: return launch<8>(grid, s, a);
-        case 9: return launch<9>(grid, s, a);
-        case 10: return launch<10>(grid, s, a);
+cudaError_t rns_launch_first(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a) {
+    switch (16 * v + logr) {
+        case 21: return launch<5, 1>(grid, s, a);
+        case 22: return launch<6, 1>(grid, s, a);
+        case 23: return launch<7, 1>(grid, s, a);
+        case 24: return launch<8, 1>(grid, s, a);
+        case 25: return launch<9, 1>(grid, s, a);
+        case 26: return launch<10, 1>(grid, s, a);
+        case 37: return launch<5, 2>(grid, s, a);
+        case 38: return launch<6, 2>(grid, s, a);
+        case 39: return launch<7, 2>(grid, s, a);
+        case 40: return launch<8, 2>(grid, s, a);
     }
     return cudaErrorInvalidValue;
 }

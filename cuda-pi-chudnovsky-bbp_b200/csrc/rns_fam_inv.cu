@@ -4,21 +4,26 @@
 
 namespace b2m {
 
-template <int LOGR>
+template <int LOGR, int V>
 static cudaError_t launch(bool first, dim3 grid, cudaStream_t s, const RnsArgs& a) {
-    if (first) k_rns_inv<LOGR, true><<<grid, RnsCol<LOGR>::THREADS, RnsCol<LOGR>::SMEM * 4, s>>>(a);
-    else k_rns_inv<LOGR, false><<<grid, RnsCol<LOGR>::THREADS, RnsCol<LOGR>::SMEM * 4, s>>>(a);
+    using G = RnsCol<LOGR, V>;
+    if (first) k_rns_inv<LOGR, V, true><<<grid, G::THREADS, G::SMEM * 4, s>>>(a);
+    else k_rns_inv<LOGR, V, false><<<grid, G::THREADS, G::SMEM * 4, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t rns_launch_inv(int logr, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a) {
-    switch (logr) {
-        case 5: return launch<5>(first, grid, s, a);
-        case 6: return launch<6>(first, grid, s, a);
-        case 7: return launch<7>(first, grid, s, a);
-        case 8: return launch<8>(first, grid, s, a);
-        case 9: return launch<9>(first, grid, s, a);
-        case 10: return launch<10>(first, grid, s, a);
+cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a) {
+    switch (16 * v + logr) {
+        case 21: return launch<5, 1>(first, grid, s, a);
+        case 22: return launch<6, 1>(first, grid, s, a);
+        case 23: return launch<7, 1>(first, grid, s, a);
+        case 24: return launch<8, 1>(first, grid, s, a);
+        case 25: return launch<9, 1>(first, grid, s, a);
+        case 26: return launch<10, 1>(first, grid, s, a);
+        case 37: return launch<5, 2>(first, grid, s, a);
+        case 38: return launch<6, 2>(first, grid, s, a);
+        case 39: return launch<7, 2>(first, grid, s, a);
+        case 40: return launch<8, 2>(first, grid, s, a);
     }
     return cudaErrorInvalidValue;
 }

@@ -39,12 +39,13 @@ namespace b2m {
 __device__ __forceinline__ uint2 rns_ld(const uint2* p) { return __ldg(p); }
 __device__ __forceinline__ uint4 rns_ld2(const uint2* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 
-// L levels below node `node` on 2^L registers (element k = position k of the
-// node's 2^L equal parts). N0: the node is node 0, whose leftmost chain has
-// w = 1. HZ (with N0): the upper half is zero, so the first level copies.
-template <int L, bool N0, bool HZ, int LEV = 0>
+// L levels below node `node` on 2^L positions of V vectors side by side
+// (x[i * V + v]; position i of the node's 2^L equal parts), which share every
+// twiddle load. N0: the node is node 0, whose leftmost chain has w = 1. HZ
+// (with N0): the upper half is zero, so the first level copies.
+template <int L, int V, bool N0, bool HZ, int LEV = 0>
 __device__ __forceinline__ void rns_dft_fwd(u32* x, const uint2* __restrict__ T, u32 node, const RnsMod& m) {
-    constexpr int half = 1 << (L - 1 - LEV);
+    constexpr int half = V << (L - 1 - LEV);
     if constexpr (LEV == 0) {
         if constexpr (N0 && HZ) {
 #pragma unroll
@@ -60,7 +61,7 @@ __device__ __forceinline__ void rns_dft_fwd(u32* x, const uint2* __restrict__ T,
     } else {
 #pragma unroll
         for (int j = 0; j < (1 << LEV); j += 2) {
-            const uint4 w = rns_ld2(T + ((u64)node << LEV) + j);
+            const uint4 w = rns_ld2(T + (node << LEV) + j);
 #pragma unroll
             for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
                 if (N0 && j == 0) rns_bfly_fwd1(x[i], x[i + half], m);
@@ -71,12 +72,12 @@ __device__ __forceinline__ void rns_dft_fwd(u32* x, const uint2* __restrict__ T,
                 rns_bfly_fwd(x[i], x[i + half], make_uint2(w.z, w.w), m);
         }
     }
-    if constexpr (LEV + 1 < L) rns_dft_fwd<L, N0, HZ, LEV + 1>(x, T, node, m);
+    if constexpr (LEV + 1 < L) rns_dft_fwd<L, V, N0, HZ, LEV + 1>(x, T, node, m);
 }
 
-template <int L, bool N0, int LEV = L - 1>
+template <int L, int V, bool N0, int LEV = L - 1>
 __device__ __forceinline__ void rns_dft_inv(u32* x, const uint2* __restrict__ T, u32 node, const RnsMod& m) {
-    constexpr int half = 1 << (L - 1 - LEV);
+    constexpr int half = V << (L - 1 - LEV);
     if constexpr (LEV == 0) {
         if constexpr (N0) {
 #pragma unroll
@@ -89,7 +90,7 @@ __device__ __forceinline__ void rns_dft_inv(u32* x, const uint2* __restrict__ T,
     } else {
 #pragma unroll
         for (int j = 0; j < (1 << LEV); j += 2) {
-            const uint4 w = rns_ld2(T + ((u64)node << LEV) + j);
+            const uint4 w = rns_ld2(T + (node << LEV) + j);
 #pragma unroll
             for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
                 if (N0 && j == 0) rns_bfly_inv1(x[i], x[i + half], m);
@@ -99,119 +100,165 @@ __device__ __forceinline__ void rns_dft_inv(u32* x, const uint2* __restrict__ T,
             for (int i = (2 * j + 2) * half; i < (2 * j + 3) * half; ++i)
                 rns_bfly_inv(x[i], x[i + half], make_uint2(w.z, w.w), m);
         }
-        rns_dft_inv<L, N0, LEV - 1>(x, T, node, m);
+        rns_dft_inv<L, V, N0, LEV - 1>(x, T, node, m);
     }
 }
 
+// V adjacent words.
+template <int V>
+__device__ __forceinline__ void rns_get(u32* x, const u32* p) {
+    if constexpr (V == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
+        x[0] = v.x, x[1] = v.y;
+    } else {
+        x[0] = *p;
+    }
+}
+template <int V>
+__device__ __forceinline__ void rns_put(u32* p, const u32* x) {
+    if constexpr (V == 2) *reinterpret_cast<uint2*>(p) = make_uint2(x[0], x[1]);
+    else *p = x[0];
+}
+
 // ---------------------------------------------------------------------------
-// Column passes. LA >= LB; a block is 256 threads: C columns x 2^LB row
-// groups. Shared memory rows get one pad row every 2^LB, so that the warp's
-// row groups (when C < 32) fall into different banks in both stages.
+// Column passes. LA >= LB; a block is 256 threads: 2^LB row groups x C / V
+// lanes of V adjacent columns. V = 2 halves the memory instructions, the
+// address arithmetic and the twiddle loads per element (a 16-byte twiddle
+// load takes the L1 four cycles even when every lane reads the same one);
+// V = 1 keeps twice as many blocks for short transforms. Shared memory rows
+// get one pad row every 2^LB, so that the row groups of a warp fall into
+// different banks in both stages. Global addresses are a block-uniform
+// 64-bit base per row plus the thread's 32-bit offset.
 // ---------------------------------------------------------------------------
-template <int LOGR>
+template <int LOGR, int V>
 struct RnsCol {
     static constexpr int LA = (LOGR + 1) / 2, LB = LOGR - LA;
     static constexpr int E = 1 << LA, U = 1 << LB, R = 1 << LOGR;
-    static constexpr int LC = 8 - LB, C = 1 << LC;
+    static constexpr int LP = 8 - LB, LC = LP + V - 1, C = 1 << LC;
     static constexpr int NB = 1 << (LA - LB);  // stage-B transforms per thread
     static constexpr int SMEM = (R + (R >> LB)) << LC;  // words
     static constexpr int THREADS = 256;
-    static constexpr int MINB = E >= 32 ? 3 : 4;
+    static constexpr int MINB = E * V >= 32 ? 3 : 4;
+    static_assert(V == 1 || V == 2, "one or two columns");
     __device__ __forceinline__ static int sa(int row, int col) { return ((row + (row >> LB)) << LC) + col; }
 };
 
-template <int LOGR>
-__device__ __forceinline__ void rns_exchange_ab(u32* sm, u32 (&x)[RnsCol<LOGR>::E], int u, int col) {
-    using G = RnsCol<LOGR>;
+// Thread coordinates of a column pass.
+template <class G, int V>
+struct RnsThread {
+    int u, col;
+    __device__ __forceinline__ RnsThread()
+        : u(threadIdx.x >> G::LP), col(((int)threadIdx.x & ((1 << G::LP) - 1)) * V) {}
+};
+
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_exchange_ab(u32* sm, u32* x, int u, int col) {
+    using G = RnsCol<LOGR, V>;
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) sm[G::sa(u + (k << G::LB), col)] = x[k];
+    for (int k = 0; k < G::E; ++k) rns_put<V>(sm + G::sa(u + (k << G::LB), col), x + k * V);
     __syncthreads();
 #pragma unroll
     for (int n = 0; n < G::NB; ++n)
 #pragma unroll
-        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = sm[G::sa(((u + (n << G::LB)) << G::LB) + k, col)];
+        for (int k = 0; k < G::U; ++k)
+            rns_get<V>(x + (n * G::U + k) * V, sm + G::sa(((u + (n << G::LB)) << G::LB) + k, col));
 }
-template <int LOGR>
-__device__ __forceinline__ void rns_exchange_ba(u32* sm, u32 (&x)[RnsCol<LOGR>::E], int u, int col) {
-    using G = RnsCol<LOGR>;
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_exchange_ba(u32* sm, u32* x, int u, int col) {
+    using G = RnsCol<LOGR, V>;
 #pragma unroll
     for (int n = 0; n < G::NB; ++n)
 #pragma unroll
-        for (int k = 0; k < G::U; ++k) sm[G::sa(((u + (n << G::LB)) << G::LB) + k, col)] = x[n * G::U + k];
+        for (int k = 0; k < G::U; ++k)
+            rns_put<V>(sm + G::sa(((u + (n << G::LB)) << G::LB) + k, col), x + (n * G::U + k) * V);
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) x[k] = sm[G::sa(u + (k << G::LB), col)];
+    for (int k = 0; k < G::E; ++k) rns_get<V>(x + k * V, sm + G::sa(u + (k << G::LB), col));
 }
 
 // Stage B of a column pass: NB transforms of LB levels at nodes node0 + s.
-template <int LOGR, bool INV>
-__device__ __forceinline__ void rns_stage_b(u32 (&x)[RnsCol<LOGR>::E], const uint2* T, u32 node0, int u,
-                                            const RnsMod& m) {
-    using G = RnsCol<LOGR>;
+template <int LOGR, int V, bool INV>
+__device__ __forceinline__ void rns_stage_b(u32* x, const uint2* T, u32 node0, int u, const RnsMod& m) {
+    using G = RnsCol<LOGR, V>;
 #pragma unroll
     for (int n = 0; n < G::NB; ++n) {
-        u32* y = x + n * G::U;
-        if constexpr (INV) rns_dft_inv<G::LB, false>(y, T, node0 + u + (n << G::LB), m);
-        else rns_dft_fwd<G::LB, false, false>(y, T, node0 + u + (n << G::LB), m);
+        u32* y = x + n * G::U * V;
+        if constexpr (INV) rns_dft_inv<G::LB, V, false>(y, T, node0 + u + (n << G::LB), m);
+        else rns_dft_fwd<G::LB, V, false, false>(y, T, node0 + u + (n << G::LB), m);
     }
 }
 
-// Global addresses are a block-uniform 64-bit base per row plus the thread's
-// 32-bit offset (the row step stays in uniform registers): one instruction
-// per access. With 64-bit indices per element, address arithmetic was more
-// than half of a pass's instructions.
-// Stage-B rows ((u + n 2^LB) 2^LB + k) of the thread's column.
-template <int LOGR>
-__device__ __forceinline__ void rns_store_b(const u32* x, u32* base, int u, int col, int logs) {
-    using G = RnsCol<LOGR>;
-    const u32 o = ((u32)u << (logs + G::LB)) + col;
+// Stage-A rows u + k 2^LB and stage-B rows (u + n 2^LB) 2^LB + k of the
+// thread's columns, from a block-uniform base.
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_store_a(const u32* x, u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR, V>;
+    const u32 o = ((u32)u << logs) + col;
 #pragma unroll
-    for (int n = 0; n < G::NB; ++n)
-#pragma unroll
-        for (int k = 0; k < G::U; ++k) (base + ((u64)((n << (2 * G::LB)) + k) << logs))[o] = x[n * G::U + k];
+    for (int k = 0; k < G::E; ++k) rns_put<V>(base + ((u64)k << (logs + G::LB)) + o, x + k * V);
 }
-template <int LOGR>
-__device__ __forceinline__ void rns_load_b(u32* x, const u32* base, int u, int col, int logs) {
-    using G = RnsCol<LOGR>;
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_load_a(u32* x, const u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR, V>;
+    const u32 o = ((u32)u << logs) + col;
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) rns_get<V>(x + k * V, base + ((u64)k << (logs + G::LB)) + o);
+}
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_store_b(const u32* x, u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR, V>;
     const u32 o = ((u32)u << (logs + G::LB)) + col;
 #pragma unroll
     for (int n = 0; n < G::NB; ++n)
 #pragma unroll
-        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = (base + ((u64)((n << (2 * G::LB)) + k) << logs))[o];
+        for (int k = 0; k < G::U; ++k)
+            rns_put<V>(base + ((u64)((n << (2 * G::LB)) + k) << logs) + o, x + (n * G::U + k) * V);
+}
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_load_b(u32* x, const u32* base, int u, int col, int logs) {
+    using G = RnsCol<LOGR, V>;
+    const u32 o = ((u32)u << (logs + G::LB)) + col;
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+        for (int k = 0; k < G::U; ++k)
+            rns_get<V>(x + (n * G::U + k) * V, base + ((u64)((n << (2 * G::LB)) + k) << logs) + o);
 }
 // K stage-A rows of limbs (j0 + k rows of 2^LB), zero at and past n, below
-// 4p (np4 = -4p). Tiles below the operand's end take no per-limb check.
-template <int LOGR, int K>
+// 4p (np4 = -4p). Operands are 4-byte aligned: limbs load one by one. Tiles
+// below the operand's end take no per-limb check.
+template <int LOGR, int V, int K>
 __device__ __forceinline__ void rns_load_limbs(u32* x, const u32* limbs, u32 j0, u32 n, int logs, u32 np4) {
-    using G = RnsCol<LOGR>;
+    using G = RnsCol<LOGR, V>;
     const int ls = logs + G::LB;
     // last position the block's K rows touch, plus one (at most 2^26)
     if (((u32)K << ls) - (1u << logs) + G::C <= n) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) x[k] = __ldg(limbs + ((u64)k << ls) + j0);
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int v = 0; v < V; ++v) x[k * V + v] = __ldg(limbs + ((u64)k << ls) + j0 + v);
     } else {
 #pragma unroll
-        for (int k = 0; k < K; ++k) x[k] = j0 + ((u32)k << ls) < n ? __ldg(limbs + ((u64)k << ls) + j0) : 0u;
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                x[k * V + v] = j0 + ((u32)k << ls) + v < n ? __ldg(limbs + ((u64)k << ls) + j0 + v) : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) x[k] = __viaddmin_u32(x[k], np4, x[k]);
+    for (int k = 0; k < K * V; ++k) x[k] = __viaddmin_u32(x[k], np4, x[k]);
 }
 
-// Buffer of operand `op` (0: A, 1: B) and the limbs it is made of.
+// Buffer of operand `op` (0: A, 1: B) of the block's job.
 __device__ __forceinline__ u32* rns_buf(const RnsArgs& a, int op) {
-    if (a.jobs) {
-        const ProdJob& J = a.jobs[blockIdx.y];
-        return reinterpret_cast<u32*>(op ? J.bufB : J.bufA);
-    }
-    return op ? a.bufB : a.bufA;
+    return op ? a.bufB + blockIdx.y * a.stride_b : a.bufA + blockIdx.y * a.stride_a;
 }
 
 // First forward pass: limbs -> residues. Grid x: tiles of the q * M points,
 // y: jobs, z: operand * 3 + prime.
-template <int LOGR>
-__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_first(const RnsArgs a) {
-    using G = RnsCol<LOGR>;
-    extern __shared__ u32 smr[];
+template <int LOGR, int V>
+__global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_first(const RnsArgs a) {
+    using G = RnsCol<LOGR, V>;
+    extern __shared__ __align__(16) u32 smr[];
     const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
     const RnsMod m(pi);
     const u32* limbs = op ? a.b : a.a;
@@ -221,112 +268,123 @@ __global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_first(const Rns
         limbs = op ? J.b : J.a;
         nd = op ? J.nb : J.na;
     }
-    u32* buf = rns_buf(a, op) + (u64)pi * a.nt;
-    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const RnsThread<G, V> t;
     const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), node = blockIdx.x >> (a.logs - G::LC);
     const u32 c0 = cg << G::LC;                           // first column of the tile
-    const u32 j0 = ((u32)u << a.logs) + col;              // this thread's first position, less c0
+    const u32 j0 = ((u32)t.u << a.logs) + t.col;          // this thread's first position, less c0
     const u32 n = (u32)nd;                                // at most 2^26
     const u32 np4 = 2 * m.np2;
-    u32 x[G::E];
+    u32 x[G::E * V];
     const uint2* T = a.tw + (u64)pi * a.ent;
     if (a.q == 1) {
         if (2 * nd <= a.nt) {
             // the upper half of the points is zero for almost every product
-            rns_load_limbs<LOGR, G::E / 2>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
-            rns_dft_fwd<G::LA, true, true>(x, T, 0, m);
+            rns_load_limbs<LOGR, V, G::E / 2>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+            rns_dft_fwd<G::LA, V, true, true>(x, T, 0, m);
         } else {
-            rns_load_limbs<LOGR, G::E>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
-            rns_dft_fwd<G::LA, true, false>(x, T, 0, m);
+            rns_load_limbs<LOGR, V, G::E>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+            rns_dft_fwd<G::LA, V, true, false>(x, T, 0, m);
         }
-        rns_exchange_ab<LOGR>(smr, x, u, col);
-        rns_stage_b<LOGR, false>(x, T, 0, u, m);
+        rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
+        rns_stage_b<LOGR, V, false>(x, T, 0, t.u, m);
     } else {
         // modulo x^M - c_t: sum over the filled M-blocks of c_t^i x_i, highest first
         const int lm = a.logs + LOGR;
         const uint2 ct = a.ct[pi][node];
         const u32 last = (n - 1) >> lm;
         const u32 b0 = (last << lm) + c0;
-        rns_load_limbs<LOGR, G::E>(x, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
+        rns_load_limbs<LOGR, V, G::E>(x, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
         for (u32 i = last; i-- > 0;) {  // blocks below the last are full
             const u32* lp = limbs + ((i << lm) + c0);
-            u32 v[G::E];
 #pragma unroll
-            for (int k = 0; k < G::E; ++k) v[k] = __ldg(lp + ((u64)k << (a.logs + G::LB)) + j0);
+            for (int h = 0; h < 2; ++h) {  // in two halves, for the registers
+                constexpr int H = G::E / 2;
+                u32 v[H * V];
 #pragma unroll
-            for (int k = 0; k < G::E; ++k)
-                x[k] = rns_red2(__viaddmin_u32(v[k], np4, v[k]), m) + rns_mul(x[k], ct, m);
+                for (int k = 0; k < H * V; ++k)
+                    v[k] = __ldg(lp + ((u64)(h * H + k / V) << (a.logs + G::LB)) + j0 + k % V);
+#pragma unroll
+                for (int k = 0; k < H * V; ++k) {
+                    u32& y = x[h * H * V + k];
+                    y = rns_red2(__viaddmin_u32(v[k], np4, v[k]), m) + rns_mul(y, ct, m);
+                }
+            }
         }
         // roots of unity as the c_t: the nodes of the common tree; otherwise
         // (weighted) each sub-transform has its own first-pass tree and
         // leaves a factor theta_t^column
         const uint2* T1 = a.wtree ? a.wtree + ((u64)(pi * a.q + node) << LOGR) : T;
         const u32 n0 = a.wtree ? 1u : node;
-        rns_dft_fwd<G::LA, false, false>(x, T1, n0, m);
-        rns_exchange_ab<LOGR>(smr, x, u, col);
-        rns_stage_b<LOGR, false>(x, T1, n0 << G::LA, u, m);
+        rns_dft_fwd<G::LA, V, false, false>(x, T1, n0, m);
+        rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
+        rns_stage_b<LOGR, V, false>(x, T1, n0 << G::LA, t.u, m);
         if (a.wtree) {
-            const uint2 w = rns_ld(a.wcol + ((u64)(pi * a.q + node) << a.logs) + c0 + col);
+            const uint2* wc = a.wcol + ((u64)(pi * a.q + node) << a.logs) + c0 + t.col;
 #pragma unroll
-            for (int k = 0; k < G::E; ++k) x[k] = rns_mul(x[k], w, m);
+            for (int v = 0; v < V; ++v) {
+                const uint2 w = rns_ld(wc + v);
+#pragma unroll
+                for (int k = 0; k < G::E; ++k) x[k * V + v] = rns_mul(x[k * V + v], w, m);
+            }
         }
     }
-    rns_store_b<LOGR>(x, buf + ((u64)node << (a.logs + LOGR)) + c0, u, col, a.logs);
+    u32* out = rns_buf(a, op) + ((u64)pi * a.nt + ((u64)node << (a.logs + LOGR)) + c0);
+    rns_store_b<LOGR, V>(x, out, t.u, t.col, a.logs);
 }
 
 // A middle forward pass, in place. Grid as above.
-template <int LOGR>
-__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_mid(const RnsArgs a) {
-    using G = RnsCol<LOGR>;
-    extern __shared__ u32 smr[];
+template <int LOGR, int V>
+__global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_mid(const RnsArgs a) {
+    using G = RnsCol<LOGR, V>;
+    extern __shared__ __align__(16) u32 smr[];
     const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
     const RnsMod m(pi);
-    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const RnsThread<G, V> t;
     const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), sub = blockIdx.x >> (a.logs - G::LC);
     const u32 node = sub & a.nmask;
-    u32* buf = rns_buf(a, op) + (u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + ((u64)cg << G::LC);
+    u32* buf = rns_buf(a, op) + ((u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + (cg << G::LC));
     const uint2* T = a.tw + (u64)pi * a.ent;
-    u32 x[G::E];
-    const u32 o = ((u32)u << a.logs) + col;
-#pragma unroll
-    for (int k = 0; k < G::E; ++k) x[k] = (buf + ((u64)k << (a.logs + G::LB)))[o];
-    rns_dft_fwd<G::LA, false, false>(x, T, node, m);
-    rns_exchange_ab<LOGR>(smr, x, u, col);
-    rns_stage_b<LOGR, false>(x, T, node << G::LA, u, m);
-    rns_store_b<LOGR>(x, buf, u, col, a.logs);
+    u32 x[G::E * V];
+    rns_load_a<LOGR, V>(x, buf, t.u, t.col, a.logs);
+    rns_dft_fwd<G::LA, V, false, false>(x, T, node, m);
+    rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
+    rns_stage_b<LOGR, V, false>(x, T, node << G::LA, t.u, m);
+    rns_store_b<LOGR, V>(x, buf, t.u, t.col, a.logs);
 }
 
 // An inverse column pass, in place. Grid z: prime. FIRST: the tree's top
 // levels (pass 0).
-template <int LOGR, bool FIRST>
-__global__ void __launch_bounds__(256, RnsCol<LOGR>::MINB) k_rns_inv(const RnsArgs a) {
-    using G = RnsCol<LOGR>;
-    extern __shared__ u32 smr[];
+template <int LOGR, int V, bool FIRST>
+__global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_inv(const RnsArgs a) {
+    using G = RnsCol<LOGR, V>;
+    extern __shared__ __align__(16) u32 smr[];
     const int pi = blockIdx.z;
     const RnsMod m(pi);
-    const int col = threadIdx.x & (G::C - 1), u = threadIdx.x >> G::LC;
+    const RnsThread<G, V> t;
     const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), sub = blockIdx.x >> (a.logs - G::LC);
-    u32* buf = rns_buf(a, 1) + (u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + ((u64)cg << G::LC);
+    u32* buf = rns_buf(a, 1) + ((u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + (cg << G::LC));
     const uint2* T = a.twi + (u64)pi * a.ent;
     u32 node = sub & a.nmask;
-    u32 x[G::E];
-    rns_load_b<LOGR>(x, buf, u, col, a.logs);
+    u32 x[G::E * V];
+    rns_load_b<LOGR, V>(x, buf, t.u, t.col, a.logs);
     if constexpr (FIRST) {
         if (a.wtree) {
             T = a.wtree + ((u64)(pi * a.q + sub) << LOGR);
             node = 1;
-            const uint2 w = rns_ld(a.wcol + ((u64)(pi * a.q + sub) << a.logs) + ((u64)cg << G::LC) + col);
+            const uint2* wc = a.wcol + ((u64)(pi * a.q + sub) << a.logs) + (cg << G::LC) + t.col;
 #pragma unroll
-            for (int k = 0; k < G::E; ++k) x[k] = rns_mul(x[k], w, m);
+            for (int v = 0; v < V; ++v) {
+                const uint2 w = rns_ld(wc + v);
+#pragma unroll
+                for (int k = 0; k < G::E; ++k) x[k * V + v] = rns_mul(x[k * V + v], w, m);
+            }
         }
     }
-    rns_stage_b<LOGR, true>(x, T, node << G::LA, u, m);
-    rns_exchange_ba<LOGR>(smr, x, u, col);
-    if (FIRST && a.q == 1) rns_dft_inv<G::LA, true>(x, T, 0, m);
-    else rns_dft_inv<G::LA, false>(x, T, node, m);
-    const u32 o = ((u32)u << a.logs) + col;
-#pragma unroll
-    for (int k = 0; k < G::E; ++k) (buf + ((u64)k << (a.logs + G::LB)))[o] = x[k];
+    rns_stage_b<LOGR, V, true>(x, T, node << G::LA, t.u, m);
+    rns_exchange_ba<LOGR, V>(smr, x, t.u, t.col);
+    if (FIRST && a.q == 1) rns_dft_inv<G::LA, V, true>(x, T, 0, m);
+    else rns_dft_inv<G::LA, V, false>(x, T, node, m);
+    rns_store_a<LOGR, V>(x, buf, t.u, t.col, a.logs);
 }
 
 // ---------------------------------------------------------------------------
@@ -350,22 +408,26 @@ struct RnsLast {
     __device__ __forceinline__ static int sa(int row) { return row + (row >> LB); }
 };
 
-template <int LOGR>
-__device__ __forceinline__ void rns_last_fwd(u32 (&x)[RnsLast<LOGR>::E], u32* sm, const uint2* T, u32 node, int u,
-                                             const RnsMod& m) {
+// The forward levels of the pass on V operands side by side (x[k * V + v]).
+template <int LOGR, int V>
+__device__ __forceinline__ void rns_last_fwd(u32* x, u32* sm, const uint2* T, u32 node, int u, const RnsMod& m) {
     using G = RnsLast<LOGR>;
-    rns_dft_fwd<G::LA, false, false>(x, T, node, m);
-    __syncwarp();
+    rns_dft_fwd<G::LA, V, false, false>(x, T, node, m);
 #pragma unroll
-    for (int k = 0; k < G::E; ++k) sm[G::sa(u + (k << G::LB))] = x[k];
-    __syncwarp();
+    for (int v = 0; v < V; ++v) {
+        __syncwarp();
 #pragma unroll
-    for (int n = 0; n < G::NB; ++n) {
+        for (int k = 0; k < G::E; ++k) sm[G::sa(u + (k << G::LB))] = x[k * V + v];
+        __syncwarp();
 #pragma unroll
-        for (int k = 0; k < G::U; ++k) x[n * G::U + k] = sm[G::sa(((u + (n << G::LB)) << G::LB) + k)];
-        u32* y = x + n * G::U;
-        rns_dft_fwd<G::LB, false, false>(y, T, (node << G::LA) + u + (n << G::LB), m);
+        for (int n = 0; n < G::NB; ++n)
+#pragma unroll
+            for (int k = 0; k < G::U; ++k)
+                x[(n * G::U + k) * V + v] = sm[G::sa(((u + (n << G::LB)) << G::LB) + k)];
     }
+#pragma unroll
+    for (int n = 0; n < G::NB; ++n)
+        rns_dft_fwd<G::LB, V, false, false>(x + n * G::U * V, T, (node << G::LA) + u + (n << G::LB), m);
 }
 
 template <int LOGR>
@@ -384,19 +446,18 @@ __global__ void __launch_bounds__(256, RnsLast<LOGR>::MINB) k_rns_fused(const Rn
     const uint2* Ti = a.twi + (u64)pi * a.ent;
     const u32 node = sub & a.nmask;
     u32 x[G::E];
-#pragma unroll
-    for (int k = 0; k < G::E; ++k) x[k] = bb[k << G::LB];
     if (!a.square) {
         const u32* ab = rns_buf(a, 0) + off;
-        u32 y[G::E];
+        u32 y[2 * G::E];
 #pragma unroll
-        for (int k = 0; k < G::E; ++k) y[k] = ab[k << G::LB];
-        rns_last_fwd<LOGR>(y, sm, T, node, u, m);
-        rns_last_fwd<LOGR>(x, sm, T, node, u, m);
+        for (int k = 0; k < G::E; ++k) y[2 * k] = bb[k << G::LB], y[2 * k + 1] = ab[k << G::LB];
+        rns_last_fwd<LOGR, 2>(y, sm, T, node, u, m);
 #pragma unroll
-        for (int k = 0; k < G::E; ++k) x[k] = rns_redc((u64)rns_red2(x[k], m) * rns_red2(y[k], m), pi, m);
+        for (int k = 0; k < G::E; ++k) x[k] = rns_redc((u64)rns_red2(y[2 * k], m) * rns_red2(y[2 * k + 1], m), pi, m);
     } else {
-        rns_last_fwd<LOGR>(x, sm, T, node, u, m);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k) x[k] = bb[k << G::LB];
+        rns_last_fwd<LOGR, 1>(x, sm, T, node, u, m);
 #pragma unroll
         for (int k = 0; k < G::E; ++k) {
             const u32 v = rns_red2(x[k], m);
@@ -406,15 +467,14 @@ __global__ void __launch_bounds__(256, RnsLast<LOGR>::MINB) k_rns_fused(const Rn
     __syncwarp();
 #pragma unroll
     for (int n = 0; n < G::NB; ++n) {
-        u32* y = x + n * G::U;
-        rns_dft_inv<G::LB, false>(y, Ti, (node << G::LA) + u + (n << G::LB), m);
+        rns_dft_inv<G::LB, 1, false>(x + n * G::U, Ti, (node << G::LA) + u + (n << G::LB), m);
 #pragma unroll
         for (int k = 0; k < G::U; ++k) sm[G::sa(((u + (n << G::LB)) << G::LB) + k)] = x[n * G::U + k];
     }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < G::E; ++k) x[k] = sm[G::sa(u + (k << G::LB))];
-    rns_dft_inv<G::LA, false>(x, Ti, node, m);
+    rns_dft_inv<G::LA, 1, false>(x, Ti, node, m);
 #pragma unroll
     for (int k = 0; k < G::E; ++k) bb[k << G::LB] = x[k];
 }
