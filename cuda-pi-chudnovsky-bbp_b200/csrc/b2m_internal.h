@@ -237,9 +237,6 @@ cudaError_t launch_r3_fwd(cudaStream_t s, const u32* limbs, u64 ndig, u64* out, 
                           const ProdJob* jobs = nullptr, unsigned njobs = 1, int operand = 0);
 cudaError_t launch_r3_inv(cudaStream_t s, u64* buf, int logm, const RootTables& tw, const ProdJob* jobs = nullptr,
                           unsigned njobs = 1);
-cudaError_t launch_mul_small(int logn, const PassGeo& g, cudaStream_t s, const u32* a, u64 na, const u32* b, u64 nb,
-                             u32* out, u64 nout, unsigned long long* out_len, u64 ninv, const RootTables& tw,
-                             const ProdJob* jobs = nullptr, unsigned njobs = 1);
 // The coefficients in `coef` are the unscaled inverse transform of `points`
 // points (N * c mod p); the carry scales them by points^-1 (points = 1: as
 // they are).
@@ -276,12 +273,15 @@ cudaError_t rns_launch_mid(int logr, int v, dim3 grid, cudaStream_t s, const Rns
 cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_configure();
+// Whole products of up to 2^12 points, one cluster each (rns_small.cu).
+cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out,
+                             unsigned long long* out_len, const RnsCrt& crt);
+cudaError_t rns_configure_small();
 
 cudaError_t configure_first();
 cudaError_t configure_mid();
 cudaError_t configure_inv();
 cudaError_t configure_last();
 cudaError_t configure_fused();
-cudaError_t configure_small();
 
 }  // namespace b2m

@@ -51,17 +51,9 @@ FAMILIES = [
          "(bbuf, aspec, ninv, tw, jobs, g.zstride)", "dim3(g.grid, njobs, g.zdim)")]),
 ]
 
-SMALL = ("ntt_fam_small.cu", "single-CTA products, N <= 2^13", "small", "k_mul_small", range(2, 14),
-         "launch_mul_small",
-         "(int logn, const PassGeo& g, cudaStream_t s, const u32* a, u64 na, const u32* b, u64 nb, u32* out, "
-         "u64 nout, unsigned long long* out_len, u64 ninv, const RootTables& tw, const ProdJob* jobs, "
-         "unsigned njobs)",
-         "(a, na, b, nb, out, nout, out_len, ninv, tw, jobs)", "dim3(g.grid * njobs)")
-
 HEAD = ("// {fn} -- instantiations and launchers: {desc}.\n"
         "// Written by gen_families.py; kernel bodies are in ntt_kernels.cuh. With a\n"
-        "// job table the grid's second dimension (the first, for single-CTA\n"
-        "// products) runs over the jobs.\n"
+        "// job table the grid's second dimension runs over the jobs.\n"
         "#include \"ntt_kernels.cuh\"\n\nnamespace b2m {{\n")
 
 
@@ -80,25 +72,8 @@ def pass_family(fn, desc, tag, kerns):
     return "".join(out)
 
 
-def small_family():
-    fn, desc, tag, kern, rng, launcher, sig, args, grid = SMALL
-    out = [HEAD.format(fn=fn, desc=desc)]
-    out.append(f"\ncudaError_t {launcher}{sig} {{\n    switch (logn) {{\n")
-    cfg = []
-    for n in rng:
-        out.append(f"        case {n}: {kern}<{n}><<<{grid}, g.block, g.smem, s>>>{args}; break;\n")
-        cfg.append(f"    if (e == cudaSuccess) e = cudaFuncSetAttribute({kern}<{n}>, "
-                   f"cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);\n")
-    out.append("        default: return cudaErrorInvalidConfiguration;\n    }\n    return cudaGetLastError();\n}\n")
-    out.append(f"\ncudaError_t configure_{tag}() {{\n    cudaError_t e = cudaSuccess;\n" + "".join(cfg)
-               + "    return e;\n}\n\n}  // namespace b2m\n")
-    return "".join(out)
-
-
 if __name__ == "__main__":
     for fn, desc, tag, kerns in FAMILIES:
         with open(os.path.join(HERE, fn), "w") as f:
             f.write(pass_family(fn, desc, tag, kerns))
-    with open(os.path.join(HERE, SMALL[0]), "w") as f:
-        f.write(small_family())
-    print("wrote", ", ".join([x[0] for x in FAMILIES] + [SMALL[0]]))
+    print("wrote", ", ".join(x[0] for x in FAMILIES))

@@ -1,7 +1,6 @@
 // ntt_fam_last.cu -- instantiations and launchers: last forward pass of operand A.
 // Written by gen_families.py; kernel bodies are in ntt_kernels.cuh. With a
-// job table the grid's second dimension (the first, for single-CTA
-// products) runs over the jobs.
+// job table the grid's second dimension runs over the jobs.
 #include "ntt_kernels.cuh"
 
 namespace b2m {

@@ -9,7 +9,6 @@
 //   inverse: k_inv_mid for the remaining passes (pass 1 yields N times the
 //      coefficients in natural order), k_carry (scale by 1/N, then the
 //      decoupled-lookback carry into u32 limbs + trimmed length).
-// For N <= 2^13 one CTA does the whole product (k_mul_small).
 //
 // Every pass kernel: a cooperative, coalesced load of its R x C tile into
 // shared memory, the column DFTs in shared memory (ntt_engine.cuh), and a
@@ -24,9 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "b2m_internal.h"
-#include "carry.cuh"
 #include "ntt_engine.cuh"
-#include "school.cuh"
 
 namespace b2m {
 
@@ -429,103 +426,6 @@ k_fused_last(u64* __restrict__ bbuf, const u64* __restrict__ aspec, u64 ninv, Ro
     tile_inv<TL>(sm, tw.dtw);
 #pragma unroll
     for (int k = 0; k < G::PER; ++k) base[k * TL::T] = sm[gp.sa0 + G::soff(k)];
-}
-
-// ---------------------------------------------------------------------------
-// Whole product in one CTA for N = 2^LOGN <= 2^13: both transforms live in
-// shared memory, the carry is a block scan. max(1, N/16) threads; thread t
-// owns coefficients [t*G, (t+1)*G), G = min(16, N). A product whose
-// schoolbook cost is lower (school_cheaper) is computed that way instead, by
-// the same threads in the same shared memory.
-// ---------------------------------------------------------------------------
-constexpr int small_threads(int logn) { return logn >= 4 ? 1 << (logn - 4) : 1; }
-constexpr int small_min_blocks(int logn) {
-    return PASS_THREADS_MAX / small_threads(logn) < 32 ? PASS_THREADS_MAX / small_threads(logn) : 32;
-}
-
-template <int LOGN>
-__global__ void __launch_bounds__(small_threads(LOGN), small_min_blocks(LOGN)) k_mul_small(const u32* __restrict__ a, u64 na, const u32* __restrict__ b,
-                                                   u64 nb, u32* __restrict__ out, u64 nout,
-                                                   unsigned long long* out_len, u64 ninv, RootTables tw,
-                                                   const ProdJob* __restrict__ jobs) {
-    if (jobs) {
-        const ProdJob& J = jobs[blockIdx.x];
-        a = J.a;
-        b = J.b;
-        na = J.na;
-        nb = J.nb;
-        out = J.out;
-        nout = J.na + J.nb;
-        out_len = J.out_len;
-    }
-    using TL = Tile<LOGN, 0, MAP_ROW>;
-    constexpr int N = 1 << LOGN, RP = TL::RP, G = N < 16 ? N : 16;
-    extern __shared__ u64 sm[];
-    u64* smA = sm;
-    u64* smB = sm + RP;
-    CState* s_st = reinterpret_cast<CState*>(sm + 2 * RP);
-    __shared__ unsigned long long s_top;
-    if (school_cheaper(na, nb, LOGN)) {
-        school_cta(a, na, b, nb, out, out_len, reinterpret_cast<unsigned char*>(sm), s_st, &s_top);
-        return;
-    }
-    const u64 nda = 2 * na, ndb = 2 * nb;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        smA[TL::saddr(i, 0)] = digit_of(a, nda, i);
-        smB[TL::saddr(i, 0)] = digit_of(b, ndb, i);
-    }
-    if (threadIdx.x == 0) s_top = 0;
-    __syncthreads();
-    tile_fwd<TL, true>(smA, tw.dtw);
-    tile_fwd<TL, true>(smB, tw.dtw);
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const int s = TL::saddr(i, 0);
-        smB[s] = gl_mul(gl_mul(smB[s], smA[s]), ninv);
-    }
-    __syncthreads();
-    tile_inv<TL>(smB, tw.dtw);
-
-    // Carry: thread t owns G consecutive coefficients.
-    const int T = blockDim.x;
-    u64 v[G];
-#pragma unroll
-    for (int i = 0; i < G; ++i) v[i] = smB[TL::saddr((int)threadIdx.x * G + i, 0)];
-    u32 lm[G / 2];
-    const CState st = group_carry<G>(v, lm);
-    u64 cin;
-    if (T >= 32) {
-        bool has;
-        CState agg;
-        const CState ex = block_scan_carry(st, &has, &agg, s_st);
-        cin = has ? cs_eval(ex, 0) : 0;
-    } else {
-        s_st[threadIdx.x] = st;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            // Serial exclusive scan: s_st[t].h becomes the carry into t.
-            u64 c = 0;
-            for (int t = 0; t < T; ++t) {
-                const CState f = s_st[t];
-                s_st[t].h = c;
-                c = cs_eval(f, c);
-            }
-        }
-        __syncthreads();
-        cin = s_st[threadIdx.x].h;
-    }
-    group_add_carry<G / 2>(lm, cin);
-    const u64 lbase = (u64)threadIdx.x * (G / 2);
-    unsigned long long top = 0;
-#pragma unroll
-    for (int i = 0; i < G / 2; ++i) {
-        if (lbase + i < nout) {
-            out[lbase + i] = lm[i];
-            if (lm[i]) top = lbase + i + 1;
-        }
-    }
-    if (top) atomicMax(&s_top, top);
-    __syncthreads();
-    if (threadIdx.x == 0 && out_len) *out_len = s_top;
 }
 
 }  // namespace b2m

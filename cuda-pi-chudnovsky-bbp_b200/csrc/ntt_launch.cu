@@ -7,7 +7,7 @@
 //      pointwise product with A's spectrum and N^-1, first inverse pass);
 //   inverse middle/first passes (pass 1 yields the coefficients), then the
 //   decoupled-lookback carry into u32 limbs and the trimmed length.
-// For N <= 2^13 a single CTA does everything.
+// For N <= 2^13 one launch does everything (rns_small.cu).
 //
 // Reference counterpart: mul_ntt_cuda (src/ntt_cuda.cu:179-243) -- host
 // repack (include/ntt.h:56-64), bit reversal + log2 N radix-2 launches per
@@ -361,7 +361,7 @@ cudaError_t configure_kernels() {
     if (e == cudaSuccess) e = configure_inv();
     if (e == cudaSuccess) e = configure_last();
     if (e == cudaSuccess) e = configure_fused();
-    if (e == cudaSuccess) e = configure_small();
+    if (e == cudaSuccess) e = rns_configure_small();
     if (e == cudaSuccess) e = rns_configure();
     return e;
 }
@@ -401,25 +401,10 @@ cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb,
                            cudaEvent_t b_ready) {
     const int logn = p.logn;
     const uint64_t n = plan_points(p);
-    const u64 ninv = gl_inv(n);
     const u64 nout = na + nb;
-    if (p.npass == 0) {
-        PassGeo g{};
-        const int T = logn >= 4 ? (1 << (logn - 4)) : 1;
-        const size_t rp = (size_t)(1 << logn) + (size_t)((1 << logn) >> 6);
-        g.grid = 1;
-        g.block = (unsigned)T;
-        g.smem = 2 * rp * sizeof(u64) + (size_t)T * 2 * sizeof(u64);
-        if (b_ready) {
-            cudaError_t e = cudaStreamWaitEvent(s, b_ready, 0);
-            if (e != cudaSuccess) return e;
-        }
-        if (tr) tr->mark(s, B2M_K_SMALL, logn);
-        cudaError_t e = launch_mul_small(logn, g, s, a, na, b, nb, out, nout,
-                                         reinterpret_cast<unsigned long long*>(out_len), ninv, tw);
-        if (tr) tr->end(s);
-        return e;
-    }
+    if (p.npass == 0)
+        return rns_launch_product(a, na, b, nb, out, nout, nullptr, nullptr, nullptr, nullptr,
+                                  reinterpret_cast<unsigned long long*>(out_len), p, err, s, tr, b_ready);
     u64* bufA = static_cast<u64*>(ws);
     u64* bufB = bufA + n;
     unsigned char* scratch = reinterpret_cast<unsigned char*>(bufB + n);
@@ -435,7 +420,6 @@ cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb,
     if (p.rns) {
         e = rns_launch_product(a, na, b, nb, out, nout, reinterpret_cast<u32*>(bufA), reinterpret_cast<u32*>(bufB), slots,
                                ticket, ol, p, err, s, tr, b_ready);
-        if (tr) tr->end(s);
         return e;
     }
     if (a == b && na == nb) {
@@ -493,16 +477,7 @@ cudaError_t launch_bucket_spectrum(const Plan& p, const ProdJob* jobs, unsigned 
 cudaError_t launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
                           const RootTables& tw, u32* err, cudaStream_t s, bool a_ready) {
     const int logn = p.logn;
-    const u64 ninv = gl_inv(plan_points(p));
-    if (p.npass == 0) {
-        PassGeo g{};
-        const int T = logn >= 4 ? (1 << (logn - 4)) : 1;
-        const size_t rp = (size_t)(1 << logn) + (size_t)((1 << logn) >> 6);
-        g.grid = 1;
-        g.block = (unsigned)T;
-        g.smem = 2 * rp * sizeof(u64) + (size_t)T * 2 * sizeof(u64);
-        return launch_mul_small(logn, g, s, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, ninv, tw, jobs, njobs);
-    }
+    if (p.npass == 0) return rns_launch_bucket(p, jobs, njobs, bufs, err, s, a_ready);
     if (p.rns) return rns_launch_bucket(p, jobs, njobs, bufs, err, s, a_ready);
     cudaError_t e = cudaSuccess;
     for (int op = a_ready ? 1 : 0; op < 2 && e == cudaSuccess; ++op)

@@ -3,12 +3,8 @@
 //
 // Same decoupled-lookback scan as ntt_carry.cu (one CTA of 256 threads per
 // 2048 limbs, eight consecutive digits per thread), reading 12 bytes of
-// residues per digit instead of two 8-byte coefficients, with the CRT in
-// front of it. With y_i = r_i (scale P / p_i)^-1 mod p_i,
-//     c = sum y_i P / p_i - t P,   t = floor(sum y_i / p_i) in {0, 1, 2}.
-// t comes from the top 16 bits of each y_i: the estimate of the sum is low by
-// less than 2^-11.7, and c / P <= 2^89 / P = 0.79 leaves room for the 2^-11
-// added back.
+// residues per digit instead of two 8-byte coefficients, with the CRT
+// (rns_crt.cuh) in front of it.
 //
 // Reference counterpart: carry_propagate (include/ntt.h:70-91).
 #include <cuda_runtime.h>
@@ -16,20 +12,14 @@
 #include "b2m_internal.h"
 #include "carry.cuh"
 #include "carry_lookback.cuh"
-#include "rns_field.cuh"
+#include "rns_crt.cuh"
 
 namespace b2m {
 
 constexpr int RCARRY_G = 8;  // digits per thread: CARRY_CHUNK / 2 limbs per CTA, as ntt_carry.cu
 static_assert(CARRY_THREADS * RCARRY_G * 2 == CARRY_CHUNK, "one lookback slot per 2048 limbs");
 
-constexpr u64 RNS_P01 = (u64)RNS_P0 * RNS_P1;
-constexpr u32 RNS_PLO = (u32)((u64)(u32)RNS_P01 * RNS_P2);                                   // P mod 2^32
-constexpr u64 RNS_PHI = (RNS_P01 >> 32) * RNS_P2 + (((u64)(u32)RNS_P01 * RNS_P2) >> 32);     // P >> 32
-__host__ __device__ constexpr u32 rns_kt(int i) { return (u32)((1ull << 44) / rns_prime(i)); }
-
-// One digit: c + carry -> limb and the new carry. The carry in and out is
-// below 2^59.
+// One digit from its residues: c + carry -> limb and the new carry.
 __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& carry) {
     u32 y[3];
 #pragma unroll
@@ -37,26 +27,7 @@ __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& car
         const u32 v = r[i] * k.kap[i].x - __umulhi(r[i], k.kap[i].y) * rns_prime(i);  // [0, 2p)
         y[i] = __viaddmin_u32(v, 0u - rns_prime(i), v);                               // [0, p)
     }
-    u32 s = 1u << 19;  // 2^30 * 2^-11
-#pragma unroll
-    for (int i = 0; i < 3; ++i) s += (y[i] >> 14) * rns_kt(i);
-    const u32 t = s >> 30;
-    u64 lo = 0, hi = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        lo += (u64)y[i] * k.qlo[i];  // three terms below 2^62
-        hi += (u64)y[i] * k.qhi[i];
-    }
-    // (hi : lo) - t P + carry, in words w0 and v
-    const u64 tl = (u64)t * RNS_PLO;
-    u64 v = hi + (lo >> 32) - (u64)t * RNS_PHI - (tl >> 32) + (carry >> 32);
-    u32 w = (u32)lo;
-    v -= w < (u32)tl;
-    w -= (u32)tl;
-    w += (u32)carry;
-    v += w < (u32)carry;
-    carry = v;
-    return w;
+    return rns_crt_digit(y, k, carry);
 }
 
 __global__ void __launch_bounds__(CARRY_THREADS, 6)

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_first(cons
         // modulo x^M - c_t: sum over the filled M-blocks of c_t^i x_i, highest first
         const int lm = a.logs + LOGR;
         const uint2 ct = a.ct[pi][node];
-        const u32 last = (n - 1) >> lm;
+        const u32 last = n ? (n - 1) >> lm : 0u;
         const u32 b0 = (last << lm) + c0;
         rns_load_limbs<LOGR, V, G::E>(x, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
         for (u32 i = last; i-- > 0;) {  // blocks below the last are full

@@ -60,7 +60,11 @@ constexpr u64 RNS_V2_POINTS = 1ull << 21;
 // The shape of a plan's length, q = 0 when these transforms do not take it.
 RnsShape rns_shape(const Plan& p) {
     RnsShape r;
-    if (p.npass < 2) return r;
+    if (p.npass < 2) {  // one launch
+        r.q = 1;
+        r.m = p.logn - 1;
+        return r;
+    }
     int m = p.logn - 1, q = p.three ? 3 : 1;  // 32-bit digits
     while (m > RNS_MAX_M) {
         --m;
@@ -406,6 +410,7 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
 
 int rns_launches(const Plan& p) {
     const RnsShape sh = rns_shape(p);
+    if (sh.npass == 0) return 1;
     return 2 * sh.npass - 1 + (sh.q > 1) + 1;
 }
 
@@ -419,7 +424,9 @@ struct RnsRun {
     cudaStream_t s;
     Tracer* tr = nullptr;
 
-    RnsRun(const Plan& p, cudaStream_t st) : sh(rns_shape(p)), s(st) {
+    bool small;  // one launch (rns_small.cu)
+
+    RnsRun(const Plan& p, cudaStream_t st) : sh(rns_shape(p)), s(st), small(sh.q == 1 && sh.npass == 0) {
         Context* c = ctx();
         std::lock_guard<std::mutex> lk(c->twt_mu);
         a.nt = sh.points();
@@ -520,6 +527,13 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
     r.a.bufB = bufB;
     r.a.square = a == b && na == nb;
     cudaError_t e = cudaSuccess;
+    if (r.small) {
+        if (b_ready && (e = cudaStreamWaitEvent(s, b_ready, 0)) != cudaSuccess) return e;
+        if (tr) tr->mark(s, B2M_K_SMALL, p.logn);
+        e = rns_launch_small(r.sh.m, 1, s, r.a, out, out_len, shape_const(r.sh).crt);
+        if (tr) tr->end(s);
+        return e;
+    }
     if (r.a.square || !b_ready) {
         if (b_ready) e = cudaStreamWaitEvent(s, b_ready, 0);
         if (e == cudaSuccess) e = r.forward(r.a.square ? 1 : 0, r.a.square ? 1 : 2);
@@ -530,7 +544,9 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
         if (e == cudaSuccess) e = r.forward(1, 1);
     }
     if (e == cudaSuccess) e = r.finish();
-    return e == cudaSuccess ? r.carry(out, nout, slots, ticket, out_len, err) : e;
+    if (e == cudaSuccess) e = r.carry(out, nout, slots, ticket, out_len, err);
+    if (tr) tr->end(s);
+    return e;
 }
 
 // Operand a of each job up to the last forward pass, which the fused pass
@@ -538,6 +554,7 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
 cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
                                 cudaStream_t s) {
     RnsRun r(p, s);
+    if (r.small) return cudaSuccess;  // transforms both operands itself
     r.batch(jobs, njobs, bufs);
     return r.forward(0, 1);
 }
@@ -546,6 +563,7 @@ cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs
                               cudaStream_t s, bool a_ready) {
     RnsRun r(p, s);
     r.batch(jobs, njobs, bufs);
+    if (r.small) return rns_launch_small(r.sh.m, njobs, s, r.a, nullptr, nullptr, shape_const(r.sh).crt);
     cudaError_t e = a_ready ? r.forward(1, 1) : r.forward(0, 2);
     if (e == cudaSuccess) e = r.finish();
     return e == cudaSuccess ? r.carry(nullptr, 0, nullptr, nullptr, nullptr, err) : e;

@@ -1,10 +1,8 @@
 // school.cuh -- schoolbook product of two small u32-limb numbers by one CTA.
 //
-// The one-CTA NTT product (k_mul_small) costs about N log2 N * 75 integer
-// instructions for N transform points; a schoolbook product costs about
-// 4.5 instructions per limb multiply-add, so for the smaller and the
-// unbalanced products of up to 2^13 points (na + nb <= 4096 limbs) it is the
-// cheaper of the two. Reference
+// A schoolbook product costs about 4.5 instructions per limb multiply-add, so
+// for the smaller and the unbalanced products of one launch (rns_small.cu) it
+// is cheaper than the transforms. Reference
 // counterpart: mul_schoolbook (src/bignum.cpp:125-143), the same column
 // products, here with every column sum of a thread's four-column block
 // accumulated in 96 bits by one carry chain per multiply-add, and the carries
@@ -14,19 +12,15 @@
 
 namespace b2m {
 
-// A product takes the schoolbook path when na * nb <= SCHOOL_MACS_PER_POINT * N
-// for the N-point one-CTA NTT it would otherwise use. Measured on a B200 in
-// batches of 4096 products: schoolbook ~0.28 us per 10^6 limb multiply-adds,
-// one-CTA NTT ~4e-5 us per transform point (2^11..2^13 points), so the two
-// cost the same near na * nb = 140 N; below ~256 limbs the schoolbook is 2-4x
-// faster, at 2048 x 2048 limbs 3x slower.
+// A product of up to 2^m limbs takes the schoolbook path when na * nb <=
+// SCHOOL_MACS_PER_POINT * 2^m.
 #ifndef B2M_SCHOOL_MACS_PER_POINT
-#define B2M_SCHOOL_MACS_PER_POINT 128
+#define B2M_SCHOOL_MACS_PER_POINT 16
 #endif
 constexpr unsigned long long SCHOOL_MACS_PER_POINT = B2M_SCHOOL_MACS_PER_POINT;
 
-__device__ __forceinline__ bool school_cheaper(u64 na, u64 nb, int logn) {
-    return na * nb <= (1ull << logn) * SCHOOL_MACS_PER_POINT;
+__device__ __forceinline__ bool school_cheaper(u64 na, u64 nb, int m) {
+    return na * nb <= (1ull << m) * SCHOOL_MACS_PER_POINT;
 }
 
 // (lo, mid, hi) += x * y as one 96-bit carry chain.
