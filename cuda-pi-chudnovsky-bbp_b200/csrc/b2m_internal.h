@@ -114,6 +114,9 @@ struct RnsArgs {
     int q;
     int op0;                  // operand of grid z 0..2
     int square;
+    unsigned long long* zero;      // first pass of a single product: scratch it zeroes
+    unsigned long long* zero_len;  // and the length
+    u32 nzero;                     // words of it
     uint2 ct[3][8];           // c_t of the q sub-transforms
 };
 

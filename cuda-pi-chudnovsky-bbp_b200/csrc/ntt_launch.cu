@@ -412,16 +412,14 @@ cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb,
     LookbackSlot* slots = reinterpret_cast<LookbackSlot*>(scratch);
     u32* ticket = reinterpret_cast<u32*>(scratch + nchunks * sizeof(LookbackSlot));
     unsigned long long* len_tmp = reinterpret_cast<unsigned long long*>(ticket + 2);
+    unsigned long long* ol = out_len ? reinterpret_cast<unsigned long long*>(out_len) : len_tmp;
+    if (p.rns)  // zeroes its scratch and *ol itself
+        return rns_launch_product(a, na, b, nb, out, nout, reinterpret_cast<u32*>(bufA), reinterpret_cast<u32*>(bufB), slots,
+                                  ticket, ol, p, err, s, tr, b_ready);
     cudaError_t e = cudaMemsetAsync(scratch, 0, carry_scratch_bytes_n(n), s);
     if (e != cudaSuccess) return e;
-    unsigned long long* ol = out_len ? reinterpret_cast<unsigned long long*>(out_len) : len_tmp;
     if (out_len && (e = cudaMemsetAsync(out_len, 0, sizeof(uint64_t), s)) != cudaSuccess) return e;
 
-    if (p.rns) {
-        e = rns_launch_product(a, na, b, nb, out, nout, reinterpret_cast<u32*>(bufA), reinterpret_cast<u32*>(bufB), slots,
-                               ticket, ol, p, err, s, tr, b_ready);
-        return e;
-    }
     if (a == b && na == nb) {
         // a square: one forward transform, its spectrum squared in the fused pass
         if (b_ready && (e = cudaStreamWaitEvent(s, b_ready, 0)) != cudaSuccess) return e;

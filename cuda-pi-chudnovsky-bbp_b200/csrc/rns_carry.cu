@@ -12,6 +12,7 @@
 #include "b2m_internal.h"
 #include "carry.cuh"
 #include "carry_lookback.cuh"
+#include "pdl.cuh"
 #include "rns_crt.cuh"
 
 namespace b2m {
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
     k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout, u32 nchunks,
                 LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                 const ProdJob* __restrict__ jobs, const RnsCrt crt) {
+    pdl_enter();
     if (jobs) {
         const ProdJob& J = jobs[blockIdx.y];
         coef = reinterpret_cast<const u32*>(J.bufB);
@@ -134,9 +136,8 @@ cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, 
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                              const ProdJob* jobs, unsigned njobs, const RnsCrt& crt) {
     if (nchunks == 0 || njobs == 0) return cudaSuccess;
-    k_rns_carry<<<dim3(nchunks, njobs), CARRY_THREADS, 0, s>>>(coef, nt, out, nout, nchunks, slots, ticket, out_len,
-                                                               err, jobs, crt);
-    return cudaGetLastError();
+    return launch_pdl(k_rns_carry, dim3(nchunks, njobs), CARRY_THREADS, 0, s, coef, nt, out, nout, nchunks, slots, ticket,
+                      out_len, err, jobs, crt);
 }
 
 }  // namespace b2m

@@ -6,8 +6,7 @@ namespace b2m {
 
 template <int LOGR, int V>
 static cudaError_t launch(dim3 grid, cudaStream_t s, const RnsArgs& a) {
-    k_rns_first<LOGR, V><<<grid, RnsCol<LOGR, V>::THREADS, RnsCol<LOGR, V>::SMEM * 4, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(k_rns_first<LOGR, V>, grid, RnsCol<LOGR, V>::THREADS, RnsCol<LOGR, V>::SMEM * 4, s, a);
 }
 
 cudaError_t rns_launch_first(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a) {

@@ -20,8 +20,7 @@ template <int LOGR>
 static cudaError_t launch(dim3 grid, cudaStream_t s, const RnsArgs& a) {
     const u64 per = (u64)RnsLast<LOGR>::SUBS << LOGR;
     grid.x = (unsigned)((a.nt + per - 1) / per);
-    k_rns_fused<LOGR><<<grid, RnsLast<LOGR>::THREADS, RnsLast<LOGR>::SMEM * 4, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(k_rns_fused<LOGR>, grid, RnsLast<LOGR>::THREADS, RnsLast<LOGR>::SMEM * 4, s, a);
 }
 
 cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a) {

@@ -7,9 +7,8 @@ namespace b2m {
 template <int LOGR, int V>
 static cudaError_t launch(bool first, dim3 grid, cudaStream_t s, const RnsArgs& a) {
     using G = RnsCol<LOGR, V>;
-    if (first) k_rns_inv<LOGR, V, true><<<grid, G::THREADS, G::SMEM * 4, s>>>(a);
-    else k_rns_inv<LOGR, V, false><<<grid, G::THREADS, G::SMEM * 4, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(first ? k_rns_inv<LOGR, V, true> : k_rns_inv<LOGR, V, false>, grid, G::THREADS, G::SMEM * 4, s,
+                      a);
 }
 
 cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a) {

@@ -32,6 +32,7 @@
 // the product is the same integer.
 #pragma once
 #include "b2m_internal.h"
+#include "pdl.cuh"
 #include "rns_field.cuh"
 
 namespace b2m {
@@ -261,6 +262,13 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_first(cons
     extern __shared__ __align__(16) u32 smr[];
     const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
     const RnsMod m(pi);
+    pdl_enter();
+    // single products: the carry's scratch and the length start at zero
+    if (a.zero && blockIdx.z == 0) {
+        const u32 i = blockIdx.x * 256 + threadIdx.x;
+        if (i < a.nzero) a.zero[i] = 0;
+        if (i == 0) *a.zero_len = 0;
+    }
     const u32* limbs = op ? a.b : a.a;
     u64 nd = op ? a.nb : a.na;
     if (a.jobs) {
@@ -345,6 +353,7 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_mid(const 
     u32* buf = rns_buf(a, op) + ((u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + (cg << G::LC));
     const uint2* T = a.tw + (u64)pi * a.ent;
     u32 x[G::E * V];
+    pdl_enter();
     rns_load_a<LOGR, V>(x, buf, t.u, t.col, a.logs);
     rns_dft_fwd<G::LA, V, false, false>(x, T, node, m);
     rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
@@ -366,6 +375,7 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_inv(const 
     const uint2* T = a.twi + (u64)pi * a.ent;
     u32 node = sub & a.nmask;
     u32 x[G::E * V];
+    pdl_enter();
     rns_load_b<LOGR, V>(x, buf, t.u, t.col, a.logs);
     if constexpr (FIRST) {
         if (a.wtree) {
@@ -446,6 +456,7 @@ __global__ void __launch_bounds__(256, RnsLast<LOGR>::MINB) k_rns_fused(const Rn
     const uint2* Ti = a.twi + (u64)pi * a.ent;
     const u32 node = sub & a.nmask;
     u32 x[G::E];
+    pdl_enter();
     if (!a.square) {
         const u32* ab = rns_buf(a, 0) + off;
         u32 y[2 * G::E];

@@ -23,6 +23,7 @@
 #include "b2m.h"
 #include "b2m_context.h"
 #include "b2m_internal.h"
+#include "pdl.cuh"
 #include "rns_field.cuh"
 
 namespace b2m {
@@ -91,15 +92,29 @@ struct RootSet {
 
 __device__ __forceinline__ u32 dmulmod(u32 a, u32 b, u32 p) { return (u32)((u64)a * b % p); }
 
-__global__ void k_rns_build(uint2* __restrict__ t, u32 ent, const RootSet fwd, const RootSet inv) {
+// T[k] = T[k mod 2^11] * T[(k div 2^11) 2^11], from the two short tables.
+constexpr int RNS_BUILD_LOG = 11;
+
+__global__ void __launch_bounds__(1 << RNS_BUILD_LOG >> 1) k_rns_build(uint2* __restrict__ t, u32 ent,
+                                                                      const RootSet fwd, const RootSet inv) {
+    __shared__ u32 lo[1 << RNS_BUILD_LOG];
     const int i = blockIdx.y % 3;
     const u32 p = rns_prime(i);
     const RootSet& r = blockIdx.y < 3 ? fwd : inv;
     uint2* dst = t + (u64)blockIdx.y * ent;
-    for (u32 k = blockIdx.x * blockDim.x + threadIdx.x; k < ent; k += gridDim.x * blockDim.x) {
+    for (u32 k = threadIdx.x; k < (1u << RNS_BUILD_LOG); k += blockDim.x) {
         u32 v = 1;
         for (u32 b = k; b; b &= b - 1) v = dmulmod(v, r.w[i][__ffs(b) - 1], p);
-        dst[k] = make_uint2(v, (u32)(((u64)v << 32) / p));
+        lo[k] = v;
+    }
+    __syncthreads();
+    for (u32 h = blockIdx.x; (h << RNS_BUILD_LOG) < ent; h += gridDim.x) {
+        u32 w = 1;
+        for (u32 b = h; b; b &= b - 1) w = dmulmod(w, r.w[i][RNS_BUILD_LOG + __ffs(b) - 1], p);
+        for (u32 k = threadIdx.x; k < (1u << RNS_BUILD_LOG); k += blockDim.x) {
+            const u32 v = dmulmod(w, lo[k], p);
+            dst[((u64)h << RNS_BUILD_LOG) + k] = make_uint2(v, (u32)(((u64)v << 32) / p));
+        }
     }
 }
 
@@ -238,6 +253,7 @@ __global__ void __launch_bounds__(256) k_rns_combine(u32* buf, u64 stride, int q
     const int i = blockIdx.z;
     const RnsMod m(i);
     const u64 M = 1ull << m_log;
+    pdl_enter();
     buf += blockIdx.y * stride + (u64)i * q * M;
     for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < M; j += (u64)gridDim.x * blockDim.x) {
         u32 z[8];
@@ -267,7 +283,8 @@ cudaError_t build_tables(uint2** out, int log_ent, cudaStream_t s) {
     cudaError_t e = cudaMalloc(out, bytes);
     if (e != cudaSuccess) return e;
     const u32 ent = 1u << log_ent;
-    k_rns_build<<<dim3(std::min<u32>(4096, ent / 256), 6), 256, 0, s>>>(*out, ent, root_set(false), root_set(true));
+    k_rns_build<<<dim3(std::min<u32>(148, ent >> RNS_BUILD_LOG), 6), 1 << RNS_BUILD_LOG >> 1, 0, s>>>(
+        *out, ent, root_set(false), root_set(true));
     if ((e = cudaGetLastError()) == cudaSuccess) e = cudaStreamSynchronize(s);  // complete before anyone sees it
     if (e != cudaSuccess) {
         cudaFree(*out);
@@ -499,9 +516,8 @@ struct RnsRun {
         if (sh.q > 1 && e == cudaSuccess) {
             if (tr) tr->mark(s, B2M_K_R3_INV, 0);
             const unsigned blocks = (unsigned)std::min<u64>(4096, (1ull << sh.m) / 256);
-            k_rns_combine<<<dim3(blocks, njobs, 3), 256, 0, s>>>(a.bufB, a.stride_b, sh.q, sh.m,
-                                                                 shape_const(sh).comb);
-            e = cudaGetLastError();
+            e = launch_pdl(k_rns_combine, dim3(blocks, njobs, 3), 256, 0, s, a.bufB, a.stride_b, sh.q, sh.m,
+                           shape_const(sh).comb);
         }
         return e;
     }
@@ -534,6 +550,10 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
         if (tr) tr->end(s);
         return e;
     }
+    // lookback slots, then the ticket: one word per 1024 points and a few
+    r.a.zero = reinterpret_cast<unsigned long long*>(slots);
+    r.a.nzero = (u32)(carry_scratch_bytes_n(plan_points(p)) / 8);
+    r.a.zero_len = out_len;
     if (r.a.square || !b_ready) {
         if (b_ready) e = cudaStreamWaitEvent(s, b_ready, 0);
         if (e == cudaSuccess) e = r.forward(r.a.square ? 1 : 0, r.a.square ? 1 : 2);
@@ -541,6 +561,7 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
         // operand B may still be on its way: A's passes go first
         e = r.forward(0, 1);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b_ready, 0);
+        r.a.zero = nullptr;
         if (e == cudaSuccess) e = r.forward(1, 1);
     }
     if (e == cudaSuccess) e = r.finish();

@@ -6,8 +6,8 @@
 // memory, and leaves its CRT terms there; each block then reads a third of
 // all terms through distributed shared memory, forms those coefficients and
 // resolves their carries with a block scan and the other blocks' aggregates.
-// Products of few limb
-// multiply-adds are schoolbook columns in block 0 alone (school.cuh).
+// Products of at most 128 limbs are
+// schoolbook columns (school.cuh).
 //
 // What bounds it: latency. A 2048 x 2048-limb product by one block in the
 // 64-bit field took 48 us on one SM; here three SMs share it.
@@ -30,6 +30,10 @@ namespace cg = cooperative_groups;
 // operand per thread.
 template <int M>
 struct SmallCfg;
+template <>
+struct SmallCfg<8> {
+    static constexpr int LE = 3, NS = 3, l[3] = {3, 3, 2};
+};
 template <>
 struct SmallCfg<9> {
     static constexpr int LE = 3, NS = 3, l[3] = {3, 3, 3};
@@ -126,10 +130,8 @@ __device__ __forceinline__ void small_inv(u32* x, u32* sx, const uint2* T, const
 template <int M>
 struct SmallShape {
     static constexpr int N = 1 << M, T = 1 << (M - SmallCfg<M>::LE), PAD = N + N / 16;
-    // pairs, then the product, and one carry state per thread; the
-    // schoolbook path lays its columns over all of it
-    static constexpr int SMEM = PAD * 12 + T * 16;
-    static constexpr int BYTES = SMEM > 16 * N + 64 + T * 16 ? SMEM : 16 * N + 64 + T * 16;
+    // pairs, then the product, and one carry state per warp
+    static constexpr int BYTES = PAD * 12 + T / 32 * 16;
     static constexpr int D = (N + 3 * T - 1) / (3 * T);  // digits per thread of the cluster
     static constexpr int MINB = T >= 256 ? 3 : (T >= 128 ? 6 : 10);
 };
@@ -145,6 +147,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, Sm
     __shared__ unsigned long long s_tops[3];
     __shared__ CState s_agg[2];  // of the blocks before this one
     const int pi = blockIdx.x % 3;
+    pdl_enter();
     const u32 *la = a.a, *lb = a.b;
     u64 na = a.na, nb = a.nb;
     if (a.jobs) {
@@ -158,11 +161,7 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, Sm
     }
     uint2* sp = reinterpret_cast<uint2*>(smem);
     u32* sx = reinterpret_cast<u32*>(sp + G::PAD);
-    CState* st_scan = reinterpret_cast<CState*>(smem + G::BYTES - G::T * 16);
-    if (school_cheaper(na, nb, M)) {  // the same for the whole cluster
-        if (pi == 0) school_cta(la, na, lb, nb, out, out_len, smem, st_scan, &s_top);
-        return;
-    }
+    CState* st_scan = reinterpret_cast<CState*>(sx + G::PAD);
     const RnsMod m(pi);
     const uint2* T = a.tw + (u64)pi * a.ent;
     const uint2* Ti = a.twi + (u64)pi * a.ent;
@@ -250,12 +249,15 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, Sm
         *out_len = s_tops[2] ? s_tops[2] : (s_tops[1] ? s_tops[1] : s_tops[0]);
 }
 
-// Products of at most 256 limbs in all: schoolbook columns.
+// Products of at most 128 limbs in all (256 in large batches): schoolbook
+// columns. (Above that the transforms win at every shape: 500 x 8 limbs 16.6 us a call against 10.4,
+// 2,048 of them 97 against 56 us; 250 x 250 18.6 against 8.3.)
 template <int T>
 __global__ void __launch_bounds__(T) k_school(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len) {
     __shared__ __align__(16) unsigned char smem[16 * 256 + 64];
     __shared__ CState st[T];
     __shared__ unsigned long long s_top;
+    pdl_enter();
     const u32 *la = a.a, *lb = a.b;
     u64 na = a.na, nb = a.nb;
     if (a.jobs) {
@@ -275,7 +277,8 @@ static cudaError_t configure() {
     return cudaFuncSetAttribute(k_rns_small<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmallShape<M>::BYTES);
 }
 cudaError_t rns_configure_small() {
-    cudaError_t e = configure<9>();
+    cudaError_t e = configure<8>();
+    if (e == cudaSuccess) e = configure<9>();
     if (e == cudaSuccess) e = configure<10>();
     if (e == cudaSuccess) e = configure<11>();
     if (e == cudaSuccess) e = configure<12>();
@@ -283,23 +286,28 @@ cudaError_t rns_configure_small() {
 }
 
 template <int M>
-static void launch(unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out, unsigned long long* out_len,
+static cudaError_t launch(unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out, unsigned long long* out_len,
                    const RnsCrt& crt) {
-    k_rns_small<M><<<3 * njobs, SmallShape<M>::T, SmallShape<M>::BYTES, s>>>(a, out, out_len, crt);
+    return launch_pdl(k_rns_small<M>, 3 * njobs, SmallShape<M>::T, SmallShape<M>::BYTES, s, a, out, out_len, crt);
 }
 
 cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out,
                              unsigned long long* out_len, const RnsCrt& crt) {
     switch (m) {
-        case 9: launch<9>(njobs, s, a, out, out_len, crt); break;
-        case 10: launch<10>(njobs, s, a, out, out_len, crt); break;
-        case 11: launch<11>(njobs, s, a, out, out_len, crt); break;
-        case 12: launch<12>(njobs, s, a, out, out_len, crt); break;
+        case 8:
+            // one after the other the cluster is faster (128 x 128 limbs 8.5
+            // against 12.4 us a call), thousands at once the schoolbook
+            // (0.015 against 0.021 us each); 512 jobs fill the SMs
+            if (njobs >= 512) return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len);
+            return launch<8>(njobs, s, a, out, out_len, crt);
+        case 9: return launch<9>(njobs, s, a, out, out_len, crt);
+        case 10: return launch<10>(njobs, s, a, out, out_len, crt);
+        case 11: return launch<11>(njobs, s, a, out, out_len, crt);
+        case 12: return launch<12>(njobs, s, a, out, out_len, crt);
         default:
-            if (m > 8) return cudaErrorInvalidValue;
-            k_school<64><<<njobs, 64, 0, s>>>(a, out, out_len);
+            if (m > 7) return cudaErrorInvalidValue;
+            return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace b2m

@@ -1,8 +1,8 @@
 // school.cuh -- schoolbook product of two small u32-limb numbers by one CTA.
 //
 // A schoolbook product costs about 4.5 instructions per limb multiply-add, so
-// for the smaller and the unbalanced products of one launch (rns_small.cu) it
-// is cheaper than the transforms. Reference
+// for the smallest products (rns_small.cu) it is cheaper than the transforms.
+// Reference
 // counterpart: mul_schoolbook (src/bignum.cpp:125-143), the same column
 // products, here with every column sum of a thread's four-column block
 // accumulated in 96 bits by one carry chain per multiply-add, and the carries
@@ -11,17 +11,6 @@
 #include "carry.cuh"
 
 namespace b2m {
-
-// A product of up to 2^m limbs takes the schoolbook path when na * nb <=
-// SCHOOL_MACS_PER_POINT * 2^m.
-#ifndef B2M_SCHOOL_MACS_PER_POINT
-#define B2M_SCHOOL_MACS_PER_POINT 16
-#endif
-constexpr unsigned long long SCHOOL_MACS_PER_POINT = B2M_SCHOOL_MACS_PER_POINT;
-
-__device__ __forceinline__ bool school_cheaper(u64 na, u64 nb, int m) {
-    return na * nb <= (1ull << m) * SCHOOL_MACS_PER_POINT;
-}
 
 // (lo, mid, hi) += x * y as one 96-bit carry chain.
 __device__ __forceinline__ void mac96(u32& lo, u32& mid, u32& hi, u32 x, u32 y) {
