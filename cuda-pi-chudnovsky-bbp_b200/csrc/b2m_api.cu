@@ -82,6 +82,7 @@ static void destroy_context(Context* c) {
     if (c->host_dev) cudaFree(c->host_dev);
     twtable_free_all(c);
     rns_free_tables(c);
+    if (c->hw) cudaFreeHost(c->hw);
     if (c->d_tables) cudaFree(c->d_tables);
     if (c->d_err) cudaFree(c->d_err);
     if (c->hstream) cudaStreamDestroy(c->hstream);
@@ -163,6 +164,7 @@ b2m_status b2m_init(int device, uint64_t hbm_budget_bytes) {
     }
     if ((e = cudaMemcpy(c->d_tables, tables.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = rns_init_tables(c)) != cudaSuccess ||
+        (e = cudaHostAlloc(reinterpret_cast<void**>(&c->hw), 64 * 64, cudaHostAllocMapped)) != cudaSuccess ||
         (e = cudaMalloc(&c->d_err, 256)) != cudaSuccess || (e = cudaMemset(c->d_err, 0, 256)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->hstream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->hcopy, cudaStreamNonBlocking)) != cudaSuccess ||

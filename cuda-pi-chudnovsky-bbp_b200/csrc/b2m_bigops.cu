@@ -25,7 +25,10 @@
 #include "b2m.h"
 #include "b2m_context.h"
 #include "b2m_internal.h"
+#include "carry_lookback.cuh"
 #include "gp_scan.cuh"
+#include "pdl.cuh"
+#include "publish.cuh"
 
 namespace b2m {
 namespace big {
@@ -44,32 +47,63 @@ inline void ck(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw Err{cuda_status(e, what)};
 }
 
-// Stream-ordered allocations of one API call, released when it returns.
+// Stream-ordered memory of one API call, released when it returns: vectors
+// are carved from a few growing blocks (an allocation call per vector was a
+// large part of the host's time between kernels), one product workspace
+// serves all products, which the stream runs one after the other.
 class Scope {
 public:
-    Scope(Context* c, cudaStream_t s) : c_(c), s_(s) { w_ = static_cast<unsigned long long*>(raw(64)); }
-    ~Scope() {
-        for (auto& a : v_) {
-            cudaFreeAsync(a.first, s_);
-            budget_release(c_, a.second);
+    Scope(Context* c, cudaStream_t s) : c_(c), s_(s), host_(c) {
+        if (!host_.words()) {
+            set_error("cannot pin host memory");
+            throw Err{B2M_ERR_OUT_OF_MEMORY};
+        }
+        w_ = static_cast<unsigned long long*>(raw(256));
+        const cudaError_t e = cudaMemsetAsync(w_, 0, 256, s);
+        if (e != cudaSuccess) {
+            release();
+            throw Err{cuda_status(e, "cudaMemsetAsync")};
         }
     }
+    ~Scope() { release(); }
     Scope(const Scope&) = delete;
     Scope& operator=(const Scope&) = delete;
     void* raw(uint64_t bytes) {
         bytes = (std::max<uint64_t>(bytes, 16) + 255) & ~255ull;
-        if (!budget_reserve(c_, bytes)) {
-            set_error("HBM budget exhausted");
-            throw Err{B2M_ERR_OUT_OF_MEMORY};
+        if (bytes > left_) {
+            // blocks double from 1 MiB to 64 MiB; what does not fit the
+            // budget rounded up is taken as it is
+            uint64_t block = std::max(bytes, next_);
+            void* p = grab(block);
+            if (!p && block > bytes) p = grab(block = bytes);
+            if (!p) throw Err{st_};
+            next_ = std::min<uint64_t>(2 * next_, 64ull << 20);
+            if (block - bytes < left_) return p;  // the old block has more room left: keep carving it
+            cur_ = static_cast<unsigned char*>(p);
+            left_ = block;
         }
-        void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, bytes, s_);
-        if (e != cudaSuccess) {
-            budget_release(c_, bytes);
-            throw Err{cuda_status(e, "cudaMallocAsync")};
-        }
-        v_.push_back({p, bytes});
+        void* p = cur_;
+        cur_ += bytes;
+        left_ -= bytes;
         return p;
+    }
+    // The workspace of products, which use it one after the other on s().
+    void* workspace(uint64_t bytes) {
+        if (bytes > ws_cap_) {
+            ws_ = raw(bytes);
+            ws_cap_ = bytes;
+        }
+        return ws_;
+    }
+    // Lookback slots of add/subtract kernels, zero between kernels.
+    LookbackSlot* slots(uint64_t n) {
+        if (n > slots_cap_) {
+            const uint64_t cap = std::max<uint64_t>(64, 2 * n);
+            slots_ = static_cast<LookbackSlot*>(raw(cap * sizeof(LookbackSlot)));
+            slots_cap_ = cap;
+            ck(cudaMemsetAsync(slots_, 0, cap * sizeof(LookbackSlot), s_), "cudaMemsetAsync");
+        }
+        return slots_;
     }
     DV vec(uint64_t n) { return {static_cast<u32*>(raw(4 * std::max<uint64_t>(n, 1))), n}; }
     DV zeros(uint64_t n) {
@@ -79,13 +113,51 @@ public:
     }
     cudaStream_t s() const { return s_; }
     Context* c() const { return c_; }
-    unsigned long long* word() const { return w_; }  // 64 bytes of device scratch
+    unsigned long long* word() const { return w_; }  // device scratch: words 8.. are a PubState
+    HostLen publication() { return host_.next(); }
+    // The words of the last publication (values from [1]).
+    const u64* published() {
+        ck(host_.wait(s_), "waiting for a kernel's result");
+        return host_.words();
+    }
 
 private:
+    void* grab(uint64_t bytes) {
+        if (!budget_reserve(c_, bytes)) {
+            set_error("HBM budget exhausted");
+            st_ = B2M_ERR_OUT_OF_MEMORY;
+            return nullptr;
+        }
+        void* p = nullptr;
+        const cudaError_t e = cudaMallocAsync(&p, bytes, s_);
+        if (e != cudaSuccess) {
+            budget_release(c_, bytes);
+            cudaGetLastError();
+            st_ = cuda_status(e, "cudaMallocAsync");
+            return nullptr;
+        }
+        v_.push_back({p, bytes});
+        return p;
+    }
+    void release() {
+        for (auto& a : v_) {
+            cudaFreeAsync(a.first, s_);
+            budget_release(c_, a.second);
+        }
+        v_.clear();
+    }
     Context* c_;
     cudaStream_t s_;
+    HostWords host_;
     unsigned long long* w_ = nullptr;
     std::vector<std::pair<void*, uint64_t>> v_;
+    unsigned char* cur_ = nullptr;
+    uint64_t left_ = 0, next_ = 1ull << 20;
+    void* ws_ = nullptr;
+    uint64_t ws_cap_ = 0;
+    LookbackSlot* slots_ = nullptr;
+    uint64_t slots_cap_ = 0;
+    b2m_status st_ = B2M_OK;
 };
 
 // ---------------------------------------------------------------------------- kernels
@@ -180,24 +252,149 @@ __global__ void __launch_bounds__(AS_T) k_as_apply(const u32* A, u64 la, const u
     }
 }
 
-// out[k] = (a * 2^(32*wl + bits))[k], k < nout (bits in [0, 32)).
-__global__ void k_shl(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout) {
+// Device words of a call's publishing kernels, all zero between kernels: the
+// last block of a kernel to finish publishes and zeroes them again.
+struct PubState {
+    unsigned long long top;
+    u32 done, ticket, carry, pad;
+};
+
+// All threads of the block: `top` is the thread's candidate for the trimmed
+// length. The last block publishes (length, carry).
+__device__ __forceinline__ void publish_top(unsigned long long top, PubState* st, unsigned nblocks, LookbackSlot* slots,
+                                            const HostLen& hl) {
+    __shared__ bool s_last;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
+        top = o > top ? o : top;
+    }
+    if ((threadIdx.x & 31) == 0 && top) atomicMax(&st->top, top);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->done, 1u) == nblocks - 1;
+    __syncthreads();
+    if (!s_last) return;
+    if (slots)
+        for (unsigned i = threadIdx.x; i < nblocks; i += blockDim.x) slots[i].word = 0;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned long long t = atomicMax(&st->top, 0ull);
+        const u32 c = *(volatile u32*)&st->carry;
+        st->top = 0;
+        st->done = st->ticket = st->carry = 0;
+        publish(hl, t, c);
+    }
+}
+
+__global__ void k_top_pub(const u32* __restrict__ a, u64 n, PubState* st, const HostLen hl) {
+    pdl_enter();
+    unsigned long long t = 0;
+    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
+        if (a[k]) t = k + 1;
+    publish_top(t, st, gridDim.x, nullptr, hl);
+}
+
+__global__ void k_limb_pub(const u32* a, u64 k, const HostLen hl) {
+    pdl_enter();
+    publish(hl, a[k]);
+}
+
+// out = a 2^(32 a_off) +- b mod 2^(32n) in one pass, the trimmed length and
+// the carry or borrow out published. out may be a (a_off = 0) or b. One block
+// per 2048 limbs; the carry into a block comes by decoupled lookback, as in
+// the carry kernels.
+__global__ void __launch_bounds__(AS_T) k_addsub_pub(const u32* A, u64 a_off, u64 la, const u32* B, u64 lb, u64 n,
+                                                     int sub, u32* out, LookbackSlot* slots, PubState* st,
+                                                     const HostLen hl, u32* err) {
+    __shared__ GP ws[AS_T / 32 + 1];
+    __shared__ u32 s_chunk, s_cin;
+    pdl_enter();
+    u32 chunk = 0;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) s_chunk = atomicAdd(&st->ticket, 1u);
+        __syncthreads();
+        chunk = s_chunk;
+    }
+    const u64 base = (u64)chunk * AS_CH + (u64)threadIdx.x * AS_L;
+    u32 av[AS_L], bv[AS_L];
+    GP g{0, 1};
+#pragma unroll
+    for (int w = 0; w < AS_L; ++w) {
+        const u64 k = base + w;
+        av[w] = k >= a_off && k - a_off < la && k < n ? A[k - a_off] : 0u;
+        bv[w] = k < lb && k < n ? B[k] : 0u;
+        if (k < n) g = gp_then(g, limb_gp(av[w], bv[w], sub));
+    }
+    GP tot;
+    const GP ex = block_scan_gp(g, ws, &tot);
+    u32 cin = 0;
+    if (gridDim.x > 1) {
+        if (threadIdx.x < 32) {
+            // the block as a carry function: constant, or passing 0 and 1 through
+            const CState agg{tot.g, tot.p && !tot.g ? 1ull : CS_NEVER};
+            const u64 c = warp_lookback(slots, chunk, agg, err);
+            if (threadIdx.x == 0) {
+                if (agg.t != CS_NEVER) st_release(&slots[chunk].word, (cs_eval(agg, c) << 2) | SLOT_INCL);
+                s_cin = (u32)c;
+            }
+        }
+        __syncthreads();
+        cin = s_cin;
+    }
+    u32 c = ex.g | (ex.p & cin);
+    unsigned long long top = 0;
+#pragma unroll
+    for (int w = 0; w < AS_L; ++w) {
+        const u64 k = base + w;
+        if (k >= n) break;
+        u32 r;
+        if (!sub) {
+            const u64 x = (u64)av[w] + bv[w] + c;
+            r = (u32)x;
+            c = (u32)(x >> 32);
+        } else {
+            const u64 d = (u64)av[w] - bv[w] - c;
+            r = (u32)d;
+            c = (u32)((d >> 63) & 1);
+        }
+        out[k] = r;
+        if (r) top = k + 1;
+    }
+    if (chunk == gridDim.x - 1 && threadIdx.x == 0) st->carry = tot.g | (tot.p & cin);
+    publish_top(top, st, gridDim.x, gridDim.x > 1 ? slots : nullptr, hl);
+}
+
+// out[k] = (a * 2^(32*wl + bits))[k], k < nout (bits in [0, 32)); publishes
+// the trimmed length.
+__global__ void k_shl(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout,
+                      PubState* st, const HostLen hl) {
+    pdl_enter();
+    unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < nout; k += (u64)gridDim.x * blockDim.x) {
         u32 v = 0;
         if (k >= wl && k - wl < na) v = a[k - wl] << bits;
         if (bits && k >= wl + 1 && k - wl - 1 < na) v |= a[k - wl - 1] >> (32 - bits);
         out[k] = v;
+        if (v) t = k + 1;
     }
+    publish_top(t, st, gridDim.x, nullptr, hl);
 }
 
-// out[k] = floor(a / 2^(32*wl + bits))[k], k < nout (bits in [0, 32)).
-__global__ void k_shr(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout) {
+// out[k] = floor(a / 2^(32*wl + bits))[k], k < nout (bits in [0, 32));
+// publishes the trimmed length.
+__global__ void k_shr(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout,
+                      PubState* st, const HostLen hl) {
+    pdl_enter();
+    unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < nout; k += (u64)gridDim.x * blockDim.x) {
         u32 v = 0;
         if (k + wl < na) v = a[k + wl] >> bits;
         if (bits && k + wl + 1 < na) v |= a[k + wl + 1] << (32 - bits);
         out[k] = v;
+        if (v) t = k + 1;
     }
+    publish_top(t, st, gridDim.x, nullptr, hl);
 }
 
 inline unsigned grid_for(uint64_t n, unsigned threads = 256) {
@@ -205,35 +402,35 @@ inline unsigned grid_for(uint64_t n, unsigned threads = 256) {
 }
 
 // ---------------------------------------------------------------------------- host ops
+PubState* pub(Scope& S) { return reinterpret_cast<PubState*>(S.word() + 8); }
+
+// Grids of publishing kernels: each block ends in an atomic on one word.
+inline unsigned pub_grid(uint64_t n) { return std::min(grid_for(n), 1024u); }
+
 uint64_t top_len(Scope& S, DV a) {
     if (a.n == 0) return 0;
-    ck(cudaMemsetAsync(S.word(), 0, 8, S.s()), "cudaMemsetAsync");
-    k_top<<<grid_for(a.n), 256, 0, S.s()>>>(a.p, a.n, S.word());
-    ck(cudaGetLastError(), "k_top");
-    unsigned long long h = 0;
-    ck(cudaMemcpyAsync(&h, S.word(), 8, cudaMemcpyDeviceToHost, S.s()), "cudaMemcpyAsync");
-    ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
-    return h;
+    ck(launch_pdl(k_top_pub, pub_grid(a.n), 256, 0, S.s(), a.p, a.n, pub(S), S.publication()), "k_top_pub");
+    return S.published()[1];
 }
 
 DV trim(Scope& S, DV a) { return {a.p, top_len(S, a)}; }
 
-// out = a +- b mod 2^(32 out.n); returns the carry (add) or borrow (sub) out.
-u32 addsub(Scope& S, DV a, DV b, DV out, bool sub) {
+// out = a 2^(32 a_off) +- b mod 2^(32 out.n): the carry (add) or borrow (sub)
+// out, and the trimmed result.
+struct Sum {
+    u32 carry;
+    DV v;
+};
+Sum addsub(Scope& S, DV a, DV b, DV out, bool sub, uint64_t a_off = 0) {
     const uint64_t n = out.n;
-    if (n == 0) return 0;
+    if (n == 0) return {0, out};
     const uint64_t nb = (n + AS_CH - 1) / AS_CH;
-    GP* agg = static_cast<GP*>(S.raw(nb * sizeof(GP)));
-    u32* cin = static_cast<u32*>(S.raw(nb * 4));
-    u32* cout = reinterpret_cast<u32*>(S.word() + 1);
-    k_as_reduce<<<(unsigned)nb, AS_T, 0, S.s()>>>(a.p, a.n, b.p, b.n, n, sub, agg);
-    k_as_scan<<<1, 1024, 0, S.s()>>>(agg, nb, cin, cout);
-    k_as_apply<<<(unsigned)nb, AS_T, 0, S.s()>>>(a.p, a.n, b.p, b.n, n, sub, cin, out.p);
-    ck(cudaGetLastError(), "add/subtract kernels");
-    u32 h = 0;
-    ck(cudaMemcpyAsync(&h, cout, 4, cudaMemcpyDeviceToHost, S.s()), "cudaMemcpyAsync");
-    ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
-    return h;
+    LookbackSlot* slots = nb > 1 ? S.slots(nb) : nullptr;
+    ck(launch_pdl(k_addsub_pub, (unsigned)nb, AS_T, 0, S.s(), a.p, a_off, a.n, b.p, b.n, n, sub ? 1 : 0, out.p, slots,
+                  pub(S), S.publication(), S.c()->d_err),
+       "k_addsub_pub");
+    const u64* h = S.published();
+    return {(u32)h[2], {out.p, h[1]}};
 }
 
 DV upload(Scope& S, const std::vector<u32>& h) {
@@ -251,10 +448,8 @@ std::vector<u32> download(Scope& S, DV d) {
 }
 
 u32 limb_at(Scope& S, DV d, uint64_t k) {
-    u32 h = 0;
-    ck(cudaMemcpyAsync(&h, d.p + k, 4, cudaMemcpyDeviceToHost, S.s()), "D2H");
-    ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
-    return h;
+    ck(launch_pdl(k_limb_pub, 1, 1, 0, S.s(), d.p, k, S.publication()), "k_limb_pub");
+    return (u32)S.published()[1];
 }
 
 DV copy(Scope& S, DV a, uint64_t cap) {
@@ -269,9 +464,8 @@ DV shl(Scope& S, DV a, uint64_t wl, int bits) {
     if (a.n == 0) return a;
     const uint64_t n = a.n + wl + 1;
     DV d = S.vec(n);
-    k_shl<<<grid_for(n), 256, 0, S.s()>>>(a.p, a.n, bits, wl, d.p, n);
-    ck(cudaGetLastError(), "k_shl");
-    return trim(S, d);
+    ck(launch_pdl(k_shl, pub_grid(n), 256, 0, S.s(), a.p, a.n, bits, wl, d.p, n, pub(S), S.publication()), "k_shl");
+    return {d.p, S.published()[1]};
 }
 
 // floor(a / 2^(32 wl + bits)), trimmed.
@@ -279,9 +473,8 @@ DV shr(Scope& S, DV a, uint64_t wl, int bits) {
     if (a.n <= wl) return {a.p, 0};
     const uint64_t n = a.n - wl;
     DV d = S.vec(n);
-    k_shr<<<grid_for(n), 256, 0, S.s()>>>(a.p, a.n, bits, wl, d.p, n);
-    ck(cudaGetLastError(), "k_shr");
-    return trim(S, d);
+    ck(launch_pdl(k_shr, pub_grid(n), 256, 0, S.s(), a.p, a.n, bits, wl, d.p, n, pub(S), S.publication()), "k_shr");
+    return {d.p, S.published()[1]};
 }
 
 // a + delta for delta in {-1, +1} (a + 1 may grow by one limb; a - 1 needs a > 0).
@@ -289,9 +482,7 @@ DV add_one(Scope& S, DV a, bool minus) {
     static const u32 one_h = 1;
     DV one = S.vec(1);
     ck(cudaMemcpyAsync(one.p, &one_h, 4, cudaMemcpyHostToDevice, S.s()), "H2D");
-    DV d = S.vec(a.n + 1);
-    addsub(S, a, one, d, minus);
-    return trim(S, d);
+    return addsub(S, a, one, S.vec(a.n + 1), minus).v;
 }
 
 // The NTT product, trimmed.
@@ -304,9 +495,16 @@ DV mul(Scope& S, DV a, DV b) {
     Plan p = product_plan(c, a.n, b.n);
     ck(twtable_ensure(c, p, S.s()), "twiddle table");
     DV out = S.vec(a.n + b.n);
-    void* ws = p.npass ? S.raw(workspace_bytes_plan(p)) : nullptr;
+    void* ws = p.npass ? S.workspace(workspace_bytes_plan(p)) : nullptr;
     uint64_t* d_len = reinterpret_cast<uint64_t*>(S.word() + 2);
-    ck(launch_product(a.p, a.n, b.p, b.n, out.p, d_len, ws, p, c->tw, c->d_err, S.s()), "product");
+    const bool published = p.npass == 0 || p.rns;
+    ck(launch_product(a.p, a.n, b.p, b.n, out.p, d_len, ws, p, c->tw, c->d_err, S.s(), nullptr, nullptr,
+                      published ? S.publication() : HostLen{}),
+       "product");
+    if (published) {
+        out.n = S.published()[1];
+        return out;
+    }
     unsigned long long h = 0;
     ck(cudaMemcpyAsync(&h, d_len, 8, cudaMemcpyDeviceToHost, S.s()), "D2H");
     ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
@@ -416,24 +614,18 @@ DV recip(Scope& S, DV Bn, uint64_t h) {
     DV E;
     bool neg = false;
     if (T.n <= e) {  // E = 2^(32e) - T >= 0
-        E = S.vec(e);
-        addsub(S, DV{T.p, 0}, T, E, true);
+        E = addsub(S, DV{T.p, 0}, T, S.vec(e), true).v;
     } else {  // T = 2^(32e) + E', 0 <= E' < 2^(32e)
         if (T.n != e + 1 || limb_at(S, T, e) != 1) {
             set_error("Newton reciprocal diverged");
             throw Err{B2M_ERR_INTERNAL};
         }
-        E = {T.p, e};
+        E = trim(S, {T.p, e});
         neg = true;
     }
-    E = trim(S, E);
     DV D = mul(S, Xl, E);
     DV corr = D.n > 2 * l ? DV{D.p + 2 * l, D.n - 2 * l} : DV{D.p, 0};
-    DV Xs = S.zeros(h + 2);
-    ck(cudaMemcpyAsync(Xs.p + (h - l), Xl.p, 4 * Xl.n, cudaMemcpyDeviceToDevice, S.s()), "D2D");
-    DV X = S.vec(h + 2);
-    addsub(S, Xs, corr, X, neg);
-    return trim(S, X);
+    return addsub(S, Xl, corr, S.vec(h + 2), neg, h - l).v;
 }
 
 // ---------------------------------------------------------------------------- division
@@ -468,17 +660,21 @@ void divmod(Scope& S, DV a, DV b, DV* q, DV* r) {
     DV QB = mul(S, Q, b);
     const uint64_t w = std::max(a.n, QB.n) + 1;
     DV R = S.vec(w);
-    bool negative = addsub(S, a, QB, R, true) != 0;
+    Sum rs = addsub(S, a, QB, R, true);
+    bool negative = rs.carry != 0;
     int it = 0;
     while (negative) {  // two's complement R < 0: add b back
-        if (addsub(S, R, b, R, false)) negative = false;
+        rs = addsub(S, R, b, R, false);
+        if (rs.carry) negative = false;
         Q = add_one(S, Q, true);
         if (++it > MAX_FIX) break;
     }
     while (it <= MAX_FIX) {  // R >= b: subtract it
         DV T = S.vec(w);
-        if (addsub(S, R, b, T, true)) break;
+        const Sum ts = addsub(S, R, b, T, true);
+        if (ts.carry) break;
         R = T;
+        rs = ts;
         Q = add_one(S, Q, false);
         ++it;
     }
@@ -487,7 +683,7 @@ void divmod(Scope& S, DV a, DV b, DV* q, DV* r) {
         throw Err{B2M_ERR_INTERNAL};
     }
     *q = Q;
-    *r = trim(S, R);
+    *r = rs.v;
 }
 
 // ---------------------------------------------------------------------------- square root
@@ -507,9 +703,7 @@ DV sqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     if (x0.n == 0) return x0;
     DV qv, rv;
     divmod(S, Nh, x0, &qv, &rv);
-    DV s = S.vec(std::max(x0.n, qv.n) + 1);
-    addsub(S, x0, qv, s, false);
-    return shr(S, trim(S, s), 0, 1);
+    return shr(S, addsub(S, x0, qv, S.vec(std::max(x0.n, qv.n) + 1), false).v, 0, 1);
 }
 
 DV isqrt(Scope& S, DV N);
@@ -536,20 +730,17 @@ DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     DV E;
     bool neg = false;
     if (U.n <= e) {  // E = 2^(32e) - U >= 0
-        E = S.vec(e);
-        addsub(S, DV{U.p, 0}, U, E, true);
+        E = addsub(S, DV{U.p, 0}, U, S.vec(e), true).v;
     } else {  // U = 2^(32e) + E'
         if (U.n != e + 1 || limb_at(S, U, e) != 1) {
             set_error("Newton reciprocal square root diverged");
             throw Err{B2M_ERR_INTERNAL};
         }
-        E = {U.p, e};
+        E = trim(S, {U.p, e});
         neg = true;
     }
-    DV corr = shr(S, mul(S, Y0, trim(S, E)), e, 1);  // Y0 |E| / 2^(32e + 1)
-    DV Y = S.vec(std::max(Y0.n, corr.n) + 1);
-    addsub(S, Y0, corr, Y, neg);
-    return trim(S, Y);
+    DV corr = shr(S, mul(S, Y0, E), e, 1);  // Y0 |E| / 2^(32e + 1)
+    return addsub(S, Y0, corr, S.vec(std::max(Y0.n, corr.n) + 1), neg).v;
 }
 
 // floor(sqrt(N)) for trimmed N: an estimate -- N * Y / 2^(64k) from the
@@ -569,19 +760,19 @@ DV isqrt(Scope& S, DV N) {
     DV SQ = mul(S, s, s);
     const uint64_t w = std::max(N.n, SQ.n) + 2;
     DV R = S.vec(w);
-    bool negative = addsub(S, N, SQ, R, true) != 0;
+    bool negative = addsub(S, N, SQ, R, true).carry != 0;
     int it = 0;
     while (negative && it <= MAX_FIX) {  // N - (s-1)^2 = R + 2s - 1
         DV twice = shl(S, s, 0, 1);
         DV d = add_one(S, twice, true);
-        if (addsub(S, R, d, R, false)) negative = false;
+        if (addsub(S, R, d, R, false).carry) negative = false;
         s = add_one(S, s, true);
         ++it;
     }
     while (it <= MAX_FIX) {  // N - (s+1)^2 = R - (2s + 1)
         DV d = add_one(S, shl(S, s, 0, 1), false);
         DV T = S.vec(w);
-        if (addsub(S, R, d, T, true)) break;
+        if (addsub(S, R, d, T, true).carry) break;
         R = T;
         s = add_one(S, s, false);
         ++it;
@@ -840,15 +1031,15 @@ void fix_node_grid(Scope& S, const u32* V, uint64_t sin, const u32* U, uint64_t 
     const uint64_t n = Pj.n;
     ck(cudaMemsetAsync(Q.p, 0, 4 * (nq + 1), S.s()), "cudaMemsetAsync");
     ck(cudaMemcpyAsync(Q.p, QE, 4 * nq, cudaMemcpyDeviceToDevice, S.s()), "D2D");
-    u32 neg = addsub(S, {const_cast<u32*>(V), sin}, {const_cast<u32*>(U), su}, R, true);
+    u32 neg = addsub(S, {const_cast<u32*>(V), sin}, {const_cast<u32*>(U), su}, R, true).carry;
     int it = 0;
     while (neg && it < 64) {
-        if (addsub(S, R, Pj, R, false)) neg = 0;
+        if (addsub(S, R, Pj, R, false).carry) neg = 0;
         addsub(S, Q, one, Q, true);
         ++it;
     }
     while (it < 64) {
-        if (addsub(S, R, Pj, T, true)) break;
+        if (addsub(S, R, Pj, T, true).carry) break;
         std::swap(R, T);
         addsub(S, Q, one, Q, false);
         ++it;
@@ -872,9 +1063,8 @@ constexpr uint64_t DC_GRID_MIN_LIMBS = 1 << 15;
 // -1, 0, 1 as a <, ==, > b (trimmed).
 int cmp(Scope& S, DV a, DV b) {
     if (a.n != b.n) return a.n < b.n ? -1 : 1;
-    DV t = S.vec(a.n);
-    if (addsub(S, a, b, t, true)) return -1;
-    return top_len(S, t) ? 1 : 0;
+    const Sum d = addsub(S, a, b, S.vec(a.n), true);
+    return d.carry ? -1 : (d.v.n ? 1 : 0);
 }
 
 // Decimal digits of trimmed X, no leading zeros ("0" for zero).

@@ -26,6 +26,11 @@ struct Context {
     std::mutex host_mu;                  // serialises b2m_mul_host (shared buffers)
     void* host_dev = nullptr;            // device buffers of b2m_mul_host, grown on demand
     uint64_t host_dev_cap = 0;
+    // Pinned host words that kernels publish lengths and carries in
+    // (HostWords below): 64 slots of eight words, a bit per slot in use.
+    u64* hw = nullptr;
+    uint64_t hw_used = 0;
+    std::mutex hw_mu;
     // Inter-pass twiddle tables (twtable_ensure), keyed by (logm, logr).
     struct TwTable {
         int logm, logr;
@@ -89,6 +94,58 @@ inline void set_tuned(Context* c, int logn, const Plan& p) {
     c->tuned[logn] = p;
     c->has_tuned[logn] = true;
 }
+
+// A slot of pinned host words for one call: a kernel writes values 1..7, a
+// system-wide fence and then the tag in word 0; the host polls the tag. Any
+// number of calls may hold slots; past 64 at a time a call pins its own.
+class HostWords {
+public:
+    explicit HostWords(Context* c) : c_(c) {
+        std::lock_guard<std::mutex> lk(c->hw_mu);
+        for (int i = 0; i < 64 && c->hw; ++i)
+            if (!((c->hw_used >> i) & 1)) {
+                c->hw_used |= 1ull << i;
+                slot_ = i;
+                p_ = c->hw + 8 * i;
+                break;
+            }
+        if (!p_ && cudaHostAlloc(reinterpret_cast<void**>(&p_), 64, cudaHostAllocMapped) != cudaSuccess) p_ = nullptr;
+        if (p_) p_[0] = 0;
+    }
+    ~HostWords() {
+        if (slot_ >= 0) {
+            std::lock_guard<std::mutex> lk(c_->hw_mu);
+            c_->hw_used &= ~(1ull << slot_);
+        } else if (p_) {
+            cudaFreeHost(p_);
+        }
+    }
+    HostWords(const HostWords&) = delete;
+    HostWords& operator=(const HostWords&) = delete;
+    u64* words() const { return p_; }  // null: pinning failed
+    // The next publication; its kernel gets words() and the tag.
+    HostLen next() { return {reinterpret_cast<unsigned long long*>(p_), ++tag_}; }
+    // Waits for the last one. The stream is asked now and then, so that a
+    // failed or finished stream without the tag is an error, not a hang.
+    cudaError_t wait(cudaStream_t s) {
+        volatile u64* v = p_;
+        for (uint32_t n = 1; v[0] != tag_; ++n) {
+            if ((n & 0xFFF) == 0) {
+                const cudaError_t q = cudaStreamQuery(s);
+                if (q == cudaSuccess) return v[0] == tag_ ? cudaSuccess : cudaErrorUnknown;
+                if (q != cudaErrorNotReady) return q;
+            }
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return cudaSuccess;
+    }
+
+private:
+    Context* c_;
+    int slot_ = -1;
+    u64* p_ = nullptr;
+    u64 tag_ = 0;
+};
 
 extern Context* g_ctx;
 extern std::mutex g_ctx_mu;

@@ -138,6 +138,13 @@ struct Tracer {
     void end(cudaStream_t s) { cudaEventRecord(ev[n], s); }
 };
 
+// Where a kernel publishes a result for the polling host (HostWords in
+// b2m_context.h): value words from host[1], then tag in host[0].
+struct HostLen {
+    unsigned long long* host = nullptr;
+    u64 tag = 0;
+};
+
 // Kernel launch sequence for one product on `stream`.
 //   a, b: device limbs; out: na+nb limbs; out_len: device u64 (may be null).
 //   ws: workspace of workspace_bytes_for(logn) bytes; err: device error word.
@@ -184,7 +191,8 @@ cudaError_t launch_gen_operand(cudaStream_t s, u64 seed, u64 n, u32 kind, u32* o
 cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out,
                            uint64_t* out_len, void* ws, const Plan& plan, const RootTables& tw,
                            u32* err, cudaStream_t stream, Tracer* tr = nullptr,
-                           cudaEvent_t b_ready = nullptr);  // operand B waited for just before its transform
+                           cudaEvent_t b_ready = nullptr,  // operand B waited for just before its transform
+                           HostLen hl = {});  // residue and one-launch products also publish their length
 // Kernels one product launches under plan p.
 int plan_launches(const Plan& p);
 
@@ -256,7 +264,8 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build);
 int rns_launches(const Plan& p);
 cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout,
                                u32* bufA, u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,
-                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready);
+                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready,
+                               HostLen hl);
 cudaError_t rns_launch_spectrum(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs,
                                 cudaStream_t s);
 cudaError_t rns_launch_bucket(const Plan& p, const ProdJob* jobs, unsigned njobs, const JobBufs& bufs, u32* err,
@@ -269,7 +278,7 @@ struct RnsCrt {
 };
 cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
-                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt);
+                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt, HostLen hl = {});
 // v: columns per thread (1; or 2 up to logr = 8)
 cudaError_t rns_launch_first(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_launch_mid(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
@@ -278,7 +287,7 @@ cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs&
 cudaError_t rns_configure();
 // Whole products of up to 2^12 points, one cluster each (rns_small.cu).
 cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out,
-                             unsigned long long* out_len, const RnsCrt& crt);
+                             unsigned long long* out_len, const RnsCrt& crt, HostLen hl = {});
 cudaError_t rns_configure_small();
 
 cudaError_t configure_first();

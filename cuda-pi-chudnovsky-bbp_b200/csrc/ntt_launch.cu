@@ -398,13 +398,13 @@ static cudaError_t launch_forward(const u32* limbs, uint64_t nlimbs, u64* buf, c
 
 cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, uint64_t* out_len,
                            void* ws, const Plan& p, const RootTables& tw, u32* err, cudaStream_t s, Tracer* tr,
-                           cudaEvent_t b_ready) {
+                           cudaEvent_t b_ready, HostLen hl) {
     const int logn = p.logn;
     const uint64_t n = plan_points(p);
     const u64 nout = na + nb;
     if (p.npass == 0)
         return rns_launch_product(a, na, b, nb, out, nout, nullptr, nullptr, nullptr, nullptr,
-                                  reinterpret_cast<unsigned long long*>(out_len), p, err, s, tr, b_ready);
+                                  reinterpret_cast<unsigned long long*>(out_len), p, err, s, tr, b_ready, hl);
     u64* bufA = static_cast<u64*>(ws);
     u64* bufB = bufA + n;
     unsigned char* scratch = reinterpret_cast<unsigned char*>(bufB + n);
@@ -415,7 +415,7 @@ cudaError_t launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb,
     unsigned long long* ol = out_len ? reinterpret_cast<unsigned long long*>(out_len) : len_tmp;
     if (p.rns)  // zeroes its scratch and *ol itself
         return rns_launch_product(a, na, b, nb, out, nout, reinterpret_cast<u32*>(bufA), reinterpret_cast<u32*>(bufB), slots,
-                                  ticket, ol, p, err, s, tr, b_ready);
+                                  ticket, ol, p, err, s, tr, b_ready, hl);
     cudaError_t e = cudaMemsetAsync(scratch, 0, carry_scratch_bytes_n(n), s);
     if (e != cudaSuccess) return e;
     if (out_len && (e = cudaMemsetAsync(out_len, 0, sizeof(uint64_t), s)) != cudaSuccess) return e;

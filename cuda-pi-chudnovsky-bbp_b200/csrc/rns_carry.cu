@@ -13,6 +13,7 @@
 #include "carry.cuh"
 #include "carry_lookback.cuh"
 #include "pdl.cuh"
+#include "publish.cuh"
 #include "rns_crt.cuh"
 
 namespace b2m {
@@ -34,7 +35,7 @@ __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& car
 __global__ void __launch_bounds__(CARRY_THREADS, 6)
     k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout, u32 nchunks,
                 LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
-                const ProdJob* __restrict__ jobs, const RnsCrt crt) {
+                const ProdJob* __restrict__ jobs, const RnsCrt crt, const HostLen hl) {
     pdl_enter();
     if (jobs) {
         const ProdJob& J = jobs[blockIdx.y];
@@ -129,15 +130,19 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
 #pragma unroll
         for (int w = 0; w < CARRY_THREADS / 32; ++w) top = s_top[w] > top ? s_top[w] : top;
         if (top) atomicMax(out_len, top);
+        if (hl.host) {  // a single product: the last block to finish publishes the length
+            __threadfence();
+            if (atomicAdd(ticket + 1, 1u) == nchunks - 1) publish(hl, atomicMax(out_len, 0ull));
+        }
     }
 }
 
 cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
-                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt) {
+                             const ProdJob* jobs, unsigned njobs, const RnsCrt& crt, HostLen hl) {
     if (nchunks == 0 || njobs == 0) return cudaSuccess;
     return launch_pdl(k_rns_carry, dim3(nchunks, njobs), CARRY_THREADS, 0, s, coef, nt, out, nout, nchunks, slots, ticket,
-                      out_len, err, jobs, crt);
+                      out_len, err, jobs, crt, hl);
 }
 
 }  // namespace b2m

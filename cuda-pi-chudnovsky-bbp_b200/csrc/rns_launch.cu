@@ -521,10 +521,11 @@ struct RnsRun {
         }
         return e;
     }
-    cudaError_t carry(u32* out, u64 nout, LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err) {
+    cudaError_t carry(u32* out, u64 nout, LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
+                      HostLen hl = {}) {
         if (tr) tr->mark(s, B2M_K_CARRY, 0);
         return rns_launch_carry((unsigned)(a.nt / (CARRY_CHUNK / 2)), s, a.bufB, a.nt, out, nout, slots, ticket,
-                                out_len, err, a.jobs, njobs, shape_const(sh).crt);
+                                out_len, err, a.jobs, njobs, shape_const(sh).crt, hl);
     }
 };
 
@@ -532,7 +533,8 @@ struct RnsRun {
 
 cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout, u32* bufA,
                                u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,
-                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready) {
+                               const Plan& p, u32* err, cudaStream_t s, Tracer* tr, cudaEvent_t b_ready,
+                               HostLen hl) {
     RnsRun r(p, s);
     r.tr = tr;
     r.a.a = a;
@@ -546,7 +548,7 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
     if (r.small) {
         if (b_ready && (e = cudaStreamWaitEvent(s, b_ready, 0)) != cudaSuccess) return e;
         if (tr) tr->mark(s, B2M_K_SMALL, p.logn);
-        e = rns_launch_small(r.sh.m, 1, s, r.a, out, out_len, shape_const(r.sh).crt);
+        e = rns_launch_small(r.sh.m, 1, s, r.a, out, out_len, shape_const(r.sh).crt, hl);
         if (tr) tr->end(s);
         return e;
     }
@@ -565,7 +567,7 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
         if (e == cudaSuccess) e = r.forward(1, 1);
     }
     if (e == cudaSuccess) e = r.finish();
-    if (e == cudaSuccess) e = r.carry(out, nout, slots, ticket, out_len, err);
+    if (e == cudaSuccess) e = r.carry(out, nout, slots, ticket, out_len, err, hl);
     if (tr) tr->end(s);
     return e;
 }

@@ -18,6 +18,7 @@
 
 #include "b2m_context.h"
 #include "carry.cuh"
+#include "publish.cuh"
 #include "rns_crt.cuh"
 #include "rns_kernels.cuh"
 #include "school.cuh"
@@ -138,7 +139,8 @@ struct SmallShape {
 
 template <int M>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, SmallShape<M>::MINB)
-    k_rns_small(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len, const RnsCrt crt) {
+    k_rns_small(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len, const RnsCrt crt,
+                const HostLen hl) {
     using G = SmallShape<M>;
     using C = SmallCfg<M>;
     constexpr int E = 1 << C::LE;
@@ -245,15 +247,19 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, Sm
     __syncthreads();
     if (threadIdx.x == 0) cluster.map_shared_rank(s_tops, 0)[pi] = s_top;
     cluster.sync();
-    if (pi == 0 && threadIdx.x == 0 && out_len)
-        *out_len = s_tops[2] ? s_tops[2] : (s_tops[1] ? s_tops[1] : s_tops[0]);
+    if (pi == 0 && threadIdx.x == 0) {
+        const unsigned long long n = s_tops[2] ? s_tops[2] : (s_tops[1] ? s_tops[1] : s_tops[0]);
+        if (out_len) *out_len = n;
+        if (hl.host) publish(hl, n);
+    }
 }
 
 // Products of at most 128 limbs in all (256 in large batches): schoolbook
 // columns. (Above that the transforms win at every shape: 500 x 8 limbs 16.6 us a call against 10.4,
 // 2,048 of them 97 against 56 us; 250 x 250 18.6 against 8.3.)
 template <int T>
-__global__ void __launch_bounds__(T) k_school(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len) {
+__global__ void __launch_bounds__(T) k_school(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len,
+                                              const HostLen hl) {
     __shared__ __align__(16) unsigned char smem[16 * 256 + 64];
     __shared__ CState st[T];
     __shared__ unsigned long long s_top;
@@ -270,6 +276,7 @@ __global__ void __launch_bounds__(T) k_school(const RnsArgs a, u32* __restrict__
         out_len = J.out_len;
     }
     school_cta(la, na, lb, nb, out, out_len, smem, st, &s_top);
+    if (threadIdx.x == 0 && hl.host) publish(hl, s_top);
 }
 
 template <int M>
@@ -287,26 +294,26 @@ cudaError_t rns_configure_small() {
 
 template <int M>
 static cudaError_t launch(unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out, unsigned long long* out_len,
-                   const RnsCrt& crt) {
-    return launch_pdl(k_rns_small<M>, 3 * njobs, SmallShape<M>::T, SmallShape<M>::BYTES, s, a, out, out_len, crt);
+                          const RnsCrt& crt, HostLen hl) {
+    return launch_pdl(k_rns_small<M>, 3 * njobs, SmallShape<M>::T, SmallShape<M>::BYTES, s, a, out, out_len, crt, hl);
 }
 
 cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArgs& a, u32* out,
-                             unsigned long long* out_len, const RnsCrt& crt) {
+                             unsigned long long* out_len, const RnsCrt& crt, HostLen hl) {
     switch (m) {
         case 8:
             // one after the other the cluster is faster (128 x 128 limbs 8.5
             // against 12.4 us a call), thousands at once the schoolbook
             // (0.015 against 0.021 us each); 512 jobs fill the SMs
-            if (njobs >= 512) return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len);
-            return launch<8>(njobs, s, a, out, out_len, crt);
-        case 9: return launch<9>(njobs, s, a, out, out_len, crt);
-        case 10: return launch<10>(njobs, s, a, out, out_len, crt);
-        case 11: return launch<11>(njobs, s, a, out, out_len, crt);
-        case 12: return launch<12>(njobs, s, a, out, out_len, crt);
+            if (njobs >= 512) return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len, hl);
+            return launch<8>(njobs, s, a, out, out_len, crt, hl);
+        case 9: return launch<9>(njobs, s, a, out, out_len, crt, hl);
+        case 10: return launch<10>(njobs, s, a, out, out_len, crt, hl);
+        case 11: return launch<11>(njobs, s, a, out, out_len, crt, hl);
+        case 12: return launch<12>(njobs, s, a, out, out_len, crt, hl);
         default:
             if (m > 7) return cudaErrorInvalidValue;
-            return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len);
+            return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len, hl);
     }
 }
 
