@@ -112,6 +112,7 @@ struct RnsArgs {
     u32 nmask;                // sub-problem index -> tree node
     int logs;                 // log2 S of the pass
     int q;
+    u32 pper;                 // first pass in parts: parts per block
     int op0;                  // operand of grid z 0..2
     int square;
     unsigned long long* zero;      // first pass of a single product: scratch it zeroes
@@ -282,6 +283,11 @@ cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, 
 // v: columns per thread (1; or 2 up to logr = 8)
 cudaError_t rns_launch_first(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_launch_mid(int logr, int v, dim3 grid, cudaStream_t s, const RnsArgs& a);
+// Inverse Vandermonde matrices of a transform in parts.
+struct RnsCombine {
+    u32 v[3][8][8];
+};
+cudaError_t rns_launch_inv_parts(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a, const RnsCombine& c);
 cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a);
 cudaError_t rns_configure();

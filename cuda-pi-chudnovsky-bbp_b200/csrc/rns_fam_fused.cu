@@ -1,5 +1,5 @@
 // rns_fam_fused.cu -- instantiations of the residue transforms' last forward
-// pass + pointwise product + first inverse pass (radix exponents 7..10).
+// pass + pointwise product + first inverse pass (radix exponents 7..9).
 #include "rns_kernels.cuh"
 
 namespace b2m {
@@ -12,7 +12,6 @@ cudaError_t rns_configure() {
     cudaError_t e = configure<7>();
     if (e == cudaSuccess) e = configure<8>();
     if (e == cudaSuccess) e = configure<9>();
-    if (e == cudaSuccess) e = configure<10>();
     return e;
 }
 
@@ -28,7 +27,6 @@ cudaError_t rns_launch_fused(int logr, dim3 grid, cudaStream_t s, const RnsArgs&
         case 7: return launch<7>(grid, s, a);
         case 8: return launch<8>(grid, s, a);
         case 9: return launch<9>(grid, s, a);
-        case 10: return launch<10>(grid, s, a);
     }
     return cudaErrorInvalidValue;
 }

@@ -1,5 +1,6 @@
 // rns_fam_inv.cu -- instantiations of the residue transforms' inverse column
-// passes (radix exponents 5..10; the top pass and the others).
+// passes (radix exponents 5..8; the top pass, the others, and the top pass of
+// a transform in parts).
 #include "rns_kernels.cuh"
 
 namespace b2m {
@@ -17,12 +18,31 @@ cudaError_t rns_launch_inv(int logr, int v, bool first, dim3 grid, cudaStream_t 
         case 22: return launch<6, 1>(first, grid, s, a);
         case 23: return launch<7, 1>(first, grid, s, a);
         case 24: return launch<8, 1>(first, grid, s, a);
-        case 25: return launch<9, 1>(first, grid, s, a);
-        case 26: return launch<10, 1>(first, grid, s, a);
         case 37: return launch<5, 2>(first, grid, s, a);
         case 38: return launch<6, 2>(first, grid, s, a);
         case 39: return launch<7, 2>(first, grid, s, a);
         case 40: return launch<8, 2>(first, grid, s, a);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <int LOGR, int Q>
+static cudaError_t parts(dim3 grid, cudaStream_t s, const RnsArgs& a, const RnsCombine& c) {
+    using G = RnsCol<LOGR, 1>;
+    return launch_pdl(k_rns_inv_parts<LOGR, Q>, grid, G::THREADS, 2 * G::SMEM * 4, s, a, c);
+}
+
+// 3 parts at any radix; 2, 4, 6 and 8 only divide 2^23-point parts.
+cudaError_t rns_launch_inv_parts(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a, const RnsCombine& c) {
+    switch (16 * a.q + logr) {
+        case 39: return parts<7, 2>(grid, s, a, c);
+        case 53: return parts<5, 3>(grid, s, a, c);
+        case 54: return parts<6, 3>(grid, s, a, c);
+        case 55: return parts<7, 3>(grid, s, a, c);
+        case 56: return parts<8, 3>(grid, s, a, c);
+        case 71: return parts<7, 4>(grid, s, a, c);
+        case 102: return parts<6, 6>(grid, s, a, c);
+        case 134: return parts<6, 8>(grid, s, a, c);
     }
     return cudaErrorInvalidValue;
 }

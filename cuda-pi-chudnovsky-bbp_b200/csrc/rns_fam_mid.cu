@@ -1,5 +1,5 @@
 // rns_fam_mid.cu -- instantiations of the residue transforms' middle forward
-// pass (radix exponents 5..10).
+// pass (radix exponents 5..8).
 #include "rns_kernels.cuh"
 
 namespace b2m {
@@ -15,8 +15,6 @@ cudaError_t rns_launch_mid(int logr, int v, dim3 grid, cudaStream_t s, const Rns
         case 22: return launch<6, 1>(grid, s, a);
         case 23: return launch<7, 1>(grid, s, a);
         case 24: return launch<8, 1>(grid, s, a);
-        case 25: return launch<9, 1>(grid, s, a);
-        case 26: return launch<10, 1>(grid, s, a);
         case 37: return launch<5, 2>(grid, s, a);
         case 38: return launch<6, 2>(grid, s, a);
         case 39: return launch<7, 2>(grid, s, a);

@@ -39,6 +39,20 @@ namespace b2m {
 
 __device__ __forceinline__ uint2 rns_ld(const uint2* p) { return __ldg(p); }
 __device__ __forceinline__ uint4 rns_ld2(const uint2* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+// Four twiddles in one 32-byte load (32-byte aligned): a warp's lanes read
+// runs of eight that lie 64 bytes apart, and every load instruction looks up
+// each 128-byte line it touches.
+struct Tw4 {
+    uint2 w[4];
+};
+__device__ __forceinline__ Tw4 rns_ld4(const uint2* p) {
+    Tw4 t;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(t.w[0].x), "=r"(t.w[0].y), "=r"(t.w[1].x), "=r"(t.w[1].y), "=r"(t.w[2].x), "=r"(t.w[2].y),
+          "=r"(t.w[3].x), "=r"(t.w[3].y)
+        : "l"(p));
+    return t;
+}
 
 // L levels below node `node` on 2^L positions of V vectors side by side
 // (x[i * V + v]; position i of the node's 2^L equal parts), which share every
@@ -60,17 +74,25 @@ __device__ __forceinline__ void rns_dft_fwd(u32* x, const uint2* __restrict__ T,
             for (int i = 0; i < half; ++i) rns_bfly_fwd(x[i], x[i + half], w, m);
         }
     } else {
+        constexpr int W = LEV == 1 ? 2 : 4;  // twiddles per load
 #pragma unroll
-        for (int j = 0; j < (1 << LEV); j += 2) {
-            const uint4 w = rns_ld2(T + (node << LEV) + j);
+        for (int j0 = 0; j0 < (1 << LEV); j0 += W) {
+            uint2 w[W];
+            if constexpr (W == 2) {
+                const uint4 v = rns_ld2(T + (node << LEV) + j0);
+                w[0] = make_uint2(v.x, v.y), w[1] = make_uint2(v.z, v.w);
+            } else {
+                const Tw4 v = rns_ld4(T + (node << LEV) + j0);
 #pragma unroll
-            for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
-                if (N0 && j == 0) rns_bfly_fwd1(x[i], x[i + half], m);
-                else rns_bfly_fwd(x[i], x[i + half], make_uint2(w.x, w.y), m);
+                for (int j = 0; j < W; ++j) w[j] = v.w[j];
             }
 #pragma unroll
-            for (int i = (2 * j + 2) * half; i < (2 * j + 3) * half; ++i)
-                rns_bfly_fwd(x[i], x[i + half], make_uint2(w.z, w.w), m);
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int i = 2 * (j0 + j) * half; i < (2 * (j0 + j) + 1) * half; ++i) {
+                    if (N0 && j0 + j == 0) rns_bfly_fwd1(x[i], x[i + half], m);
+                    else rns_bfly_fwd(x[i], x[i + half], w[j], m);
+                }
         }
     }
     if constexpr (LEV + 1 < L) rns_dft_fwd<L, V, N0, HZ, LEV + 1>(x, T, node, m);
@@ -89,17 +111,25 @@ __device__ __forceinline__ void rns_dft_inv(u32* x, const uint2* __restrict__ T,
             for (int i = 0; i < half; ++i) rns_bfly_inv(x[i], x[i + half], w, m);
         }
     } else {
+        constexpr int W = LEV == 1 ? 2 : 4;  // twiddles per load
 #pragma unroll
-        for (int j = 0; j < (1 << LEV); j += 2) {
-            const uint4 w = rns_ld2(T + (node << LEV) + j);
+        for (int j0 = 0; j0 < (1 << LEV); j0 += W) {
+            uint2 w[W];
+            if constexpr (W == 2) {
+                const uint4 v = rns_ld2(T + (node << LEV) + j0);
+                w[0] = make_uint2(v.x, v.y), w[1] = make_uint2(v.z, v.w);
+            } else {
+                const Tw4 v = rns_ld4(T + (node << LEV) + j0);
 #pragma unroll
-            for (int i = 2 * j * half; i < (2 * j + 1) * half; ++i) {
-                if (N0 && j == 0) rns_bfly_inv1(x[i], x[i + half], m);
-                else rns_bfly_inv(x[i], x[i + half], make_uint2(w.x, w.y), m);
+                for (int j = 0; j < W; ++j) w[j] = v.w[j];
             }
 #pragma unroll
-            for (int i = (2 * j + 2) * half; i < (2 * j + 3) * half; ++i)
-                rns_bfly_inv(x[i], x[i + half], make_uint2(w.z, w.w), m);
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+                for (int i = 2 * (j0 + j) * half; i < (2 * (j0 + j) + 1) * half; ++i) {
+                    if (N0 && j0 + j == 0) rns_bfly_inv1(x[i], x[i + half], m);
+                    else rns_bfly_inv(x[i], x[i + half], w[j], m);
+                }
         }
         rns_dft_inv<L, V, N0, LEV - 1>(x, T, node, m);
     }
@@ -254,80 +284,119 @@ __device__ __forceinline__ u32* rns_buf(const RnsArgs& a, int op) {
     return op ? a.bufB + blockIdx.y * a.stride_b : a.bufA + blockIdx.y * a.stride_a;
 }
 
-// First forward pass: limbs -> residues. Grid x: tiles of the q * M points,
-// y: jobs, z: operand * 3 + prime.
-template <int LOGR, int V>
+// The operand of a first pass, and for single products the zeroing of the
+// carry's scratch and length. JOBS: from the job table (kept apart so that
+// single products address their limbs from uniform registers).
+template <bool JOBS>
+__device__ __forceinline__ const u32* rns_operand(const RnsArgs& a, int op, u32* n) {
+    if constexpr (JOBS) {
+        const ProdJob& J = a.jobs[blockIdx.y];
+        *n = (u32)(op ? J.nb : J.na);  // at most 2^26
+        return op ? J.b : J.a;
+    } else {
+        if (a.zero && blockIdx.z == 0) {
+            const u32 i = blockIdx.x * 256 + threadIdx.x;
+            if (i < a.nzero) a.zero[i] = 0;
+            if (i == 0) *a.zero_len = 0;
+        }
+        *n = (u32)(op ? a.nb : a.na);
+        return op ? a.b : a.a;
+    }
+}
+
+// First forward pass: limbs -> residues. Grid x: tiles, y: jobs, z: operand *
+// 3 + prime.
+template <int LOGR, int V, bool JOBS>
 __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_first(const RnsArgs a) {
     using G = RnsCol<LOGR, V>;
     extern __shared__ __align__(16) u32 smr[];
     const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
     const RnsMod m(pi);
     pdl_enter();
-    // single products: the carry's scratch and the length start at zero
-    if (a.zero && blockIdx.z == 0) {
-        const u32 i = blockIdx.x * 256 + threadIdx.x;
-        if (i < a.nzero) a.zero[i] = 0;
-        if (i == 0) *a.zero_len = 0;
-    }
-    const u32* limbs = op ? a.b : a.a;
-    u64 nd = op ? a.nb : a.na;
-    if (a.jobs) {
-        const ProdJob& J = a.jobs[blockIdx.y];
-        limbs = op ? J.b : J.a;
-        nd = op ? J.nb : J.na;
-    }
+    u32 n;
+    const u32* limbs = rns_operand<JOBS>(a, op, &n);
     const RnsThread<G, V> t;
-    const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), node = blockIdx.x >> (a.logs - G::LC);
-    const u32 c0 = cg << G::LC;                           // first column of the tile
-    const u32 j0 = ((u32)t.u << a.logs) + t.col;          // this thread's first position, less c0
-    const u32 n = (u32)nd;                                // at most 2^26
+    const u32 c0 = blockIdx.x << G::LC;            // first column of the tile
+    const u32 j0 = ((u32)t.u << a.logs) + t.col;   // this thread's first position, less c0
     const u32 np4 = 2 * m.np2;
     u32 x[G::E * V];
     const uint2* T = a.tw + (u64)pi * a.ent;
-    if (a.q == 1) {
-        if (2 * nd <= a.nt) {
-            // the upper half of the points is zero for almost every product
-            rns_load_limbs<LOGR, V, G::E / 2>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
-            rns_dft_fwd<G::LA, V, true, true>(x, T, 0, m);
-        } else {
-            rns_load_limbs<LOGR, V, G::E>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
-            rns_dft_fwd<G::LA, V, true, false>(x, T, 0, m);
-        }
-        rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
-        rns_stage_b<LOGR, V, false>(x, T, 0, t.u, m);
+    if (2 * (u64)n <= a.nt) {
+        // the upper half of the points is zero for almost every product
+        rns_load_limbs<LOGR, V, G::E / 2>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+        rns_dft_fwd<G::LA, V, true, true>(x, T, 0, m);
     } else {
-        // modulo x^M - c_t: sum over the filled M-blocks of c_t^i x_i, highest first
-        const int lm = a.logs + LOGR;
-        const uint2 ct = a.ct[pi][node];
-        const u32 last = n ? (n - 1) >> lm : 0u;
+        rns_load_limbs<LOGR, V, G::E>(x, limbs + c0, j0, n > c0 ? n - c0 : 0u, a.logs, np4);
+        rns_dft_fwd<G::LA, V, true, false>(x, T, 0, m);
+    }
+    rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
+    rns_stage_b<LOGR, V, false>(x, T, 0, t.u, m);
+    rns_store_b<LOGR, V>(x, rns_buf(a, op) + ((u64)pi * a.nt + c0), t.u, t.col, a.logs);
+}
+
+// The same for a transform in q parts: the operand modulo x^M - c_t, that is
+// the sum over the filled M-blocks of c_t^i x_i (highest first), then the
+// part's levels. A block runs a.pper parts of its tile one after the other on
+// the limbs it loaded once (the two blocks that a balanced product's operand
+// fills; further ones are read again). Grid x: tiles of M, then part groups.
+template <int LOGR, int V, bool JOBS>
+__global__ void __launch_bounds__(256, 3) k_rns_first_parts(const RnsArgs a) {
+    using G = RnsCol<LOGR, V>;
+    extern __shared__ __align__(16) u32 smr[];
+    const int pi = blockIdx.z % 3, op = a.op0 + blockIdx.z / 3;
+    const RnsMod m(pi);
+    pdl_enter();
+    u32 n;
+    const u32* limbs = rns_operand<JOBS>(a, op, &n);
+    const RnsThread<G, V> t;
+    const u32 c0 = (blockIdx.x & ((1u << (a.logs - G::LC)) - 1)) << G::LC;
+    const u32 j0 = ((u32)t.u << a.logs) + t.col;
+    const u32 np4 = 2 * m.np2;
+    const int lm = a.logs + LOGR;
+    const u32 last = n ? (n - 1) >> lm : 0u;
+    u32 hi[G::E * V], lo[G::E * V];
+    {
         const u32 b0 = (last << lm) + c0;
-        rns_load_limbs<LOGR, V, G::E>(x, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
-        for (u32 i = last; i-- > 0;) {  // blocks below the last are full
-            const u32* lp = limbs + ((i << lm) + c0);
+        rns_load_limbs<LOGR, V, G::E>(hi, limbs + b0, j0, n > b0 ? n - b0 : 0u, a.logs, np4);
+        if (last) {  // blocks below the last are full
+            rns_load_limbs<LOGR, V, G::E>(lo, limbs + (((last - 1) << lm) + c0), j0, ~0u, a.logs, np4);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {  // in two halves, for the registers
-                constexpr int H = G::E / 2;
-                u32 v[H * V];
+            for (int k = 0; k < G::E * V; ++k) lo[k] = rns_red2(lo[k], m);
+        }
+    }
+    const u32 t0 = (blockIdx.x >> (a.logs - G::LC)) * a.pper;
+#pragma unroll 1
+    for (u32 part = t0; part < t0 + a.pper; ++part) {
+        const uint2 ct = a.ct[pi][part];
+        u32 x[G::E * V];
+        if (last == 0) {
 #pragma unroll
-                for (int k = 0; k < H * V; ++k)
-                    v[k] = __ldg(lp + ((u64)(h * H + k / V) << (a.logs + G::LB)) + j0 + k % V);
+            for (int k = 0; k < G::E * V; ++k) x[k] = hi[k];
+        } else if (part == 0) {  // c_0 = 1
 #pragma unroll
-                for (int k = 0; k < H * V; ++k) {
-                    u32& y = x[h * H * V + k];
-                    y = rns_red2(__viaddmin_u32(v[k], np4, v[k]), m) + rns_mul(y, ct, m);
-                }
+            for (int k = 0; k < G::E * V; ++k) x[k] = lo[k] + rns_red2(hi[k], m);
+        } else {
+#pragma unroll
+            for (int k = 0; k < G::E * V; ++k) x[k] = lo[k] + rns_mul(hi[k], ct, m);
+        }
+        for (u32 i = last; i-- > 1;) {
+            const u32* lp = limbs + (((i - 1) << lm) + c0);
+#pragma unroll
+            for (int k = 0; k < G::E * V; ++k) {
+                const u32 v = __ldg(lp + ((u64)(k / V) << (a.logs + G::LB)) + j0 + k % V);
+                x[k] = rns_red2(__viaddmin_u32(v, np4, v), m) + rns_mul(x[k], ct, m);
             }
         }
         // roots of unity as the c_t: the nodes of the common tree; otherwise
-        // (weighted) each sub-transform has its own first-pass tree and
-        // leaves a factor theta_t^column
-        const uint2* T1 = a.wtree ? a.wtree + ((u64)(pi * a.q + node) << LOGR) : T;
-        const u32 n0 = a.wtree ? 1u : node;
-        rns_dft_fwd<G::LA, V, false, false>(x, T1, n0, m);
-        rns_exchange_ab<LOGR, V>(smr, x, t.u, t.col);
-        rns_stage_b<LOGR, V, false>(x, T1, n0 << G::LA, t.u, m);
-        if (a.wtree) {
-            const uint2* wc = a.wcol + ((u64)(pi * a.q + node) << a.logs) + c0 + t.col;
+        // (weighted) each part has its own first-pass tree and leaves a
+        // factor theta_t^column (theta_0 = 1)
+        const uint2* T = a.wtree ? a.wtree + ((u64)(pi * a.q + part) << LOGR) : a.tw + (u64)pi * a.ent;
+        const u32 n0 = a.wtree ? 1u : part;
+        rns_dft_fwd<G::LA, V, false, false>(x, T, n0, m);
+        rns_exchange_ab<LOGR, V>(smr + (part & 1) * G::SMEM, x, t.u, t.col);  // two buffers in turn
+        rns_stage_b<LOGR, V, false>(x, T, n0 << G::LA, t.u, m);
+        if (a.wtree && part) {
+            const uint2* wc = a.wcol + ((u64)(pi * a.q + part) << a.logs) + c0 + t.col;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const uint2 w = rns_ld(wc + v);
@@ -335,9 +404,8 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_first(cons
                 for (int k = 0; k < G::E; ++k) x[k * V + v] = rns_mul(x[k * V + v], w, m);
             }
         }
+        rns_store_b<LOGR, V>(x, rns_buf(a, op) + ((u64)pi * a.nt + ((u64)part << lm) + c0), t.u, t.col, a.logs);
     }
-    u32* out = rns_buf(a, op) + ((u64)pi * a.nt + ((u64)node << (a.logs + LOGR)) + c0);
-    rns_store_b<LOGR, V>(x, out, t.u, t.col, a.logs);
 }
 
 // A middle forward pass, in place. Grid as above.
@@ -362,7 +430,7 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_mid(const 
 }
 
 // An inverse column pass, in place. Grid z: prime. FIRST: the tree's top
-// levels (pass 0).
+// levels (pass 0) of an undivided transform.
 template <int LOGR, int V, bool FIRST>
 __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_inv(const RnsArgs a) {
     using G = RnsCol<LOGR, V>;
@@ -373,28 +441,74 @@ __global__ void __launch_bounds__(256, (RnsCol<LOGR, V>::MINB)) k_rns_inv(const 
     const u32 cg = blockIdx.x & ((1u << (a.logs - G::LC)) - 1), sub = blockIdx.x >> (a.logs - G::LC);
     u32* buf = rns_buf(a, 1) + ((u64)pi * a.nt + ((u64)sub << (a.logs + LOGR)) + (cg << G::LC));
     const uint2* T = a.twi + (u64)pi * a.ent;
-    u32 node = sub & a.nmask;
+    const u32 node = FIRST ? 0u : sub & a.nmask;
     u32 x[G::E * V];
     pdl_enter();
     rns_load_b<LOGR, V>(x, buf, t.u, t.col, a.logs);
-    if constexpr (FIRST) {
-        if (a.wtree) {
-            T = a.wtree + ((u64)(pi * a.q + sub) << LOGR);
-            node = 1;
-            const uint2* wc = a.wcol + ((u64)(pi * a.q + sub) << a.logs) + (cg << G::LC) + t.col;
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const uint2 w = rns_ld(wc + v);
-#pragma unroll
-                for (int k = 0; k < G::E; ++k) x[k * V + v] = rns_mul(x[k * V + v], w, m);
-            }
-        }
-    }
     rns_stage_b<LOGR, V, true>(x, T, node << G::LA, t.u, m);
     rns_exchange_ba<LOGR, V>(smr, x, t.u, t.col);
-    if (FIRST && a.q == 1) rns_dft_inv<G::LA, V, true>(x, T, 0, m);
-    else rns_dft_inv<G::LA, V, false>(x, T, node, m);
+    rns_dft_inv<G::LA, V, FIRST>(x, T, node, m);
     rns_store_a<LOGR, V>(x, buf, t.u, t.col, a.logs);
+}
+
+// Inverse pass 0 of a transform in Q parts: each block runs its tile of every
+// part, then puts the parts together in registers,
+//     f_s[j] = sum_t V^-1[s][t] z_t[j]
+// (V the Vandermonde matrix of the c_t), one wide sum and one reduction per
+// value: z_t is brought below p, so Q <= 8 terms below 2^59.8 fit 64 bits. As
+// a kernel of its own the last step read and wrote all residues once more
+// (215 us of the 2^24-limb product, 88 us at 3 * 2^22 points).
+template <int LOGR, int Q>
+__global__ void __launch_bounds__(256, (RnsCol<LOGR, 1>::E * Q >= 48 ? 2 : 3))
+    k_rns_inv_parts(const RnsArgs a, const RnsCombine c) {
+    using G = RnsCol<LOGR, 1>;
+    extern __shared__ __align__(16) u32 smr[];
+    const int pi = blockIdx.z;
+    const RnsMod m(pi);
+    const RnsThread<G, 1> t;
+    const u32 c0 = blockIdx.x << G::LC;
+    const u64 M = 1ull << (a.logs + LOGR);
+    u32* buf = rns_buf(a, 1) + ((u64)pi * a.nt + c0);
+    u32 z[Q][G::E];
+    pdl_enter();
+#pragma unroll
+    for (int s = 0; s < Q; ++s) {
+        u32* x = z[s];
+        rns_load_b<LOGR, 1>(x, buf + s * M, t.u, t.col, a.logs);
+        const uint2* T = a.twi + (u64)pi * a.ent;
+        u32 node = s;
+        if (a.wtree) {
+            T = a.wtree + ((u64)(pi * Q + s) << LOGR);
+            node = 1;
+            if (s) {  // theta_0 = 1
+                const uint2 w = rns_ld(a.wcol + ((u64)(pi * Q + s) << a.logs) + c0 + t.col);
+#pragma unroll
+                for (int k = 0; k < G::E; ++k) x[k] = rns_mul(x[k], w, m);
+            }
+        }
+        rns_stage_b<LOGR, 1, true>(x, T, node << G::LA, t.u, m);
+        // two buffers in turn: a part's writes never meet the previous part's
+        // reads, which end before the barrier in between
+        rns_exchange_ba<LOGR, 1>(smr + (s & 1) * G::SMEM, x, t.u, t.col);
+        rns_dft_inv<G::LA, 1, false>(x, T, node, m);
+#pragma unroll
+        for (int k = 0; k < G::E; ++k) x[k] = __viaddmin_u32(x[k], 0u - m.p, x[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < G::E; ++k) {
+        u32 y[Q];
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            u64 acc = 0;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) acc += (u64)z[i][k] * c.v[pi][s][i];
+            y[s] = rns_redc(acc, pi, m);
+        }
+#pragma unroll
+        for (int s = 0; s < Q; ++s) z[s][k] = y[s];
+    }
+#pragma unroll
+    for (int s = 0; s < Q; ++s) rns_store_a<LOGR, 1>(z[s], buf + s * M, t.u, t.col, a.logs);
 }
 
 // ---------------------------------------------------------------------------

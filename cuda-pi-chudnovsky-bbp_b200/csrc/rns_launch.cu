@@ -11,7 +11,7 @@
 // c_t = theta_t^M with theta_t a power of the generator, the first pass runs
 // the tree of theta_t and its columns take a factor theta_t^column
 // ("weighted"). The parts of the inverse are put together by the inverse
-// Vandermonde matrix of the c_t (k_rns_combine).
+// Vandermonde matrix of the c_t (k_rns_inv_parts).
 //
 // Reference counterpart: mul_ntt_cuda (src/ntt_cuda.cu:179-243).
 #include <cuda_runtime.h>
@@ -40,23 +40,29 @@ struct RnsShape {
 // Pass radices of a 2^m-point part.
 constexpr int RNS_MIN_M = 13, RNS_MAX_M = RNS_TWO_ADICITY;
 constexpr int kSplit[RNS_MAX_M - RNS_MIN_M + 1][3] = {
-    {6, 0, 7},   // 2^13
-    {6, 0, 8},   // 2^14
-    {7, 0, 8},   // 2^15
-    {8, 0, 8},   // 2^16
-    {9, 0, 8},   // 2^17
-    {10, 0, 8},  // 2^18
-    {10, 0, 9},  // 2^19
-    {6, 6, 8},   // 2^20
-    {6, 7, 8},   // 2^21
-    {7, 7, 8},   // 2^22
-    {7, 8, 8},   // 2^23
+    {6, 0, 7},  // 2^13
+    {6, 0, 8},  // 2^14
+    {7, 0, 8},  // 2^15
+    {8, 0, 8},  // 2^16
+    {5, 5, 7},  // 2^17
+    {5, 6, 7},  // 2^18
+    {6, 6, 7},  // 2^19
+    {6, 6, 8},  // 2^20
+    {6, 7, 8},  // 2^21
+    {6, 8, 8},  // 2^22
+    {7, 8, 8},  // 2^23
 };
+// 6 and 8 parts: eight values per thread and part in the first pass (the
+// inverse holds all parts of its tile in registers).
+constexpr int kSplitParts23[3] = {6, 8, 9};
 
 // Launches of at least this many points (over all jobs) take two columns per
-// thread, shorter ones twice as many blocks: at 2^21 points 128.5 -> 120.7 us
-// a product, at 2^20 the same within 1%.
-constexpr u64 RNS_V2_POINTS = 1ull << 21;
+// thread, shorter ones twice as many blocks: at 2^20 points 57.6 against
+// 61.4 us a product, at 2^18 31.7 against 28.5.
+constexpr u64 RNS_V2_POINTS = 1ull << 19;
+
+// Blocks that keep the SMs busy (three per SM) several times over.
+constexpr u64 RNS_FULL_GRID = 148 * 6;
 
 // The shape of a plan's length, q = 0 when these transforms do not take it.
 RnsShape rns_shape(const Plan& p) {
@@ -77,7 +83,7 @@ RnsShape rns_shape(const Plan& p) {
     r.q = q;
     r.m = m;
     r.weighted = q > 1 && m + lq > RNS_TWO_ADICITY;
-    const int* s = kSplit[m - RNS_MIN_M];
+    const int* s = q > 4 ? kSplitParts23 : kSplit[m - RNS_MIN_M];
     for (int k = 0; k < 3; ++k)
         if (s[k]) r.logr[r.npass++] = s[k];
     return r;
@@ -182,12 +188,9 @@ u32 part_constant(const RnsShape& sh, int i, int t) {
 }
 
 // Host constants of a shape, computed once.
-struct CombineArgs {
-    u32 v[3][8][8];  // inverse Vandermonde matrix of the c_t
-};
 struct RnsConst {
     uint2 ct[3][8];
-    CombineArgs comb;
+    RnsCombine comb;
     RnsCrt crt;
 };
 
@@ -225,7 +228,7 @@ RnsConst make_const(const RnsShape& sh) {
         for (int s = 0; s < q; ++s)
             for (int t = 0; t < q; ++t) k.comb.v[i][s][t] = a[s][q + t];
         // residues arrive as c * 2^m * 2^-32 (Montgomery pointwise product),
-        // times 2^-32 again when k_rns_combine ran
+        // times 2^-32 again where parts were put together
         u32 scale = rns_invmod(rns_powmod(2, 32, p), p);
         if (q > 1) scale = rns_mulmod(scale, scale, p);
         scale = rns_mulmod(scale, rns_powmod(2, sh.m, p), p);
@@ -244,35 +247,6 @@ const RnsConst& shape_const(const RnsShape& sh) {
     auto it = cache.find({sh.q, sh.m});
     if (it == cache.end()) it = cache.emplace(std::make_pair(sh.q, sh.m), make_const(sh)).first;
     return it->second;
-}
-
-// The parts' remainders z_t = f mod (x^M - c_t) -> the M-blocks of f:
-// f_s[j] = sum_t V^-1[s][t] z_t[j], one wide sum and one reduction each.
-// In place; z_t < 2p is brought below p, so q <= 8 terms below 2^59.8 fit.
-__global__ void __launch_bounds__(256) k_rns_combine(u32* buf, u64 stride, int q, int m_log, const CombineArgs c) {
-    const int i = blockIdx.z;
-    const RnsMod m(i);
-    const u64 M = 1ull << m_log;
-    pdl_enter();
-    buf += blockIdx.y * stride + (u64)i * q * M;
-    for (u64 j = (u64)blockIdx.x * blockDim.x + threadIdx.x; j < M; j += (u64)gridDim.x * blockDim.x) {
-        u32 z[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (t < q) {
-                z[t] = buf[t * M + j];
-                z[t] = __viaddmin_u32(z[t], 0u - m.p, z[t]);
-            }
-#pragma unroll
-        for (int s = 0; s < 8; ++s)
-            if (s < q) {
-                u64 acc = 0;
-#pragma unroll
-                for (int t = 0; t < 8; ++t)
-                    if (t < q) acc += (u64)z[t] * c.v[i][s][t];
-                buf[s * M + j] = rns_redc(acc, i, m);
-            }
-    }
 }
 
 // ---- context tables --------------------------------------------------------------
@@ -428,7 +402,7 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
 int rns_launches(const Plan& p) {
     const RnsShape sh = rns_shape(p);
     if (sh.npass == 0) return 1;
-    return 2 * sh.npass - 1 + (sh.q > 1) + 1;
+    return 2 * sh.npass - 1 + 1;
 }
 
 namespace {
@@ -482,16 +456,22 @@ struct RnsRun {
         a.wcol = on ? wcol[dir] : nullptr;
     }
     // Columns per thread of pass k, and its tiles: blocks of 256 threads with
-    // V 2^LA elements each.
-    int cols(int k) const { return sh.logr[k] <= 8 && a.nt * njobs >= RNS_V2_POINTS ? 2 : 1; }
+    // V 2^LA elements each. First passes in parts have 16 elements.
+    int cols(int k) const { return a.nt * njobs >= RNS_V2_POINTS ? 2 : 1; }
     unsigned tiles(int k) const { return (unsigned)(a.nt >> (7 + cols(k) + (sh.logr[k] + 1) / 2)); }
+    unsigned part_tiles() const { return (unsigned)((1ull << sh.m) >> 12); }
     // Forward passes but the last, operands op0 .. op0 + nops - 1.
     cudaError_t forward(int op0, int nops) {
         cudaError_t e = cudaSuccess;
         a.op0 = op0;
         for (int k = 0; k + 1 < sh.npass && e == cudaSuccess; ++k) {
             pass(k);
-            const dim3 grid(tiles(k), njobs, 3 * nops);
+            dim3 grid(tiles(k), njobs, 3 * nops);
+            if (k == 0 && sh.q > 1) {
+                // all parts in one block where that leaves enough blocks
+                a.pper = (u64)part_tiles() * njobs * 3 * nops >= RNS_FULL_GRID ? sh.q : 1;
+                grid.x = part_tiles() * (sh.q / a.pper);
+            }
             if (tr) tr->mark(s, k == 0 ? B2M_K_FWD_FIRST : B2M_K_FWD_MID, sh.logr[k]);
             weights(0, k == 0);
             e = k == 0 ? rns_launch_first(sh.logr[k], cols(k), grid, s, a)
@@ -510,15 +490,12 @@ struct RnsRun {
             pass(k);
             if (tr) tr->mark(s, B2M_K_INV_MID, sh.logr[k]);
             weights(1, k == 0);
-            e = rns_launch_inv(sh.logr[k], cols(k), k == 0, dim3(tiles(k), njobs, 3), s, a);
+            if (k == 0 && sh.q > 1)
+                e = rns_launch_inv_parts(sh.logr[0], dim3((unsigned)((1ull << sh.m) >> (8 + (sh.logr[0] + 1) / 2)), njobs, 3), s, a, shape_const(sh).comb);
+            else
+                e = rns_launch_inv(sh.logr[k], cols(k), k == 0, dim3(tiles(k), njobs, 3), s, a);
         }
         weights(1, false);
-        if (sh.q > 1 && e == cudaSuccess) {
-            if (tr) tr->mark(s, B2M_K_R3_INV, 0);
-            const unsigned blocks = (unsigned)std::min<u64>(4096, (1ull << sh.m) / 256);
-            e = launch_pdl(k_rns_combine, dim3(blocks, njobs, 3), 256, 0, s, a.bufB, a.stride_b, sh.q, sh.m,
-                           shape_const(sh).comb);
-        }
         return e;
     }
     cudaError_t carry(u32* out, u64 nout, LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,

@@ -371,8 +371,7 @@ enum {
     B2M_K_CARRY = 6,       /* decoupled-lookback carry into u32 limbs */
     B2M_K_SMALL = 7,       /* whole product in one CTA (transform length <= 2^13) */
     B2M_K_R3_FWD = 8,      /* radix-3 step of a 3 * 2^k-point transform (digits in) */
-    B2M_K_R3_INV = 9       /* inverse radix-3 step, or the parts of a residue transform put
-                              together (coefficients out, natural order) */
+    B2M_K_R3_INV = 9       /* inverse radix-3 step (coefficients out, natural order) */
 };
 
 typedef struct b2m_plan_desc {
