@@ -263,13 +263,13 @@ b2m_status b2m_mul_device(const uint32_t* d_a, uint64_t na, const uint32_t* d_b,
         return B2M_ERR_OUT_OF_MEMORY;
     }
     void* ws = nullptr;
-    cudaError_t e = cudaMallocAsync(&ws, wsb, s);
+    cudaError_t e = p.npass ? cudaMallocAsync(&ws, wsb, s) : cudaSuccess;  // one-launch products need none
     if (e != cudaSuccess) {
         budget_release(c, wsb);
         return cuda_status(e, "cudaMallocAsync(workspace)");
     }
     e = launch_product(d_a, na, d_b, nb, d_out, d_out_len, ws, p, c->tw, c->d_err, s);
-    cudaError_t e2 = cudaFreeAsync(ws, s);
+    cudaError_t e2 = ws ? cudaFreeAsync(ws, s) : cudaSuccess;
     budget_release(c, wsb);
     if (e != cudaSuccess) return cuda_status(e, "kernel launch");
     return cuda_status(e2, "cudaFreeAsync(workspace)");

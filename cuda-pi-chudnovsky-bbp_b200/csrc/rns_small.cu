@@ -134,7 +134,7 @@ struct SmallShape {
     // pairs, then the product, and one carry state per warp
     static constexpr int BYTES = PAD * 12 + T / 32 * 16;
     static constexpr int D = (N + 3 * T - 1) / (3 * T);  // digits per thread of the cluster
-    static constexpr int MINB = T >= 256 ? 3 : (T >= 128 ? 6 : 10);
+    static constexpr int MINB = T >= 256 ? 3 : (T >= 128 ? 6 : (SmallCfg<M>::LE == 4 ? 12 : (T == 64 ? 16 : 28)));
 };
 
 template <int M>
@@ -257,11 +257,10 @@ __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M>::T, Sm
 // Products of at most 128 limbs in all (256 in large batches): schoolbook
 // columns. (Above that the transforms win at every shape: 500 x 8 limbs 16.6 us a call against 10.4,
 // 2,048 of them 97 against 56 us; 250 x 250 18.6 against 8.3.)
-template <int T>
-__global__ void __launch_bounds__(T) k_school(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len,
-                                              const HostLen hl) {
-    __shared__ __align__(16) unsigned char smem[16 * 256 + 64];
-    __shared__ CState st[T];
+__global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const RnsArgs a, u32* __restrict__ out,
+                                                           unsigned long long* out_len, const HostLen hl) {
+    __shared__ u32 smem[SCHOOL_SMEM_WORDS];
+    __shared__ CState st[SCHOOL_WARPS_CTA];
     __shared__ unsigned long long s_top;
     pdl_enter();
     const u32 *la = a.a, *lb = a.b;
@@ -305,7 +304,7 @@ cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArg
             // one after the other the cluster is faster (128 x 128 limbs 8.5
             // against 12.4 us a call), thousands at once the schoolbook
             // (0.015 against 0.021 us each); 512 jobs fill the SMs
-            if (njobs >= 512) return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len, hl);
+            if (njobs >= 512) return launch_pdl(k_school, njobs, SCHOOL_THREADS, 0, s, a, out, out_len, hl);
             return launch<8>(njobs, s, a, out, out_len, crt, hl);
         case 9: return launch<9>(njobs, s, a, out, out_len, crt, hl);
         case 10: return launch<10>(njobs, s, a, out, out_len, crt, hl);
@@ -313,7 +312,7 @@ cudaError_t rns_launch_small(int m, unsigned njobs, cudaStream_t s, const RnsArg
         case 12: return launch<12>(njobs, s, a, out, out_len, crt, hl);
         default:
             if (m > 7) return cudaErrorInvalidValue;
-            return launch_pdl(k_school<64>, njobs, 64, 0, s, a, out, out_len, hl);
+            return launch_pdl(k_school, njobs, SCHOOL_THREADS, 0, s, a, out, out_len, hl);
     }
 }
 
