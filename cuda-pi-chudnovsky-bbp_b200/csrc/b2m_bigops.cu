@@ -287,8 +287,10 @@ __device__ __forceinline__ void publish_top(unsigned long long top, PubState* st
     }
 }
 
-__global__ void k_top_pub(const u32* __restrict__ a, u64 n, PubState* st, const HostLen hl) {
+// `limb` (may be null): a limb published beside the length.
+__global__ void k_top_pub(const u32* __restrict__ a, u64 n, const u32* limb, PubState* st, const HostLen hl) {
     pdl_enter();
+    if (limb && blockIdx.x == 0 && threadIdx.x == 0) st->carry = *limb;
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
         if (a[k]) t = k + 1;
@@ -409,11 +411,20 @@ inline unsigned pub_grid(uint64_t n) { return std::min(grid_for(n), 1024u); }
 
 uint64_t top_len(Scope& S, DV a) {
     if (a.n == 0) return 0;
-    ck(launch_pdl(k_top_pub, pub_grid(a.n), 256, 0, S.s(), a.p, a.n, pub(S), S.publication()), "k_top_pub");
+    ck(launch_pdl(k_top_pub, pub_grid(a.n), 256, 0, S.s(), a.p, a.n, nullptr, pub(S), S.publication()),
+       "k_top_pub");
     return S.published()[1];
 }
 
 DV trim(Scope& S, DV a) { return {a.p, top_len(S, a)}; }
+
+// The low n limbs of a, trimmed, and limb n.
+DV split_at(Scope& S, DV a, uint64_t n, u32* limb) {
+    ck(launch_pdl(k_top_pub, pub_grid(n), 256, 0, S.s(), a.p, n, a.p + n, pub(S), S.publication()), "k_top_pub");
+    const u64* h = S.published();
+    *limb = (u32)h[2];
+    return {a.p, h[1]};
+}
 
 // out = a 2^(32 a_off) +- b mod 2^(32 out.n): the carry (add) or borrow (sub)
 // out, and the trimmed result.
@@ -616,11 +627,12 @@ DV recip(Scope& S, DV Bn, uint64_t h) {
     if (T.n <= e) {  // E = 2^(32e) - T >= 0
         E = addsub(S, DV{T.p, 0}, T, S.vec(e), true).v;
     } else {  // T = 2^(32e) + E', 0 <= E' < 2^(32e)
-        if (T.n != e + 1 || limb_at(S, T, e) != 1) {
+        u32 top = 0;
+        if (T.n == e + 1) E = split_at(S, T, e, &top);
+        if (top != 1) {
             set_error("Newton reciprocal diverged");
             throw Err{B2M_ERR_INTERNAL};
         }
-        E = trim(S, {T.p, e});
         neg = true;
     }
     DV D = mul(S, Xl, E);
@@ -732,11 +744,12 @@ DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     if (U.n <= e) {  // E = 2^(32e) - U >= 0
         E = addsub(S, DV{U.p, 0}, U, S.vec(e), true).v;
     } else {  // U = 2^(32e) + E'
-        if (U.n != e + 1 || limb_at(S, U, e) != 1) {
+        u32 top = 0;
+        if (U.n == e + 1) E = split_at(S, U, e, &top);
+        if (top != 1) {
             set_error("Newton reciprocal square root diverged");
             throw Err{B2M_ERR_INTERNAL};
         }
-        E = trim(S, {U.p, e});
         neg = true;
     }
     DV corr = shr(S, mul(S, Y0, E), e, 1);  // Y0 |E| / 2^(32e + 1)
@@ -803,6 +816,7 @@ constexpr int DC_LEAF_GROUPS = 8;
 __global__ void k_dc_jobs(const u32* a, u64 sa, u64 na, const u32* b, u64 sb, u64 nb, u32* out, u64 so,
                           unsigned long long* lens, ProdJob* jobs, u64 njobs, unsigned char* ws, u64 wss, u64 npts,
                           u64* spec) {
+    pdl_enter();
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= njobs) return;
     ProdJob J{};
@@ -839,6 +853,7 @@ __global__ void k_dc_jobs(const u32* a, u64 sa, u64 na, const u32* b, u64 sb, u6
 
 // The one-job table that transforms b into spec.
 __global__ void k_dc_spec_job(const u32* b, u64 nb, u64* spec, ProdJob* job) {
+    pdl_enter();
     ProdJob J{};
     J.a = b;
     J.na = nb;
@@ -847,6 +862,7 @@ __global__ void k_dc_spec_job(const u32* b, u64 nb, u64* spec, ProdJob* job) {
 }
 
 __global__ void k_dc_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 scratch_words) {
+    pdl_enter();
     const u64 j = blockIdx.x;
     if (j >= njobs) return;
     unsigned long long* s = reinterpret_cast<unsigned long long*>(jobs[j].slots);
@@ -872,8 +888,7 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
     if (sb == 0 && m > 1 && p.npass > 0) {
         spec = static_cast<u64*>(S.raw(8 * npts));
         ProdJob* sj = static_cast<ProdJob*>(S.raw(sizeof(ProdJob)));
-        k_dc_spec_job<<<1, 1, 0, S.s()>>>(b, nb, spec, sj);
-        ck(cudaGetLastError(), "spectrum job");
+        ck(launch_pdl(k_dc_spec_job, 1, 1, 0, S.s(), b, nb, spec, sj), "spectrum job");
         ck(launch_bucket_spectrum(p, sj, 1, {spec, 0, nullptr, 0}, c->tw, S.s()), "shared spectrum");
     }
     const uint64_t wss = !p.npass ? 0
@@ -887,11 +902,13 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
         ProdJob* jobs = static_cast<ProdJob*>(S.raw(nj * sizeof(ProdJob)));
         unsigned long long* lens = static_cast<unsigned long long*>(S.raw(nj * 8));
         unsigned char* ws = wss ? static_cast<unsigned char*>(S.raw(nj * wss)) : nullptr;
-        k_dc_jobs<<<(unsigned)((nj + 255) / 256), 256, 0, S.s()>>>(a + off * sa, sa, na, b + off * sb, sb, nb,
-                                                                  out + off * so, so, lens, jobs, nj, ws, wss, npts,
-                                                                  spec);
-        if (wss) k_dc_zero_ws<<<(unsigned)nj, 256, 0, S.s()>>>(jobs, nj, carry_scratch_bytes_n(npts) / 8);
-        ck(cudaGetLastError(), "job tables");
+        ck(launch_pdl(k_dc_jobs, (unsigned)((nj + 255) / 256), 256, 0, S.s(), a + off * sa, sa, na, b + off * sb, sb, nb,
+                      out + off * so, so, lens, jobs, nj, ws, wss, npts, spec),
+           "job tables");
+        // (residue products zero their scratch and lengths themselves)
+        if (wss && !p.rns)
+            ck(launch_pdl(k_dc_zero_ws, (unsigned)nj, 256, 0, S.s(), jobs, nj, carry_scratch_bytes_n(npts) / 8),
+               "carry scratch");
         JobBufs bufs;
         if (wss) bufs = spec ? JobBufs{spec, 0, ws, wss} : JobBufs{ws, wss, ws + 8 * npts, wss};
         ck(launch_bucket(p, jobs, (unsigned)nj, bufs, c->tw, c->d_err, S.s(), spec != nullptr), "batched product");
@@ -902,6 +919,7 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
 // a compact array of stride nq.
 __global__ void k_dc_extract(const u32* __restrict__ prod, u64 sp, u64 pl, u64 s, u64 nq, u32* __restrict__ q,
                              u64 m) {
+    pdl_enter();
     const u64 total = m * nq;
     for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (u64)gridDim.x * blockDim.x) {
         const u64 i = t / nq, k = t % nq;
@@ -961,6 +979,7 @@ __device__ u32 cta_addsub(const u32* A, u64 la, const u32* B, u64 lb, u32 bsmall
 __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restrict__ U, u64 su,
                          const u32* __restrict__ QE, u64 nq, const u32* __restrict__ P, u64 n, u32* scr, u64 w,
                          u32* __restrict__ out, u64 sout, u32* err) {
+    pdl_enter();
     __shared__ GP ws[33];
     __shared__ u32 s_carry;
     const u64 i = blockIdx.x;
@@ -997,6 +1016,7 @@ __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restri
 
 // One thread per leaf (a value below 10^72 in 8 limbs): 72 decimal digits.
 __global__ void k_dc_leaf(const u32* __restrict__ nodes, u64 stride, u64 m, char* __restrict__ out) {
+    pdl_enter();
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     u32 x[DC_LEAF_LIMBS];
@@ -1122,8 +1142,7 @@ std::string to_decimal(Scope& S, DV X) {
         batched_mul(S, in.p + k, sin, na, R.p, 0, R.n, prod.p, sp, m);
         const uint64_t s = E - k, nq = n + 1;
         DV qe = S.vec(m * nq);
-        k_dc_extract<<<grid_for(m * nq), 256, 0, S.s()>>>(prod.p, sp, sp, s, nq, qe.p, m);
-        ck(cudaGetLastError(), "k_dc_extract");
+        ck(launch_pdl(k_dc_extract, grid_for(m * nq), 256, 0, S.s(), prod.p, sp, sp, s, nq, qe.p, m), "k_dc_extract");
         const uint64_t su = nq + n;
         DV U = S.vec(m * su);
         batched_mul(S, qe.p, nq, nq, Pj.p, 0, n, U.p, su, m);
@@ -1143,9 +1162,9 @@ std::string to_decimal(Scope& S, DV X) {
             DV scr = S.vec(m * (2 * w + nq + 1));
             unsigned threads = 32;
             while (threads < 1024 && (uint64_t)threads * ADD_LPT < w) threads <<= 1;
-            k_dc_fix<<<(unsigned)m, threads, 0, S.s()>>>(in.p, sin, U.p, su, qe.p, nq, Pj.p, n, scr.p, w, out.p,
-                                                         sout, err);
-            ck(cudaGetLastError(), "k_dc_fix");
+            ck(launch_pdl(k_dc_fix, (unsigned)m, threads, 0, S.s(), in.p, sin, U.p, su, qe.p, nq, Pj.p, n, scr.p, w,
+                          out.p, sout, err),
+               "k_dc_fix");
         }
         in = out;
         sin = sout;
@@ -1154,8 +1173,7 @@ std::string to_decimal(Scope& S, DV X) {
     // leaves: m nodes below 10^72 in 8-limb slots
     const uint64_t digits = m * 9 * DC_LEAF_GROUPS;
     char* d_str = static_cast<char*>(S.raw(digits));
-    k_dc_leaf<<<(unsigned)((m + 127) / 128), 128, 0, S.s()>>>(in.p, sin, m, d_str);
-    ck(cudaGetLastError(), "k_dc_leaf");
+    ck(launch_pdl(k_dc_leaf, (unsigned)((m + 127) / 128), 128, 0, S.s(), in.p, sin, m, d_str), "k_dc_leaf");
     std::string str(digits, '0');
     ck(cudaMemcpyAsync(&str[0], d_str, digits, cudaMemcpyDeviceToHost, S.s()), "D2H");
     u32 h_err = 0;

@@ -29,6 +29,7 @@
 #include "b2m_context.h"
 #include "b2m_internal.h"
 #include "gp_scan.cuh"
+#include "pdl.cuh"
 
 namespace b2m {
 
@@ -136,6 +137,7 @@ __device__ __forceinline__ MergeProd merge_prod(const LevelView& L, const LevelV
 // lane resolves the carries. For operands of at most SCHOOL_MAX limbs.
 __global__ void __launch_bounds__(SCHOOL_WARPS * 32) k_bs_school(LevelView L, LevelView Ln, ScratchXY S,
                                                                  u64 m2, u32 kinds_mask) {
+    pdl_enter();
     __shared__ u64 s_lo[SCHOOL_WARPS][2 * SCHOOL_MAX];
     __shared__ u32 s_hi[SCHOOL_WARPS][2 * SCHOOL_MAX];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -186,6 +188,7 @@ __global__ void __launch_bounds__(SCHOOL_WARPS * 32) k_bs_school(LevelView L, Le
 __global__ void k_bs_build_jobs(LevelView L, LevelView Ln, ScratchXY S, u64 m2, int kind, ProdJob* jobs,
                                 unsigned char* ntt_ws, u64 ws_stride, u64 npts, unsigned char* spec_ws,
                                 u64 spec_stride) {
+    pdl_enter();
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m2) return;
     const MergeProd p = merge_prod(L, Ln, S, i, kind);
@@ -220,6 +223,7 @@ __global__ void k_bs_zero(unsigned long long* p, u64 n) {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) p[i] = 0;
 }
 __global__ void k_bs_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 scratch_words) {
+    pdl_enter();
     // one block per job: its lookback slots + ticket, and its length
     const u64 j = blockIdx.x;
     if (j >= njobs) return;
@@ -231,6 +235,7 @@ __global__ void k_bs_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 sc
 // ---------------------------------------------------------------------------- T = sx*X + sy*Y
 // One CTA per merge: T' = sign(TL)*X + sign(TR)*Y (X = TL*QR, Y = PL*TR).
 __global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln, u64 m2) {
+    pdl_enter();
     __shared__ GP s_ws[33];
     __shared__ u32 s_carry;
     __shared__ unsigned long long s_top;
@@ -565,8 +570,8 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
         if (std::max(ka[k], kb[k]) <= SCHOOL_MAX) school_mask |= 1u << k;
     if (m2 && school_mask) {
         const uint64_t blocks = (4 * m2 + SCHOOL_WARPS - 1) / SCHOOL_WARPS;
-        k_bs_school<<<(unsigned)blocks, SCHOOL_WARPS * 32, 0, s>>>(L, *Ln, S, m2, school_mask);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_pdl(k_bs_school, (unsigned)blocks, SCHOOL_WARPS * 32, 0, s, L, *Ln, S, m2, school_mask);
+        if (e != cudaSuccess) return e;
     }
     std::vector<void*> tmp;
     std::vector<uint64_t> tmpb;
@@ -627,13 +632,12 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
         tmpb.push_back(tb);
         ProdJob* jobs = static_cast<ProdJob*>(t);
         unsigned char* ws = wss ? static_cast<unsigned char*>(t) + al(m2 * sizeof(ProdJob)) : nullptr;
-        k_bs_build_jobs<<<(unsigned)((m2 + 255) / 256), 256, 0, s>>>(L, *Ln, S, m2, k, jobs, ws, wss, npts,
-                                                                    use_spec ? pair_ws : nullptr, pair_wss);
-        if (wss) {
-            const uint64_t scratch_words = carry_scratch_bytes_n(npts) / 8;
-            k_bs_zero_ws<<<(unsigned)m2, 256, 0, s>>>(jobs, m2, scratch_words);
-        }
-        if ((e = cudaGetLastError()) != cudaSuccess) break;
+        e = launch_pdl(k_bs_build_jobs, (unsigned)((m2 + 255) / 256), 256, 0, s, L, *Ln, S, m2, k, jobs, ws, wss, npts,
+                       use_spec ? pair_ws : nullptr, pair_wss);
+        // (residue products zero their scratch and lengths themselves)
+        if (e == cudaSuccess && wss && !p.rns)
+            e = launch_pdl(k_bs_zero_ws, (unsigned)m2, 256, 0, s, jobs, m2, carry_scratch_bytes_n(npts) / 8);
+        if (e != cudaSuccess) break;
         for (uint64_t off = 0; off < m2 && e == cudaSuccess; off += 65535) {
             const unsigned nj = (unsigned)std::min<uint64_t>(65535, m2 - off);
             JobBufs bufs;
@@ -654,8 +658,7 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
         const uint64_t maxn = capT;
         unsigned threads = 32;
         while (threads < 1024 && (uint64_t)threads * ADD_LPT < maxn) threads <<= 1;
-        k_bs_signed_add<<<(unsigned)m2, threads, 0, s>>>(S, L.sign, *Ln, m2);
-        e = cudaGetLastError();
+        e = launch_pdl(k_bs_signed_add, (unsigned)m2, threads, 0, s, S, L.sign, *Ln, m2);
     }
     if (e == cudaSuccess && (m & 1)) {
         k_bs_copy_node<<<64, 256, 0, s>>>(L, m - 1, *Ln, mn - 1);

@@ -115,9 +115,9 @@ struct RnsArgs {
     u32 pper;                 // first pass in parts: parts per block
     int op0;                  // operand of grid z 0..2
     int square;
-    unsigned long long* zero;      // first pass of a single product: scratch it zeroes
+    unsigned long long* zero;      // single products: the carry scratch that the first pass zeroes
     unsigned long long* zero_len;  // and the length
-    u32 nzero;                     // words of it
+    u32 nzero;                     // words of carry scratch
     uint2 ct[3][8];           // c_t of the q sub-transforms
 };
 

@@ -19,29 +19,29 @@ __device__ __forceinline__ GP gp_then(GP lo, GP hi) { return {hi.g | (hi.p & lo.
 constexpr int ADD_LPT = 8;  // limbs per thread
 
 // Exclusive block scan of GP (low threads first). blockDim multiple of 32.
+// A warp's carry chain is an integer addition: with G the lanes that generate
+// and P those that only propagate, the carries into the lanes are the carries
+// of (G | P) + G, that is P ^ ((G | P) + G [+ 1 with a carry in]). The warps'
+// aggregates go the same way, by every warp: one barrier, no loop over lanes
+// or warps. Callers synchronise before writing `ws` again.
 __device__ __forceinline__ GP block_scan_gp(GP v, GP* ws, GP* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    GP inc = v;
-    for (int off = 1; off < 32; off <<= 1) {
-        GP o{__shfl_up_sync(0xFFFFFFFFu, inc.g, off), __shfl_up_sync(0xFFFFFFFFu, inc.p, off)};
-        if (lane >= off) inc = gp_then(o, inc);
-    }
-    GP ex{__shfl_up_sync(0xFFFFFFFFu, inc.g, 1), __shfl_up_sync(0xFFFFFFFFu, inc.p, 1)};
-    if (lane == 0) ex = {0, 1};
-    if (lane == 31) ws[warp] = inc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        GP acc{0, 1};
-        for (int w = 0; w < nw; ++w) {
-            GP t = ws[w];
-            ws[w] = acc;
-            acc = gp_then(acc, t);
-        }
-        ws[nw] = acc;
+    const u32 G = __ballot_sync(0xFFFFFFFFu, v.g != 0), P = __ballot_sync(0xFFFFFFFFu, v.p && !v.g);
+    const u64 s0 = (u64)(G | P) + G;
+    if (lane == 0) {
+        const u32 c0 = (u32)(s0 >> 32), c1 = (u32)((s0 + 1) >> 32);
+        ws[warp] = {c0, c1 & ~c0};
     }
     __syncthreads();
-    *total = ws[nw];
-    return gp_then(ws[warp], ex);
+    const GP w = lane < nw ? ws[lane] : GP{0, 0};
+    const u32 WG = __ballot_sync(0xFFFFFFFFu, w.g != 0), WP = __ballot_sync(0xFFFFFFFFu, w.p != 0);
+    const u64 t0 = (u64)(WG | WP) + WG, t1 = t0 + 1;
+    const u32 o0 = (u32)(t0 >> nw) & 1, o1 = (u32)(t1 >> nw) & 1;
+    *total = {o0, o1 & ~o0};
+    // carry into this warp, then into this lane, for a block carry-in of 0 and 1
+    const u32 w0 = ((WP ^ (u32)t0) >> warp) & 1, w1 = ((WP ^ (u32)t1) >> warp) & 1;
+    const u32 c0 = ((P ^ (u32)(s0 + w0)) >> lane) & 1, c1 = ((P ^ (u32)(s0 + w1)) >> lane) & 1;
+    return {c0, c1 & ~c0};
 }
 
 }  // namespace b2m

@@ -284,17 +284,22 @@ __device__ __forceinline__ u32* rns_buf(const RnsArgs& a, int op) {
     return op ? a.bufB + blockIdx.y * a.stride_b : a.bufA + blockIdx.y * a.stride_a;
 }
 
-// The operand of a first pass, and for single products the zeroing of the
-// carry's scratch and length. JOBS: from the job table (kept apart so that
+// The operand of a first pass, and the zeroing of the product's carry scratch
+// and length by the pass's first grid layer. JOBS: from the job table (kept apart so that
 // single products address their limbs from uniform registers).
 template <bool JOBS>
 __device__ __forceinline__ const u32* rns_operand(const RnsArgs& a, int op, u32* n) {
     if constexpr (JOBS) {
         const ProdJob& J = a.jobs[blockIdx.y];
+        if (blockIdx.z == 0 && J.slots) {  // (null: only the spectrum is wanted)
+            const u32 i = blockIdx.x * 256 + threadIdx.x;
+            if (i < a.nzero) reinterpret_cast<unsigned long long*>(J.slots)[i] = 0;
+            if (i == 0) *J.out_len = 0;
+        }
         *n = (u32)(op ? J.nb : J.na);  // at most 2^26
         return op ? J.b : J.a;
     } else {
-        if (a.zero && blockIdx.z == 0) {
+        if (blockIdx.z == 0 && a.zero) {
             const u32 i = blockIdx.x * 256 + threadIdx.x;
             if (i < a.nzero) a.zero[i] = 0;
             if (i == 0) *a.zero_len = 0;

@@ -421,6 +421,7 @@ struct RnsRun {
         Context* c = ctx();
         std::lock_guard<std::mutex> lk(c->twt_mu);
         a.nt = sh.points();
+        a.nzero = (u32)(carry_scratch_bytes_n(plan_points(p)) / 8);
         a.tw = c->rns_t;
         a.ent = 1u << c->rns_log;
         a.twi = a.tw + 3ull * a.ent;
@@ -531,7 +532,6 @@ cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t
     }
     // lookback slots, then the ticket: one word per 1024 points and a few
     r.a.zero = reinterpret_cast<unsigned long long*>(slots);
-    r.a.nzero = (u32)(carry_scratch_bytes_n(plan_points(p)) / 8);
     r.a.zero_len = out_len;
     if (r.a.square || !b_ready) {
         if (b_ready) e = cudaStreamWaitEvent(s, b_ready, 0);
