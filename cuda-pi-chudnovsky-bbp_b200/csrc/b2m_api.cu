@@ -358,7 +358,10 @@ b2m_status b2m_autotune(uint64_t na, uint64_t nb, b2m_stream stream, b2m_tune_en
     int three = 0;
     choose_length(2 * (na + nb), &logn, &three);  // candidates for the (sub-)transform length
     std::vector<Plan> cands = plan_candidates(logn);
-    for (Plan& cp : cands) cp.three = three;
+    for (Plan& cp : cands) {
+        cp.three = three;
+        cp.need = na + nb;
+    }
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t ba = al(4 * na), bb = al(4 * nb), bo = al(4 * (na + nb)), wsb = al(workspace_bytes_plan(cands[0]));
     const uint64_t need = ba + bb + bo + 256 + wsb;
@@ -428,7 +431,8 @@ b2m_status b2m_autotune(uint64_t na, uint64_t nb, b2m_stream stream, b2m_tune_en
     st = take_device_error(c);
     if (st != B2M_OK) return st;
     Plan kept = cands[best_i];
-    kept.three = kept.rns = 0;  // tuned plans are kept per power-of-two length
+    kept.three = kept.rns = 0;
+    kept.need = 0;  // tuned plans are kept per power-of-two length
     set_tuned(c, logn, kept);
     if (best_i < cnt) out[best_i].chosen = 1;
     if (n) *n = cnt;

@@ -100,11 +100,14 @@ static cudaError_t autotune_bucket(b2m_batch* bt, Bucket& b, cudaStream_t s) {
     {
         std::lock_guard<std::mutex> lk(c->tune_mu);
         if (c->has_tuned[b.logn]) {
+            const uint64_t need = b.plan.need;
             b.plan = c->tuned[b.logn];  // its tables: b2m_batch_create
+            b.plan.need = need;
             return cudaSuccess;
         }
     }
     std::vector<Plan> cands = plan_candidates(b.logn);
+    for (Plan& p : cands) p.need = b.plan.need;
     if (cands.size() < 2) return cudaSuccess;
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);
@@ -150,7 +153,9 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
         return B2M_ERR_INVALID_ARGUMENT;
     *out = nullptr;
     // Validate and bucket.
-    std::map<uint64_t, std::vector<unsigned>> by_pts;  // transform points -> job indices
+    // transform points -> job indices, products that 5/6 of a 3 * 2^k length
+    // holds apart from the others
+    std::map<std::pair<uint64_t, int>, std::vector<unsigned>> by_pts;
     std::vector<unsigned> empty;
     for (uint64_t i = 0; i < njobs; ++i) {
         const b2m_job& j = jobs[i];
@@ -165,7 +170,8 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
         b2m_status st = check_sizes(j.na, j.nb, &logn);
         if (st != B2M_OK) return st;
         choose_length(2 * (j.na + j.nb), &logn, &three);
-        by_pts[(three ? 3ull : 1ull) << logn].push_back((unsigned)i);
+        const uint64_t pts = (three ? 3ull : 1ull) << logn;
+        by_pts[{pts, !three || 12 * (j.na + j.nb) > 5 * pts}].push_back((unsigned)i);
     }
     cudaSetDevice(c->device);
     b2m_batch* bt = new b2m_batch();
@@ -176,9 +182,10 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
     const uint64_t lens = al(njobs * sizeof(uint64_t));
     uint64_t bufs = 0, scr = 0;
     for (auto& kv : by_pts) {
-        if (kv.first <= (1ull << SMALL_MAX_LOGN)) continue;
-        bufs += kv.second.size() * 2 * 8 * kv.first;
-        scr += kv.second.size() * al(carry_scratch_bytes_n(kv.first));
+        const uint64_t n = kv.first.first;
+        if (n <= (1ull << SMALL_MAX_LOGN)) continue;
+        bufs += kv.second.size() * 2 * 8 * n;
+        scr += kv.second.size() * al(carry_scratch_bytes_n(n));
     }
     bt->dbytes = tab + lens + bufs + scr;
     if (!budget_reserve(c, bt->dbytes)) {
@@ -216,7 +223,7 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
     };
     constexpr unsigned MAX_GRID_Y = 65535;  // a bucket launch covers at most this many jobs
     for (auto it = by_pts.rbegin(); it != by_pts.rend(); ++it) {
-      const uint64_t n = it->first;
+      const uint64_t n = it->first.first;
       const int three = (n & (n - 1)) ? 1 : 0;  // 3 * 2^k is no power of two
       const uint64_t sub = three ? n / 3 : n;      // the (sub-)transform length 2^k
       int lg = 0;
@@ -224,7 +231,9 @@ b2m_status b2m_batch_create(const b2m_job* jobs, uint64_t njobs, uint32_t flags,
       for (size_t off = 0; off < it->second.size(); off += MAX_GRID_Y) {
         Bucket b;
         b.logn = lg;
-        b.plan = plan_for(c, b.logn, three);
+        uint64_t need = 0;
+        for (unsigned i : it->second) need = std::max(need, jobs[i].na + jobs[i].nb);
+        b.plan = plan_for(c, b.logn, three, need);
         b.first = (unsigned)hj.size();
         b.njobs = (unsigned)std::min<size_t>(MAX_GRID_Y, it->second.size() - off);
         if (n > (1ull << SMALL_MAX_LOGN)) b.bufs = {pbuf, 16 * n, pbuf + 8 * n, 16 * n};

@@ -580,7 +580,7 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
     auto kind_plan = [&](int k) {
         int logn = 0, three = 0;
         choose_length(2 * cap[k], &logn, &three);
-        return plan_for(c, logn, three);
+        return plan_for(c, logn, three, cap[k]);
     };
     // Pairs that share a forward spectrum: Q = QR*QL then X = QR*TL (QR), and
     // P = PL*PR then Y = PL*TR (PL). A shared pair runs both products under
@@ -604,7 +604,9 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
                 const Plan q = kind_plan(partner);
                 const uint64_t n1 = plan_points(p), n2 = plan_points(q), nmax = std::max(n1, n2);
                 if (5 * nmax < 3 * (n1 + n2)) {
+                    const uint64_t need = std::max(p.need, q.need);
                     if (n2 > n1) p = q;
+                    p.need = need;
                     pair_share = p.npass > 0;
                 }
             }

@@ -70,14 +70,16 @@ struct Context {
 };
 
 // The plan products of (sub-)transform length 2^logn use: the tuned one if
-// any, else the default (three: the radix-3 products' default).
-inline Plan plan_for(Context* c, int logn, int three = 0) {
+// any, else the default (three: the radix-3 products' default). need: the
+// limbs of the longest product, when known.
+inline Plan plan_for(Context* c, int logn, int three = 0, uint64_t need = 0) {
     Plan p;
     {
         std::lock_guard<std::mutex> lk(c->tune_mu);
         p = c->has_tuned[logn] ? c->tuned[logn] : make_plan(logn, three);
     }
     p.three = three;
+    p.need = need;
     rns_resolve(c, p, nullptr, false);
     return p;
 }
@@ -87,11 +89,12 @@ inline Plan plan_for(Context* c, int logn, int three = 0) {
 inline Plan product_plan(Context* c, uint64_t na, uint64_t nb) {
     int logn = 0, three = 0;
     choose_length(2 * (na + nb), &logn, &three);
-    return plan_for(c, logn, three);
+    return plan_for(c, logn, three, na + nb);
 }
 inline void set_tuned(Context* c, int logn, const Plan& p) {
     std::lock_guard<std::mutex> lk(c->tune_mu);
     c->tuned[logn] = p;
+    c->tuned[logn].need = 0;
     c->has_tuned[logn] = true;
 }
 

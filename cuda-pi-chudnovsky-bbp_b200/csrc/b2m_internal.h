@@ -44,6 +44,9 @@ struct Plan {
     // logc then only name the length and the workspace. Set where the tables
     // of that path exist (rns_resolve).
     int rns = 0;
+    // Limbs of the longest product that runs under this copy of the plan (0:
+    // any that fits): the residue transforms have lengths in between.
+    uint64_t need = 0;
 };
 
 // Points of a plan's transform, and the workspace and carry scratch a

@@ -106,6 +106,16 @@ struct Req {
     uint64_t t_submit = 0, t_admit = 0, t_done = 0;
 };
 
+// Products of a 3 * 2^k length that 5/6 of it holds run on shorter transforms,
+// in launches of their own.
+static bool above_five_sixths(const Req& q) { return !q.three || 12 * (q.r.na + q.r.nb) > 5 * q.pts; }
+
+// Order of a dispatch's jobs (of its job table and of its results).
+static bool runs_before(const Req& x, const Req& y) {
+    if (x.pts != y.pts) return x.pts > y.pts;
+    return above_five_sixths(x) > above_five_sixths(y);
+}
+
 struct Slot {
     cudaStream_t s = nullptr;
     cudaEvent_t ev = nullptr;
@@ -166,7 +176,7 @@ static cudaError_t launch_dispatch(b2m_server* S, Slot& sl, std::vector<Req>& rv
     // Dispatch block: [job table][lengths][residues][buffers][carry scratch].
     std::vector<size_t> order(n);
     for (size_t i = 0; i < n; ++i) order[i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return rs[x]->pts > rs[y]->pts; });
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return runs_before(*rs[x], *rs[y]); });
     const uint64_t tab = al(n * sizeof(ProdJob)), lens = al(n * 8), res = al(n * RES_WORDS * 8);
     uint64_t bufs = 0, scr = 0;
     for (Req* q : rs)
@@ -245,8 +255,11 @@ static cudaError_t launch_dispatch(b2m_server* S, Slot& sl, std::vector<Req>& rv
     for (size_t k0 = 0; k0 < n;) {
         const uint64_t pts = rs[order[k0]]->pts;
         size_t k1 = k0;
-        while (k1 < n && rs[order[k1]]->pts == pts && k1 - k0 < 65535) ++k1;
-        Plan p = plan_for(S->c, rs[order[k0]]->logn, rs[order[k0]]->three);
+        const bool above = above_five_sixths(*rs[order[k0]]);
+        uint64_t need = 0;
+        for (; k1 < n && rs[order[k1]]->pts == pts && above_five_sixths(*rs[order[k1]]) == above && k1 - k0 < 65535; ++k1)
+            need = std::max(need, rs[order[k1]]->r.na + rs[order[k1]]->r.nb);
+        Plan p = plan_for(S->c, rs[order[k0]]->logn, rs[order[k0]]->three, need);
         if ((e = twtable_ensure(S->c, p, s)) != cudaSuccess) return e;
         JobBufs bufs;  // as laid out above: two buffers of pts elements per job, jobs back to back
         if (pts > (1ull << SMALL_MAX_LOGN)) bufs = {hj[k0].bufA, 16 * pts, hj[k0].bufB, 16 * pts};
@@ -362,7 +375,7 @@ static void scheduler(b2m_server* S) {
             // launch_dispatch sorted the jobs by size: record ids in that order
             std::vector<size_t> order(rs.size());
             for (size_t i = 0; i < order.size(); ++i) order[i] = i;
-            std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return rs[x].pts > rs[y].pts; });
+            std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return runs_before(rs[x], rs[y]); });
             sl.ids.resize(rs.size());
             for (size_t k = 0; k < order.size(); ++k) sl.ids[k] = ids[order[k]];
             sl.busy = true;
@@ -422,6 +435,8 @@ b2m_status b2m_server_start(const b2m_server_config* cfg, b2m_server** out) {
         Plan p = plan_for(c, logn);
         if (twtable_ensure(c, p, S->release_stream) != cudaSuccess) break;
         // the sub-transform plan of 3 * 2^logn points may differ
+        p = plan_for(c, logn, 1, (5 * pts) / 4);  // in five parts
+        if (6 * 8 * pts <= S->cfg.hbm_budget_bytes && twtable_ensure(c, p, S->release_stream) != cudaSuccess) break;
         p = plan_for(c, logn, 1);
         if (6 * 8 * pts <= S->cfg.hbm_budget_bytes && twtable_ensure(c, p, S->release_stream) != cudaSuccess) break;
     }

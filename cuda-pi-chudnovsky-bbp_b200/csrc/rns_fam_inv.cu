@@ -32,7 +32,7 @@ static cudaError_t parts(dim3 grid, cudaStream_t s, const RnsArgs& a, const RnsC
     return launch_pdl(k_rns_inv_parts<LOGR, Q>, grid, G::THREADS, 2 * G::SMEM * 4, s, a, c);
 }
 
-// 3 parts at any radix; 2, 4, 6 and 8 only divide 2^23-point parts.
+// 3 parts at any radix, 5 at 2^6 and below; 2, 4, 6 and 8 have 2^23-point parts.
 cudaError_t rns_launch_inv_parts(int logr, dim3 grid, cudaStream_t s, const RnsArgs& a, const RnsCombine& c) {
     switch (16 * a.q + logr) {
         case 39: return parts<7, 2>(grid, s, a, c);
@@ -41,6 +41,8 @@ cudaError_t rns_launch_inv_parts(int logr, dim3 grid, cudaStream_t s, const RnsA
         case 55: return parts<7, 3>(grid, s, a, c);
         case 56: return parts<8, 3>(grid, s, a, c);
         case 71: return parts<7, 4>(grid, s, a, c);
+        case 85: return parts<5, 5>(grid, s, a, c);
+        case 86: return parts<6, 5>(grid, s, a, c);
         case 102: return parts<6, 6>(grid, s, a, c);
         case 134: return parts<6, 8>(grid, s, a, c);
     }

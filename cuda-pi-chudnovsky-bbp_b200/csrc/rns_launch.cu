@@ -2,8 +2,9 @@
 // tables and launch sequences (kernels: rns_kernels.cuh, rns_carry.cu).
 //
 // A product whose 16-bit-digit length is 2^L or 3 * 2^k points takes half as
-// many 32-bit digits: N = q * 2^m with q = 1 or 3, as long as the roots of
-// unity last (q * 2^m <= 2^23); beyond that N splits into q <= 8 parts of at
+// many 32-bit digits: N = q * 2^m with q = 1 or 3 -- or 5/6 of the latter, q =
+// 5, where that holds it -- as long as the roots of unity last (q * 2^m <=
+// 2^23); beyond that N splits into q <= 8 parts of at
 // most 2^23 points (N <= 2^26, the CRT's bound on the coefficients: at most
 // 2^25 terms below 2^64 each). Parts evaluate modulo x^M - c_t. Where the
 // 2^23 roots allow, c_t is the constant of tree node t and the parts are the
@@ -56,6 +57,11 @@ constexpr int kSplit[RNS_MAX_M - RNS_MIN_M + 1][3] = {
 // inverse holds all parts of its tile in registers).
 constexpr int kSplitParts23[3] = {6, 8, 9};
 
+// Part lengths of transforms in five parts (first radix 2^6 and below: the
+// inverse holds five values per row in registers).
+constexpr bool five_parts(int m) { return m >= 13 && m <= 22 && m != 15; }
+constexpr int kSplitFive16[3] = {5, 5, 6};
+
 // Launches of at least this many points (over all jobs) take two columns per
 // thread, shorter ones twice as many blocks: at 2^20 points 57.6 against
 // 61.4 us a product, at 2^18 31.7 against 28.5.
@@ -78,12 +84,16 @@ RnsShape rns_shape(const Plan& p) {
         q *= 2;
     }
     if (m < RNS_MIN_M || q > 8) return r;
+    if (p.three && q == 3 && p.need && p.need <= 5ull << (m - 1) && five_parts(m - 1)) {
+        q = 5;
+        --m;
+    }
     int lq = 0;
     while ((1 << lq) < q) ++lq;
     r.q = q;
     r.m = m;
     r.weighted = q > 1 && m + lq > RNS_TWO_ADICITY;
-    const int* s = q > 4 ? kSplitParts23 : kSplit[m - RNS_MIN_M];
+    const int* s = q > 5 ? kSplitParts23 : (q == 5 && m == 16 ? kSplitFive16 : kSplit[m - RNS_MIN_M]);
     for (int k = 0; k < 3; ++k)
         if (s[k]) r.logr[r.npass++] = s[k];
     return r;
@@ -458,7 +468,12 @@ struct RnsRun {
     }
     // Columns per thread of pass k, and its tiles: blocks of 256 threads with
     // V 2^LA elements each. First passes in parts have 16 elements.
-    int cols(int k) const { return a.nt * njobs >= RNS_V2_POINTS ? 2 : 1; }
+    // (two columns: 2^(9 - LB) columns a tile, which must fit the stride S).
+    int cols(int k) const {
+        int logs = sh.m;
+        for (int i = 0; i <= k; ++i) logs -= sh.logr[i];
+        return a.nt * njobs >= RNS_V2_POINTS && logs >= 9 - sh.logr[k] / 2 ? 2 : 1;
+    }
     unsigned tiles(int k) const { return (unsigned)(a.nt >> (7 + cols(k) + (sh.logr[k] + 1) / 2)); }
     unsigned part_tiles() const { return (unsigned)((1ull << sh.m) >> 12); }
     // Forward passes but the last, operands op0 .. op0 + nops - 1.
