@@ -33,16 +33,19 @@
 #include "b2m.h"
 #include "b2m_context.h"
 #include "b2m_internal.h"
+#include "pdl.cuh"
 
 namespace b2m {
 
 constexpr int RES_WORDS = 9;  // per job: (sum, even, odd) of a, b and the product
 
 // res[j*9 + 3*w + k]: array w (a, b, out) limb sum (k=0), even-index sum (1),
-// odd-index sum (2). Grid: x over 4096-limb chunks, y over jobs.
+// odd-index sum (2). Grid: x strides over 4096-limb chunks, y over jobs.
 __global__ void k_residues(const ProdJob* __restrict__ jobs, unsigned long long* res) {
     const ProdJob& J = jobs[blockIdx.y];
-    const u64 base = (u64)blockIdx.x * 4096;
+    pdl_enter();
+    const u64 first = (u64)blockIdx.x * 4096, step = (u64)gridDim.x * 4096;
+    if (first >= J.na + J.nb) return;
     __shared__ unsigned long long s[RES_WORDS];
     if (threadIdx.x < RES_WORDS) s[threadIdx.x] = 0;
     __syncthreads();
@@ -50,11 +53,12 @@ __global__ void k_residues(const ProdJob* __restrict__ jobs, unsigned long long*
         const u32* p = w == 0 ? J.a : (w == 1 ? J.b : J.out);
         const u64 n = w == 0 ? J.na : (w == 1 ? J.nb : J.na + J.nb);
         unsigned long long even = 0, odd = 0;
-        for (u64 i = base + threadIdx.x; i < n && i < base + 4096; i += blockDim.x) {
-            const u32 v = p[i];
-            if (i & 1) odd += v;
-            else even += v;
-        }
+        for (u64 base = first; base < n; base += step)
+            for (u64 i = base + threadIdx.x; i < n && i < base + 4096; i += blockDim.x) {
+                const u32 v = p[i];
+                if (i & 1) odd += v;
+                else even += v;
+            }
         for (int off = 16; off > 0; off >>= 1) {
             even += __shfl_xor_sync(0xFFFFFFFFu, even, off);
             odd += __shfl_xor_sync(0xFFFFFFFFu, odd, off);
@@ -265,14 +269,17 @@ static cudaError_t launch_dispatch(b2m_server* S, Slot& sl, std::vector<Req>& rv
         if (pts > (1ull << SMALL_MAX_LOGN)) bufs = {hj[k0].bufA, 16 * pts, hj[k0].bufB, 16 * pts};
         if ((e = launch_bucket(p, djobs + k0, (unsigned)(k1 - k0), bufs, S->c->tw, S->c->d_err, s)) != cudaSuccess)
             return e;
-        // Residue check of the bucket's products, its grid sized to the
-        // bucket's longest operands (not the dispatch's).
-        uint64_t maxlen = 0;
-        for (size_t k = k0; k < k1; ++k) maxlen = std::max<uint64_t>(maxlen, rs[order[k]]->r.na + rs[order[k]]->r.nb);
-        const unsigned gx = (unsigned)((maxlen + 4095) / 4096);
-        k_residues<<<dim3(gx, (unsigned)(k1 - k0)), 256, 0, s>>>(djobs + k0, dres + k0 * RES_WORDS);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         k0 = k1;
+    }
+    // Residue check of all products in one launch (a launch per bucket was an
+    // eighth of the scheduler's enqueueing).
+    uint64_t maxlen = 0;
+    for (size_t k = 0; k < n; ++k) maxlen = std::max<uint64_t>(maxlen, rs[k]->r.na + rs[k]->r.nb);
+    for (size_t k = 0; k < n; k += 65535) {
+        const unsigned nj = (unsigned)std::min<size_t>(65535, n - k);
+        const unsigned gx = (unsigned)std::min<uint64_t>((maxlen + 4095) / 4096, 512);
+        if ((e = launch_pdl(k_residues, dim3(gx, nj), 256, 0, s, djobs + k, dres + k * RES_WORDS)) != cudaSuccess)
+            return e;
     }
     // Results to pinned host memory.
     unsigned char* h = static_cast<unsigned char*>(sl.host);
