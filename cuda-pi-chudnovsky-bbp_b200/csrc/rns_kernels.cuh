@@ -566,7 +566,11 @@ __global__ void __launch_bounds__(256, RnsLast<LOGR>::MINB) k_rns_fused(const Rn
     const int pi = blockIdx.z;
     const RnsMod m(pi);
     const int u = threadIdx.x & (G::U - 1), sl = threadIdx.x >> G::LB;
-    const u32 sub = blockIdx.x * G::SUBS + sl;
+    // Weighted parts read the same twiddles: blocks go round the parts, so that
+    // the copies in L2 serve all of them. (A twiddle per point and direction:
+    // with part after part each came from memory q times.)
+    u32 sub = blockIdx.x * G::SUBS + sl;
+    if (a.nmask != ~0u) sub = (blockIdx.x % a.q) * (a.nmask + 1) + (blockIdx.x / a.q) * G::SUBS + sl;
     if (((u64)sub << LOGR) >= a.nt) return;  // whole sub-problems: whole groups of U lanes
     u32* sm = smr + sl * G::BS;
     const u64 off = (u64)pi * a.nt + ((u64)sub << LOGR) + u;
