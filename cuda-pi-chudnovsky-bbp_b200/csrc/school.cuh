@@ -1,12 +1,11 @@
-// school.cuh -- schoolbook product of two small u32-limb numbers by one CTA.
+// school.cuh -- schoolbook product of two small u32-limb numbers.
 //
 // A schoolbook product costs about 4.5 instructions per limb multiply-add, so
 // for the smallest products (rns_small.cu) it is cheaper than the transforms.
-// Reference
-// counterpart: mul_schoolbook (src/bignum.cpp:125-143), the same column
-// products, here with every column sum of a thread's four-column block
+// Reference counterpart: mul_schoolbook (src/bignum.cpp:125-143), the same
+// column products, here with every column sum of a thread's four columns
 // accumulated in 96 bits by one carry chain per multiply-add, and the carries
-// resolved by a block scan of carry functions (carry.cuh).
+// resolved by a scan of carry functions (carry.cuh).
 #pragma once
 #include "carry.cuh"
 
@@ -21,58 +20,63 @@ __device__ __forceinline__ void mac96(u32& lo, u32& mid, u32& hi, u32 x, u32 y) 
         : "r"(x), "r"(y));
 }
 
-// Limits of school_cta: columns (na + nb) and threads, and its shared memory
-// in words: both operands (b padded by up to seven words) and three words of
-// every column sum, from each of the parts the terms are split into.
-constexpr int SCHOOL_MAX_COLS = 256, SCHOOL_THREADS = 128, SCHOOL_WARPS_CTA = SCHOOL_THREADS / 32;
-__host__ __device__ constexpr int school_parts(int nc) {
-    return nc <= 128 ? SCHOOL_WARPS_CTA : SCHOOL_WARPS_CTA / 2;  // warps per block of 128 columns
-}
-constexpr int SCHOOL_SMEM_WORDS = SCHOOL_MAX_COLS + 12 + 3 * 128 * SCHOOL_WARPS_CTA;
+// Limits of school_product: columns (na + nb), and its shared memory in words
+// per product: both operands (b padded by up to seven words), and from W > 1
+// warps three words of every column sum of each.
+constexpr int SCHOOL_MAX_COLS = 128, SCHOOL_WARPS_CTA = 4, SCHOOL_THREADS = 32 * SCHOOL_WARPS_CTA;
+template <int W>
+constexpr int SCHOOL_SMEM_WORDS = SCHOOL_MAX_COLS + 12 + (W > 1 ? 3 * SCHOOL_MAX_COLS * W : 0);
 
-// out[0, na + nb) = a * b and *out_len = its trimmed length (when out_len is
-// not null), by the SCHOOL_THREADS threads of the block. `smem`:
-// SCHOOL_SMEM_WORDS words; `st`: one CState per warp.
-static __device__ __forceinline__ void school_cta(const u32* __restrict__ a, u64 na, const u32* __restrict__ b, u64 nb,
-                                                  u32* __restrict__ out, unsigned long long* out_len, u32* smem,
-                                                  CState* st, unsigned long long* s_top) {
-    constexpr int T = SCHOOL_THREADS;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int la = (int)na, lb = (int)nb, nc = la + lb;
-    const int parts = school_parts(nc), pstride = 3 * nc;
+// Exclusive scan of carry functions over a warp (nothing valid on lane 0).
+__device__ __forceinline__ CState warp_scan_carry(CState st, int lane) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const CState o = cs_shfl_up(st, off);
+        if (lane >= off) st = cs_then(o, st);
+    }
+    return cs_shfl_up(st, 1);
+}
+
+// out[0, na + nb) = a * b by W warps (one, or the whole block); returns its
+// trimmed length, on lane 0 of each warp. `smem`: SCHOOL_SMEM_WORDS<W> words
+// of the product; `st`, `s_top`: one per warp, and one, of the block (W > 1).
+//
+// Column sums: lane l takes the four columns at 4l and warp w a W-th of the
+// range of i (one product alone on one warp stepped through up to 128
+// dependent iterations); terms outside a lane's own range read b as zero, so
+// the loop is warp-uniform. Window w[c] = b[k0 + c - i] slides down a limb a
+// step.
+template <int W>
+static __device__ __forceinline__ unsigned long long school_product(const u32* __restrict__ a, int la,
+                                                                    const u32* __restrict__ b, int lb,
+                                                                    u32* __restrict__ out, u32* smem, CState* st,
+                                                                    unsigned long long* s_top) {
+    constexpr int T = 32 * W;
+    const int t = threadIdx.x % T, lane = t & 31, warp = t >> 5, nc = la + lb;
     // b is stored as four interleaved quarter arrays, b[j] at (j & 3) * qb +
     // (j >> 2), so that lanes reading b[k0 + c - i] with k0 = 4 * lane read
     // consecutive words.
     const int qb = (lb + 3) / 4 + 1;
     u32* sa = smem;
     u32* sb = sa + la;
-    u32* cs = sb + 4 * qb;  // part p's column sums: cs[p * 3 nc + w * nc + column]
+    u32* cs = sb + 4 * qb;  // warp p's column sums: cs[(3 p + word) * nc + column]
     for (int i = t; i < la; i += T) sa[i] = __ldg(a + i);
     for (int j = t; j < lb; j += T) sb[(j & 3) * qb + (j >> 2)] = __ldg(b + j);
-    if (t == 0) *s_top = 0;
-    __syncthreads();
+    if (W > 1 && t == 0) *s_top = 0;
+    if constexpr (W > 1) __syncthreads();
+    else __syncwarp();
 
-    // Column sums. A warp takes a block of 128 consecutive columns, lane l the
-    // four at k0 = K0 + 4l, and a part of the block's range of i (the parts
-    // side by side on the block's warps: one warp alone stepped through up to
-    // 128 dependent iterations); terms outside a lane's own range read b as
-    // zero, so the loop is warp-uniform. Window w[c] = b[k0 + c - i] slides
-    // down a limb a step.
+    u32 lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
     {
-        const int part = warp % parts, K0 = 128 * (warp / parts);
-        const int k0 = K0 + 4 * lane;
-        const int lo_i = K0 - lb + 1 > 0 ? K0 - lb + 1 : 0;
-        const int hi_i = K0 + 127 < la - 1 ? K0 + 127 : la - 1;
-        const int cnt = hi_i >= lo_i ? hi_i - lo_i + 1 : 0, per = (cnt + parts - 1) / parts;
-        const int i0 = lo_i + part * per, i1 = i0 + per - 1 < hi_i ? i0 + per - 1 : hi_i;
-        u32 lo[4] = {0, 0, 0, 0}, mid[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+        const int k0 = 4 * lane, per = (la + W - 1) / W;
+        const int i0 = warp * per, i1 = i0 + per < la ? i0 + per : la;
         u32 w[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int j = k0 + c - i0;
             w[c] = (j >= 0 && j < lb) ? sb[(j & 3) * qb + (j >> 2)] : 0u;
         }
-        for (int i = i0; i <= i1; ++i) {
+        for (int i = i0; i < i1; ++i) {
             const u32 x = sa[i];
 #pragma unroll
             for (int c = 0; c < 4; ++c) mac96(lo[c], mid[c], hi[c], x, w[c]);
@@ -82,69 +86,70 @@ static __device__ __forceinline__ void school_cta(const u32* __restrict__ a, u64
             const int j = k0 - i - 1;
             w[0] = (j >= 0 && j < lb) ? sb[(j & 3) * qb + (j >> 2)] : 0u;
         }
-        u32* c0 = cs + part * pstride;
+    }
+
+    // Carries: a thread owns CPT >= 2 consecutive columns, so that a carry in
+    // (< 2^45) changes a range's carry out by at most one; columns from nc on
+    // are zero.
+    constexpr int CPT = W > 1 ? 2 : 4;
+    const int k_beg = CPT * t;
+    u32 limb[CPT];
+    u64 carry = 0;
+    if constexpr (W > 1) {
+        u32* c0 = cs + 3 * warp * nc + 4 * lane;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if (k0 + c < nc) {
-                c0[k0 + c] = lo[c];
-                c0[nc + k0 + c] = mid[c];
-                c0[2 * nc + k0 + c] = hi[c];
+            if (4 * lane + c < nc) {
+                c0[c] = lo[c];
+                c0[nc + c] = mid[c];
+                c0[2 * nc + c] = hi[c];
             }
         }
+        __syncthreads();
     }
-    __syncthreads();
-
-    // Carries: thread t owns two consecutive columns, so that a carry in
-    // (< 2^45) changes a range's carry out by at most one. Its limbs with no
-    // carry in and its carry function f(c) = h + [c >= th]. Only the last
-    // non-empty range can be one limb long, and only empty ranges, whose
-    // functions nothing uses, follow it.
-    static_assert(2 * T >= SCHOOL_MAX_COLS, "two columns per thread");
-    const int k_beg = 2 * t, n_own = k_beg + 2 <= nc ? 2 : (k_beg < nc ? 1 : 0);
-    u32 limb[2] = {0, 0};
-    u64 carry = 0;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        if (m < n_own) {
-            const int k = k_beg + m;
-            u64 s0 = 0, s1 = 0, s2 = 0;
-            for (int p = 0; p < parts; ++p) {
-                const u32* c0 = cs + p * pstride + k;
-                s0 += c0[0];
-                s1 += c0[nc];
-                s2 += c0[2 * nc];
-            }
-            s0 += carry;  // carry < 2^45: column sums are below 2^76
-            limb[m] = (u32)s0;
-            carry = (s0 >> 32) + s1 + (s2 << 32);
+    for (int c = 0; c < CPT; ++c) {
+        u64 s0 = 0, s1 = 0, s2 = 0;
+        if constexpr (W > 1) {
+            if (k_beg + c < nc)
+                for (int p = 0; p < W; ++p) {
+                    const u32* c0 = cs + 3 * p * nc + k_beg + c;
+                    s0 += c0[0];
+                    s1 += c0[nc];
+                    s2 += c0[2 * nc];
+                }
+        } else {
+            s0 = lo[c], s1 = mid[c], s2 = hi[c];
+        }
+        s0 += carry;  // carry < 2^45: column sums are below 2^76
+        limb[c] = (u32)s0;
+        carry = (s0 >> 32) + s1 + (s2 << 32);
+    }
+    const CState f = group_state<CPT>(limb, carry);
+    bool has = lane > 0;
+    CState ex;
+    if constexpr (W > 1) {
+        CState agg;
+        ex = block_scan_carry(f, &has, &agg, st);
+    } else {
+        ex = warp_scan_carry(f, lane);
+    }
+    group_add_carry<CPT>(limb, has ? cs_eval(ex, 0) : 0);
+    unsigned top = 0;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+        if (k_beg + c < nc) {
+            out[k_beg + c] = limb[c];
+            if (limb[c]) top = k_beg + c + 1;
         }
     }
-    CState f{carry, CS_NEVER};
-    const u64 dl = (u64)limb[0] | ((u64)limb[1] << 32);
-    if (n_own == 2 && dl != 0) {
-        const u64 tt = 0ull - dl;  // 2^64 less the two limbs
-        if (tt < (1ull << 62)) f.t = tt;
+    top = __reduce_max_sync(0xFFFFFFFFu, top);
+    if constexpr (W > 1) {
+        if (lane == 0 && top) atomicMax(s_top, (unsigned long long)top);
+        __syncthreads();
+        return *s_top;
     }
-    bool has;
-    CState agg;
-    const CState ex = block_scan_carry(f, &has, &agg, st);
-    u64 cin = has ? cs_eval(ex, 0) : 0;
-    // Add the carry in and store; the carry out of the range is f(cin).
-    unsigned long long top = 0;
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        if (m < n_own) {
-            const u64 s0 = (u64)limb[m] + (cin & 0xFFFFFFFFull);
-            const u32 v = (u32)s0;
-            cin = (cin >> 32) + (s0 >> 32);
-            out[k_beg + m] = v;
-            if (v) top = (unsigned long long)(k_beg + m) + 1;
-        }
-    }
-    const unsigned any = __ballot_sync(0xFFFFFFFFu, top != 0);
-    if (any && lane == 31 - __clz(any)) atomicMax(s_top, top);
-    __syncthreads();
-    if (t == 0 && out_len) *out_len = *s_top;
+    return top;
 }
 
 }  // namespace b2m

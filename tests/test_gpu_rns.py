@@ -151,3 +151,40 @@ def test_served_lengths_belong_to_their_requests(b2m_gpu):
                 srv.release(t)
     finally:
         srv.stop()
+
+
+# lengths of 2^7 (schoolbook) to 2^12 points: the longest, the shortest,
+# unbalanced, and operands longer than half of the length
+ONE_LAUNCH = [
+    [(1, 1), (64, 64), (1, 127), (127, 1), (33, 2), (3, 5), (100, 28), (31, 32)],
+    [(128, 128), (65, 64), (255, 1), (1, 200), (130, 100)],
+    [(256, 256), (129, 128), (511, 1), (200, 150), (3, 300)],
+    [(512, 512), (257, 256), (1, 1023), (700, 300), (600, 60)],
+    [(1024, 1024), (513, 512), (2047, 1), (1500, 400), (90, 1300)],
+    [(2048, 2048), (1025, 1024), (1, 4095), (3000, 1000), (4000, 90)],
+]
+
+
+@pytest.mark.parametrize("sizes", ONE_LAUNCH)
+@pytest.mark.parametrize("njobs", [1, 63, 64, 255, 511, 514])
+def test_batches_of_one_launch_products_match_oracle(b2m_gpu, sizes, njobs):
+    """On either side of the counts at which a batch takes another kernel."""
+    torch = pytest.importorskip("torch")
+    ops = [(gen_operand(5 * i + na, na, kind), gen_operand(7 * i + nb, nb, kind))
+           for i, (na, nb) in enumerate(sizes) for kind in (0, 1)]
+    dev = [(_dev(torch, a), _dev(torch, b)) for a, b in ops]
+    want = [oracle.mul_port(a, b) for a, b in ops]
+    jobs, outs = [], []
+    lens = torch.full((njobs,), -1, dtype=torch.int64, device="cuda")
+    for j in range(njobs):
+        a, b = dev[j % len(ops)]
+        na, nb = a.numel(), b.numel()
+        outs.append(torch.full((na + nb + 1,), -1, dtype=torch.int32, device="cuda"))
+        jobs.append((a.data_ptr(), na, b.data_ptr(), nb, outs[j].data_ptr(), na + nb, lens[j:].data_ptr()))
+    b2m_gpu.mul_batch(jobs, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    lens = lens.cpu().numpy()
+    for j, o in enumerate(outs):
+        w, got = want[j % len(ops)], o.cpu().numpy().view(np.uint32)
+        assert lens[j] == w.size and np.array_equal(got[:w.size], w)
+        assert not got[w.size:-1].any() and got[-1] == 0xFFFFFFFF
