@@ -253,26 +253,42 @@ __global__ void __launch_bounds__(AS_T) k_as_apply(const u32* A, u64 la, const u
 }
 
 // Device words of a call's publishing kernels, all zero between kernels: the
-// last block of a kernel to finish publishes and zeroes them again.
+// last block of a kernel to finish zeroes them again.
 struct PubState {
     unsigned long long top;
-    u32 done, ticket, carry, pad;
+    u32 done, ticket, carry, early;
 };
 
 // All threads of the block: `top` is the thread's candidate for the trimmed
-// length. The last block publishes (length, carry).
-__device__ __forceinline__ void publish_top(unsigned long long top, PubState* st, unsigned nblocks, LookbackSlot* slots,
-                                            const HostLen& hl) {
+// length; (length, *word) is published, word null for none. A block whose top
+// lies above `last` -- the elements from there on are its own -- has the
+// length, and publishes without waiting for the others; without such a block
+// (the result is short) the last one to finish does. The host launches the
+// next step meanwhile, and that is ordered by the stream. Waiting for all
+// blocks, a chain of three atomics and two fences, cost a step of a
+// 400,003 / 200,001-limb division about 2 us.
+__device__ __forceinline__ void publish_top(unsigned long long top, u64 last, const u32* word, PubState* st,
+                                            unsigned nblocks, LookbackSlot* slots, const HostLen& hl) {
     __shared__ bool s_last;
+    __shared__ unsigned long long s_tops[32];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
         top = o > top ? o : top;
     }
-    if ((threadIdx.x & 31) == 0 && top) atomicMax(&st->top, top);
-    __threadfence();
+    if ((threadIdx.x & 31) == 0) s_tops[threadIdx.x >> 5] = top;
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&st->done, 1u) == nblocks - 1;
+    if (threadIdx.x == 0) {
+        for (unsigned w = 1; w < blockDim.x / 32; ++w) top = s_tops[w] > top ? s_tops[w] : top;
+        if (top > last) {
+            publish(hl, top, word ? *(volatile const u32*)word : 0);
+            st->early = 1;
+        } else if (top) {
+            atomicMax(&st->top, top);
+        }
+        __threadfence();
+        s_last = atomicAdd(&st->done, 1u) == nblocks - 1;
+    }
     __syncthreads();
     if (!s_last) return;
     if (slots)
@@ -280,21 +296,19 @@ __device__ __forceinline__ void publish_top(unsigned long long top, PubState* st
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned long long t = atomicMax(&st->top, 0ull);
-        const u32 c = *(volatile u32*)&st->carry;
+        if (!*(volatile u32*)&st->early) publish(hl, t, word ? *(volatile const u32*)word : 0);
         st->top = 0;
-        st->done = st->ticket = st->carry = 0;
-        publish(hl, t, c);
+        st->done = st->ticket = st->carry = st->early = 0;
     }
 }
 
 // `limb` (may be null): a limb published beside the length.
 __global__ void k_top_pub(const u32* __restrict__ a, u64 n, const u32* limb, PubState* st, const HostLen hl) {
     pdl_enter();
-    if (limb && blockIdx.x == 0 && threadIdx.x == 0) st->carry = *limb;
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
         if (a[k]) t = k + 1;
-    publish_top(t, st, gridDim.x, nullptr, hl);
+    publish_top(t, (n - 1) / blockDim.x * blockDim.x, limb, st, gridDim.x, nullptr, hl);
 }
 
 __global__ void k_limb_pub(const u32* a, u64 k, const HostLen hl) {
@@ -364,7 +378,7 @@ __global__ void __launch_bounds__(AS_T) k_addsub_pub(const u32* A, u64 a_off, u6
         if (r) top = k + 1;
     }
     if (chunk == gridDim.x - 1 && threadIdx.x == 0) st->carry = tot.g | (tot.p & cin);
-    publish_top(top, st, gridDim.x, gridDim.x > 1 ? slots : nullptr, hl);
+    publish_top(top, (u64)(gridDim.x - 1) * AS_CH, &st->carry, st, gridDim.x, gridDim.x > 1 ? slots : nullptr, hl);
 }
 
 // out[k] = (a * 2^(32*wl + bits))[k], k < nout (bits in [0, 32)); publishes
@@ -380,7 +394,7 @@ __global__ void k_shl(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* 
         out[k] = v;
         if (v) t = k + 1;
     }
-    publish_top(t, st, gridDim.x, nullptr, hl);
+    publish_top(t, (nout - 1) / blockDim.x * blockDim.x, nullptr, st, gridDim.x, nullptr, hl);
 }
 
 // out[k] = floor(a / 2^(32*wl + bits))[k], k < nout (bits in [0, 32));
@@ -396,7 +410,7 @@ __global__ void k_shr(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* 
         out[k] = v;
         if (v) t = k + 1;
     }
-    publish_top(t, st, gridDim.x, nullptr, hl);
+    publish_top(t, (nout - 1) / blockDim.x * blockDim.x, nullptr, st, gridDim.x, nullptr, hl);
 }
 
 inline unsigned grid_for(uint64_t n, unsigned threads = 256) {

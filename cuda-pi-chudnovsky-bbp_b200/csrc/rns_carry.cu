@@ -130,7 +130,12 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
 #pragma unroll
         for (int w = 0; w < CARRY_THREADS / 32; ++w) top = s_top[w] > top ? s_top[w] : top;
         if (top) atomicMax(out_len, top);
-        if (hl.host) {  // a single product: the last block to finish publishes the length
+        // A single product: the block of the last limbs publishes the length
+        // (and the host launches what follows, in stream order) unless those
+        // are zero; then the last block to finish does.
+        if (hl.host && top > (nout - 1) / (CARRY_THREADS * RCARRY_G) * (CARRY_THREADS * RCARRY_G)) {
+            publish(hl, top);
+        } else if (hl.host) {
             __threadfence();
             if (atomicAdd(ticket + 1, 1u) == nchunks - 1) publish(hl, atomicMax(out_len, 0ull));
         }
