@@ -280,7 +280,7 @@ struct RnsCrt {
     uint2 kap[3];   // (scale * P / p_i)^-1 mod p_i
     u32 qlo[3], qhi[3];  // P / p_i
 };
-cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
+cudaError_t rns_launch_carry(cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                              const ProdJob* jobs, unsigned njobs, const RnsCrt& crt, HostLen hl = {});
 // v: columns per thread (1; or 2 up to logr = 8)

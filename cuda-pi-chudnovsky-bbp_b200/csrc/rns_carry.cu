@@ -18,8 +18,9 @@
 
 namespace b2m {
 
+constexpr int CHUNK = CARRY_CHUNK / 2;  // limbs per block
 constexpr int RCARRY_G = 8;  // digits per thread: CARRY_CHUNK / 2 limbs per CTA, as ntt_carry.cu
-static_assert(CARRY_THREADS * RCARRY_G * 2 == CARRY_CHUNK, "one lookback slot per 2048 limbs");
+static_assert(CARRY_THREADS * RCARRY_G == CHUNK, "one lookback slot per 2048 limbs");
 
 // One digit from its residues: c + carry -> limb and the new carry.
 __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& carry) {
@@ -33,7 +34,7 @@ __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& car
 }
 
 __global__ void __launch_bounds__(CARRY_THREADS, 6)
-    k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout, u32 nchunks,
+    k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout,
                 LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                 const ProdJob* __restrict__ jobs, const RnsCrt crt, const HostLen hl) {
     pdl_enter();
@@ -54,6 +55,8 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
     if (threadIdx.x == 0) s_chunk = atomicAdd(ticket, 1u);
     __syncthreads();
     const u32 chunk = s_chunk;
+    // digits from na + nb on are zero: no block for them alone
+    const u32 nchunks = (u32)((nout + CHUNK - 1) / CHUNK);
     if (chunk >= nchunks) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const u64 base = ((u64)chunk * CARRY_THREADS + threadIdx.x) * RCARRY_G;
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
         // A single product: the block of the last limbs publishes the length
         // (and the host launches what follows, in stream order) unless those
         // are zero; then the last block to finish does.
-        if (hl.host && top > (nout - 1) / (CARRY_THREADS * RCARRY_G) * (CARRY_THREADS * RCARRY_G)) {
+        if (hl.host && top > (u64)(nchunks - 1) * CHUNK) {
             publish(hl, top);
         } else if (hl.host) {
             __threadfence();
@@ -142,12 +145,13 @@ __global__ void __launch_bounds__(CARRY_THREADS, 6)
     }
 }
 
-cudaError_t rns_launch_carry(unsigned nchunks, cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
+cudaError_t rns_launch_carry(cudaStream_t s, const u32* coef, u64 nt, u32* out, u64 nout,
                              LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                              const ProdJob* jobs, unsigned njobs, const RnsCrt& crt, HostLen hl) {
-    if (nchunks == 0 || njobs == 0) return cudaSuccess;
-    return launch_pdl(k_rns_carry, dim3(nchunks, njobs), CARRY_THREADS, 0, s, coef, nt, out, nout, nchunks, slots, ticket,
-                      out_len, err, jobs, crt, hl);
+    const u64 n = jobs ? nt : nout;
+    if (n == 0 || njobs == 0) return cudaSuccess;
+    return launch_pdl(k_rns_carry, dim3((unsigned)((n + CHUNK - 1) / CHUNK), njobs), CARRY_THREADS, 0, s, coef, nt, out,
+                      nout, slots, ticket, out_len, err, jobs, crt, hl);
 }
 
 }  // namespace b2m

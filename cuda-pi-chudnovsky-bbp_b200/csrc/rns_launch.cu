@@ -517,7 +517,7 @@ struct RnsRun {
     cudaError_t carry(u32* out, u64 nout, LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
                       HostLen hl = {}) {
         if (tr) tr->mark(s, B2M_K_CARRY, 0);
-        return rns_launch_carry((unsigned)(a.nt / (CARRY_CHUNK / 2)), s, a.bufB, a.nt, out, nout, slots, ticket,
+        return rns_launch_carry(s, a.bufB, a.nt, out, nout, slots, ticket,
                                 out_len, err, a.jobs, njobs, shape_const(sh).crt, hl);
     }
 };
