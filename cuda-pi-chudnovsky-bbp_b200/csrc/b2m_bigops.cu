@@ -983,7 +983,11 @@ __device__ u32 cta_addsub(const u32* A, u64 la, const u32* B, u64 lb, u32 bsmall
         if (threadIdx.x == 0) *s_carry = tot.g | (tot.p & cin_chunk);
         __syncthreads();
     }
-    return *s_carry;
+    // every thread has read the carry before the next call clears it: callers
+    // branch on it, and then meet barriers
+    const u32 carry = *s_carry;
+    __syncthreads();
+    return carry;
 }
 
 // One CTA per node i: R = V_i - U_i (U_i = q~_i P), then q~ and R move one
