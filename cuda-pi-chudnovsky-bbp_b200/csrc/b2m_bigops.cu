@@ -990,46 +990,61 @@ __device__ u32 cta_addsub(const u32* A, u64 la, const u32* B, u64 lb, u32 bsmall
     return carry;
 }
 
+// A >= B over n limbs, by the CTA: from the top, a limb a thread, until some
+// limb differs (nearly always in the first round).
+__device__ bool cta_ge(const u32* A, const u32* B, u64 n) {
+    __shared__ u32 s_key;
+    for (u64 hi = n; hi > 0; hi -= hi < blockDim.x ? hi : (u64)blockDim.x) {
+        const u32 x = threadIdx.x < hi ? A[hi - 1 - threadIdx.x] : 0u, y = threadIdx.x < hi ? B[hi - 1 - threadIdx.x] : 0u;
+        if (threadIdx.x == 0) s_key = 0xFFFFFFFFu;
+        if (__syncthreads_or(x != y)) {
+            if (x != y) atomicMin(&s_key, 2 * threadIdx.x + (x > y));
+            __syncthreads();
+            return s_key & 1;
+        }
+    }
+    return true;
+}
+
 // One CTA per node i: R = V_i - U_i (U_i = q~_i P), then q~ and R move one
 // unit at a time until 0 <= R < P; writes q (node 2i) and R (node 2i + 1) of
-// the next level, zero-padded to its stride. A correction count above the
-// bound sets bit 2 of *err (reported as an internal error).
+// the next level, zero-padded to its stride sout >= n. q~ is within a few
+// units of the quotient, so R lies within 64 P of zero and its n limbs and
+// one more, in two's complement, hold it: the upper half of V - U is not
+// formed. A correction count above the bound sets bit 2 of *err (reported as
+// an internal error).
+// What bounds it: the chain of rounds of 8192 limbs, one CTA a node. Four
+// nodes of 13,000 limbs take 25 us, and took 69 over all limbs of V - U, with
+// R - P formed to see its sign and the results copied to their place.
 __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restrict__ U, u64 su,
-                         const u32* __restrict__ QE, u64 nq, const u32* __restrict__ P, u64 n, u32* scr, u64 w,
-                         u32* __restrict__ out, u64 sout, u32* err) {
+                         const u32* __restrict__ QE, u64 nq, const u32* __restrict__ P, u64 n, u32* out, u64 sout,
+                         u32* err) {
     pdl_enter();
     __shared__ GP ws[33];
     __shared__ u32 s_carry;
     const u64 i = blockIdx.x;
     V += i * sin;
     U += i * su;
-    u32* R = scr + i * (2 * w + nq + 1);
-    u32* T = R + w;
-    u32* Q = T + w;  // nq + 1 limbs
-    for (u64 k = threadIdx.x; k <= nq; k += blockDim.x) Q[k] = k < nq ? QE[i * nq + k] : 0u;
-    __syncthreads();
-    u32 neg = cta_addsub(V, sin, U, su, 0, R, w, 1, ws, &s_carry);
+    u32* Q = out + 2 * i * sout;
+    u32* R = Q + sout;
+    for (u64 k = threadIdx.x; k < sout; k += blockDim.x) {
+        Q[k] = k < n && k < nq ? QE[i * nq + k] : 0u;
+        if (k >= n) R[k] = 0;
+    }
+    u32 top = (n < sin ? V[n] : 0u) - (n < su ? U[n] : 0u);
+    top -= cta_addsub(V, sin, U, su, 0, R, n, 1, ws, &s_carry);
     int it = 0;
-    while (neg && it < 64) {
-        if (cta_addsub(R, w, P, n, 0, R, w, 0, ws, &s_carry)) neg = 0;
-        cta_addsub(Q, nq + 1, nullptr, 0, 1, Q, nq + 1, 1, ws, &s_carry);
+    while ((int)top < 0 && it < 64) {
+        top += cta_addsub(R, n, P, n, 0, R, n, 0, ws, &s_carry);
+        cta_addsub(Q, n, nullptr, 0, 1, Q, n, 1, ws, &s_carry);
         ++it;
     }
-    while (it < 64) {
-        if (cta_addsub(R, w, P, n, 0, T, w, 1, ws, &s_carry)) break;
-        u32* t = R;
-        R = T;
-        T = t;
-        cta_addsub(Q, nq + 1, nullptr, 0, 1, Q, nq + 1, 0, ws, &s_carry);
+    while (it < 64 && (top || cta_ge(R, P, n))) {
+        top -= cta_addsub(R, n, P, n, 0, R, n, 1, ws, &s_carry);
+        cta_addsub(Q, n, nullptr, 0, 1, Q, n, 0, ws, &s_carry);
         ++it;
     }
     if (it >= 64 && threadIdx.x == 0) atomicOr(err, 2u);
-    u32* oq = out + (2 * i) * sout;
-    u32* orr = out + (2 * i + 1) * sout;
-    for (u64 k = threadIdx.x; k < sout; k += blockDim.x) {
-        oq[k] = k < n ? Q[k] : 0u;
-        orr[k] = k < n ? R[k] : 0u;
-    }
 }
 
 // One thread per leaf (a value below 10^72 in 8 limbs): 72 decimal digits.
@@ -1093,10 +1108,11 @@ void fix_node_grid(Scope& S, const u32* V, uint64_t sin, const u32* U, uint64_t 
     ck(cudaMemcpyAsync(orr, R.p, 4 * std::min(k, R.n), cudaMemcpyDeviceToDevice, S.s()), "D2D");
 }
 
-// Levels with at most this many nodes, of at least DC_GRID_MIN_LIMBS limbs,
-// fix their nodes with grid-wide passes (fix_node_grid).
-constexpr uint64_t DC_GRID_MAX_NODES = 16;
-constexpr uint64_t DC_GRID_MIN_LIMBS = 1 << 15;
+// Levels whose V - U has at least this many limbs per node, times the number
+// of nodes, fix them with grid-wide passes (fix_node_grid), one node after the
+// other at about 45 us each; k_dc_fix takes all nodes of a level side by side
+// at about 1.5 us per 2,000 limbs.
+constexpr uint64_t DC_GRID_MIN_LIMBS = 1 << 16;
 
 // -1, 0, 1 as a <, ==, > b (trimmed).
 int cmp(Scope& S, DV a, DV b) {
@@ -1168,7 +1184,7 @@ std::string to_decimal(Scope& S, DV X) {
         const uint64_t sout = j - 1 > DC_LEAF_J ? 2 * P[j - 1].n : DC_LEAF_LIMBS;
         DV out = S.vec(2 * m * sout);
         const uint64_t w = std::max(sin, su) + 1;
-        if (m <= DC_GRID_MAX_NODES && w >= DC_GRID_MIN_LIMBS) {
+        if (w >= DC_GRID_MIN_LIMBS * m) {
             DV R = S.vec(w), T = S.vec(w), Q = S.vec(nq + 1);
             DV one = S.vec(1);
             static const u32 one_h = 1;
@@ -1177,11 +1193,10 @@ std::string to_decimal(Scope& S, DV X) {
                 fix_node_grid(S, in.p + i * sin, sin, U.p + i * su, su, qe.p + i * nq, nq, Pj, R, T, Q, one,
                               out.p + (2 * i) * sout, out.p + (2 * i + 1) * sout, sout);
         } else {
-            DV scr = S.vec(m * (2 * w + nq + 1));
             unsigned threads = 32;
-            while (threads < 1024 && (uint64_t)threads * ADD_LPT < w) threads <<= 1;
-            ck(launch_pdl(k_dc_fix, (unsigned)m, threads, 0, S.s(), in.p, sin, U.p, su, qe.p, nq, Pj.p, n, scr.p, w,
-                          out.p, sout, err),
+            while (threads < 1024 && (uint64_t)threads * ADD_LPT < n) threads <<= 1;
+            ck(launch_pdl(k_dc_fix, (unsigned)m, threads, 0, S.s(), in.p, sin, U.p, su, qe.p, nq, Pj.p, n, out.p, sout,
+                          err),
                "k_dc_fix");
         }
         in = out;
