@@ -161,96 +161,7 @@ private:
 };
 
 // ---------------------------------------------------------------------------- kernels
-__global__ void k_top(const u32* __restrict__ a, u64 n, unsigned long long* out) {
-    unsigned long long t = 0;
-    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
-        if (a[k]) t = k + 1;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, t, off);
-        t = o > t ? o : t;
-    }
-    if ((threadIdx.x & 31) == 0 && t) atomicMax(out, t);
-}
-
 constexpr int AS_T = 256, AS_L = ADD_LPT, AS_CH = AS_T * AS_L;  // limbs per block
-
-__device__ __forceinline__ GP limb_gp(u32 a, u32 b, int sub) {
-    if (!sub) {
-        const u64 s = (u64)a + b;
-        return {(u32)(s >> 32), (u32)((u32)s == 0xFFFFFFFFu)};
-    }
-    return {(u32)(a < b), (u32)(a == b)};
-}
-
-// Carry / borrow (generate, propagate) of each block's limbs.
-__global__ void __launch_bounds__(AS_T) k_as_reduce(const u32* __restrict__ A, u64 la, const u32* __restrict__ B,
-                                                    u64 lb, u64 n, int sub, GP* __restrict__ agg) {
-    __shared__ GP ws[AS_T / 32 + 1];
-    const u64 base = (u64)blockIdx.x * AS_CH + (u64)threadIdx.x * AS_L;
-    GP g{0, 1};
-#pragma unroll
-    for (int w = 0; w < AS_L; ++w) {
-        const u64 k = base + w;
-        if (k < n) g = gp_then(g, limb_gp(k < la ? A[k] : 0u, k < lb ? B[k] : 0u, sub));
-    }
-    GP tot;
-    block_scan_gp(g, ws, &tot);
-    if (threadIdx.x == 0) agg[blockIdx.x] = tot;
-}
-
-// Carry into each block (all blocks' aggregates scanned in one CTA), and the
-// carry out of the top limb.
-__global__ void __launch_bounds__(1024) k_as_scan(const GP* __restrict__ agg, u64 nb, u32* __restrict__ cin,
-                                                  u32* __restrict__ cout) {
-    __shared__ GP ws[33];
-    GP acc{0, 1};
-    for (u64 c0 = 0; c0 < nb; c0 += blockDim.x) {
-        const u64 i = c0 + threadIdx.x;
-        GP tot;
-        const GP ex = block_scan_gp(i < nb ? agg[i] : GP{0, 1}, ws, &tot);
-        if (i < nb) cin[i] = gp_then(acc, ex).g;
-        acc = gp_then(acc, tot);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *cout = acc.g;
-}
-
-// out = A +- B (mod 2^(32n)); out may be A or B (each limb is read before it
-// is written, by the same thread).
-__global__ void __launch_bounds__(AS_T) k_as_apply(const u32* A, u64 la, const u32* B, u64 lb, u64 n, int sub,
-                                                   const u32* __restrict__ cin, u32* out) {
-    __shared__ GP ws[AS_T / 32 + 1];
-    const u64 base = (u64)blockIdx.x * AS_CH + (u64)threadIdx.x * AS_L;
-    u32 av[AS_L], bv[AS_L];
-    GP g{0, 1};
-#pragma unroll
-    for (int w = 0; w < AS_L; ++w) {
-        const u64 k = base + w;
-        av[w] = k < la && k < n ? A[k] : 0u;
-        bv[w] = k < lb && k < n ? B[k] : 0u;
-        if (k < n) g = gp_then(g, limb_gp(av[w], bv[w], sub));
-    }
-    GP tot;
-    const GP ex = block_scan_gp(g, ws, &tot);
-    u32 c = ex.g | (ex.p & cin[blockIdx.x]);
-#pragma unroll
-    for (int w = 0; w < AS_L; ++w) {
-        const u64 k = base + w;
-        if (k >= n) break;
-        u32 r;
-        if (!sub) {
-            const u64 s = (u64)av[w] + bv[w] + c;
-            r = (u32)s;
-            c = (u32)(s >> 32);
-        } else {
-            const u64 d = (u64)av[w] - bv[w] - c;
-            r = (u32)d;
-            c = (u32)((d >> 63) & 1);
-        }
-        out[k] = r;
-    }
-}
 
 // Device words of a call's publishing kernels, all zero between kernels: the
 // last block of a kernel to finish zeroes them again.
@@ -1255,50 +1166,6 @@ void put(Scope& S, DV v, uint32_t* dst, uint64_t cap, uint64_t* len) {
 }
 
 }  // namespace big
-
-// ---------------------------------------------------------------------------- launchers for other files
-namespace {
-__global__ void k_top_diff(const u32* __restrict__ a, const u32* __restrict__ b, u64 n, unsigned long long* out) {
-    unsigned long long t = 0;
-    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
-        if (a[k] != b[k]) t = k + 1;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, t, off);
-        t = o > t ? o : t;
-    }
-    if ((threadIdx.x & 31) == 0 && t) atomicMax(out, t);
-}
-}  // namespace
-
-uint64_t addsub_scratch_bytes(uint64_t n) {
-    const uint64_t nb = (n + big::AS_CH - 1) / big::AS_CH;
-    return ((nb * sizeof(GP) + 255) & ~255ull) + ((nb * 4 + 255) & ~255ull);
-}
-
-cudaError_t launch_addsub(const u32* a, uint64_t la, const u32* b, uint64_t lb, uint64_t n, int sub, u32* out,
-                          void* scratch, u32* flag, cudaStream_t s) {
-    if (n == 0) return cudaMemsetAsync(flag, 0, 4, s);
-    const uint64_t nb = (n + big::AS_CH - 1) / big::AS_CH;
-    GP* agg = static_cast<GP*>(scratch);
-    u32* cin = reinterpret_cast<u32*>(static_cast<unsigned char*>(scratch) + ((nb * sizeof(GP) + 255) & ~255ull));
-    big::k_as_reduce<<<(unsigned)nb, big::AS_T, 0, s>>>(a, la, b, lb, n, sub, agg);
-    big::k_as_scan<<<1, 1024, 0, s>>>(agg, nb, cin, flag);
-    big::k_as_apply<<<(unsigned)nb, big::AS_T, 0, s>>>(a, la, b, lb, n, sub, cin, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_top(const u32* a, uint64_t n, unsigned long long* out, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    big::k_top<<<big::grid_for(n), 256, 0, s>>>(a, n, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_top_diff(const u32* a, const u32* b, uint64_t n, unsigned long long* out, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_top_diff<<<big::grid_for(n), 256, 0, s>>>(a, b, n, out);
-    return cudaGetLastError();
-}
 
 }  // namespace b2m
 

@@ -28,6 +28,8 @@
 #include "b2m.h"
 #include "b2m_context.h"
 #include "b2m_internal.h"
+#include "carry.cuh"
+#include "carry_lookback.cuh"
 #include "gp_scan.cuh"
 #include "pdl.cuh"
 
@@ -233,23 +235,24 @@ __global__ void k_bs_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 sc
 }
 
 // ---------------------------------------------------------------------------- T = sx*X + sy*Y
-// One CTA per merge: T' = sign(TL)*X + sign(TR)*Y (X = TL*QR, Y = PL*TR).
-__global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln, u64 m2) {
-    pdl_enter();
-    __shared__ GP s_ws[33];
-    __shared__ u32 s_carry;
-    __shared__ unsigned long long s_top;
+// T' = sign(TL)*X + sign(TR)*Y (X = TL*QR, Y = PL*TR) as A + B or A - B with
+// |A| >= |B|: the operands, the limbs of the result at most (0: it is zero)
+// and its sign; and what the blocks of k_bs_add_wide share.
+struct SignedAdd {
+    const u32 *A, *B;
+    u64 la, lb, n;
+    int sub, sign;
+    u32 ticket, done;
+    unsigned long long top;
+};
+
+// Merge i's operation, by all threads of a block.
+__device__ SignedAdd signed_add_of(const ScratchXY& S, const int* __restrict__ sign_l, u64 i) {
     __shared__ long long s_diff;
-    const u64 i = blockIdx.x;
-    if (i >= m2) return;
     const u32* X = S.x + i * S.sx;
     const u32* Y = S.y + i * S.sy;
     u64 lx = S.lx[i], ly = S.ly[i];
-    int sx = sign_l[2 * i], sy = sign_l[2 * i + 1];
-    if (lx == 0) sx = 0;
-    if (ly == 0) sy = 0;
-    u32* out = Ln.limbs[2] + i * Ln.stride[2];
-    // Choose the operation: add (same signs), or big - small with big's sign.
+    const int sx = lx ? sign_l[2 * i] : 0, sy = ly ? sign_l[2 * i + 1] : 0;
     bool sub = false, swap = false;
     int sres;
     if (sx == 0) {
@@ -282,20 +285,34 @@ __global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_
             const long long d = s_diff;
             if (d >= 0) c = X[d] > Y[d] ? 1 : -1;
         }
-        if (c == 0) {  // exact cancellation
-            if (threadIdx.x == 0) {
-                Ln.len[2 * Ln.m + i] = 0;
-                Ln.sign[i] = 0;
-            }
-            return;
-        }
+        if (c == 0) return {};  // exact cancellation
         swap = c < 0;
         sres = swap ? sy : sx;
     }
-    const u32* A = swap ? Y : X;  // the larger magnitude when subtracting
-    const u32* B = swap ? X : Y;
-    const u64 la = swap ? ly : lx, lb = swap ? lx : ly;
-    const u64 n = (la > lb ? la : lb) + (sub ? 0 : 1);
+    SignedAdd r{};
+    r.A = swap ? Y : X;  // the larger magnitude when subtracting
+    r.B = swap ? X : Y;
+    r.la = swap ? ly : lx;
+    r.lb = swap ? lx : ly;
+    r.n = (r.la > r.lb ? r.la : r.lb) + (sub ? 0 : 1);
+    r.sub = sub;
+    r.sign = sres;
+    return r;
+}
+
+// One CTA per merge.
+__global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln, u64 m2) {
+    pdl_enter();
+    __shared__ GP s_ws[33];
+    __shared__ u32 s_carry;
+    __shared__ unsigned long long s_top;
+    const u64 i = blockIdx.x;
+    if (i >= m2) return;
+    u32* out = Ln.limbs[2] + i * Ln.stride[2];
+    const SignedAdd op = signed_add_of(S, sign_l, i);
+    const u32 *A = op.A, *B = op.B;
+    const u64 la = op.la, lb = op.lb, n = op.n;
+    const int sub = op.sub, sres = op.sign;
     if (threadIdx.x == 0) {
         s_carry = 0;
         s_top = 0;
@@ -311,14 +328,7 @@ __global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_
             const u64 k = base + w;
             av[w] = k < la ? A[k] : 0;
             bv[w] = k < lb ? B[k] : 0;
-            GP e;
-            if (!sub) {
-                const u64 s = (u64)av[w] + bv[w];
-                e = {(u32)(s >> 32), (u32)((u32)s == 0xFFFFFFFFu)};
-            } else {
-                e = {(u32)(av[w] < bv[w]), (u32)(av[w] == bv[w])};
-            }
-            g = gp_then(g, e);
+            g = gp_then(g, limb_gp(av[w], bv[w], sub));
         }
         GP tot;
         const GP ex = block_scan_gp(g, s_ws, &tot);
@@ -351,6 +361,107 @@ __global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_
     if (threadIdx.x == 0) {
         Ln.len[2 * Ln.m + i] = s_top;
         Ln.sign[i] = s_top ? sres : 0;
+    }
+}
+
+// The same for few long merges, as one pass over all SMs: k_bs_plan_add
+// chooses each merge's operation and zeroes its lookback slots, k_bs_add_wide
+// (a row of blocks per merge, 2048 limbs each) adds with the carry into a
+// block by decoupled lookback, as the carry kernels do, and its last block
+// writes length and sign.
+constexpr int ADD_T = 256, ADD_CH = ADD_T * ADD_LPT;
+
+__global__ void __launch_bounds__(ADD_T) k_bs_plan_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln,
+                                                       SignedAdd* ops, LookbackSlot* slots, u32 nch) {
+    pdl_enter();
+    const u64 i = blockIdx.x;
+    const SignedAdd op = signed_add_of(S, sign_l, i);
+    for (u32 k = threadIdx.x; k < nch; k += ADD_T) slots[i * nch + k].word = 0;
+    if (threadIdx.x == 0) {
+        ops[i] = op;
+        if (op.n == 0) {
+            Ln.len[2 * Ln.m + i] = 0;
+            Ln.sign[i] = 0;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(ADD_T) k_bs_add_wide(SignedAdd* ops, LevelView Ln, LookbackSlot* slots, u32 nch,
+                                                       u32* err) {
+    pdl_enter();
+    __shared__ GP s_ws[ADD_T / 32 + 1];
+    __shared__ u32 s_chunk, s_cin;
+    __shared__ unsigned long long s_tops[ADD_T / 32];
+    const u64 i = blockIdx.y;
+    SignedAdd* op = ops + i;
+    slots += i * nch;
+    const u32 *A = op->A, *B = op->B;
+    const u64 la = op->la, lb = op->lb, n = op->n;
+    const int sub = op->sub;
+    u32* out = Ln.limbs[2] + i * Ln.stride[2];
+    const u32 nchunks = (u32)((n + ADD_CH - 1) / ADD_CH);
+    if (threadIdx.x == 0) s_chunk = atomicAdd(&op->ticket, 1u);
+    __syncthreads();
+    const u32 chunk = s_chunk;
+    if (chunk >= nchunks) return;
+    const u64 base = (u64)chunk * ADD_CH + (u64)threadIdx.x * ADD_LPT;
+    u32 av[ADD_LPT], bv[ADD_LPT];
+    GP g{0, 1};
+#pragma unroll
+    for (int w = 0; w < ADD_LPT; ++w) {
+        const u64 k = base + w;
+        av[w] = k < la ? A[k] : 0u;
+        bv[w] = k < lb ? B[k] : 0u;
+        g = gp_then(g, limb_gp(av[w], bv[w], sub));
+    }
+    GP tot;
+    const GP ex = block_scan_gp(g, s_ws, &tot);
+    if (threadIdx.x < 32) {
+        // the block as a carry function: constant, or passing 0 and 1 through
+        const CState agg{tot.g, tot.p && !tot.g ? 1ull : CS_NEVER};
+        const u64 c = warp_lookback(slots, chunk, agg, err);
+        if (threadIdx.x == 0) {
+            if (agg.t != CS_NEVER) st_release(&slots[chunk].word, (cs_eval(agg, c) << 2) | SLOT_INCL);
+            s_cin = (u32)c;
+        }
+    }
+    __syncthreads();
+    u32 c = ex.g | (ex.p & s_cin);
+    unsigned long long top = 0;
+#pragma unroll
+    for (int w = 0; w < ADD_LPT; ++w) {
+        const u64 k = base + w;
+        u32 r;
+        if (!sub) {
+            const u64 s = (u64)av[w] + bv[w] + c;
+            r = (u32)s;
+            c = (u32)(s >> 32);
+        } else {
+            const u64 d = (u64)av[w] - bv[w] - c;
+            r = (u32)d;
+            c = (u32)((d >> 63) & 1);
+        }
+        if (k < n) {
+            out[k] = r;
+            if (r) top = k + 1;
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, top, off);
+        top = o > top ? o : top;
+    }
+    if ((threadIdx.x & 31) == 0) s_tops[threadIdx.x >> 5] = top;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < ADD_T / 32; ++w) top = s_tops[w] > top ? s_tops[w] : top;
+    if (top) atomicMax(&op->top, top);
+    __threadfence();
+    if (atomicAdd(&op->done, 1u) == nchunks - 1) {
+        __threadfence();
+        const unsigned long long t = atomicMax(&op->top, 0ull);
+        Ln.len[2 * Ln.m + i] = t;
+        Ln.sign[i] = t ? op->sign : 0;
     }
 }
 
@@ -437,99 +548,13 @@ static int ceil_log2(uint64_t x) {
     return l;
 }
 
+// Results of more than this many limbs are added by k_bs_add_wide: at two
+// rounds of one CTA, whose rounds follow each other, the two launches cost the
+// same (17 merges of 13,000 limbs 18 us either way, 9 of 26,000 34 against 14,
+// and 4 of 52,000, done one after the other from the host, 250).
+constexpr uint64_t BS_WIDE_MIN_LIMBS = 1 << 13;
+
 // One level: L (m nodes, max lengths mx) -> Ln.
-// k_bs_signed_add's operation as grid-wide passes driven from the host, for
-// levels of a few merges with up to millions of limbs (the top of the tree),
-// where one CTA a merge would leave the GPU idle. Reads each merge's lengths
-// and signs back, compares |X| and |Y| when it subtracts, and writes T's
-// magnitude, length and sign.
-constexpr uint64_t BS_GRID_MAX_MERGES = 8;
-constexpr uint64_t BS_GRID_MIN_LIMBS = 1 << 15;
-
-static cudaError_t signed_add_grid(Context* c, const ScratchXY& S, const int* sign_l, const LevelView& Ln,
-                                   uint64_t m2, uint64_t capT, cudaStream_t s) {
-    std::vector<u64> lx(m2), ly(m2);
-    std::vector<int> sg(2 * m2);
-    cudaError_t e = cudaMemcpyAsync(lx.data(), S.lx, 8 * m2, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ly.data(), S.ly, 8 * m2, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(sg.data(), sign_l, sizeof(int) * 2 * m2, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    const uint64_t sb = addsub_scratch_bytes(capT) + 256;
-    if (!budget_reserve(c, sb)) return cudaErrorMemoryAllocation;
-    void* scratch = nullptr;
-    if ((e = cudaMallocAsync(&scratch, sb, s)) != cudaSuccess) {
-        budget_release(c, sb);
-        return e;
-    }
-    unsigned long long* word = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(scratch) + sb - 256);
-    u32* flag = reinterpret_cast<u32*>(word + 1);
-    auto read_word = [&](unsigned long long* h) {
-        cudaError_t r = cudaMemcpyAsync(h, word, 8, cudaMemcpyDeviceToHost, s);
-        return r == cudaSuccess ? cudaStreamSynchronize(s) : r;
-    };
-    for (uint64_t i = 0; i < m2 && e == cudaSuccess; ++i) {
-        const u32* X = S.x + i * S.sx;
-        const u32* Y = S.y + i * S.sy;
-        uint64_t la = lx[i], lb = ly[i];
-        int sx = la ? sg[2 * i] : 0, sy = lb ? sg[2 * i + 1] : 0;
-        u32* out = Ln.limbs[2] + i * Ln.stride[2];
-        bool sub = false, swap = false, cancel = false;
-        int sres = 0;
-        if (sx == 0) {
-            sres = sy;
-            swap = true;
-            la = 0;
-        } else if (sy == 0) {
-            sres = sx;
-            lb = 0;
-        } else if (sx == sy) {
-            sres = sx;
-        } else {
-            sub = true;
-            int cmpv = 0;
-            if (la != lb) {
-                cmpv = la > lb ? 1 : -1;
-            } else {
-                unsigned long long d = 0;
-                if ((e = cudaMemsetAsync(word, 0, 8, s)) == cudaSuccess && (e = launch_top_diff(X, Y, la, word, s)) ==
-                    cudaSuccess)
-                    e = read_word(&d);
-                if (e == cudaSuccess && d) {
-                    u32 xv = 0, yv = 0;
-                    e = cudaMemcpyAsync(&xv, X + d - 1, 4, cudaMemcpyDeviceToHost, s);
-                    if (e == cudaSuccess) e = cudaMemcpyAsync(&yv, Y + d - 1, 4, cudaMemcpyDeviceToHost, s);
-                    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-                    cmpv = xv > yv ? 1 : -1;
-                }
-            }
-            if (cmpv == 0) cancel = true;  // exact cancellation (or an error, reported below)
-            swap = cmpv < 0;
-            sres = swap ? sy : sx;
-        }
-        if (e != cudaSuccess) break;
-        unsigned long long top = 0;
-        if (!cancel) {
-            const u32* A = swap ? Y : X;  // the larger magnitude when subtracting
-            const u32* B = swap ? X : Y;
-            const uint64_t na = swap ? lb : la, nb = swap ? la : lb;
-            const uint64_t n = std::max(na, nb) + (sub ? 0 : 1);
-            e = launch_addsub(A, na, B, nb, n, sub ? 1 : 0, out, scratch, flag, s);
-            if (e == cudaSuccess) e = cudaMemsetAsync(word, 0, 8, s);
-            if (e == cudaSuccess) e = launch_top(out, n, word, s);
-            if (e == cudaSuccess) e = read_word(&top);
-        }
-        const u64 len = top;
-        const int sign = top ? sres : 0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(Ln.len + 2 * Ln.m + i, &len, 8, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(Ln.sign + i, &sign, sizeof(int), cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // len and sign are stack values
-    }
-    cudaFreeAsync(scratch, s);
-    budget_release(c, sb);
-    return e;
-}
-
 static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx[3], LevelView* Ln, void** mem_n,
                                uint64_t* bytes_n, uint64_t* products, cudaStream_t s) {
     const uint64_t m = L.m, m2 = m / 2, mn = m2 + (m & 1);
@@ -543,7 +568,9 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
     // Scratch: X, Y and their lengths.
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     const uint64_t xb = al(m2 * capX * 4), yb = al(m2 * capY * 4), lb = al(2 * m2 * 8);
-    const uint64_t sbytes = xb + yb + lb;
+    const uint64_t nch = capT > BS_WIDE_MIN_LIMBS && m2 <= 65535 ? (capT + ADD_CH - 1) / ADD_CH : 0;
+    const uint64_t ab = nch ? al(m2 * sizeof(SignedAdd)) : 0, slb = al(m2 * nch * sizeof(LookbackSlot));
+    const uint64_t sbytes = xb + yb + lb + ab + slb;
     void* smem = nullptr;
     if (m2) {
         if (!budget_reserve(c, sbytes)) return cudaErrorMemoryAllocation;
@@ -654,8 +681,13 @@ static cudaError_t merge_level(Context* c, const LevelView& L, const uint64_t mx
         }
     }
     *products += 4 * m2;
-    if (e == cudaSuccess && m2 && m2 <= BS_GRID_MAX_MERGES && capT >= BS_GRID_MIN_LIMBS) {
-        e = signed_add_grid(c, S, L.sign, *Ln, m2, capT, s);
+    if (e == cudaSuccess && m2 && nch) {
+        SignedAdd* ops = reinterpret_cast<SignedAdd*>(static_cast<unsigned char*>(smem) + xb + yb + lb);
+        LookbackSlot* slots = reinterpret_cast<LookbackSlot*>(static_cast<unsigned char*>(smem) + xb + yb + lb + ab);
+        e = launch_pdl(k_bs_plan_add, (unsigned)m2, ADD_T, 0, s, S, L.sign, *Ln, ops, slots, (u32)nch);
+        if (e == cudaSuccess)
+            e = launch_pdl(k_bs_add_wide, dim3((unsigned)nch, (unsigned)m2), ADD_T, 0, s, ops, *Ln, slots, (u32)nch,
+                           c->d_err);
     } else if (e == cudaSuccess && m2) {
         const uint64_t maxn = capT;
         unsigned threads = 32;

@@ -16,6 +16,15 @@ struct GP {
 };
 __device__ __forceinline__ GP gp_then(GP lo, GP hi) { return {hi.g | (hi.p & lo.g), hi.p & lo.p}; }
 
+// One limb's pair, of a + b or (sub) a - b.
+__device__ __forceinline__ GP limb_gp(u32 a, u32 b, int sub) {
+    if (!sub) {
+        const u64 s = (u64)a + b;
+        return {(u32)(s >> 32), (u32)((u32)s == 0xFFFFFFFFu)};
+    }
+    return {(u32)(a < b), (u32)(a == b)};
+}
+
 constexpr int ADD_LPT = 8;  // limbs per thread
 
 // Exclusive block scan of GP (low threads first). blockDim multiple of 32.
