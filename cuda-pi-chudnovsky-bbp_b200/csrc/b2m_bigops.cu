@@ -19,7 +19,6 @@
 #include <chrono>
 #include <cstring>
 #include <exception>
-#include <string>
 #include <vector>
 
 #include "b2m.h"
@@ -985,6 +984,20 @@ __global__ void k_dc_leaf(const u32* __restrict__ nodes, u64 stride, u64 m, char
     }
 }
 
+// The n digits without their leading zeros: publishes how many are left, and
+// *err. n is a multiple of 8 and the digits are 8-byte aligned; block 0's
+// first words are the leading ones, and nearly always decide.
+__global__ void k_dc_count(const u64* __restrict__ digits, u64 n, const u32* err, PubState* st, const HostLen hl) {
+    pdl_enter();
+    unsigned long long t = 0;
+    for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n / 8 && !t; k += (u64)gridDim.x * blockDim.x) {
+        const u64 w = digits[k] ^ 0x3030303030303030ull;
+        if (w) t = n - (8 * k + (__ffsll((long long)w) - 1) / 8);
+    }
+    const u64 head = 8 * (u64)blockDim.x;
+    publish_top(t, n > head ? n - head : 0, err, st, gridDim.x, nullptr, hl);
+}
+
 // k_dc_fix's steps for one node as grid-wide passes driven from the host:
 // for the top levels, whose few nodes have up to millions of limbs, one CTA
 // a node would leave the GPU idle. R = V - U over w limbs, then R += P with
@@ -1032,9 +1045,19 @@ int cmp(Scope& S, DV a, DV b) {
     return d.carry ? -1 : (d.v.n ? 1 : 0);
 }
 
-// Decimal digits of trimmed X, no leading zeros ("0" for zero).
-std::string to_decimal(Scope& S, DV X) {
-    if (X.n == 0) return "0";
+// Decimal digits of trimmed X, no leading zeros ("0" for zero), left on the
+// device: callers copy them straight to where they are wanted (by way of
+// strings on the host ten million digits took 10 ms longer).
+struct Digits {
+    const char* d;  // on the device
+    uint64_t n;
+};
+Digits to_decimal(Scope& S, DV X) {
+    if (X.n == 0) {
+        char* z = static_cast<char*>(S.raw(1));
+        ck(cudaMemsetAsync(z, '0', 1, S.s()), "cudaMemsetAsync");
+        return {z, 1};
+    }
     std::vector<DV> P;  // P[j] = 10^(9 2^j)
     P.push_back(upload(S, {1000000000u}));
     P[0] = trim(S, P[0]);
@@ -1118,19 +1141,31 @@ std::string to_decimal(Scope& S, DV X) {
     const uint64_t digits = m * 9 * DC_LEAF_GROUPS;
     char* d_str = static_cast<char*>(S.raw(digits));
     ck(launch_pdl(k_dc_leaf, (unsigned)((m + 127) / 128), 128, 0, S.s(), in.p, sin, m, d_str), "k_dc_leaf");
-    std::string str(digits, '0');
-    ck(cudaMemcpyAsync(&str[0], d_str, digits, cudaMemcpyDeviceToHost, S.s()), "D2H");
-    u32 h_err = 0;
-    ck(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, S.s()), "D2H");
-    ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
-    if (h_err) {
+    ck(launch_pdl(k_dc_count, pub_grid(digits / 8), 256, 0, S.s(), reinterpret_cast<const u64*>(d_str), digits, err,
+                  pub(S), S.publication()),
+       "k_dc_count");
+    const u64* h = S.published();
+    const uint64_t left = h[1];
+    if (h[2]) {
         set_error("decimal conversion: a quotient correction did not converge");
         throw Err{B2M_ERR_INTERNAL};
     }
     const b2m_status e = take_device_error(S.c());
     if (e != B2M_OK) throw Err{e};
-    const size_t first = str.find_first_not_of('0');
-    return first == std::string::npos ? std::string("0") : str.substr(first);
+    if (left == 0) return {d_str, 1};  // all zeros
+    return {d_str + (digits - left), left};
+}
+
+// The digits and a NUL to out (cap bytes).
+void put_digits(Scope& S, Digits v, char* out, uint64_t cap, uint64_t* len) {
+    if (v.n + 1 > cap) {
+        set_error("decimal output buffer too small");
+        throw Err{B2M_ERR_OUTPUT_TOO_SMALL};
+    }
+    ck(cudaMemcpyAsync(out, v.d, v.n, cudaMemcpyDeviceToHost, S.s()), "D2H");
+    ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
+    out[v.n] = 0;
+    *len = v.n;
 }
 
 // Wraps an API body: context, device, error translation.
@@ -1241,19 +1276,18 @@ b2m_status b2m_compute_pi(uint64_t digits, char* out, uint64_t cap, uint64_t* le
         big::DV q, r;
         big::divmod(S, num, T, &q, &r);
         t3 = clk::now();
-        const std::string str = big::to_decimal(S, q);
+        const big::Digits d = big::to_decimal(S, q);
+        // "3." and `digits` digits, or "3": the first digit moves in front of the point
+        const uint64_t n = digits ? std::min(d.n, digits + 1) : 1;
+        big::ck(cudaMemcpyAsync(digits ? out + 1 : out, d.d, n, cudaMemcpyDeviceToHost, S.s()), "D2H");
+        big::ck(cudaStreamSynchronize(S.s()), "cudaStreamSynchronize");
         t4 = clk::now();
-        std::string res;
-        if (digits == 0) {
-            res = "3";
-        } else {
-            res.reserve(digits + 2);
-            res.push_back(str[0]);
-            res.push_back('.');
-            res.append(str, 1, (size_t)digits);
+        if (digits) {
+            out[0] = out[1];
+            out[1] = '.';
         }
-        std::memcpy(out, res.c_str(), res.size() + 1);
-        *len = res.size();
+        *len = digits ? n + 1 : 1;
+        out[*len] = 0;
     });
     b2m_pqt_free(tree);
     if (st != B2M_OK) return st;
@@ -1272,13 +1306,7 @@ b2m_status b2m_to_decimal_device(const uint32_t* d_a, uint64_t na, char* out, ui
                                  b2m_stream stream) {
     if ((na && !d_a) || !out || !len) return B2M_ERR_INVALID_ARGUMENT;
     return big::run_op(stream, [&](big::Scope& S) {
-        const std::string str = big::to_decimal(S, big::trim(S, {const_cast<u32*>(d_a), na}));
-        if (str.size() + 1 > cap) {
-            set_error("decimal output buffer too small");
-            throw big::Err{B2M_ERR_OUTPUT_TOO_SMALL};
-        }
-        std::memcpy(out, str.c_str(), str.size() + 1);
-        *len = str.size();
+        big::put_digits(S, big::to_decimal(S, big::trim(S, {const_cast<u32*>(d_a), na})), out, cap, len);
     });
 }
 
@@ -1317,13 +1345,7 @@ b2m_status b2m_isqrt_host(const uint32_t* a, uint64_t na, uint32_t* out, uint64_
 b2m_status b2m_to_decimal_host(const uint32_t* a, uint64_t na, char* out, uint64_t cap, uint64_t* len) {
     if ((na && !a) || !out || !len) return B2M_ERR_INVALID_ARGUMENT;
     return big::run_op(nullptr, [&](big::Scope& S) {
-        const std::string str = big::to_decimal(S, host_in(S, a, na));
-        if (str.size() + 1 > cap) {
-            set_error("decimal output buffer too small");
-            throw big::Err{B2M_ERR_OUTPUT_TOO_SMALL};
-        }
-        std::memcpy(out, str.c_str(), str.size() + 1);
-        *len = str.size();
+        big::put_digits(S, big::to_decimal(S, host_in(S, a, na)), out, cap, len);
     });
 }
 
