@@ -839,18 +839,6 @@ void batched_mul(Scope& S, const u32* a, uint64_t sa, uint64_t na, const u32* b,
     }
 }
 
-// q~_i = limbs [s, s + nq) of product i (stride sp, pl limbs written), into
-// a compact array of stride nq.
-__global__ void k_dc_extract(const u32* __restrict__ prod, u64 sp, u64 pl, u64 s, u64 nq, u32* __restrict__ q,
-                             u64 m) {
-    pdl_enter();
-    const u64 total = m * nq;
-    for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (u64)gridDim.x * blockDim.x) {
-        const u64 i = t / nq, k = t % nq;
-        q[t] = s + k < pl ? prod[i * sp + s + k] : 0u;
-    }
-}
-
 // CTA-wide out = A +- B over n limbs (A: la limbs, B: lb limbs, or B null and
 // the one-limb value bsmall), carry / borrow out returned to every thread.
 // out may be A. blockDim a multiple of 32.
@@ -927,7 +915,7 @@ __device__ bool cta_ge(const u32* A, const u32* B, u64 n) {
 // nodes of 13,000 limbs take 25 us, and took 69 over all limbs of V - U, with
 // R - P formed to see its sign and the results copied to their place.
 __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restrict__ U, u64 su,
-                         const u32* __restrict__ QE, u64 nq, const u32* __restrict__ P, u64 n, u32* out, u64 sout,
+                         const u32* __restrict__ QE, u64 sq, u64 nq, const u32* __restrict__ P, u64 n, u32* out, u64 sout,
                          u32* err) {
     pdl_enter();
     __shared__ GP ws[33];
@@ -938,7 +926,7 @@ __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restri
     u32* Q = out + 2 * i * sout;
     u32* R = Q + sout;
     for (u64 k = threadIdx.x; k < sout; k += blockDim.x) {
-        Q[k] = k < n && k < nq ? QE[i * nq + k] : 0u;
+        Q[k] = k < n && k < nq ? QE[i * sq + k] : 0u;
         if (k >= n) R[k] = 0;
     }
     u32 top = (n < sin ? V[n] : 0u) - (n < su ? U[n] : 0u);
@@ -1108,12 +1096,17 @@ Digits to_decimal(Scope& S, DV X) {
         const uint64_t na = sin - k, sp = na + R.n;
         DV prod = S.vec(m * sp);
         batched_mul(S, in.p + k, sin, na, R.p, 0, R.n, prod.p, sp, m);
-        const uint64_t s = E - k, nq = n + 1;
-        DV qe = S.vec(m * nq);
-        ck(launch_pdl(k_dc_extract, grid_for(m * nq), 256, 0, S.s(), prod.p, sp, sp, s, nq, qe.p, m), "k_dc_extract");
+        // q~ are limbs [s, s + nq) of each product, read where they are
+        const uint64_t s = E - k;
+        if (s >= sp) {
+            set_error("decimal conversion: reciprocal scale above the product");
+            throw Err{B2M_ERR_INTERNAL};
+        }
+        const uint64_t nq = std::min(n + 1, sp - s);
+        const u32* qe = prod.p + s;
         const uint64_t su = nq + n;
         DV U = S.vec(m * su);
-        batched_mul(S, qe.p, nq, nq, Pj.p, 0, n, U.p, su, m);
+        batched_mul(S, qe, sp, nq, Pj.p, 0, n, U.p, su, m);
         // next level: 2m nodes below P_j = P_{j-1}^2, stride 2 len(P_{j-1})
         const uint64_t sout = j - 1 > DC_LEAF_J ? 2 * P[j - 1].n : DC_LEAF_LIMBS;
         DV out = S.vec(2 * m * sout);
@@ -1124,12 +1117,12 @@ Digits to_decimal(Scope& S, DV X) {
             static const u32 one_h = 1;
             ck(cudaMemcpyAsync(one.p, &one_h, 4, cudaMemcpyHostToDevice, S.s()), "H2D");
             for (uint64_t i = 0; i < m; ++i)
-                fix_node_grid(S, in.p + i * sin, sin, U.p + i * su, su, qe.p + i * nq, nq, Pj, R, T, Q, one,
+                fix_node_grid(S, in.p + i * sin, sin, U.p + i * su, su, qe + i * sp, nq, Pj, R, T, Q, one,
                               out.p + (2 * i) * sout, out.p + (2 * i + 1) * sout, sout);
         } else {
             unsigned threads = 32;
             while (threads < 1024 && (uint64_t)threads * ADD_LPT < n) threads <<= 1;
-            ck(launch_pdl(k_dc_fix, (unsigned)m, threads, 0, S.s(), in.p, sin, U.p, su, qe.p, nq, Pj.p, n, out.p, sout,
+            ck(launch_pdl(k_dc_fix, (unsigned)m, threads, 0, S.s(), in.p, sin, U.p, su, qe, sp, nq, Pj.p, n, out.p, sout,
                           err),
                "k_dc_fix");
         }
