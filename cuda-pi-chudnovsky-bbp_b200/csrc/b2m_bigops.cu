@@ -226,6 +226,66 @@ __global__ void k_limb_pub(const u32* a, u64 k, const HostLen hl) {
     publish(hl, a[k]);
 }
 
+// a >= b over the warp's limbs (one a lane); *d = a - b. The borrows into the
+// lanes by one integer addition, as in block_scan_gp.
+__device__ __forceinline__ bool warp_ge_sub(u32 a, u32 b, int lane, u32* d) {
+    const u32 G = __ballot_sync(0xFFFFFFFFu, a < b), P = __ballot_sync(0xFFFFFFFFu, a == b);
+    const u64 s = (u64)(G | P) + G;
+    *d = a - b - (((P ^ (u32)s) >> lane) & 1);
+    return (s >> 32) == 0;
+}
+
+// One warp, a limb a lane: the root r = floor(sqrt(a)) of n <= 32 limbs (h =
+// 0), or the seed floor((2^(64h) - 1) / r) of its reciprocal (h <= 16); the
+// result's 32 limbs to out, its length published. A bit of the root, then of
+// the quotient, a step (the schoolbook methods in base 2), each a compare and
+// subtract of one integer addition's carries.
+// What bounds it: the chain of at most 512 and 545 steps of about 70 cycles,
+// 40 us. The same by nested Newton divisions from the host was 40 launches
+// and synchronisations or more for 16 limbs, about 0.7 ms.
+constexpr int SEED_LIMBS = 32;
+__global__ void __launch_bounds__(32) k_seed_sqrt(const u32* __restrict__ a, int n, int h, u32* __restrict__ out,
+                                                  const HostLen hl) {
+    pdl_enter();
+    const int lane = threadIdx.x;
+    u32 v = lane < n ? a[lane] : 0u, res = 0, d;
+    const u32 nz = __ballot_sync(0xFFFFFFFFu, v != 0);
+    const int tl = nz ? 31 - __clz(nz) : 0;
+    const u32 tv = __shfl_sync(0xFFFFFFFFu, v, tl);
+    // res holds the bits found so far, shifted; p walks the even positions
+    for (int p = nz ? (32 * tl + 31 - __clz(tv)) & ~1 : -1; p >= 0; p -= 2) {
+        const u32 bit = lane == p >> 5 ? 1u << (p & 31) : 0u;
+        const bool ge = warp_ge_sub(v, res | bit, lane, &d);
+        const u32 up = __shfl_down_sync(0xFFFFFFFFu, res, 1);
+        res = (res >> 1) | (lane < 31 ? up << 31 : 0u);
+        if (ge) {
+            v = d;
+            res |= bit;
+        }
+    }
+    u32 q = res;
+    if (h > 0 && nz) {
+        const u32 rz = __ballot_sync(0xFFFFFFFFu, res != 0);
+        const int rl = 31 - __clz(rz);
+        const int L = 32 * rl + 32 - __clz(__shfl_sync(0xFFFFFFFFu, res, rl));  // bits of the root
+        // the first L - 1 ones of the numerator give no quotient bit
+        const int ones = L - 1 - 32 * lane;
+        u32 rem = ones >= 32 ? 0xFFFFFFFFu : (ones > 0 ? (1u << ones) - 1 : 0u);
+        q = 0;
+        for (int i = 64 * h - L; i >= 0; --i) {
+            const u32 dn = __shfl_up_sync(0xFFFFFFFFu, rem, 1);
+            rem = (rem << 1) | (lane > 0 ? dn >> 31 : 1u);
+            if (warp_ge_sub(rem, res, lane, &d)) {
+                rem = d;
+                if (lane == i >> 5) q |= 1u << (i & 31);
+            }
+        }
+    }
+    out[lane] = q;
+    const u32 qz = __ballot_sync(0xFFFFFFFFu, q != 0);
+    if (lane == 0) publish(hl, 32 - __clz(qz));
+}
+
 // out = a 2^(32 a_off) +- b mod 2^(32n) in one pass, the trimmed length and
 // the carry or borrow out published. out may be a (a_off = 0) or b. One block
 // per 2048 limbs; the carry into a block comes by decoupled lookback, as in
@@ -495,37 +555,6 @@ std::vector<u32> recip_small(const std::vector<u32>& Y) {
     while (!q.empty() && q.back() == 0) q.pop_back();
     return q;
 }
-// floor(sqrt(v)) for v < 2^128 (bit by bit).
-unsigned __int128 isqrt128(unsigned __int128 v) {
-    unsigned __int128 res = 0, bit = (unsigned __int128)1 << 126;
-    while (bit > v) bit >>= 2;
-    while (bit) {
-        if (v >= res + bit) {
-            v -= res + bit;
-            res = (res >> 1) + bit;
-        } else {
-            res >>= 1;
-        }
-        bit >>= 2;
-    }
-    return res;
-}
-
-std::vector<u32> from128(unsigned __int128 v) {
-    std::vector<u32> h;
-    while (v) {
-        h.push_back((u32)v);
-        v >>= 32;
-    }
-    return h;
-}
-
-unsigned __int128 to128(const std::vector<u32>& h) {
-    unsigned __int128 v = 0;
-    for (size_t i = h.size(); i-- > 0;) v = (v << 32) | h[i];
-    return v;
-}
-
 // ---------------------------------------------------------------------------- Newton reciprocal
 // Top h limbs of the normalized Bn (n limbs), or Bn * 2^(32(h - n)) if h > n.
 DV top_limbs(Scope& S, DV Bn, uint64_t h) {
@@ -623,42 +652,21 @@ void divmod(Scope& S, DV a, DV b, DV* q, DV* r) {
 }
 
 // ---------------------------------------------------------------------------- square root
-// ~ sqrt(floor(N / 2^(32(2k - 2h)))) to h limbs (N has at most 2k limbs):
-// one Newton step x = (x0 + floor(N_h / x0)) / 2 from the root of the top
-// 2l limbs, l = floor((h + 2) / 2).
-DV sqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
-    const uint64_t drop = 2 * k - 2 * h;
-    DV Nh = N.n > drop ? DV{N.p + drop, N.n - drop} : DV{N.p, 0};
-    if (h <= 2) {
-        std::vector<u32> v = download(S, Nh);
-        return trim(S, upload(S, from128(isqrt128(to128(v)))));
-    }
-    const uint64_t l = (h + 2) / 2;
-    DV xl = sqrt_approx(S, N, k, l);
-    DV x0 = shl(S, xl, h - l, 0);
-    if (x0.n == 0) return x0;
-    DV qv, rv;
-    divmod(S, Nh, x0, &qv, &rv);
-    return shr(S, addsub(S, x0, qv, S.vec(std::max(x0.n, qv.n) + 1), false).v, 0, 1);
+// floor(sqrt(N)) of at most 32 limbs (h = 0), or floor((2^(64h) - 1) / that).
+DV seed_sqrt(Scope& S, DV N, uint64_t h) {
+    DV d = S.vec(SEED_LIMBS);
+    ck(launch_pdl(k_seed_sqrt, 1, 32, 0, S.s(), N.p, (int)N.n, (int)h, d.p, S.publication()), "k_seed_sqrt");
+    return {d.p, S.published()[1]};
 }
-
-DV isqrt(Scope& S, DV N);
 
 // Y ~ 2^(64h) / sqrt(N_h), N_h = floor(N / 2^(32(2k - 2h))), by Newton on the
 // reciprocal square root, y <- y + y (1 - N y^2) / 2: three products a step
-// and no division. The seed (h <= 8) is floor((2^(64h) - 1) / isqrt(N_h))
+// and no division. The seed (h <= 16) is floor((2^(64h) - 1) / isqrt(N_h))
 // from the exact root; each step starts from l = floor((h + 3) / 2) limbs.
 DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     const uint64_t drop = 2 * k - 2 * h;
     DV Nh = N.n > drop ? DV{N.p + drop, N.n - drop} : DV{N.p, 0};
-    if (h <= 8) {
-        DV root = isqrt(S, Nh);
-        DV num = S.vec(2 * h);
-        ck(cudaMemsetAsync(num.p, 0xFF, 8 * h, S.s()), "cudaMemsetAsync");  // 2^(64h) - 1
-        DV q, r;
-        divmod(S, num, root, &q, &r);
-        return q;
-    }
+    if (2 * h <= SEED_LIMBS) return seed_sqrt(S, Nh, h);
     const uint64_t l = (h + 3) / 2;
     DV Y0 = shl(S, rsqrt_approx(S, N, k, l), h - l, 0);
     DV U = mul(S, Nh, mul(S, Y0, Y0));  // ~ 2^(128h)
@@ -685,15 +693,9 @@ DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
 // root -- then the remainder R = N - s^2 moves s until 0 <= R <= 2s.
 DV isqrt(Scope& S, DV N) {
     if (N.n == 0) return N;
-    if (N.n <= 4) return trim(S, upload(S, from128(isqrt128(to128(download(S, N))))));
+    if (N.n <= SEED_LIMBS) return seed_sqrt(S, N, 0);
     const uint64_t k = (N.n + 1) / 2;
-    DV s;
-    if (N.n <= 16) {
-        s = sqrt_approx(S, N, k, k);
-    } else {
-        DV Y = rsqrt_approx(S, N, k, k);
-        s = shr(S, mul(S, N, Y), 2 * k, 0);
-    }
+    DV s = shr(S, mul(S, N, rsqrt_approx(S, N, k, k)), 2 * k, 0);
     DV SQ = mul(S, s, s);
     const uint64_t w = std::max(N.n, SQ.n) + 2;
     DV R = S.vec(w);
