@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Benchmark of the B200 Goldilocks-NTT big-integer multiply.
+"""Benchmark of the B200 number-theoretic-transform big-integer multiply.
 
 Headline metric: ms per 2^24 x 2^24-limb multiply (seeded uniform random u32
 limbs), device-resident operands, bit-exact product. One "step" is one full
@@ -379,8 +379,8 @@ def run_ours(args) -> None:
                          "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": round(dom_ms, 4),
                          "peak_source": peak_src,
                          # what the ncu captures show holds the transform kernels
-                         "binding_unit": "integer ALU pipe, 79-83% of its peak in every transform kernel "
-                                         "(ncu; profiles/kernels_2e23_instructions_traffic.md)",
+                         "binding_unit": "FMA pipe (32-bit multiplies), 55-67% of its heavy half's peak, and the "
+                                         "exchange between stages (ncu; profiles/residue_kernels.md)",
                          "product": {"algorithmic_bytes": prod_bytes,
                                      "achieved_gbs": round(prod_bytes / (step_ms * 1e-3) / 1e9, 1),
                                      "frac": round(prod_bytes / (step_ms * 1e-3) / 1e9 / peak, 4)},
@@ -391,7 +391,7 @@ def run_ours(args) -> None:
             "e2e": {"value": round(e2e_ms, 3), "unit": "ms", "h2d_bytes_per_step": 4 * (na + nb) * world,
                     "d2h_bytes_per_step": (4 * (na + nb) + 8) * world,
                     "path": "b2m_mul_host (C ABI), pinned host buffers, wall clock per call"},
-            "gpu_launches": plan["launches"] * args.steps,
+            "gpu_launches": sum(v["launches_per_product"] for v in kinds.values()) * args.steps,
             "clocks": clocks,
             "batch": batch,
             "serve": serve,
@@ -524,7 +524,7 @@ def measure_batch(rk, args) -> dict:
         "unit": "Glimbs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(batched_ms, 4), "higher_is_better": True,
         "scaling": "strong" if (args.batch_split and world > 1) else "weak",
-        "vs_baseline": None, "dtype": "u64 (GF(p), p=2^64-2^32+1)",
+        "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
         "data": "synthetic: seeded uniform random u32 limbs; lengths floor(2^(6+10u)), u uniform",
         "config": {"workload": "4096 independent products, na and nb log-uniform in [64, 65536] limbs",
                    "parallelism": ("one batch partitioned over the ranks by cost (LPT)"
@@ -632,7 +632,7 @@ def run_chudnovsky(args) -> None:
             "value": round(statistics.median(walls) * 1e3, 2), "unit": "ms", "n_gpus": rk.world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(dev_ms, 2),
             "higher_is_better": False, "scaling": "strong" if rk.world > 1 else "weak",
-            "vs_baseline": None, "dtype": "u32 limbs / u64 GF(p)",
+            "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
             "data": "deterministic: the Chudnovsky series terms",
             "config": {"workload": f"chudnovsky_bs(0, {terms}) for {args.digits} digits, level-wise on device",
                        "parallelism": (f"{rk.world} subtrees (one per rank), roots merged pairwise into rank 0"
@@ -699,7 +699,7 @@ def run_pi(args) -> None:
         "metric": f"ms per {args.digits}-digit pi string (compute_pi_chudnovsky on the device)",
         "value": round(med["total_ms"], 1), "unit": "ms", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(med["total_ms"], 1), "higher_is_better": False, "scaling": "weak",
-        "vs_baseline": None, "dtype": "u32 limbs / u64 GF(p)", "data": "deterministic: the Chudnovsky series",
+        "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)", "data": "deterministic: the Chudnovsky series",
         "config": {"workload": f"compute_pi({args.digits}): tree, isqrt, division, decimal on device",
                    "terms": med["terms"]},
         "split_ms": {k: round(med[k], 1) for k in ("tree_ms", "sqrt_ms", "div_ms", "decimal_ms")},
@@ -837,7 +837,7 @@ def measure_serve(rk, args, rate: float | None = None) -> dict:
         "value": round(float(np.percentile(lat, 50)), 2), "unit": "ms",
         "p99_ms": round(float(np.percentile(lat, 99)), 2), "mean_ms": round(float(lat.mean()), 2),
         "n_gpus": rk.world, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u64 (GF(p), p=2^64-2^32+1)",
+        "dtype": "u32 (three primes c*2^23+1 < 2^30)",
         "data": "synthetic: seeded random limbs generated on the device per request",
         "config": {"workload": f"{rate} req/s Poisson for {args.duration} s per GPU", "requests": n_req,
                    "hbm_budget_gb": args.serve_budget_gb, "streams": args.serve_streams,

@@ -6,9 +6,9 @@
 // allocation, copies and ~2 log2 N launches (src/ntt_cuda.cu:179-243).
 //
 // A batch buckets its jobs by transform length. A bucket is one set of
-// launches whose grid's second dimension runs over the bucket's jobs (one CTA
-// per job for transform lengths <= 2^13), so thousands of small products fill
-// the GPU instead of one SM each. Buckets are independent and run on forked
+// launches whose grid's second dimension runs over the bucket's jobs (one
+// launch for transform lengths <= 2^13, rns_small.cu), so thousands of small
+// products fill the GPU instead of a few SMs each. Buckets are independent and run on forked
 // streams; the whole sequence (prep kernel, buckets, join) can be captured
 // once into a CUDA graph and replayed. With B2M_BATCH_AUTOTUNE the pass split
 // and tile size of every multi-pass bucket is chosen by timing the candidates

@@ -12,7 +12,7 @@ namespace b2m {
 struct Context;
 
 constexpr int MAX_LOGN = 30;      // coefficients stay below p for N <= 2^32
-constexpr int SMALL_MAX_LOGN = 13; // one CTA holds both transforms up to here
+constexpr int SMALL_MAX_LOGN = 13; // products of one launch (rns_small.cu) up to here
 constexpr int CARRY_THREADS = 256;
 constexpr int CARRY_G = 16;       // coefficients per thread in the carry kernel
 constexpr int CARRY_CHUNK = CARRY_THREADS * CARRY_G;
@@ -33,7 +33,7 @@ struct RootTables {
 // Pass plan of one transform length.
 struct Plan {
     int logn = 0;
-    int npass = 0;   // 0 = single-CTA multiply
+    int npass = 0;   // 0 = product in one launch (rns_small.cu)
     int logr[3] = {0, 0, 0};
     int logc[3] = {0, 0, 0};
     // 1: 3 * 2^logn points -- a radix-3 step (ntt_radix3.cu) around three
@@ -80,7 +80,7 @@ struct LookbackSlot {
 uint64_t workspace_bytes_for(int logn);
 
 // One product's device pointers. Batched launches give kernels a table of
-// these and each CTA reads jobs[blockIdx.y] (blockIdx.x for the single-CTA
+// these and each CTA reads jobs[blockIdx.y] (blockIdx.x for the one-launch
 // kernel); single products pass a null table and plain arguments.
 struct ProdJob {
     const u32* a;
@@ -224,7 +224,7 @@ void twtable_free_all(Context* c);
 // Per-family launchers (ntt_fam_*.cu, ntt_carry.cu); each dispatches on the
 // radix exponent to the matching template instantiation.
 // `jobs` (device table, may be null) and `njobs` select batched launches:
-// grid.y (grid.x for the single-CTA kernel) runs over the jobs.
+// grid.y (grid.x for the one-launch kernels) runs over the jobs.
 cudaError_t launch_fwd_first(int logr, const PassGeo& g, cudaStream_t s, const u32* limbs, u64 ndig, u64* out,
                              const RootTables& tw, const ProdJob* jobs = nullptr, unsigned njobs = 1,
                              int operand = 0);

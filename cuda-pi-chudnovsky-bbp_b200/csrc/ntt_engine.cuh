@@ -352,8 +352,7 @@ __device__ __forceinline__ void group64(u64* sm, const u64* __restrict__ dtw) {
         if constexpr (RT && TL::LC >= 1) {
             // run-time shifts: a thread's two tasks are instances inst and
             // inst + NI/2 of the same u1, so one call shifts both (tiles of
-            // one column, the single-CTA products among them, keep single
-            // tasks: two live tasks there spill)
+            // one column keep single tasks: two live tasks there spill)
             for_tasks<TASKS / 2, TL::T>([&](int p) {
                 const int u1 = p >> (LOGNI - 1);
                 const int inst = p & (NI / 2 - 1);

@@ -1,6 +1,9 @@
 // ntt_kernels.cuh -- kernel bodies of one big-integer product (templates;
 // instantiated per radix in ntt_fam_*.cu).
 //
+// The transforms over the 64-bit prime: products under a plan that was fixed
+// or tuned (default plans run rns_kernels.cuh), and the no-allocation path.
+//
 // Launch sequence for N = 2^L >= 2^14 (a 2- or 3-pass plan, see make_plan):
 //   A: k_fwd_first (u32 limbs -> 16-bit digits -> pass 1), k_fwd_mid ...,
 //      k_fwd_last (last pass)

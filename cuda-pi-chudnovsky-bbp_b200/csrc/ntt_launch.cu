@@ -109,7 +109,7 @@ Plan make_plan_custom(int logn, int r0, int tile) {
 }
 
 // Explicit pass radices r[0..npass) (sum logn) with one tile size (log2
-// elements, <= 0 for the default); npass = 0 is the single-CTA product.
+// elements, <= 0 for the default); npass = 0 is the one-launch product.
 Plan make_plan_split(int logn, const int* r, int npass, int tile) {
     Plan p;
     p.logn = logn;

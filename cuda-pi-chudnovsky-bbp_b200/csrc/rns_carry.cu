@@ -6,6 +6,11 @@
 // residues per digit instead of two 8-byte coefficients, with the CRT
 // (rns_crt.cuh) in front of it.
 //
+// What bounds it: the CRT's multiplies and the latency of its serial part
+// (ticket, loads, lookback), FMA heavy 35%, ALU 41%, DRAM 37% of their peaks at
+// 2^24 digits, 82 us. Four digits a thread took 65 against 47 us at 2^23, blocks
+// in index order without a ticket the same as with one.
+//
 // Reference counterpart: carry_propagate (include/ntt.h:70-91).
 #include <cuda_runtime.h>
 

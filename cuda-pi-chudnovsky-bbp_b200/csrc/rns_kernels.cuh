@@ -26,7 +26,14 @@
 // launches for both operands and all primes together.
 //
 // What bounds them: the multiply-add pipe (8 cycles of it per butterfly) with
-// the ALU pipe close behind; see rns_field.cuh.
+// the ALU pipe close behind (rns_field.cuh), both at 50 to 65% of their peak,
+// and the exchange between the stages; DRAM is at 30 to 60% of its bandwidth.
+// Three blocks of 256 threads at 80 registers an SM; four of 64 registers
+// gained 1%. Measured at 2^24 x 2^24 limbs (four parts of 2^23 points), ms, and
+// the same passes of the 64-bit transform: first 0.45 (2 x 0.46), middle 0.29
+// (2 x 0.47), fused 0.43 (0.74, and the other operand's last pass besides),
+// inverse 0.15 and 0.28 with the parts put together (2 x 0.50), carry 0.16
+// (0.18).
 //
 // Reference counterpart: the per-stage launches of src/ntt_cuda.cu:99-128;
 // the product is the same integer.

@@ -38,7 +38,10 @@ struct RnsShape {
     u64 points() const { return (u64)q << m; }
 };
 
-// Pass radices of a 2^m-point part.
+// Pass radices of a 2^m-point part, from a sweep over the splits of each
+// length (us a product): 2^17 [5, 5, 7] 24.5 against 26.5 to 31.7 in two passes
+// (64 at once 4.9 each against 4.7); 2^19 [6, 6, 7] 37.3 against [10, 9] 43.4;
+// 2^22 [6, 8, 8] 195 against [7, 7, 8] 199.
 constexpr int RNS_MIN_M = 13, RNS_MAX_M = RNS_TWO_ADICITY;
 constexpr int kSplit[RNS_MAX_M - RNS_MIN_M + 1][3] = {
     {6, 0, 7},  // 2^13

@@ -369,14 +369,14 @@ enum {
     B2M_K_FUSED_LAST = 4,  /* operand B's last forward pass + pointwise + first inverse pass */
     B2M_K_INV_MID = 5,     /* an inverse pass (pass 1 yields the coefficients) */
     B2M_K_CARRY = 6,       /* decoupled-lookback carry into u32 limbs */
-    B2M_K_SMALL = 7,       /* whole product in one CTA (transform length <= 2^13) */
+    B2M_K_SMALL = 7,       /* whole product in one launch (transform length <= 2^13) */
     B2M_K_R3_FWD = 8,      /* radix-3 step of a 3 * 2^k-point transform (digits in) */
     B2M_K_R3_INV = 9       /* inverse radix-3 step (coefficients out, natural order) */
 };
 
 typedef struct b2m_plan_desc {
     uint32_t ntt_log2;      /* log2 of the transform length */
-    uint32_t npass;         /* 0 = single-CTA product, else 2 or 3 passes */
+    uint32_t npass;         /* 0 = product in one launch, else 2 or 3 passes */
     uint32_t logr[3];       /* radix exponent of each pass */
     uint32_t logc[3];       /* columns per CTA (log2) of each pass */
     uint32_t launches;      /* kernels launched per product */
