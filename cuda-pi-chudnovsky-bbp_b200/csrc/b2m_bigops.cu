@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(32) k_seed_sqrt(const u32* __restrict__ a, int
     }
     out[lane] = q;
     const u32 qz = __ballot_sync(0xFFFFFFFFu, q != 0);
-    if (lane == 0) publish(hl, 32 - __clz(qz));
+    if (lane == 0 && hl.host) publish(hl, 32 - __clz(qz));
 }
 
 // CTA-wide out = A +- B over n limbs (A: la limbs, B: lb limbs, or B null and
@@ -423,6 +423,23 @@ __device__ int cta_top(const u32* v, int n) {
     return r;
 }
 
+// st[0, e) = |2^(32e) - T| for the T < 2^(32(e + 1)) in st, whose limb e is top.
+__device__ void cta_error(u32* st, int e, u32 top) {
+    __shared__ int s_low;
+    if (top) return;  // the low limbs are it
+    if (threadIdx.x == 0) s_low = e;
+    __syncthreads();
+    for (int k = threadIdx.x; k < e; k += RECIP_T)
+        if (st[k]) {
+            atomicMin(&s_low, k);
+            break;
+        }
+    __syncthreads();
+    const int low = s_low;
+    for (int k = threadIdx.x; k < e; k += RECIP_T) st[k] = k > low ? ~st[k] : 0u - st[k];
+    __syncthreads();
+}
+
 // recip's steps for the top limbs y[0, h[nlev - 1]) of a divisor, one level
 // after the other, the same integers as from the host: X_h = X_l 2^(32(h-l)) +
 // X_l (2^(32(h+l)) - Y_h X_l) / 2^(64 l). X to out (h + 2 limbs of the last
@@ -437,7 +454,6 @@ __global__ void __launch_bounds__(RECIP_T) k_recip(const u32* __restrict__ y, co
     __shared__ CState sc[RECIP_W];
     __shared__ GP ws[33];
     __shared__ u32 s_carry;
-    __shared__ int s_low;
     pdl_enter();
     const int t = threadIdx.x, H = a.h[a.nlev - 1];
     for (int k = t; k < H; k += RECIP_T) sy[k] = y[k];
@@ -446,25 +462,12 @@ __global__ void __launch_bounds__(RECIP_T) k_recip(const u32* __restrict__ y, co
     for (int lev = 0; lev < a.nlev; ++lev) {
         const int h = a.h[lev], l = (h + 3) / 2, e = h + l;
         cta_mul(sx, l + 2, sy + (H - h), h, st, cs, sc);  // Y_h X_l: e + 2 limbs
-        // |2^(32e) - T| into st: T's low limbs, or their two's complement
         const u32 top = st[e];
         if (top > 1 || st[e + 1]) {
             if (t == 0) publish(hl, 0);
             return;
         }
-        if (top == 0) {
-            if (t == 0) s_low = e;
-            __syncthreads();
-            for (int k = t; k < e; k += RECIP_T)
-                if (st[k]) {
-                    atomicMin(&s_low, k);
-                    break;
-                }
-            __syncthreads();
-            const int low = s_low;
-            for (int k = t; k < e; k += RECIP_T) st[k] = k > low ? ~st[k] : 0u - st[k];
-            __syncthreads();
-        }
+        cta_error(st, e, top);
         const int en = cta_top(st, e);
         if (en > h + 2) {
             if (t == 0) publish(hl, 0);
@@ -486,6 +489,57 @@ __global__ void __launch_bounds__(RECIP_T) k_recip(const u32* __restrict__ y, co
     const int n = cta_top(sx, H + 2);
     for (int k = t; k < H + 2; k += RECIP_T) out[k] = sx[k];
     if (t == 0) publish(hl, n);
+}
+
+// rsqrt_approx's steps up to RSQRT_MAX limbs for nh, the top 2 h[nlev - 1]
+// limbs (n of them not zero above), from the seed of (h[0] + 3) / 2 limbs, the
+// same integers as from the host: with y of l limbs,
+//     U = N_h y^2, y_h = y 2^(32(h-l)) +- y |2^(32(2h+2l)) - U| / 2^(32(h+3l) + 1).
+// Bounded as k_recip; from the host a level is seven launches.
+constexpr int RSQRT_MAX = 224;
+struct RsqrtArgs {
+    int nlev, h[6];
+};
+__global__ void __launch_bounds__(RECIP_T) k_rsqrt(const u32* __restrict__ nh, int n, const u32* __restrict__ seed,
+                                                   const RsqrtArgs a, u32* __restrict__ out, const HostLen hl) {
+    __shared__ u32 sn[2 * RSQRT_MAX], sy[RSQRT_MAX + 2], ss[RSQRT_MAX + 16], su[2 * RECIP_T], sd[2 * RECIP_T];
+    __shared__ u32 cs[3 * 128 * RECIP_W];
+    __shared__ CState sc[RECIP_W];
+    __shared__ GP ws[33];
+    __shared__ u32 s_carry;
+    pdl_enter();
+    const int t = threadIdx.x, H = a.h[a.nlev - 1];
+    for (int k = t; k < 2 * H; k += RECIP_T) sn[k] = k < n ? nh[k] : 0u;
+    for (int k = t; k < RSQRT_MAX + 2; k += RECIP_T) sy[k] = k < SEED_LIMBS ? seed[k] : 0u;
+    __syncthreads();
+    for (int lev = 0; lev < a.nlev; ++lev) {
+        const int h = a.h[lev], l = (h + 3) / 2, e = 2 * h + 2 * l;
+        cta_mul(sy, l + 2, sy, l + 2, ss, cs, sc);
+        cta_mul(ss, 2 * l + 4, sn + 2 * (H - h), 2 * h, su, cs, sc);  // e + 4 limbs
+        const u32 top = su[e];
+        if (top > 1 || (su[e + 1] | su[e + 2] | su[e + 3])) {
+            if (t == 0) publish(hl, 0);
+            return;
+        }
+        cta_error(su, e, top);
+        const int en = cta_top(su, e), sh = h + 3 * l;
+        int cn = 0;
+        if (en) {
+            cta_mul(sy, l + 2, su, en, sd, cs, sc);
+            cn = l + 2 + en > sh ? l + 2 + en - sh : 0;
+            for (int k = t; k < cn; k += RECIP_T)
+                ss[k] = sd[sh + k] >> 1 | (k + 1 < cn ? sd[sh + k + 1] << 31 : 0u);
+        }
+        for (int k = t; k < h + 2; k += RECIP_T) su[k] = k >= h - l ? sy[k - (h - l)] : 0u;
+        __syncthreads();
+        if (cn) cta_addsub(su, h + 2, ss, cn, 0, sy, h + 2, top != 0, ws, &s_carry);
+        else
+            for (int k = t; k < h + 2; k += RECIP_T) sy[k] = su[k];
+        __syncthreads();
+    }
+    const int m = cta_top(sy, H + 2);
+    for (int k = t; k < H + 2; k += RECIP_T) out[k] = sy[k];
+    if (t == 0) publish(hl, m);
 }
 
 // out = a 2^(32 a_off) +- b mod 2^(32n) in one pass, the trimmed length and
@@ -891,6 +945,28 @@ DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     const uint64_t drop = 2 * k - 2 * h;
     DV Nh = N.n > drop ? DV{N.p + drop, N.n - drop} : DV{N.p, 0};
     if (2 * h <= SEED_LIMBS) return seed_sqrt(S, Nh, h);
+    if (h <= RSQRT_MAX) {
+        uint64_t hs[8] = {h};
+        int n = 1;
+        while (2 * hs[n - 1] > SEED_LIMBS) {
+            hs[n] = (hs[n - 1] + 3) / 2;
+            ++n;
+        }
+        RsqrtArgs a{};
+        a.nlev = n - 1;
+        for (int i = 0; i < a.nlev; ++i) a.h[i] = (int)hs[a.nlev - 1 - i];
+        const uint64_t cut = 2 * k - 2 * hs[n - 1];
+        DV seed = S.vec(SEED_LIMBS), Y = S.vec(h + 2);
+        ck(launch_pdl(k_seed_sqrt, 1, 32, 0, S.s(), N.p + cut, (int)(N.n - cut), (int)hs[n - 1], seed.p, HostLen{}),
+           "k_seed_sqrt");
+        ck(launch_pdl(k_rsqrt, 1, RECIP_T, 0, S.s(), Nh.p, (int)Nh.n, seed.p, a, Y.p, S.publication()), "k_rsqrt");
+        Y.n = S.published()[1];
+        if (Y.n == 0) {
+            set_error("Newton reciprocal square root diverged");
+            throw Err{B2M_ERR_INTERNAL};
+        }
+        return Y;
+    }
     const uint64_t l = (h + 3) / 2;
     DV Y0 = shl(S, rsqrt_approx(S, N, k, l), h - l, 0);
     DV U = mul(S, Nh, mul(S, Y0, Y0));  // ~ 2^(128h)
