@@ -711,12 +711,14 @@ DV copy(Scope& S, DV a, uint64_t cap) {
 }
 
 // a * 2^(32 wl + bits), trimmed.
-DV shl(Scope& S, DV a, uint64_t wl, int bits) {
+// normalizes: bits take the top limb's leading zeros (wl = 0), so the length
+// stays and is not waited for.
+DV shl(Scope& S, DV a, uint64_t wl, int bits, bool normalizes = false) {
     if (a.n == 0) return a;
     const uint64_t n = a.n + wl + 1;
     DV d = S.vec(n);
     ck(launch_pdl(k_shl, pub_grid(n), 256, 0, S.s(), a.p, a.n, bits, wl, d.p, n, pub(S), S.publication()), "k_shl");
-    return {d.p, S.published()[1]};
+    return {d.p, normalizes ? a.n : S.published()[1]};
 }
 
 // floor(a / 2^(32 wl + bits)), trimmed.
@@ -889,7 +891,7 @@ void divmod(Scope& S, DV a, DV b, DV* q, DV* r) {
         return;
     }
     const int sh = __builtin_clz(limb_at(S, b, b.n - 1));
-    DV Bn = sh ? shl(S, b, 0, sh) : b;
+    DV Bn = sh ? shl(S, b, 0, sh, true) : b;
     DV An = sh ? shl(S, a, 0, sh) : a;
     const uint64_t n = b.n;
     const uint64_t m = An.n - n + 1;  // quotient limbs, at most
@@ -898,8 +900,7 @@ void divmod(Scope& S, DV a, DV b, DV* q, DV* r) {
     const uint64_t k = An.n > L + 1 ? An.n - (L + 1) : 0;
     DV P = mul(S, DV{An.p + k, An.n - k}, X);
     const uint64_t s = L + n - k;
-    DV Q = copy(S, P.n > s ? DV{P.p + s, P.n - s} : DV{P.p, 0}, m + 2);
-    Q = trim(S, Q);
+    DV Q{P.p + std::min(s, P.n), P.n > s ? P.n - s : 0};
     DV QB = mul(S, Q, b);
     const uint64_t w = std::max(a.n, QB.n) + 1;
     DV R = S.vec(w);
@@ -1328,7 +1329,7 @@ Digits to_decimal(Scope& S, DV X) {
         const uint64_t L = n + 3;
         if (j == J) {
             const int sh = __builtin_clz(limb_at(S, Pj, n - 1));
-            DV Pn = sh ? shl(S, Pj, 0, sh) : Pj;
+            DV Pn = sh ? shl(S, Pj, 0, sh, true) : Pj;
             R = recip(S, Pn, L);  // ~ 2^(32 (L + n)) / Pn, Pn = P_j 2^sh
             if (sh) R = shl(S, R, 0, sh);
             E = L + n;
