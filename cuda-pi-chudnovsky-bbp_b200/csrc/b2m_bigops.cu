@@ -176,8 +176,8 @@ struct PubState {
 // length, and publishes without waiting for the others; without such a block
 // (the result is short) the last one to finish does. The host launches the
 // next step meanwhile, and that is ordered by the stream. Waiting for all
-// blocks, a chain of three atomics and two fences, cost a step of a
-// 400,003 / 200,001-limb division about 2 us.
+// blocks, a chain of three atomics and two fences, made a division of
+// 400,003 / 200,001 limbs 1171 us long instead of 1135.
 __device__ __forceinline__ void publish_top(unsigned long long top, u64 last, const u32* word, PubState* st,
                                             unsigned nblocks, LookbackSlot* slots, const HostLen& hl) {
     __shared__ bool s_last;
@@ -241,9 +241,9 @@ __device__ __forceinline__ bool warp_ge_sub(u32 a, u32 b, int lane, u32* d) {
 // result's 32 limbs to out, its length published. A bit of the root, then of
 // the quotient, a step (the schoolbook methods in base 2), each a compare and
 // subtract of one integer addition's carries.
-// What bounds it: the chain of at most 512 and 545 steps of about 70 cycles,
-// 40 us. The same by nested Newton divisions from the host was 40 launches
-// and synchronisations or more for 16 limbs, about 0.7 ms.
+// What bounds it: the chain of at most 512 and 545 steps, each a few dependent
+// ballots, shuffles and additions. The same by nested Newton divisions from the
+// host, for the top 16 limbs, made square roots 0.6 to 0.7 ms longer.
 constexpr int SEED_LIMBS = 32;
 __global__ void __launch_bounds__(32) k_seed_sqrt(const u32* __restrict__ a, int n, int h, u32* __restrict__ out,
                                                   const HostLen hl) {
@@ -1276,8 +1276,9 @@ void fix_node_grid(Scope& S, const u32* V, uint64_t sin, const u32* U, uint64_t 
 
 // Levels whose V - U has at least this many limbs per node, times the number
 // of nodes, fix them with grid-wide passes (fix_node_grid), one node after the
-// other at about 45 us each; k_dc_fix takes all nodes of a level side by side
-// at about 1.5 us per 2,000 limbs.
+// other, two waits of the host and eight launches and copies each; k_dc_fix
+// takes all nodes of a level side by side, 25 us at 26,000 limbs of V - U and
+// about 0.7 us more per 1,000.
 constexpr uint64_t DC_GRID_MIN_LIMBS = 1 << 16;
 
 // -1, 0, 1 as a <, ==, > b (trimmed).

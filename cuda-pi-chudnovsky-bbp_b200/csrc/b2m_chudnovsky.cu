@@ -548,10 +548,11 @@ static int ceil_log2(uint64_t x) {
     return l;
 }
 
-// Results of more than this many limbs are added by k_bs_add_wide: at two
-// rounds of one CTA, whose rounds follow each other, the two launches cost the
-// same (17 merges of 13,000 limbs 18 us either way, 9 of 26,000 34 against 14,
-// and 4 of 52,000, done one after the other from the host, 250).
+// Results of more than this many limbs are added by k_bs_add_wide: one CTA a
+// merge takes more than one round from there, and its rounds follow each other
+// (34 merges of 6,500 limbs 11 us by a CTA each; 17 of 13,000 18 against 13 in
+// the two launches, 9 of 26,000 34 against 13). The longest, which the host
+// drove one merge after the other, made pi to 1M digits 1.1 ms longer.
 constexpr uint64_t BS_WIDE_MIN_LIMBS = 1 << 13;
 
 // One level: L (m nodes, max lengths mx) -> Ln.
