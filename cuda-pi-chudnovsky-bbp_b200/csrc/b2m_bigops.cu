@@ -214,7 +214,7 @@ __device__ __forceinline__ void publish_top(unsigned long long top, u64 last, co
 }
 
 // `limb` (may be null): a limb published beside the length.
-__global__ void k_top_pub(const u32* __restrict__ a, u64 n, const u32* limb, PubState* st, const HostLen hl) {
+__global__ void k_top_pub(const u32* a, u64 n, const u32* limb, PubState* st, const HostLen hl) {
     pdl_enter();
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (u64)gridDim.x * blockDim.x)
@@ -245,8 +245,7 @@ __device__ __forceinline__ bool warp_ge_sub(u32 a, u32 b, int lane, u32* d) {
 // ballots, shuffles and additions. The same by nested Newton divisions from the
 // host, for the top 16 limbs, made square roots 0.6 to 0.7 ms longer.
 constexpr int SEED_LIMBS = 32;
-__global__ void __launch_bounds__(32) k_seed_sqrt(const u32* __restrict__ a, int n, int h, u32* __restrict__ out,
-                                                  const HostLen hl) {
+__global__ void __launch_bounds__(32) k_seed_sqrt(const u32* a, int n, int h, u32* out, const HostLen hl) {
     pdl_enter();
     const int lane = threadIdx.x;
     u32 v = lane < n ? a[lane] : 0u, res = 0, d;
@@ -447,8 +446,7 @@ __device__ void cta_error(u32* st, int e, u32 top) {
 // What bounds it: the products' multiply-adds on one SM, 2 x 512 x 257 of them
 // at the last level. From the host a level is four launches, each waited for:
 // the division of pi to 10,000 digits, 1,000 limbs, 0.48 ms, and 0.34 so.
-__global__ void __launch_bounds__(RECIP_T) k_recip(const u32* __restrict__ y, const RecipArgs a, u32* __restrict__ out,
-                                                   const HostLen hl) {
+__global__ void __launch_bounds__(RECIP_T) k_recip(const u32* y, const RecipArgs a, u32* out, const HostLen hl) {
     __shared__ u32 sy[RECIP_MAX], sx[RECIP_MAX + 2], st[RECIP_MAX + RECIP_MAX / 2 + 16], sd[2 * RECIP_T];
     __shared__ u32 cs[3 * 128 * RECIP_W];
     __shared__ CState sc[RECIP_W];
@@ -500,8 +498,8 @@ constexpr int RSQRT_MAX = 224;
 struct RsqrtArgs {
     int nlev, h[6];
 };
-__global__ void __launch_bounds__(RECIP_T) k_rsqrt(const u32* __restrict__ nh, int n, const u32* __restrict__ seed,
-                                                   const RsqrtArgs a, u32* __restrict__ out, const HostLen hl) {
+__global__ void __launch_bounds__(RECIP_T) k_rsqrt(const u32* nh, int n, const u32* seed, const RsqrtArgs a,
+                                                   u32* out, const HostLen hl) {
     __shared__ u32 sn[2 * RSQRT_MAX], sy[RSQRT_MAX + 2], ss[RSQRT_MAX + 16], su[2 * RECIP_T], sd[2 * RECIP_T];
     __shared__ u32 cs[3 * 128 * RECIP_W];
     __shared__ CState sc[RECIP_W];
@@ -609,8 +607,7 @@ __global__ void __launch_bounds__(AS_T) k_addsub_pub(const u32* A, u64 a_off, u6
 
 // out[k] = (a * 2^(32*wl + bits))[k], k < nout (bits in [0, 32)); publishes
 // the trimmed length.
-__global__ void k_shl(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout,
-                      PubState* st, const HostLen hl) {
+__global__ void k_shl(const u32* a, u64 na, int bits, u64 wl, u32* out, u64 nout, PubState* st, const HostLen hl) {
     pdl_enter();
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < nout; k += (u64)gridDim.x * blockDim.x) {
@@ -625,8 +622,7 @@ __global__ void k_shl(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* 
 
 // out[k] = floor(a / 2^(32*wl + bits))[k], k < nout (bits in [0, 32));
 // publishes the trimmed length.
-__global__ void k_shr(const u32* __restrict__ a, u64 na, int bits, u64 wl, u32* __restrict__ out, u64 nout,
-                      PubState* st, const HostLen hl) {
+__global__ void k_shr(const u32* a, u64 na, int bits, u64 wl, u32* out, u64 nout, PubState* st, const HostLen hl) {
     pdl_enter();
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < nout; k += (u64)gridDim.x * blockDim.x) {
@@ -1088,7 +1084,7 @@ __global__ void k_dc_spec_job(const u32* b, u64 nb, u64* spec, ProdJob* job) {
     *job = J;
 }
 
-__global__ void k_dc_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 scratch_words) {
+__global__ void k_dc_zero_ws(const ProdJob* jobs, u64 njobs, u64 scratch_words) {
     pdl_enter();
     const u64 j = blockIdx.x;
     if (j >= njobs) return;
@@ -1168,9 +1164,8 @@ __device__ bool cta_ge(const u32* A, const u32* B, u64 n) {
 // What bounds it: the chain of rounds of 8192 limbs, one CTA a node. Four
 // nodes of 13,000 limbs take 25 us, and took 69 over all limbs of V - U, with
 // R - P formed to see its sign and the results copied to their place.
-__global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restrict__ U, u64 su,
-                         const u32* __restrict__ QE, u64 sq, u64 nq, const u32* __restrict__ P, u64 n, u32* out, u64 sout,
-                         u32* err) {
+__global__ void k_dc_fix(const u32* V, u64 sin, const u32* U, u64 su, const u32* QE, u64 sq, u64 nq, const u32* P,
+                         u64 n, u32* out, u64 sout, u32* err) {
     pdl_enter();
     __shared__ GP ws[33];
     __shared__ u32 s_carry;
@@ -1200,7 +1195,7 @@ __global__ void k_dc_fix(const u32* __restrict__ V, u64 sin, const u32* __restri
 }
 
 // One thread per leaf (a value below 10^72 in 8 limbs): 72 decimal digits.
-__global__ void k_dc_leaf(const u32* __restrict__ nodes, u64 stride, u64 m, char* __restrict__ out) {
+__global__ void k_dc_leaf(const u32* nodes, u64 stride, u64 m, char* out) {
     pdl_enter();
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
@@ -1229,7 +1224,7 @@ __global__ void k_dc_leaf(const u32* __restrict__ nodes, u64 stride, u64 m, char
 // The n digits without their leading zeros: publishes how many are left, and
 // *err. n is a multiple of 8 and the digits are 8-byte aligned; block 0's
 // first words are the leading ones, and nearly always decide.
-__global__ void k_dc_count(const u64* __restrict__ digits, u64 n, const u32* err, PubState* st, const HostLen hl) {
+__global__ void k_dc_count(const u64* digits, u64 n, const u32* err, PubState* st, const HostLen hl) {
     pdl_enter();
     unsigned long long t = 0;
     for (u64 k = (u64)blockIdx.x * blockDim.x + threadIdx.x; k < n / 8 && !t; k += (u64)gridDim.x * blockDim.x) {

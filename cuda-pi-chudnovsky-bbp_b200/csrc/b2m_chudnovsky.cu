@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(SCHOOL_WARPS * 32) k_bs_school(LevelView L, Le
         const int i0 = k - (int)p.nb + 1 > 0 ? k - (int)p.nb + 1 : 0;
         const int i1 = k < (int)p.na - 1 ? k : (int)p.na - 1;
         for (int i = i0; i <= i1; ++i) {
-            const u64 prod = (u64)__ldg(p.a + i) * __ldg(p.b + k - i);
+            const u64 prod = (u64)p.a[i] * p.b[k - i];
             lo += prod;
             hi += (lo < prod);
         }
@@ -224,7 +224,7 @@ __global__ void k_bs_build_jobs(LevelView L, LevelView Ln, ScratchXY S, u64 m2, 
 __global__ void k_bs_zero(unsigned long long* p, u64 n) {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) p[i] = 0;
 }
-__global__ void k_bs_zero_ws(const ProdJob* __restrict__ jobs, u64 njobs, u64 scratch_words) {
+__global__ void k_bs_zero_ws(const ProdJob* jobs, u64 njobs, u64 scratch_words) {
     pdl_enter();
     // one block per job: its lookback slots + ticket, and its length
     const u64 j = blockIdx.x;
@@ -247,7 +247,7 @@ struct SignedAdd {
 };
 
 // Merge i's operation, by all threads of a block.
-__device__ SignedAdd signed_add_of(const ScratchXY& S, const int* __restrict__ sign_l, u64 i) {
+__device__ SignedAdd signed_add_of(const ScratchXY& S, const int* sign_l, u64 i) {
     __shared__ long long s_diff;
     const u32* X = S.x + i * S.sx;
     const u32* Y = S.y + i * S.sy;
@@ -301,7 +301,7 @@ __device__ SignedAdd signed_add_of(const ScratchXY& S, const int* __restrict__ s
 }
 
 // One CTA per merge.
-__global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln, u64 m2) {
+__global__ void k_bs_signed_add(const ScratchXY S, const int* sign_l, LevelView Ln, u64 m2) {
     pdl_enter();
     __shared__ GP s_ws[33];
     __shared__ u32 s_carry;
@@ -371,7 +371,7 @@ __global__ void k_bs_signed_add(const ScratchXY S, const int* __restrict__ sign_
 // writes length and sign.
 constexpr int ADD_T = 256, ADD_CH = ADD_T * ADD_LPT;
 
-__global__ void __launch_bounds__(ADD_T) k_bs_plan_add(const ScratchXY S, const int* __restrict__ sign_l, LevelView Ln,
+__global__ void __launch_bounds__(ADD_T) k_bs_plan_add(const ScratchXY S, const int* sign_l, LevelView Ln,
                                                        SignedAdd* ops, LookbackSlot* slots, u32 nch) {
     pdl_enter();
     const u64 i = blockIdx.x;

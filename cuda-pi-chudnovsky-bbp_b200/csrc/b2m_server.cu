@@ -41,7 +41,7 @@ constexpr int RES_WORDS = 9;  // per job: (sum, even, odd) of a, b and the produ
 
 // res[j*9 + 3*w + k]: array w (a, b, out) limb sum (k=0), even-index sum (1),
 // odd-index sum (2). Grid: x strides over 4096-limb chunks, y over jobs.
-__global__ void k_residues(const ProdJob* __restrict__ jobs, unsigned long long* res) {
+__global__ void k_residues(const ProdJob* jobs, unsigned long long* res) {
     const ProdJob& J = jobs[blockIdx.y];
     pdl_enter();
     const u64 first = (u64)blockIdx.x * 4096, step = (u64)gridDim.x * 4096;

@@ -8,6 +8,14 @@
 // pdl_enter() before it touches memory that an earlier kernel may write or
 // read: it returns once all earlier kernels have completed and their writes
 // are visible, so nothing is reordered.
+//
+// "Visible" holds for ordinary loads. Such a kernel is resident while earlier
+// ones still write, so what they write is not read-only for its lifetime, and
+// it must not promise that: no __ldg (ld.global.nc) and no __restrict__ on
+// operands, results, lengths and job tables. A load under either promise is
+// outside the guarantee, and the compiler may move it above the wait. The
+// resident twiddle tables, complete before any kernel sees them, are the only
+// memory read that way.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -39,9 +39,9 @@ __device__ __forceinline__ u32 rns_digit(const u32* r, const RnsCrt& k, u64& car
 }
 
 __global__ void __launch_bounds__(CARRY_THREADS, 6)
-    k_rns_carry(const u32* __restrict__ coef, u64 nt, u32* __restrict__ out, u64 nout,
+    k_rns_carry(const u32* coef, u64 nt, u32* out, u64 nout,
                 LookbackSlot* slots, u32* ticket, unsigned long long* out_len, u32* err,
-                const ProdJob* __restrict__ jobs, const RnsCrt crt, const HostLen hl) {
+                const ProdJob* jobs, const RnsCrt crt, const HostLen hl) {
     pdl_enter();
     if (jobs) {
         const ProdJob& J = jobs[blockIdx.y];

@@ -274,13 +274,13 @@ __device__ __forceinline__ void rns_load_limbs(u32* x, const u32* limbs, u32 j0,
 #pragma unroll
         for (int k = 0; k < K; ++k)
 #pragma unroll
-            for (int v = 0; v < V; ++v) x[k * V + v] = __ldg(limbs + ((u64)k << ls) + j0 + v);
+            for (int v = 0; v < V; ++v) x[k * V + v] = limbs[((u64)k << ls) + j0 + v];
     } else {
 #pragma unroll
         for (int k = 0; k < K; ++k)
 #pragma unroll
             for (int v = 0; v < V; ++v)
-                x[k * V + v] = j0 + ((u32)k << ls) + v < n ? __ldg(limbs + ((u64)k << ls) + j0 + v) : 0u;
+                x[k * V + v] = j0 + ((u32)k << ls) + v < n ? limbs[((u64)k << ls) + j0 + v] : 0u;
     }
 #pragma unroll
     for (int k = 0; k < K * V; ++k) x[k] = __viaddmin_u32(x[k], np4, x[k]);
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(256, 3) k_rns_first_parts(const RnsArgs a) {
             const u32* lp = limbs + (((i - 1) << lm) + c0);
 #pragma unroll
             for (int k = 0; k < G::E * V; ++k) {
-                const u32 v = __ldg(lp + ((u64)(k / V) << (a.logs + G::LB)) + j0 + k % V);
+                const u32 v = lp[((u64)(k / V) << (a.logs + G::LB)) + j0 + k % V];
                 x[k] = rns_red2(__viaddmin_u32(v, np4, v), m) + rns_mul(x[k], ct, m);
             }
         }

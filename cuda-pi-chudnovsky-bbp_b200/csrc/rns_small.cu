@@ -178,8 +178,8 @@ __device__ __forceinline__ void small_product(const u32* la, u64 na, const u32* 
             u32 va = 0, vb = 0;
             if (!hz || k < (1 << S0::L) / 2) {
                 const u32 j = S0::pos(t, i) + (k << S0::REST);
-                va = j < na ? __ldg(la + j) : 0u;
-                vb = j < nb ? __ldg(lb + j) : 0u;
+                va = j < na ? la[j] : 0u;
+                vb = j < nb ? lb[j] : 0u;
             }
             u32* y = x + (i << (S0::L + 1)) + 2 * k;
             y[0] = __viaddmin_u32(va, np4, va);
@@ -202,7 +202,7 @@ __device__ __forceinline__ void small_product(const u32* la, u64 na, const u32* 
 }
 
 template <int M, bool ONE>
-__device__ __forceinline__ void small_kernel(const RnsArgs& a, u32* __restrict__ out, unsigned long long* out_len,
+__device__ __forceinline__ void small_kernel(const RnsArgs& a, u32* out, unsigned long long* out_len,
                                              const RnsCrt& crt, const HostLen& hl) {
     using G = SmallShape<M, ONE>;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -290,14 +290,14 @@ __device__ __forceinline__ void small_kernel(const RnsArgs& a, u32* __restrict__
 
 template <int M>
 __global__ void __cluster_dims__(3, 1, 1) __launch_bounds__(SmallShape<M, false>::T, SmallShape<M, false>::MINB)
-    k_rns_small(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len, const RnsCrt crt,
+    k_rns_small(const RnsArgs a, u32* out, unsigned long long* out_len, const RnsCrt crt,
                 const HostLen hl) {
     small_kernel<M, false>(a, out, out_len, crt, hl);
 }
 
 template <int M>
 __global__ void __launch_bounds__(SmallShape<M, true>::BLOCK, SmallShape<M, true>::MINB)
-    k_rns_small_one(const RnsArgs a, u32* __restrict__ out, unsigned long long* out_len, const RnsCrt crt,
+    k_rns_small_one(const RnsArgs a, u32* out, unsigned long long* out_len, const RnsCrt crt,
                     const HostLen hl) {
     small_kernel<M, true>(a, out, out_len, crt, hl);
 }
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(SmallShape<M, true>::BLOCK, SmallShape<M, true
 // Products of at most 128 limbs in all: schoolbook columns. (Above that the
 // transforms win at every shape.) W warps a product, 4 / W products a block.
 template <int W>
-__global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const RnsArgs a, unsigned njobs, u32* __restrict__ out,
+__global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const RnsArgs a, unsigned njobs, u32* out,
                                                            unsigned long long* out_len, const HostLen hl) {
     constexpr int PER = SCHOOL_WARPS_CTA / W;
     __shared__ u32 smem[PER * SCHOOL_SMEM_WORDS<W>];

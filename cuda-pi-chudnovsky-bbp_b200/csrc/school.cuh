@@ -47,10 +47,8 @@ __device__ __forceinline__ CState warp_scan_carry(CState st, int lane) {
 // the loop is warp-uniform. Window w[c] = b[k0 + c - i] slides down a limb a
 // step.
 template <int W>
-static __device__ __forceinline__ unsigned long long school_product(const u32* __restrict__ a, int la,
-                                                                    const u32* __restrict__ b, int lb,
-                                                                    u32* __restrict__ out, u32* smem, CState* st,
-                                                                    unsigned long long* s_top) {
+static __device__ __forceinline__ unsigned long long school_product(const u32* a, int la, const u32* b, int lb, u32* out,
+                                                                    u32* smem, CState* st, unsigned long long* s_top) {
     constexpr int T = 32 * W;
     const int t = threadIdx.x % T, lane = t & 31, warp = t >> 5, nc = la + lb;
     // b is stored as four interleaved quarter arrays, b[j] at (j & 3) * qb +
@@ -60,8 +58,8 @@ static __device__ __forceinline__ unsigned long long school_product(const u32* _
     u32* sa = smem;
     u32* sb = sa + la;
     u32* cs = sb + 4 * qb;  // warp p's column sums: cs[(3 p + word) * nc + column]
-    for (int i = t; i < la; i += T) sa[i] = __ldg(a + i);
-    for (int j = t; j < lb; j += T) sb[(j & 3) * qb + (j >> 2)] = __ldg(b + j);
+    for (int i = t; i < la; i += T) sa[i] = a[i];
+    for (int j = t; j < lb; j += T) sb[(j & 3) * qb + (j >> 2)] = b[j];
     if (W > 1 && t == 0) *s_top = 0;
     if constexpr (W > 1) __syncthreads();
     else __syncwarp();
