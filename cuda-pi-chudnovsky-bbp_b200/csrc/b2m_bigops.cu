@@ -53,7 +53,7 @@ inline void ck(cudaError_t e, const char* what) {
 // serves all products, which the stream runs one after the other.
 class Scope {
 public:
-    Scope(Context* c, cudaStream_t s) : c_(c), s_(s), host_(c) {
+    Scope(Context* c, cudaStream_t s) : c_(c), s_(s), host_(c, s) {
         if (!host_.words()) {
             set_error("cannot pin host memory");
             throw Err{B2M_ERR_OUT_OF_MEMORY};
@@ -117,7 +117,7 @@ public:
     HostLen publication() { return host_.next(); }
     // The words of the last publication (values from [1]).
     const u64* published() {
-        ck(host_.wait(s_), "waiting for a kernel's result");
+        ck(host_.wait(), "waiting for a kernel's result");
         return host_.words();
     }
 

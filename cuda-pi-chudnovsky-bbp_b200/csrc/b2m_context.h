@@ -27,9 +27,11 @@ struct Context {
     void* host_dev = nullptr;            // device buffers of b2m_mul_host, grown on demand
     uint64_t host_dev_cap = 0;
     // Pinned host words that kernels publish lengths and carries in
-    // (HostWords below): 64 slots of eight words, a bit per slot in use.
+    // (HostWords below): 64 slots of eight words, a bit per slot in use, and
+    // the last tag that a slot's users gave out.
     u64* hw = nullptr;
     uint64_t hw_used = 0;
+    u64 hw_tag[64] = {};
     std::mutex hw_mu;
     // Inter-pass twiddle tables (twtable_ensure), keyed by (logm, logr).
     struct TwTable {
@@ -98,26 +100,33 @@ inline void set_tuned(Context* c, int logn, const Plan& p) {
     c->has_tuned[logn] = true;
 }
 
-// A slot of pinned host words for one call: a kernel writes values 1..7, a
-// system-wide fence and then the tag in word 0; the host polls the tag. Any
-// number of calls may hold slots; past 64 at a time a call pins its own.
+// A slot of pinned host words for one call on stream s: a kernel writes values
+// 1..7, a system-wide fence and then the tag in word 0; the host polls the tag.
+// Any number of calls may hold slots; past 64 at a time a call pins its own.
+// A slot is given back when no kernel owes it a publication any more: a call
+// that ends early, with its last one not waited for, waits for its stream.
+// (The words of that publication would land on the next call's, or in freed
+// memory.) Tags go on from the slot's last one, so none is ever met twice.
 class HostWords {
 public:
-    explicit HostWords(Context* c) : c_(c) {
+    HostWords(Context* c, cudaStream_t s) : c_(c), s_(s) {
         std::lock_guard<std::mutex> lk(c->hw_mu);
         for (int i = 0; i < 64 && c->hw; ++i)
             if (!((c->hw_used >> i) & 1)) {
                 c->hw_used |= 1ull << i;
                 slot_ = i;
                 p_ = c->hw + 8 * i;
+                tag_ = seen_ = c->hw_tag[i];
                 break;
             }
         if (!p_ && cudaHostAlloc(reinterpret_cast<void**>(&p_), 64, cudaHostAllocMapped) != cudaSuccess) p_ = nullptr;
         if (p_) p_[0] = 0;
     }
     ~HostWords() {
+        if (seen_ != tag_) cudaStreamSynchronize(s_);
         if (slot_ >= 0) {
             std::lock_guard<std::mutex> lk(c_->hw_mu);
+            c_->hw_tag[slot_] = tag_;
             c_->hw_used &= ~(1ull << slot_);
         } else if (p_) {
             cudaFreeHost(p_);
@@ -128,26 +137,29 @@ public:
     u64* words() const { return p_; }  // null: pinning failed
     // The next publication; its kernel gets words() and the tag.
     HostLen next() { return {reinterpret_cast<unsigned long long*>(p_), ++tag_}; }
-    // Waits for the last one. The stream is asked now and then, so that a
-    // failed or finished stream without the tag is an error, not a hang.
-    cudaError_t wait(cudaStream_t s) {
+    // Waits for the last one, and with it for all before it. The stream is
+    // asked now and then, so that a failed or finished stream without the tag
+    // is an error, not a hang.
+    cudaError_t wait() {
         volatile u64* v = p_;
         for (uint32_t n = 1; v[0] != tag_; ++n) {
             if ((n & 0xFFF) == 0) {
-                const cudaError_t q = cudaStreamQuery(s);
-                if (q == cudaSuccess) return v[0] == tag_ ? cudaSuccess : cudaErrorUnknown;
-                if (q != cudaErrorNotReady) return q;
+                const cudaError_t q = cudaStreamQuery(s_);
+                if (q == cudaSuccess && v[0] == tag_) break;
+                if (q != cudaErrorNotReady) return q == cudaSuccess ? cudaErrorUnknown : q;
             }
         }
+        seen_ = tag_;
         std::atomic_thread_fence(std::memory_order_acquire);
         return cudaSuccess;
     }
 
 private:
     Context* c_;
+    cudaStream_t s_;
     int slot_ = -1;
     u64* p_ = nullptr;
-    u64 tag_ = 0;
+    u64 tag_ = 0, seen_ = 0;  // given out, and waited for
 };
 
 extern Context* g_ctx;
