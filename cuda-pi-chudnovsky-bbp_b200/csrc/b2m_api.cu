@@ -283,8 +283,10 @@ b2m_status b2m_plan_describe(uint64_t na, uint64_t nb, b2m_plan_desc* d) {
     Context* c = ctx();
     int l = 0, three = 0;
     choose_length(2 * (na + nb), &l, &three);
-    Plan p = c ? plan_for(c, l, three) : make_plan(l, three);
+    Plan p = c ? plan_for(c, l, three, na + nb) : make_plan(l, three);
     p.three = three;
+    p.need = na + nb;
+    p.rns = rns_expected(c, p);
     d->ntt_log2 = (uint32_t)l;
     d->three = (uint32_t)three;
     d->npass = (uint32_t)p.npass;

@@ -253,6 +253,10 @@ cudaError_t launch_carry(unsigned nchunks, cudaStream_t s, const u64* coef, u32*
 cudaError_t rns_init_tables(Context* c);
 void rns_free_tables(Context* c);
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build);
+// Whether a product call outside of a capture would run plan p on them: the
+// missing tables, which it would build, fit the budget beside its workspace.
+// Without a context: by the plan alone.
+bool rns_expected(Context* c, const Plan& p);
 int rns_launches(const Plan& p);
 cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout,
                                u32* bufA, u32* bufB, LookbackSlot* slots, u32* ticket, unsigned long long* out_len,

@@ -361,6 +361,21 @@ static bool is_default_plan(const Plan& p) {
     return false;
 }
 
+static constexpr uint64_t kFullTableBytes = 6ull * sizeof(uint2) << RNS_FULL_LOG;
+static uint64_t weight_bytes(const RnsShape& sh) {
+    return 2 * 3ull * sh.q * sizeof(uint2) * ((1ull << sh.logr[0]) + (1ull << (sh.m - sh.logr[0])));
+}
+
+bool rns_expected(Context* c, const Plan& p) {
+    const RnsShape sh = rns_shape(p);
+    if (p.npass < 2 || sh.q == 0 || !is_default_plan(p)) return false;
+    if (!c) return true;
+    std::lock_guard<std::mutex> lk(c->twt_mu);
+    uint64_t bytes = need_log_ent(sh) > c->rns_log ? kFullTableBytes : 0;
+    if (sh.weighted && !find_weights(c, sh)) bytes += weight_bytes(sh);
+    return bytes == 0 || c->in_use.load() + bytes + workspace_bytes_plan(p) <= c->budget;
+}
+
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
     p.rns = 0;
     const RnsShape sh = rns_shape(p);
@@ -379,7 +394,7 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
         return true;
     };
     if (need > c->rns_log) {
-        const uint64_t bytes = 6ull * sizeof(uint2) << RNS_FULL_LOG;
+        const uint64_t bytes = kFullTableBytes;
         if (!build || !room(bytes)) return cudaSuccess;
         uint2* t = nullptr;
         const cudaError_t e = build_tables(&t, RNS_FULL_LOG, s);
@@ -397,7 +412,7 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
         Context::RnsWeights w{};
         w.q = sh.q;
         w.m = sh.m;
-        w.bytes = 2 * 3ull * sh.q * sizeof(uint2) * ((1ull << sh.logr[0]) + (1ull << (sh.m - sh.logr[0])));
+        w.bytes = weight_bytes(sh);
         if (!room(w.bytes)) return cudaSuccess;
         const cudaError_t e = build_weights(c, sh, &w, s);
         if (e != cudaSuccess) {

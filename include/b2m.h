@@ -390,7 +390,9 @@ typedef struct b2m_plan_desc {
  * that is fewer and k >= 14). Default plans of 2^14 to 2^27 points run on
  * half as many 32-bit digits modulo three 30-bit primes, with passes of their
  * own: logr and logc then describe the plan of 16-bit digits that they stand
- * for (and that b2m_set_plan takes), launches what is launched. */
+ * for (and that b2m_set_plan takes). launches is what b2m_mul_device
+ * would launch now for two operands (the same one twice may take fewer),
+ * outside of a stream capture, whether or not its tables exist yet. */
 b2m_status b2m_plan_describe(uint64_t na, uint64_t nb, b2m_plan_desc* desc);
 
 /* One timed candidate of b2m_autotune. */
