@@ -39,26 +39,47 @@ NA = NB = 1 << 24
 SEED_A, SEED_B = 24001, 24002
 
 
-def algorithmic_bytes(na: int, nb: int, n: int) -> int:
+RESIDUES = "u32 (three primes c*2^23+1 < 2^30)"
+WIDE = "u64 (GF(p), p=2^64-2^32+1)"
+
+
+def is_wide(kinds) -> bool:
+    """Whether a product whose kernels these are ran on the 64-bit transforms
+    (a fixed or tuned plan, a length above 2^27 points, no room for the
+    residue tables): only they finish operand A's transform in a pass of its
+    own."""
+    return "fwd_last" in kinds
+
+
+def algorithmic_bytes(na: int, nb: int, n: int, wide: bool) -> int:
     """Minimum HBM traffic of one product: u32 operands in and product out
-    (8(na+nb)) plus the residue sweeps of a two-pass schedule. n is the
-    16-bit-digit length; the residues are three u32 for each of its n/2
-    32-bit digits (6n bytes a sweep): both operands out of the first pass, in
-    and out of the fused pass (one product out), in and out of the inverse
-    pass, into the carry -- eight sweeps."""
-    return 8 * (na + nb) + 8 * 6 * n
+    (8(na+nb)) plus eight sweeps of the transforms. n is the 16-bit-digit
+    length. 64-bit: n elements of 8 bytes. Residues: three u32 for each of
+    n/2 32-bit digits (6n bytes a sweep), both operands out of the first pass,
+    in and out of the fused pass (one product out), in and out of the inverse
+    pass, into the carry."""
+    return 8 * (na + nb) + 8 * (8 if wide else 6) * n
 
 
-def kernel_bytes(kind: str, na: int, nb: int, n: int) -> int:
-    """Algorithmic bytes of one launch of each kernel kind; forward passes
-    cover both operands, residues are 6n bytes per operand."""
+def kernel_bytes(kind: str, na: int, nb: int, n: int, wide: bool) -> int:
+    """Algorithmic bytes of one launch of each kernel kind. 64-bit: a forward
+    pass covers one operand (the mean of the two), 8n bytes. Residues: it
+    covers both, 6n bytes each."""
+    if wide:
+        if kind in ("fwd_first", "r3_fwd"):
+            return 2 * (na + nb) + 8 * n
+        if kind in ("fwd_mid", "fwd_last", "inv_mid", "r3_inv"):
+            return 16 * n
+        if kind == "fused_last":
+            return 24 * n
+        return 8 * n + 4 * (na + nb)  # carry
     if kind == "fwd_first":
         return 4 * (na + nb) + 12 * n
     if kind == "fwd_mid":
         return 24 * n
     if kind == "fused_last":
         return 18 * n
-    if kind in ("inv_mid", "r3_inv"):
+    if kind == "inv_mid":
         return 12 * n
     if kind == "carry":
         return 6 * n + 4 * (na + nb)
@@ -194,7 +215,7 @@ def run_reference(args) -> None:
     out = {
         "impl": "reference", "metric": METRIC, "value": round(value, 1), "unit": "ms", "n_gpus": args.gpus,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(step * 1e3, 2),
-        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": "u64 (GF(p), p=2^64-2^32+1)",
+        "higher_is_better": False, "scaling": "weak", "vs_baseline": None, "dtype": WIDE,
         "data": "synthetic: seeded uniform random u32 limbs (splitmix64, the GPU arm's operands)",
         "config": {"workload": "2^24 x 2^24-limb product, uniform random limbs", "na": NA, "nb": NB,
                    "threads": 1, "host_threads_available": os.cpu_count()},
@@ -278,11 +299,12 @@ def run_ours(args) -> None:
                                         olen.data_ptr(), sp) for _ in range(args.trace_steps)]
     per_kind: dict[str, list[float]] = {}
     per_launch_bytes: dict[str, int] = {}
+    wide = is_wide({kind for tr in traces for kind, _, _ in tr})
     for tr in traces:
         for kind, logr, ms in tr:
             key = f"{kind}<{logr}>" if kind not in ("carry",) else kind
             per_kind.setdefault(key, []).append(ms)
-            per_launch_bytes[key] = kernel_bytes(kind, na, nb, n)
+            per_launch_bytes[key] = kernel_bytes(kind, na, nb, n, wide)
     kinds = {k: {"launches_per_product": len(v) // len(traces), "avg_ms": statistics.mean(v),
                  "share": sum(v) / sum(sum(x) for x in per_kind.values())} for k, v in per_kind.items()}
     dominant = max(kinds, key=lambda k: kinds[k]["avg_ms"] * kinds[k]["launches_per_product"])
@@ -290,10 +312,10 @@ def run_ours(args) -> None:
     dom_ms = kinds[dominant]["avg_ms"]
     dom_bytes = per_launch_bytes[dominant]
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
-    prod_bytes = algorithmic_bytes(na, nb, n)
+    prod_bytes = algorithmic_bytes(na, nb, n, wide)
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(tpath):
+    if os.path.exists(tpath) and not wide:  # of the residue kernels
         traffic = json.load(open(tpath)).get(dominant)
 
     # End to end through the public host-buffer call: pinned host operands,
@@ -361,11 +383,11 @@ def run_ours(args) -> None:
         metric = METRIC if headline else f"ms per {na} x {nb}-limb multiply"
         workload = ("2^24 x 2^24-limb product, uniform random limbs" if headline
                     else f"{na} x {nb}-limb product, uniform random limbs")
-        wset = 4 * (na + nb) * 2 + 12 * n
+        wset = 4 * (na + nb) * 2 + (16 if wide else 12) * n
         line = {
             "metric": metric, "value": round(value, 4), "unit": "ms", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": round(step_ms, 4), "higher_is_better": False,
-            "scaling": "weak", "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
+            "scaling": "weak", "vs_baseline": None, "dtype": WIDE if wide else RESIDUES,
             "data": "synthetic: seeded uniform random u32 limbs (splitmix64), top limb non-zero",
             "config": {"workload": workload, "na": na, "nb": nb,
                        "ntt_length": n, "plan": plan, "products_per_step": world,
@@ -379,8 +401,9 @@ def run_ours(args) -> None:
                          "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": round(dom_ms, 4),
                          "peak_source": peak_src,
                          # what the ncu captures show holds the transform kernels
-                         "binding_unit": "FMA pipe (32-bit multiplies), 55-67% of its heavy half's peak, and the "
-                                         "exchange between stages (ncu; profiles/residue_kernels.md)",
+                         "binding_unit": "integer ALU pipe (profiles/field_ops_instruction_counts_b200.md)" if wide
+                                         else "FMA pipe (32-bit multiplies), 55-67% of its heavy half's peak, and "
+                                              "the exchange between stages (ncu; profiles/residue_kernels.md)",
                          "product": {"algorithmic_bytes": prod_bytes,
                                      "achieved_gbs": round(prod_bytes / (step_ms * 1e-3) / 1e9, 1),
                                      "frac": round(prod_bytes / (step_ms * 1e-3) / 1e9 / peak, 4)},
@@ -524,7 +547,7 @@ def measure_batch(rk, args) -> dict:
         "unit": "Glimbs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(batched_ms, 4), "higher_is_better": True,
         "scaling": "strong" if (args.batch_split and world > 1) else "weak",
-        "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
+        "vs_baseline": None, "dtype": RESIDUES,
         "data": "synthetic: seeded uniform random u32 limbs; lengths floor(2^(6+10u)), u uniform",
         "config": {"workload": "4096 independent products, na and nb log-uniform in [64, 65536] limbs",
                    "parallelism": ("one batch partitioned over the ranks by cost (LPT)"
@@ -632,7 +655,7 @@ def run_chudnovsky(args) -> None:
             "value": round(statistics.median(walls) * 1e3, 2), "unit": "ms", "n_gpus": rk.world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(dev_ms, 2),
             "higher_is_better": False, "scaling": "strong" if rk.world > 1 else "weak",
-            "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)",
+            "vs_baseline": None, "dtype": RESIDUES,
             "data": "deterministic: the Chudnovsky series terms",
             "config": {"workload": f"chudnovsky_bs(0, {terms}) for {args.digits} digits, level-wise on device",
                        "parallelism": (f"{rk.world} subtrees (one per rank), roots merged pairwise into rank 0"
@@ -699,7 +722,7 @@ def run_pi(args) -> None:
         "metric": f"ms per {args.digits}-digit pi string (compute_pi_chudnovsky on the device)",
         "value": round(med["total_ms"], 1), "unit": "ms", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": round(med["total_ms"], 1), "higher_is_better": False, "scaling": "weak",
-        "vs_baseline": None, "dtype": "u32 (three primes c*2^23+1 < 2^30)", "data": "deterministic: the Chudnovsky series",
+        "vs_baseline": None, "dtype": RESIDUES, "data": "deterministic: the Chudnovsky series",
         "config": {"workload": f"compute_pi({args.digits}): tree, isqrt, division, decimal on device",
                    "terms": med["terms"]},
         "split_ms": {k: round(med[k], 1) for k in ("tree_ms", "sqrt_ms", "div_ms", "decimal_ms")},
@@ -837,7 +860,7 @@ def measure_serve(rk, args, rate: float | None = None) -> dict:
         "value": round(float(np.percentile(lat, 50)), 2), "unit": "ms",
         "p99_ms": round(float(np.percentile(lat, 99)), 2), "mean_ms": round(float(lat.mean()), 2),
         "n_gpus": rk.world, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u32 (three primes c*2^23+1 < 2^30)",
+        "dtype": RESIDUES,
         "data": "synthetic: seeded random limbs generated on the device per request",
         "config": {"workload": f"{rate} req/s Poisson for {args.duration} s per GPU", "requests": n_req,
                    "hbm_budget_gb": args.serve_budget_gb, "streams": args.serve_streams,
