@@ -248,14 +248,14 @@ cudaError_t launch_carry(unsigned nchunks, cudaStream_t s, const u64* coef, u32*
                          const ProdJob* jobs = nullptr, unsigned njobs = 1, u64 points = 1);
 // Residue-transform products. rns_resolve sets p.rns when p is the default
 // plan of its length, the length is in range and the tables exist; with
-// `build` it builds missing tables first (when `s` is not capturing and the
-// budget has room for them beside the product's own workspace).
+// `build` it builds missing tables first (when `s` is not capturing and they
+// take a small enough part of the budget, tables_fit in rns_launch.cu).
 cudaError_t rns_init_tables(Context* c);
 void rns_free_tables(Context* c);
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build);
 // Whether a product call outside of a capture would run plan p on them: the
-// missing tables, which it would build, fit the budget beside its workspace.
-// Without a context: by the plan alone.
+// missing tables, which it would build, fit the budget. Without a context: by
+// the plan alone.
 bool rns_expected(Context* c, const Plan& p);
 int rns_launches(const Plan& p);
 cudaError_t rns_launch_product(const u32* a, uint64_t na, const u32* b, uint64_t nb, u32* out, u64 nout,

@@ -366,14 +366,30 @@ static uint64_t weight_bytes(const RnsShape& sh) {
     return 2 * 3ull * sh.q * sizeof(uint2) * ((1ull << sh.logr[0]) + (1ull << (sh.m - sh.logr[0])));
 }
 
+// Bytes of the tables that shape sh lacks. Caller holds c->twt_mu.
+static uint64_t missing_bytes(Context* c, const RnsShape& sh) {
+    return (need_log_ent(sh) > c->rns_log ? kFullTableBytes : 0) +
+           (sh.weighted && !find_weights(c, sh) ? weight_bytes(sh) : 0);
+}
+// All the tables that a plan lacks are built, or none, where they take at most
+// a quarter of what the budget has left and leave the product its workspace.
+// They are kept, so they must not cost a call the memory that it asks for
+// after them (a tree level's other products). The 64-bit transforms, which run
+// where they do not fit, keep 24 bytes of tables a point of each length: a
+// call that finds room beside those needs 0.4 (one product, 16 bytes a point)
+// to 0.67 (3 * 2^k points) of what is left, a tree level about 0.55.
+static bool tables_fit(Context* c, const Plan& p, uint64_t bytes) {
+    const uint64_t used = c->in_use.load(), left = c->budget > used ? c->budget - used : 0;
+    return bytes <= left / 4 && bytes + workspace_bytes_plan(p) <= left;
+}
+
 bool rns_expected(Context* c, const Plan& p) {
     const RnsShape sh = rns_shape(p);
     if (p.npass < 2 || sh.q == 0 || !is_default_plan(p)) return false;
     if (!c) return true;
     std::lock_guard<std::mutex> lk(c->twt_mu);
-    uint64_t bytes = need_log_ent(sh) > c->rns_log ? kFullTableBytes : 0;
-    if (sh.weighted && !find_weights(c, sh)) bytes += weight_bytes(sh);
-    return bytes == 0 || c->in_use.load() + bytes + workspace_bytes_plan(p) <= c->budget;
+    const uint64_t bytes = missing_bytes(c, sh);
+    return bytes == 0 || tables_fit(c, p, bytes);
 }
 
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
@@ -386,16 +402,11 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
         if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) build = false;
     }
     std::lock_guard<std::mutex> lk(c->twt_mu);
-    // tables only where they leave the product its workspace
-    auto room = [&](uint64_t bytes) {
-        const uint64_t ws = workspace_bytes_plan(p);
-        if (!budget_reserve(c, bytes + ws)) return false;
-        budget_release(c, ws);
-        return true;
-    };
+    const uint64_t missing = missing_bytes(c, sh);
+    if (missing && (!build || !tables_fit(c, p, missing))) return cudaSuccess;
     if (need > c->rns_log) {
         const uint64_t bytes = kFullTableBytes;
-        if (!build || !room(bytes)) return cudaSuccess;
+        if (!budget_reserve(c, bytes)) return cudaSuccess;
         uint2* t = nullptr;
         const cudaError_t e = build_tables(&t, RNS_FULL_LOG, s);
         if (e != cudaSuccess) {
@@ -408,12 +419,11 @@ cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
         c->rns_log = RNS_FULL_LOG;
     }
     if (sh.weighted && !find_weights(c, sh)) {
-        if (!build) return cudaSuccess;
         Context::RnsWeights w{};
         w.q = sh.q;
         w.m = sh.m;
         w.bytes = weight_bytes(sh);
-        if (!room(w.bytes)) return cudaSuccess;
+        if (!budget_reserve(c, w.bytes)) return cudaSuccess;
         const cudaError_t e = build_weights(c, sh, &w, s);
         if (e != cudaSuccess) {
             budget_release(c, w.bytes);
