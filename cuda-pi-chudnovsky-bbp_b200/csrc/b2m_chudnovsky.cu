@@ -220,10 +220,8 @@ __global__ void k_bs_build_jobs(LevelView L, LevelView Ln, ScratchXY S, u64 m2, 
     jobs[i] = J;
 }
 
-// Zero the lengths the products accumulate with atomicMax and the carry scratch.
-__global__ void k_bs_zero(unsigned long long* p, u64 n) {
-    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) p[i] = 0;
-}
+// Zero the lengths that 64-bit products accumulate with atomicMax and their
+// carry scratch.
 __global__ void k_bs_zero_ws(const ProdJob* jobs, u64 njobs, u64 scratch_words) {
     pdl_enter();
     // one block per job: its lookback slots + ticket, and its length

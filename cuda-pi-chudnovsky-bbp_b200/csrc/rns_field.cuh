@@ -24,7 +24,6 @@
 
 namespace b2m {
 
-constexpr int RNS_PRIMES = 3;
 constexpr int RNS_TWO_ADICITY = 23;  // each p - 1 is divisible by 2^23
 constexpr u32 RNS_P0 = 998244353u, RNS_P1 = 897581057u, RNS_P2 = 880803841u;
 
