@@ -985,9 +985,9 @@ DV rsqrt_approx(Scope& S, DV N, uint64_t k, uint64_t h) {
     return addsub(S, Y0, corr, S.vec(std::max(Y0.n, corr.n) + 1), neg).v;
 }
 
-// floor(sqrt(N)) for trimmed N: an estimate -- N * Y / 2^(64k) from the
-// reciprocal square root above, or for small N the division-based Newton
-// root -- then the remainder R = N - s^2 moves s until 0 <= R <= 2s.
+// floor(sqrt(N)) for trimmed N: up to 32 limbs bit by bit (k_seed_sqrt), above
+// that the estimate N * Y / 2^(64k) from the reciprocal square root, whose
+// remainder R = N - s^2 then moves s until 0 <= R <= 2s.
 DV isqrt(Scope& S, DV N) {
     if (N.n == 0) return N;
     if (N.n <= SEED_LIMBS) return seed_sqrt(S, N, 0);

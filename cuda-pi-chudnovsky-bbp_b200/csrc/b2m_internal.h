@@ -156,11 +156,11 @@ struct HostLen {
 // `njobs` products of plan p whose pointers are in the device table `jobs`.
 // a_ready: every job's bufA already holds the finished forward spectrum of
 // its operand a under plan p (a spectrum several products share: the kernels
-// only read bufA), so a's forward passes are skipped. Plans of one CTA
+// only read bufA), so a's forward passes are skipped. Products of one launch
 // (npass == 0) transform both operands themselves and ignore it.
 // The jobs' transform buffers again as job 0's and the strides in bytes
 // between jobs (0: shared), so that kernels address them from uniform
-// registers; null where the plan has one CTA per product.
+// registers; null where the products are one launch (no buffers).
 struct JobBufs {
     void* a = nullptr;
     u64 stride_a = 0;

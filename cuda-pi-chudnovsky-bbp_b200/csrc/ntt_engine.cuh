@@ -31,8 +31,8 @@ namespace b2m {
 // Register DFTs on E = 2^e consecutive registers.
 // dft_fwd: natural-order input, bit-reversed output (decimation in frequency).
 // dft_inv: bit-reversed input, natural-order output (decimation in time),
-//          inverse roots, unscaled (1/N is applied by the carry kernel, or by
-//          the pointwise step of the one-CTA product).
+//          inverse roots, unscaled (1/N is applied by the inverse pass 0
+//          through its scaled twiddle table, or by the carry kernel).
 // The root of unity of order 2h is 2^(96/h).
 // ---------------------------------------------------------------------------
 // ZH: the upper half x[E/2 .. E) is known to be zero (the first level of the

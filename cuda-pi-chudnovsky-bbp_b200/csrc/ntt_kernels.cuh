@@ -2,7 +2,9 @@
 // instantiated per radix in ntt_fam_*.cu).
 //
 // The transforms over the 64-bit prime: products under a plan that was fixed
-// or tuned (default plans run rns_kernels.cuh), and the no-allocation path.
+// or tuned and is not the default, above 2^27 points, or whose residue tables
+// do not exist and do not fit the budget or cannot be built during a capture.
+// All others run rns_kernels.cuh.
 //
 // Launch sequence for N = 2^L >= 2^14 (a 2- or 3-pass plan, see make_plan):
 //   A: k_fwd_first (u32 limbs -> 16-bit digits -> pass 1), k_fwd_mid ...,

@@ -61,7 +61,8 @@ constexpr int kSplit[RNS_MAX_M - RNS_MIN_M + 1][3] = {
 constexpr int kSplitParts23[3] = {6, 8, 9};
 
 // Part lengths of transforms in five parts (first radix 2^6 and below: the
-// inverse holds five values per row in registers).
+// inverse holds five values per row in registers). 2^15 has a first radix of
+// 2^7; a split of it that would do, [6, 9], was not measured.
 constexpr bool five_parts(int m) { return m >= 13 && m <= 22 && m != 15; }
 constexpr int kSplitFive16[3] = {5, 5, 6};
 

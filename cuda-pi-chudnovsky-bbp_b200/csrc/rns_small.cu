@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(SmallShape<M, true>::BLOCK, SmallShape<M, true
 }
 
 // Products of at most 128 limbs in all: schoolbook columns. (Above that the
-// transforms win at every shape.) W warps a product, 4 / W products a block.
+// transforms were faster than columns on four warps at every shape; columns on
+// more warps were not measured.) W warps a product, 4 / W products a block.
 template <int W>
 __global__ void __launch_bounds__(SCHOOL_THREADS) k_school(const RnsArgs a, unsigned njobs, u32* out,
                                                            unsigned long long* out_len, const HostLen hl) {

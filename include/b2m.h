@@ -58,7 +58,8 @@ typedef enum b2m_status {
 /* Replaces the implicit per-call setup of src/ntt_cuda.cu:179-214 (device
  * probe, cudaMalloc, twiddle build). Selects `device`, uploads the resident
  * root tables once and sets the HBM budget the library may allocate
- * (0 = 90% of the device's free memory at init). Idempotent for the same
+ * (0 = 90% of the device's free memory at init). The tables uploaded here, 14
+ * MB, and the 16 MiB of b2m_mul_device_noalloc come on top of it. Idempotent for the same
  * device; a second call with another device re-initialises. */
 b2m_status b2m_init(int device, uint64_t hbm_budget_bytes);
 
