@@ -48,10 +48,11 @@ struct Context {
     std::mutex twt_mu;
     std::vector<TwTable> twt;
     // Residue-transform tables (rns_launch.cu, under twt_mu): T and its
-    // inverses of 2^rns_log entries per prime, small from the start, full
-    // size on first need; and the tables of weighted parts, per (q, m).
+    // inverses of 2^rns_log entries per prime, small from the start, larger on
+    // first need; and the tables of weighted parts, per (q, m).
     uint2* rns_t = nullptr;
     uint2* rns_base = nullptr;
+    std::vector<std::pair<uint2*, uint64_t>> rns_grown;  // all but the first, and their bytes
     int rns_log = 0;
     struct RnsWeights {
         int q, m;

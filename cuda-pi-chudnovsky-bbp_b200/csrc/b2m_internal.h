@@ -249,7 +249,7 @@ cudaError_t launch_carry(unsigned nchunks, cudaStream_t s, const u64* coef, u32*
 // Residue-transform products. rns_resolve sets p.rns when p is the default
 // plan of its length, the length is in range and the tables exist; with
 // `build` it builds missing tables first (when `s` is not capturing and they
-// take a small enough part of the budget, tables_fit in rns_launch.cu).
+// take a small enough part of the budget, tables_for in rns_launch.cu).
 cudaError_t rns_init_tables(Context* c);
 void rns_free_tables(Context* c);
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build);

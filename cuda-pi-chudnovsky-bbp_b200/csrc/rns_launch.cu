@@ -266,8 +266,10 @@ const RnsConst& shape_const(const RnsShape& sh) {
 // ---- context tables --------------------------------------------------------------
 constexpr int RNS_BASE_LOG = 18, RNS_FULL_LOG = RNS_TWO_ADICITY - 1;  // log2 entries per prime and direction
 
+uint64_t table_bytes(int log_ent) { return 6ull * sizeof(uint2) << log_ent; }
+
 cudaError_t build_tables(uint2** out, int log_ent, cudaStream_t s) {
-    const u64 bytes = 6ull * sizeof(uint2) << log_ent;
+    const u64 bytes = table_bytes(log_ent);
     cudaError_t e = cudaMalloc(out, bytes);
     if (e != cudaSuccess) return e;
     const u32 ent = 1u << log_ent;
@@ -337,10 +339,11 @@ cudaError_t rns_init_tables(Context* c) {
 
 void rns_free_tables(Context* c) {
     std::lock_guard<std::mutex> lk(c->twt_mu);
-    if (c->rns_t && c->rns_t != c->rns_base) {
-        cudaFree(c->rns_t);
-        budget_release(c, 6ull * sizeof(uint2) << RNS_FULL_LOG);
+    for (auto& g : c->rns_grown) {
+        cudaFree(g.first);
+        budget_release(c, g.second);
     }
+    c->rns_grown.clear();
     if (c->rns_base) cudaFree(c->rns_base);
     c->rns_t = c->rns_base = nullptr;
     for (Context::RnsWeights& w : c->rns_weights) {
@@ -362,26 +365,32 @@ static bool is_default_plan(const Plan& p) {
     return false;
 }
 
-static constexpr uint64_t kFullTableBytes = 6ull * sizeof(uint2) << RNS_FULL_LOG;
 static uint64_t weight_bytes(const RnsShape& sh) {
     return 2 * 3ull * sh.q * sizeof(uint2) * ((1ull << sh.logr[0]) + (1ull << (sh.m - sh.logr[0])));
 }
 
-// Bytes of the tables that shape sh lacks. Caller holds c->twt_mu.
-static uint64_t missing_bytes(Context* c, const RnsShape& sh) {
-    return (need_log_ent(sh) > c->rns_log ? kFullTableBytes : 0) +
-           (sh.weighted && !find_weights(c, sh) ? weight_bytes(sh) : 0);
-}
-// All the tables that a plan lacks are built, or none, where they take at most
-// a quarter of what the budget has left and leave the product its workspace.
-// They are kept, so they must not cost a call the memory that it asks for
-// after them (a tree level's other products). The 64-bit transforms, which run
-// where they do not fit, keep 24 bytes of tables a point of each length: a
-// call that finds room beside those needs 0.4 (one product, 16 bytes a point)
-// to 0.67 (3 * 2^k points) of what is left, a tree level about 0.55.
-static bool tables_fit(Context* c, const Plan& p, uint64_t bytes) {
+// log2 entries of the tables that plan p's product runs on: the present ones,
+// or those to build, full ones if they fit and else what the length needs. -1
+// where none fit: then the 64-bit transforms run. Caller holds c->twt_mu.
+//
+// What a plan lacks is built, all or none, where it takes at most a quarter of
+// what the budget has left and leaves the product its workspace. Tables are
+// kept, so they must not cost a call the memory that it asks for after them (a
+// tree level's other products). The 64-bit transforms keep 24 bytes of tables
+// a point of each length: a call that finds room beside those needs 0.4 (one
+// product, 16 bytes a point) to 0.67 (3 * 2^k points) of what is left, a tree
+// level about 0.55.
+static int tables_for(Context* c, const Plan& p, const RnsShape& sh) {
+    const int need = need_log_ent(sh);
+    const uint64_t weights = sh.weighted && !find_weights(c, sh) ? weight_bytes(sh) : 0;
+    if (need <= c->rns_log && !weights) return c->rns_log;
     const uint64_t used = c->in_use.load(), left = c->budget > used ? c->budget - used : 0;
-    return bytes <= left / 4 && bytes + workspace_bytes_plan(p) <= left;
+    for (int log : {RNS_FULL_LOG, need}) {
+        if (need <= c->rns_log) log = c->rns_log;
+        const uint64_t bytes = (log > c->rns_log ? table_bytes(log) : 0) + weights;
+        if (bytes <= left / 4 && bytes + workspace_bytes_plan(p) <= left) return log;
+    }
+    return -1;
 }
 
 bool rns_expected(Context* c, const Plan& p) {
@@ -389,35 +398,35 @@ bool rns_expected(Context* c, const Plan& p) {
     if (p.npass < 2 || sh.q == 0 || !is_default_plan(p)) return false;
     if (!c) return true;
     std::lock_guard<std::mutex> lk(c->twt_mu);
-    const uint64_t bytes = missing_bytes(c, sh);
-    return bytes == 0 || tables_fit(c, p, bytes);
+    return tables_for(c, p, sh) >= 0;
 }
 
 cudaError_t rns_resolve(Context* c, Plan& p, cudaStream_t s, bool build) {
     p.rns = 0;
     const RnsShape sh = rns_shape(p);
     if (!c || !c->rns_t || sh.q == 0 || !is_default_plan(p)) return cudaSuccess;
-    const int need = need_log_ent(sh);
     if (build) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) build = false;
     }
     std::lock_guard<std::mutex> lk(c->twt_mu);
-    const uint64_t missing = missing_bytes(c, sh);
-    if (missing && (!build || !tables_fit(c, p, missing))) return cudaSuccess;
-    if (need > c->rns_log) {
-        const uint64_t bytes = kFullTableBytes;
+    if (!build && (need_log_ent(sh) > c->rns_log || (sh.weighted && !find_weights(c, sh)))) return cudaSuccess;
+    const int log = tables_for(c, p, sh);
+    if (log < 0) return cudaSuccess;
+    if (log > c->rns_log) {
+        const uint64_t bytes = table_bytes(log);
         if (!budget_reserve(c, bytes)) return cudaSuccess;
         uint2* t = nullptr;
-        const cudaError_t e = build_tables(&t, RNS_FULL_LOG, s);
+        const cudaError_t e = build_tables(&t, log, s);
         if (e != cudaSuccess) {
             budget_release(c, bytes);
             if (e != cudaErrorMemoryAllocation) return e;
             cudaGetLastError();
             return cudaSuccess;
         }
-        c->rns_t = t;  // the base table stays: launches in flight read it
-        c->rns_log = RNS_FULL_LOG;
+        c->rns_grown.push_back({t, bytes});  // the earlier ones stay: launches in flight and captured graphs read them
+        c->rns_t = t;
+        c->rns_log = log;
     }
     if (sh.weighted && !find_weights(c, sh)) {
         Context::RnsWeights w{};

@@ -1,6 +1,7 @@
 """Tables that a call builds do not take the memory that the call itself needs:
-what a budget admitted on the 64-bit transforms' smaller or fewer tables it
-still admits. Each case in a process of its own, where no table exists yet."""
+what a budget admitted beside the 64-bit transforms' tables it still admits.
+Where the full residue tables are too large, shorter ones do, and grow later.
+Each case in a process of its own, where no table exists yet."""
 import os
 import subprocess
 import sys
@@ -24,8 +25,8 @@ def random_limbs(seed, n):
     return t
 """
 
-# 6,291,456 limbs each: 402.8 MB of workspace. The residue transforms take 201.3
-# MB of tables and 9.4 of weights (613.5 in all), the 64-bit ones 201.6 (604.4).
+# 6,291,456 limbs each: 402.8 MB of workspace. The residue transforms' full tables
+# and weights are 210.7 MB (613.5 in all), the 64-bit ones 201.6 (604.4).
 PRODUCT = HEAD + """
 b200mul.init(0, 605 * MB)
 n = 6 << 20
@@ -63,7 +64,45 @@ print("ok")
 """
 
 
-@pytest.mark.parametrize("script", [PRODUCT, MERGE], ids=["product", "merge"])
+# 2^21 points need a table of 25 MB; a graph holds it while a longer product
+# replaces it by the full one.
+GROWTH = HEAD + """
+import oracle
+b200mul.init(0, 300 * MB)
+n = 524288
+a, b = random_limbs(1, n), random_limbs(2, n)
+want = oracle.mul_port(*(t.cpu().numpy().view(np.uint32) for t in (a, b)))
+out = torch.zeros(2 * n, dtype=torch.int32, device="cuda")
+def check():
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32)[:want.size], want)
+    out.fill_(-1)
+assert b200mul.plan_describe(n, n)["launches"] == 6
+bt = b200mul.Batch([(a.data_ptr(), n, b.data_ptr(), n, out.data_ptr(), 2 * n, 0)], b200mul.BATCH_GRAPH)
+bt.launch()
+check()
+assert b200mul.plan_describe(12 * n, 12 * n)["launches"] > 6  # no room for its tables
+b200mul.init(0, 4000 * MB)
+c = random_limbs(3, 4 * n)
+for m in (2 * n, 4 * n):
+    big = torch.zeros(2 * m, dtype=torch.int32, device="cuda")
+    assert b200mul.plan_describe(m, m)["launches"] == 6
+    b200mul.mul_device(c.data_ptr(), m, c.data_ptr(), m, big.data_ptr(), 2 * m)
+    b200mul.stream_check()
+    p = [int.from_bytes(t.cpu().numpy().tobytes(), "little") for t in (c[:m], big)]
+    for q in ((1 << 61) - 1, (1 << 32) - 1, (1 << 32) + 1):
+        assert pow(p[0], 2, q) == p[1] % q
+    bt.launch()
+    check()
+    b200mul.mul_device(a.data_ptr(), n, b.data_ptr(), n, out.data_ptr(), 2 * n)
+    check()
+bt.close()
+b200mul.shutdown()
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("script", [PRODUCT, MERGE, GROWTH], ids=["product", "merge", "growth"])
 def test_tables_leave_the_call_its_memory(script):
     env = dict(os.environ, PYTHONPATH=os.pathsep.join(sys.path))
     r = subprocess.run([sys.executable, "-c", script], env=env, capture_output=True, text=True, timeout=300)

@@ -150,10 +150,11 @@ def traced(da, db):
 """
 
 SHORT_BUDGET = HEAD + """
-# 2^21 and 3 * 2^20 points (33 and 50 MB of workspace); the residue tables are
-# 201 MB
-b200mul.init(0, 240 * 1000000)
-for na, nb, kind in ((524288, 524288, 0), (600000, 600000, 0), (700000, 500000, 1), (1048575, 1, 0)):
+# 2^21 and 3 * 2^20 points: 33 and 50 MB of workspace, 50 and 25 of 64-bit tables;
+# the shortest residue tables are 25 and 50 MB, more than a quarter of what is left
+for budget, na, nb, kind in ((98, 524288, 524288, 0), (98, 1048575, 1, 0), (195, 600000, 600000, 0),
+                             (195, 700000, 500000, 1)):
+    b200mul.init(0, budget * 1000000)
     a, b, da, db = operands(na, nb, kind)
     got, wide = traced(da, db)
     assert wide and np.array_equal(got, oracle.mul_port(a, b)), (na, nb)
